@@ -93,10 +93,15 @@ std::mutex g_pin_mu;
 void *g_pin[2] = {nullptr, nullptr};
 size_t g_pin_bytes[2] = {0, 0};
 }  // namespace
+// captured graphs hold the addresses of the arena and of staging slot 1: they
+// go before either is freed (a later allocation may return the same address)
+static void drop_graphs();
+
 // slot 0: row uploads (under g_pin_mu); slot 1: solver state (under the arena lock)
 void *pinned_staging_slot(int slot, size_t bytes)
 {
     if (bytes <= g_pin_bytes[slot]) return g_pin[slot];
+    if (slot == 1) drop_graphs();
     if (g_pin[slot]) cudaFreeHost(g_pin[slot]);
     g_pin[slot] = nullptr;
     g_pin_bytes[slot] = 0;
@@ -573,6 +578,7 @@ size_t g_arena_bytes = 0;
 char *arena_reserve(size_t bytes)
 {
     if (bytes <= g_arena_bytes) return g_arena;
+    drop_graphs();
     if (g_arena) cudaFree(g_arena);
     g_arena = nullptr;
     g_arena_bytes = 0;
@@ -595,6 +601,7 @@ char *arena_reserve(size_t bytes)
 void release_arena()
 {
     std::lock_guard<std::mutex> g(g_arena_mu);
+    drop_graphs();
     if (g_arena) cudaFree(g_arena);
     g_arena = nullptr;
     g_arena_bytes = 0;
@@ -896,6 +903,17 @@ std::string graph_key(const Wave &w)
 }
 }  // namespace
 
+static void drop_graphs()
+{
+    for (auto &kv : g_graphs) {
+        if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+        if (kv.second.ev0) cudaEventDestroy(kv.second.ev0);
+        if (kv.second.ev1) cudaEventDestroy(kv.second.ev1);
+        if (kv.second.done) cudaEventDestroy(kv.second.done);
+    }
+    g_graphs.clear();
+}
+
 void graph_counts(long long *captured, long long *replayed)
 {
     if (captured) *captured = g_graph_captured.load();
@@ -905,15 +923,7 @@ void graph_counts(long long *captured, long long *replayed)
 static int wave_issue_graph(Wave &w, InstanceDesc *d_desc, int *d_block_inst, cudaStream_t s)
 {
     const std::string key = graph_key(w);
-    if (g_graphs.size() > 64) {
-        for (auto &kv : g_graphs) {
-            if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
-            if (kv.second.ev0) cudaEventDestroy(kv.second.ev0);
-            if (kv.second.ev1) cudaEventDestroy(kv.second.ev1);
-            if (kv.second.done) cudaEventDestroy(kv.second.done);
-        }
-        g_graphs.clear();
-    }
+    if (g_graphs.size() > 64) drop_graphs();
     GraphEntry &ge = g_graphs[key];
     if (!ge.ev0) {
         CK(cudaEventCreate(&ge.ev0));
