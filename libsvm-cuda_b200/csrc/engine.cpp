@@ -546,18 +546,15 @@ InstanceLayout instance_layout(int l, int nb, double cache_mb)
     (void)nb;
     InstanceLayout L;
     memset(&L, 0, sizeof(L));
-    // cache geometry: rows of l floats, at least 4, at most 2l slots
+    // cache geometry: rows of l floats, at least 4, at most one per variable
     long long slots = (long long)std::floor(cache_mb * (1 << 20) / (4.0 * std::max(l, 1)));
-    slots = std::max<long long>(slots, 4);
-    slots = std::min<long long>(slots, std::max<long long>(4, 2LL * l));
-    L.ways = (int)std::min<long long>(kMaxWays, slots);
-    L.sets = (int)(slots / L.ways);
-    const size_t ns = (size_t)L.sets * L.ways;
+    slots = std::min<long long>(std::max<long long>(slots, 4), std::max<long long>(4, l));
+    L.slots = (int)std::min<long long>(slots, kMaxSlots);
     Bump b;
     L.G = b.take<double>(l); L.Gb = b.take<double>(l); L.QD = b.take<double>(l);
     L.S = b.take<unsigned char>(l);
-    L.PL = b.take<int>(l); L.Sc = b.take<int>(2 * (size_t)l);
-    L.Data = b.take<float>(ns * (size_t)l);
+    L.PL = b.take<int>(l); L.PS = b.take<int>(l); L.Sc = b.take<int>(2 * (size_t)l);
+    L.Data = b.take<float>((size_t)L.slots * (size_t)l);
     L.bytes = (b.off + 255) & ~size_t(255);
     return L;
 }
@@ -612,8 +609,6 @@ void release_arena()
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kChunkBytes = 3 * 8 + 2 * 4 + 2;     // per position: G, alpha, QD, col, row, y, status
-
 // dynamic shared memory a solver block can use beside its static part
 long long smem_budget()
 {
@@ -654,7 +649,7 @@ StagePlan stage_plan(const DeviceRows &rows, int form, long long budget, int til
         if (p.stage_cap < 2) p.stage_cap = 0;
         // the exact form stages its source values as float64
         const long long elem = form == FORM_EXACT ? 8 : 4;
-        p.bytes = (((long long)p.stage_cap * p.stage_lds * elem) + 15) & ~15LL;
+        p.bytes = (((long long)p.stage_cap * p.stage_lds * elem) + 127) & ~127LL;
         if (!rows.dense && p.stage_cap == 0) {
             // too wide to scatter: the sources go into a column-keyed table
             p.hash_slots = kHashSlots;
@@ -813,12 +808,12 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
     w.dyn_smem = (size_t)dyn;
 
     // One device block per wave, laid out so that the host touches it with
-    // one upload, three fills and two downloads:
+    // one upload, one fill and one download:
     //   upload   [descriptors][block map][alpha][p][row ids][labels]
     //   download [outputs][alpha by local index]
-    //   zero     [group syncs][exchange records][cache epochs][cache stamps]
-    //   0xff     [cache tags]
-    //   per instance: G, G_bar, QD, status, position->local, shrink lists, Q rows
+    //   zero     [group syncs][exchange records][record words]
+    //   [cache tags]
+    //   per instance: G, G_bar, QD, status, position->local, position->slot, shrink lists, Q rows
     auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
     w.loff.assign(count + 1, 0);
     w.poff.assign(count + 1, 0);
@@ -830,7 +825,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
         w.lay[k] = instance_layout(l, w.nb[k], params_of(sp, prm).cache_mb);
         w.loff[k + 1] = w.loff[k] + (size_t)l;
         w.poff[k + 1] = w.poff[k] + 2 * (size_t)w.nb[k];
-        w.coff[k + 1] = w.coff[k] + (size_t)w.lay[k].sets * w.lay[k].ways;
+        w.coff[k + 1] = w.coff[k] + (size_t)w.lay[k].slots;
     }
     const size_t L = w.loff[count], P = w.poff[count], S = w.coff[count];
     size_t off = 0;
@@ -847,11 +842,9 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
     w.o_zero = off;
     w.o_sync = off; off = al(off + sizeof(GroupSync) * count);
     w.o_part = off; off = al(off + sizeof(Partial) * P);
-    w.o_ep = off; off = al(off + 4 * S);
-    w.o_st = off; off = al(off + 8 * S);
+    w.o_word = off; off = al(off + sizeof(RecWord) * kRecWords * (P / 2));
     w.zero_bytes = off - w.o_zero;
     w.o_tag = off; off = al(off + 4 * S);
-    w.tag_bytes = 4 * S;
     w.inst_off.resize(count);
     for (int k = 0; k < count; k++) {
         w.inst_off[k] = off;
@@ -869,7 +862,6 @@ static cudaError_t wave_issue(Wave &w, InstanceDesc *d_desc, int *d_block_inst, 
     char *dev = w.dev, *host = w.host;
     cudaError_t e = xfer_async(dev, host, w.up_bytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(dev + w.o_zero, 0, w.zero_bytes, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(dev + w.o_tag, 0xff, w.tag_bytes, s);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(w.ev0, s, rec);
     if (e == cudaSuccess)
         e = launch_smo(w.form, d_desc, d_block_inst, w.used - (w.drop_last_block ? 1 : 0), w.dyn_smem, w.cooperative, s);
@@ -896,8 +888,8 @@ std::atomic<long long> g_graph_captured{0}, g_graph_replayed{0};
 std::string graph_key(const Wave &w)
 {
     char buf[512];
-    snprintf(buf, sizeof buf, "%p:%p:%zu:%zu:%zu:%zu:%zu:%zu:%zu:%d:%zu:%d:%d", (void *)w.dev, (void *)w.host, w.up_bytes,
-             w.down_bytes, w.zero_bytes, w.tag_bytes, w.o_zero, w.o_tag, w.o_out, w.used, w.dyn_smem, w.form,
+    snprintf(buf, sizeof buf, "%p:%p:%zu:%zu:%zu:%zu:%zu:%d:%zu:%d:%d", (void *)w.dev, (void *)w.host, w.up_bytes,
+             w.down_bytes, w.zero_bytes, w.o_zero, w.o_out, w.used, w.dyn_smem, w.form,
              (int)w.cooperative);
     return std::string(buf) + ":" + std::to_string(w.o_desc) + ":" + std::to_string(w.o_bmap);
 }
@@ -1031,6 +1023,7 @@ int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, cons
         D.QD = (double *)(base + Lk.QD);
         D.status = (unsigned char *)(base + Lk.S);
         D.pos_local = (int *)(base + Lk.PL);
+        D.pos_slot = (int *)(base + Lk.PS);
         D.scratch = (int *)(base + Lk.Sc);
         D.cache.data = (float *)(base + Lk.Data);
         // initial state lives in the shared regions (positions start as local indices)
@@ -1042,11 +1035,9 @@ int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, cons
         D.alpha_local = (double *)(dev + w.o_alocal) + w.loff[k];
         D.sync = (GroupSync *)(dev + w.o_sync) + k;
         D.partials = (Partial *)(dev + w.o_part) + w.poff[k];
+        D.words = (RecWord *)(dev + w.o_word) + kRecWords * (w.poff[k] / 2);
         D.cache.tag = (int *)(dev + w.o_tag) + w.coff[k];
-        D.cache.epoch = (int *)(dev + w.o_ep) + w.coff[k];
-        D.cache.stamp = (unsigned long long *)(dev + w.o_st) + w.coff[k];
-        D.cache.nsets = Lk.sets;
-        D.cache.nways = Lk.ways;
+        D.cache.nslots = Lk.slots;
         D.cache.stride = l;
     }
     // the instances' initial state into the staging block, on all host threads

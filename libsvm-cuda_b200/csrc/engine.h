@@ -24,22 +24,24 @@ namespace svmb {
 constexpr int kThreads = SVMB_THREADS;  // threads per block of the persistent solver (a multiple of 128)
 constexpr int kWarps = kThreads / 32;
 constexpr int kSrcBatch = 8;            // source rows staged per pass in the row-block product
-constexpr int kMaxWays = 8;             // set associativity of the Q-row cache
-constexpr int kEpochFull = -2;          // cache slot holds the complete row
+// Q-row cache slots an instance may use at most (a position keeps its row's
+// slot in 16 bits), and how many of them carry a reference bit
+constexpr int kNoSlot = 0xffff;
+constexpr int kMaxSlots = 65534;
+constexpr int kRefSlots = 8192;
 constexpr int kPrefetchCand = 4;        // prefetch candidates published per block and phase
 constexpr int kPrefetchMax = 8;         // rows evaluated per fill pass (the missing row + prefetched)
-constexpr int kNoTag = -1;
 constexpr int kMaxGroupBlocks = 160;     // blocks per instance (one per SM)
 constexpr int kTileStride = 16;         // floats per row of a warp's 32x16 transpose tile (16-byte pieces swizzled)
-// shared memory shared by the transpose tiles (two per warp: the next column
-// slice loads while the current one is used) and the prefetch candidate table
+// shared memory of the transpose tiles (two per warp: the next column slice
+// loads while the current one is used)
 constexpr int kTileBytes = kWarps * 32 * kTileStride * 4;      // one tile per warp
-constexpr int kCandBytes = kMaxGroupBlocks * kPrefetchCand * (8 + 4 * 4);
-constexpr int kAuxBytes = ((2 * kTileBytes > kCandBytes ? 2 * kTileBytes : kCandBytes) + 15) / 16 * 16;
-constexpr int kAuxBytes1 = ((kTileBytes > kCandBytes ? kTileBytes : kCandBytes) + 15) / 16 * 16;
-// tensor forms: no transpose tiles; candidates or the block-product partial sums
-constexpr int kRedBytes = 8 * 128 * 8;
-constexpr int kAuxBytesTc = ((kCandBytes > kRedBytes ? kCandBytes : kRedBytes) + 15) / 16 * 16;
+constexpr int kAuxBytes = 2 * kTileBytes;
+// tensor forms: no transpose tiles; the block-product partial sums
+constexpr int kAuxBytesTc = 8 * 128 * 8;
+// a block's share of the active state, per position: G, alpha, QD, column, row id,
+// cache slot, flags (kFlag*)
+constexpr int kChunkBytes = 3 * 8 + 2 * 4 + 2 + 1;
 // transpose tiles per warp in the CUDA-core fills: a ring of up to 4 column
 // slices, all but the one in use in flight
 constexpr int kMaxTileBufs = 4;
@@ -51,7 +53,7 @@ constexpr int kMaxTileBufs = 4;
 // back to merge walks in global memory.
 constexpr int kHashSlots = 1024;
 SVMB_HD constexpr int hash_bytes(int form) { return kHashSlots * 4 + kHashSlots * kSrcBatch * (form == 0 ? 8 : 4); }
-SVMB_HD constexpr int tile_aux_bytes(int bufs) { return ((bufs * kTileBytes > kCandBytes ? bufs * kTileBytes : kCandBytes) + 15) / 16 * 16; }
+SVMB_HD constexpr int tile_aux_bytes(int bufs) { return bufs * kTileBytes; }
 SVMB_HD constexpr int aux_bytes(int form, int tile_bufs) { return (form == 2 || form == 3 || form == 4) ? kAuxBytesTc : tile_aux_bytes(tile_bufs); }
 
 // tensor-core (FORM_BF16X3) block products inside the solver
@@ -115,15 +117,13 @@ struct DevX {
     const double *xinv;         // FORM_FP16X3: per-row 2^-e undoing the split's scale (nullptr: 1)
 };
 
-// Q-row cache of one instance: `nsets` x `nways` slots of `stride` floats;
-// columns are indexed by the instance's LOCAL variable index (not position),
-// so shrinking permutations never move cached data.
+// Q-row cache of one instance: `nslots` rows of `stride` floats; columns are
+// indexed by the instance's LOCAL variable index (not position), so shrinking
+// permutations never move cached data.
 struct CacheView {
     float *data;
-    int *tag;                   // [nslots] local row held, or kNoTag
-    int *epoch;                 // [nslots] active-set epoch the row is valid for, or kEpochFull
-    unsigned long long *stamp;  // [nslots] LRU clock
-    int nsets, nways;
+    int *tag;                   // [nslots] local index of the row a slot was last given to
+    int nslots;
     long long stride;
 };
 
@@ -135,29 +135,27 @@ struct GroupSync {
     int pad[28];
 };
 
-// Cross-block reduction record (one per block per phase).  Besides the
-// reduced value and position it carries the winner's per-variable data
-// (alpha, QD, label, local index, row id) so that no block has to read
-// another block's chunk of the state arrays.
-// `seq` is written last with release semantics: a reader that observes
-// seq == k (acquire) sees the record of exchange k, so the record exchange is
-// also the group barrier.
+// Cross-block record of the collective sections (shrinking, reconstruction,
+// start and end of a solve), one per block per phase.  `seq` is written last
+// with release semantics: a reader that observes seq == k (acquire) sees the
+// record of exchange k and everything its block wrote before, so the exchange
+// is also the group barrier.
 struct Partial {
     double v[8];
     int n[8];
     float q[2];
     int seq;
     int pad[5];
-    // the block's most violating positions (prefetch candidates): priority,
-    // position, local index, row id, label
-    double cv[kPrefetchCand];
-    int cpos[kPrefetchCand];
-    int cloc[kPrefetchCand];
-    int crow[kPrefetchCand];
-    int cy[kPrefetchCand];
-    int pad2[8];
 };
-static_assert(sizeof(Partial) == 256, "Partial must stay 256 bytes");
+static_assert(sizeof(Partial) == 128, "Partial must stay 128 bytes");
+// Per-iteration records: 16-byte words {8 bytes, 4 bytes, sequence number},
+// each written and read with one 128-bit access, so a word that carries the
+// awaited number carries its data too.  Per block: the phase-A record (two
+// tracks of kWordsI), the phase-B record, the prefetch candidates.
+constexpr int kWordsI = 4, kWordsJ = 6;
+constexpr int kWordA = 0, kWordB = 2 * kWordsI, kWordCand = 14, kRecWords = kWordCand + 2 * kPrefetchCand;
+static_assert(kWordB + kWordsJ <= kWordCand, "record words overlap");
+struct alignas(16) RecWord { unsigned long long lo, hi; };
 static_assert(kPrefetchMax <= kSrcBatch, "a fill pass stages at most kSrcBatch rows");
 
 struct SolveOut {
@@ -195,6 +193,7 @@ struct InstanceDesc {
     unsigned char *status;
     int *pos_local;             // position -> local index (cache column)
     int *pos_row;               // position -> row id in DevX
+    int *pos_slot;              // position -> cache slot | flags (kSlot*), kNoSlot without a row
     // outputs
     double *alpha_local;        // [l] final alpha by local index (unsigned, unscaled)
     SolveOut *out;
@@ -202,6 +201,7 @@ struct InstanceDesc {
     int block0, nblocks;
     GroupSync *sync;
     Partial *partials;          // [2][nblocks]
+    RecWord *words;             // [nblocks][kRecWords]
     int *scratch;               // [2*l] shrink pair lists
     CacheView cache;
     // source-row staging in dynamic shared memory

@@ -98,12 +98,12 @@ struct Wave {
     std::vector<std::array<int, 5>> stage;    // stage_cap, stage_lds, tc_n, chunk_cap, hash_slots per instance
     std::vector<int> fill_path;               // SVMB_FILL_* per instance
     size_t dyn_smem = 0;
-    struct Layout { size_t G, Gb, A, P, QD, Al, Y, S, PL, PR, Sc, Out, Sync, Part, Tag, Ep, St, Data, bytes; int sets, ways; };
+    struct Layout { size_t G, Gb, QD, S, PL, PS, Sc, Data, bytes; int slots; };
     std::vector<Layout> lay;
     std::vector<size_t> loff, poff, coff, inst_off;
     size_t o_desc = 0, o_bmap = 0, o_alpha = 0, o_p = 0, o_row = 0, o_y = 0, o_out = 0, o_alocal = 0;
-    size_t o_zero = 0, o_sync = 0, o_part = 0, o_ep = 0, o_st = 0, o_tag = 0;
-    size_t up_bytes = 0, down_bytes = 0, zero_bytes = 0, tag_bytes = 0, dev_bytes = 0;
+    size_t o_zero = 0, o_sync = 0, o_part = 0, o_word = 0, o_tag = 0;
+    size_t up_bytes = 0, down_bytes = 0, zero_bytes = 0, dev_bytes = 0;
     char *dev = nullptr, *host = nullptr;
     cudaStream_t stream = nullptr;
     bool cooperative = true;   // false: plain launch (the caller guarantees the blocks are co-resident)

@@ -116,13 +116,12 @@ extern "C" int svmb_solve_dense_noalloc(int n, int ld, const float *X, const dou
         set_error("cannot query the device");
         return -1;
     }
-    constexpr int kChunkBytes = 3 * 8 + 2 * 4 + 2;
     const long long budget = (long long)smem_total - smo_static_smem() - 1024;
     int stage_cap = (int)std::min<long long>(kSrcBatch, (48LL << 10) / ((long long)ld * 4));
     if (stage_cap < 2) stage_cap = 0;
     // staged source values are float64 in the exact form
     const int elem = params->form == SVMB_FORM_EXACT ? 8 : 4;
-    long long stage_bytes = (((long long)stage_cap * ld * elem) + 15) & ~15LL;
+    long long stage_bytes = (((long long)stage_cap * ld * elem) + 127) & ~127LL;
     stage_bytes += kAuxBytes;   // transpose tiles (two per warp) / prefetch candidates
     const long long chunk_max = (budget - stage_bytes) / kChunkBytes;
     if (chunk_max < 64) { set_error("not enough shared memory for the solver state"); return -1; }
@@ -155,20 +154,16 @@ extern "C" int svmb_solve_dense_noalloc(int n, int ld, const float *X, const dou
     signed char *yy = (signed char *)take((size_t)n);
     unsigned char *status = (unsigned char *)take((size_t)n);
     int *pos_local = (int *)take(4 * (size_t)n), *pos_row = (int *)take(4 * (size_t)n);
+    int *pos_slot = (int *)take(4 * (size_t)n);
     int *lists = (int *)take(8 * (size_t)n);
+    RecWord *words = (RecWord *)take(sizeof(RecWord) * kRecWords * kNoAllocMaxBlocks);
     // cache: whatever remains, at least 4 rows
-    const int ways_max = kMaxWays;
-    const size_t meta_per_slot = 4 + 4 + 8;
-    const size_t left = kNoAllocScratchBytes - off - 3 * 256;
-    long long slots = (long long)(left / (meta_per_slot + 4 * (size_t)n));
-    slots = std::min<long long>(slots, 2LL * n);
+    const size_t left = kNoAllocScratchBytes - off - 2 * 256;
+    long long slots = (long long)(left / (4 + 4 * (size_t)n));
+    slots = std::min<long long>(slots, std::max(n, 4));
     if (slots < 4) { set_error("svmb_solve_dense_noalloc: workspace too small for the Q-row cache"); return -1; }
-    const int ways = (int)std::min<long long>(ways_max, slots);
-    const int sets = (int)(slots / ways);
-    const size_t nslots = (size_t)sets * ways;
+    const size_t nslots = (size_t)slots;
     int *tag = (int *)take(4 * nslots);
-    int *epoch = (int *)take(4 * nslots);
-    unsigned long long *stamp = (unsigned long long *)take(8 * nslots);
     float *cdata = (float *)take(4 * nslots * (size_t)n);
     if (off > kNoAllocScratchBytes) { set_error("svmb_solve_dense_noalloc: workspace overflow"); return -1; }
 
@@ -197,12 +192,11 @@ extern "C" int svmb_solve_dense_noalloc(int n, int ld, const float *X, const dou
     D.x.nchunk = 0;
     D.x.xinv = nullptr;
     D.G = G; D.G_bar = G_bar; D.alpha = alpha; D.p = pvec; D.QD = QD;
-    D.y = yy; D.status = status; D.pos_local = pos_local; D.pos_row = pos_row;
+    D.y = yy; D.status = status; D.pos_local = pos_local; D.pos_row = pos_row; D.pos_slot = pos_slot;
     D.alpha_local = alpha_local; D.out = d_out;
     D.block0 = 0; D.nblocks = nb;
-    D.sync = d_sync; D.partials = d_part; D.scratch = lists;
-    D.cache.data = cdata; D.cache.tag = tag; D.cache.epoch = epoch; D.cache.stamp = stamp;
-    D.cache.nsets = sets; D.cache.nways = ways; D.cache.stride = n;
+    D.sync = d_sync; D.partials = d_part; D.words = words; D.scratch = lists;
+    D.cache.data = cdata; D.cache.tag = tag; D.cache.nslots = (int)nslots; D.cache.stride = n;
     D.stage_cap = stage_cap;
     D.stage_lds = ld;
     D.chunk_cap = (int)chunk_cap;
@@ -226,9 +220,7 @@ extern "C" int svmb_solve_dense_noalloc(int n, int ld, const float *X, const dou
     // what must start from zero (the workspace keeps the previous call's contents)
     NA_CK(cudaMemsetAsync(d_sync, 0, sizeof(GroupSync), s));
     NA_CK(cudaMemsetAsync(d_part, 0, sizeof(Partial) * 2 * kNoAllocMaxBlocks, s));
-    NA_CK(cudaMemsetAsync(tag, 0xff, 4 * nslots, s));
-    NA_CK(cudaMemsetAsync(epoch, 0, 4 * nslots, s));
-    NA_CK(cudaMemsetAsync(stamp, 0, 8 * nslots, s));
+    NA_CK(cudaMemsetAsync(words, 0, sizeof(RecWord) * kRecWords * kNoAllocMaxBlocks, s));
     NA_CK(xfer_async(d_desc, &D, sizeof(InstanceDesc), cudaMemcpyHostToDevice, s));
     NA_CK(xfer_async(d_block_inst, block_inst, sizeof(int) * nb, cudaMemcpyHostToDevice, s));
     noalloc_init<<<(n + 255) / 256, 256, 0, s>>>(y, n, yy, alpha, pvec, pos_local, pos_row);

@@ -4,26 +4,38 @@
 // binary subproblem).  Every instance is owned by a group of `nblocks` thread
 // blocks; block `rank` of the group owns a contiguous chunk of the active
 // positions [0, A) and a chunk of the inactive tail [A, l).  The state of its
-// active chunk (G, alpha, QD, label, bound status, cache column, row id) lives
-// in the block's shared memory between shrink events.  Per SMO iteration there
-// are exactly two group exchanges:
+// active chunk (G, alpha, QD, label, bound status, cache column, row id, cache
+// slot) lives in the block's shared memory between shrink events.  Per SMO
+// iteration there are exactly two record exchanges:
 //
-//   phase A  reduce the per-block I_up maxima -> working index i (nu-SVC: the
-//            two track maxima ip/in), look up or evaluate the Q row(s) on the
-//            block's chunk, scan the chunk for the second-order j candidate
+//   phase A  take the working index i of the I_up records (nu-SVC: the two
+//            tracks' ip/in), evaluate the Q row(s) on the block's chunk where the
+//            cache has none, scan the chunk for the second-order j candidate
 //            (WSS3, reference svm.cpp:833-930 / :1076-1186)
-//   --- exchange ---
-//   phase B  reduce the j candidates, stopping test, look up or evaluate Q_j,
-//            two-variable analytic step with box clipping (svm.cpp:636-721,
-//            computed redundantly and identically by every block), gradient
-//            update G += dQ (svm.cpp:729-735) and G_bar update (:744-769) on the
-//            block's chunk, fused with the I_up scan for the next i
-//   --- exchange ---
+//   --- records ---
+//   phase B  take j, stopping test, evaluate Q_j if missing, two-variable
+//            analytic step with box clipping (svm.cpp:636-721, computed
+//            redundantly and identically by every block), gradient update
+//            G += dQ (svm.cpp:729-735) and G_bar update (:744-769) on the block's
+//            chunk, fused with the I_up scan for the next i
+//   --- records ---
 //
-// An exchange publishes a 128-byte record per block whose last field is a
-// sequence number written with release semantics; every block polls all
-// records with acquire loads.  The exchange is therefore also the group
-// barrier.  Records alternate between two buffers.
+// What bounds an iteration: not bandwidth but the chain of one block's
+// barriers, reductions, the records' trip through L2 and the row reads, so
+// the chain is kept short.
+//   - A phase ends in two block barriers: warps leave their partial results,
+//     warp 0 reduces them (three integer warp reductions per arg-max over an
+//     order-preserving key instead of five rounds of double shuffles), sends
+//     the block's record, polls the group's records and leaves the winner.
+//   - A record is a few 16-byte words that each carry the exchange's sequence
+//     number, written and read with single 128-bit accesses: a word that shows
+//     the number shows its data, so no fence precedes the store and no second
+//     round trip follows the poll.  Blocks share nothing else in the loop (a
+//     block reads only the Q columns it filled itself); the collective
+//     sections, after which chunks move, use release/acquire exchanges.
+//   - Where a variable's row is cached is kept beside its position and travels
+//     in the record, so a phase knows a hit or a miss as soon as it knows the
+//     variable; every block replays the same slot allocation.
 //
 // Shrinking (svm.cpp:932-1011), gradient reconstruction (:473-513) and the
 // initial gradient (:545-572) run inside the same launch as group-collective
@@ -60,7 +72,7 @@ constexpr double kTau = 1e-12;                     // reference svm.cpp:42
 constexpr long long kWaitTimeoutNs = 30000000000LL;  // default bound of a cross-block wait: 30 s
 // positions a thread takes at a time in the chunk scans that read Q rows from
 // global memory: their loads are issued together
-constexpr int kScanGroup = 8;
+constexpr int kScanGroup = 4;
 
 // --------------------------------------------------------------------------
 // memory-model helpers
@@ -80,6 +92,22 @@ __device__ __forceinline__ int ld_relaxed_i32(const int *p)
     int v;
     asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
+}
+
+// single-copy atomic 128-bit accesses of a record word at L2
+__device__ __forceinline__ RecWord ld_word(const RecWord *p)
+{
+    RecWord w;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(w.lo), "=l"(w.hi) : "l"(p) : "memory");
+    return w;
+}
+__device__ __forceinline__ void st_word(RecWord *p, double d, unsigned x, unsigned seq)
+{
+    const unsigned long long lo = (unsigned long long)__double_as_longlong(d);
+    const unsigned long long hi = (unsigned long long)x | ((unsigned long long)seq << 32);
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}"
+                 ::"l"(p), "l"(lo), "l"(hi) : "memory");
 }
 
 // --------------------------------------------------------------------------
@@ -258,6 +286,11 @@ __device__ void unstage_sources(const InstanceDesc &D, float *stage, StageSlots 
     }
     __syncthreads();
 }
+
+// q_value as one function: inlined at every use (up to 8 sources per target,
+// each with every kernel type's code) it made the row passes several times
+// larger than the instruction caches
+__device__ __noinline__ float q_of(int yy, double dot, double xsq_a, double xsq_b);
 
 template <int FORM>
 struct Acc {
@@ -439,37 +472,44 @@ __device__ __forceinline__ void row_dots(const InstanceDesc &D, const StageSlots
 }
 
 // --------------------------------------------------------------------------
-// block reductions with the reference's tie rules
+// reductions with the reference's tie rules
 // --------------------------------------------------------------------------
 // argmax, ties -> larger index ("if (v >= best)" scanning upward, svm.cpp:851,860)
 __device__ __forceinline__ void better_max(double &v, int &i, double v2, int i2)
 {
     if (v2 > v || (v2 == v && i2 > i)) { v = v2; i = i2; }
 }
-// argmin, ties -> larger index ("if (obj_diff <= obj_diff_min)", svm.cpp:890,914)
-__device__ __forceinline__ void better_min(double &v, int &i, double v2, int i2)
+
+// Order-preserving key of a number that is not NaN (-0 counts as +0); 0 is
+// below every number's key.
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 key_of(double v)
 {
-    if (v2 < v || (v2 == v && i2 > i)) { v = v2; i = i2; }
+    const long long b = __double_as_longlong(__dadd_rn(v, 0.0));
+    return (u64)b ^ ((u64)(b >> 63) | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double key_value(u64 k)
+{
+    const u64 b = (k >> 63) ? k ^ 0x8000000000000000ull : ~k;
+    return __longlong_as_double((long long)b);
+}
+// the largest key of the warp
+__device__ __forceinline__ u64 warp_max_key(u64 k)
+{
+    const unsigned hi = (unsigned)(k >> 32), lo = (unsigned)k;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return ((u64)mh << 32) | ml;
+}
+// the largest key of the warp and, among the lanes that hold it, the largest
+// index (ties go to the larger index); every lane gets both
+__device__ __forceinline__ void warp_best(u64 &k, int &i)
+{
+    const u64 m = warp_max_key(k);
+    i = __reduce_max_sync(0xffffffffu, k == m ? i : -1);
+    k = m;
 }
 
-__device__ __forceinline__ void warp_argmax(double &v, int &i)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-        const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-        better_max(v, i, v2, i2);
-    }
-}
-__device__ __forceinline__ void warp_argmin(double &v, int &i)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-        const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-        better_min(v, i, v2, i2);
-    }
-}
 __device__ __forceinline__ double warp_max(double v)
 {
 #pragma unroll
@@ -485,38 +525,24 @@ __device__ __forceinline__ int warp_sum_i(int v)
 
 struct RedScratch {
     double v[4][kWarps];
-    int i[4][kWarps];
+    int i[kWarps];
 };
 
-// Reduce up to 4 (value,index) pairs over the block; the result is in every
-// thread.  kind[k]: 0 argmax, 1 argmin, 2 max (index ignored).
+// Maxima of N values over the block; the result is in every thread.
 template <int N>
-__device__ void block_reduce(RedScratch &s, double (&v)[N], int (&idx)[N], const int (&kind)[N])
+__device__ void block_max(RedScratch &s, double (&v)[N])
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < N; k++) {
-        if (kind[k] == 0) warp_argmax(v[k], idx[k]);
-        else if (kind[k] == 1) warp_argmin(v[k], idx[k]);
-        else v[k] = warp_max(v[k]);
-    }
+    for (int k = 0; k < N; k++) v[k] = warp_max(v[k]);
     __syncthreads();
     if (lane == 0) {
 #pragma unroll
-        for (int k = 0; k < N; k++) { s.v[k][w] = v[k]; s.i[k][w] = idx[k]; }
+        for (int k = 0; k < N; k++) s.v[k][w] = v[k];
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < N; k++) {
-        double vv = kind[k] == 1 ? SVMB_INF : -SVMB_INF;
-        int ii = -1;
-        if (lane < kWarps) { vv = s.v[k][lane]; ii = s.i[k][lane]; }
-        if (kind[k] == 0) warp_argmax(vv, ii);
-        else if (kind[k] == 1) warp_argmin(vv, ii);
-        else vv = warp_max(vv);
-        v[k] = vv;
-        idx[k] = ii;
-    }
+    for (int k = 0; k < N; k++) v[k] = warp_max(lane < kWarps ? s.v[k][lane] : -SVMB_INF);
 }
 
 __device__ int block_sum_i(RedScratch &s, int v)
@@ -524,9 +550,9 @@ __device__ int block_sum_i(RedScratch &s, int v)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     v = warp_sum_i(v);
     __syncthreads();
-    if (lane == 0) s.i[0][w] = v;
+    if (lane == 0) s.i[w] = v;
     __syncthreads();
-    int tot = lane < kWarps ? s.i[0][lane] : 0;
+    int tot = lane < kWarps ? s.i[lane] : 0;
     tot = warp_sum_i(tot);
     __syncthreads();
     return tot;
@@ -540,11 +566,11 @@ __device__ int block_excl_scan(RedScratch &s, int flag, int *total)
     const unsigned bal = __ballot_sync(0xffffffffu, flag);
     const int in_warp = __popc(bal & ((1u << lane) - 1u));
     __syncthreads();
-    if (lane == 0) s.i[0][w] = __popc(bal);
+    if (lane == 0) s.i[w] = __popc(bal);
     __syncthreads();
     int before = 0, tot = 0;
     for (int k = 0; k < kWarps; k++) {
-        const int c = s.i[0][k];
+        const int c = s.i[k];
         if (k < w) before += c;
         tot += c;
     }
@@ -554,246 +580,89 @@ __device__ int block_excl_scan(RedScratch &s, int flag, int *total)
 }
 
 // --------------------------------------------------------------------------
-// Q-row cache (set associative, LRU within a set).  Every block makes the same
-// decisions from the same metadata; only block 0 writes metadata, one phase
-// after the decision, and every reader overlays the decisions whose writes may
-// still be in flight (prev) or are not yet issued (cur).
-// --------------------------------------------------------------------------
-struct CacheRec {
-    int set, way, tag, epoch;
-    unsigned long long stamp;
-};
-
-struct CacheState {
-    CacheRec prev[16], cur[16];
-    int nprev, ncur;
-};
-
-struct Lookup {
-    long long slot;     // -1: no slot could be taken (prefetch only)
-    int valid_active;   // positions [0,A) already valid
-    int was_prefetched; // hit on a row that a prefetch filled and nobody used yet
-};
-
-// LRU stamps: 2*iter+1 for phase A, 2*iter+2 for phase B; bit 62 marks rows
-// filled by prefetch and not yet used.
-constexpr unsigned long long kPrefetchMark = 1ull << 62;
-
-__device__ void cache_rotate(CacheState &cs, const CacheView &cv, int rank)
-{
-    // thread 0, right after an exchange: publish the previous phase's records
-    if (rank == 0) {
-        for (int k = 0; k < cs.ncur; k++) {
-            const CacheRec &r = cs.cur[k];
-            const long long s = (long long)r.set * cv.nways + r.way;
-            cv.tag[s] = r.tag;
-            cv.epoch[s] = r.epoch;
-            cv.stamp[s] = r.stamp;
-        }
-    }
-    for (int k = 0; k < cs.ncur; k++) cs.prev[k] = cs.cur[k];
-    cs.nprev = cs.ncur;
-    cs.ncur = 0;
-}
-
-// a cache set's metadata as stored in global memory, copied into shared memory
-struct SetStage {
-    int set;
-    int tag[kMaxWays], ep[kMaxWays];
-    unsigned long long st[kMaxWays];
-};
-
-// The set's metadata with this phase's and the previous phase's decisions
-// laid over it.  Ways are visited by constant index (unrolled, guarded by the
-// set's way count) so that the arrays stay in registers, and the global reads
-// of a set go out together.
-__device__ __forceinline__ void cache_read_set(const CacheState &cs, const CacheView &cv, int set, int (&tag)[kMaxWays],
-                                               int (&ep)[kMaxWays], unsigned long long (&st)[kMaxWays],
-                                               const SetStage *pre = nullptr)
-{
-    if (pre && pre->set == set) {
-#pragma unroll
-        for (int w = 0; w < kMaxWays; w++)
-            if (w < cv.nways) {
-                tag[w] = pre->tag[w];
-                ep[w] = pre->ep[w];
-                st[w] = pre->st[w];
-            }
-    } else {
-        const long long s0 = (long long)set * cv.nways;
-#pragma unroll
-        for (int w = 0; w < kMaxWays; w++)
-            if (w < cv.nways) {
-                tag[w] = __ldcg(&cv.tag[s0 + w]);
-                ep[w] = __ldcg(&cv.epoch[s0 + w]);
-                st[w] = __ldcg(&cv.stamp[s0 + w]);
-            }
-    }
-    auto overlay = [&](const CacheRec &r) {
-#pragma unroll
-        for (int w = 0; w < kMaxWays; w++)
-            if (w == r.way) {
-                tag[w] = r.tag;
-                ep[w] = r.epoch;
-                st[w] = r.stamp;
-            }
-    };
-    for (int k = 0; k < cs.nprev; k++)
-        if (cs.prev[k].set == set) overlay(cs.prev[k]);
-    for (int k = 0; k < cs.ncur; k++)
-        if (cs.cur[k].set == set) overlay(cs.cur[k]);
-}
-
-// Decide where row `local` lives; records the decision.  whole: the rows
-// evaluated now cover every position (A == l), so they are complete.
-// Victims are taken only among ways whose stamp is below `protect` (rows
-// claimed in the phases still using them are never evicted).  A prefetch
-// lookup (`prefetch`) takes a slot only if its set keeps at least two
-// evictable ways, so that the rows the solver must place later always find
-// one; otherwise it returns slot -1.
-//
-// The 32 lanes of one warp decide together: lane w reads and overlays way w
-// (the set's metadata, then the previous and this phase's decisions), and
-// the hit, the victim and the count of evictable ways come from ballots and
-// a shuffle reduction.  A hit is the highest way holding the tag; the victim
-// is the highest empty way, else the evictable way with the least stamp
-// (lowest way on equal stamps).  Every lane returns the same Lookup; lane 0
-// records the decision.  Called by all lanes of the warp with the same
-// arguments.
-__device__ Lookup cache_lookup_w(CacheState &cs, const CacheView &cv, int local, int cur_epoch,
-                                 unsigned long long clk, int whole, unsigned long long protect, int prefetch,
-                                 const SetStage *pre = nullptr)
-{
-    const int lane = threadIdx.x & 31;
-    const int set = local % cv.nsets;
-    const bool mine = lane < cv.nways;
-    int tag = kNoTag, ep = 0;
-    unsigned long long st = 0;
-    if (mine) {
-        if (pre && pre->set == set) {
-            tag = pre->tag[lane];
-            ep = pre->ep[lane];
-            st = pre->st[lane];
-        } else {
-            const long long s = (long long)set * cv.nways + lane;
-            tag = __ldcg(&cv.tag[s]);
-            ep = __ldcg(&cv.epoch[s]);
-            st = __ldcg(&cv.stamp[s]);
-        }
-    }
-    // the previous phase's decisions, then this phase's, in order
-    const int nprev = cs.nprev, ncur = cs.ncur;
-    for (int k = 0; k < nprev; k++) {
-        const CacheRec &r = cs.prev[k];
-        if (r.set == set && r.way == lane) {
-            tag = r.tag;
-            ep = r.epoch;
-            st = r.stamp;
-        }
-    }
-    for (int k = 0; k < ncur; k++) {
-        const CacheRec &r = cs.cur[k];
-        if (r.set == set && r.way == lane) {
-            tag = r.tag;
-            ep = r.epoch;
-            st = r.stamp;
-        }
-    }
-    Lookup L;
-    L.was_prefetched = 0;
-    CacheRec rec;
-    rec.set = set;
-    rec.stamp = prefetch ? (clk | kPrefetchMark) : clk;
-    rec.tag = local;
-    int way;
-    const unsigned hit = __ballot_sync(0xffffffffu, mine && tag == local);
-    if (hit) {
-        way = 31 - __clz(hit);
-        const int ep_hit = __shfl_sync(0xffffffffu, ep, way);
-        const unsigned long long st_hit = __shfl_sync(0xffffffffu, st, way);
-        const int va = ep_hit == kEpochFull || ep_hit == cur_epoch;
-        L.valid_active = va;
-        L.was_prefetched = va && (st_hit & kPrefetchMark) ? 1 : 0;
-        if (prefetch && va) rec.stamp = st_hit;   // a prefetch hit changes nothing
-        rec.way = way;
-        rec.epoch = whole ? kEpochFull : (va ? ep_hit : cur_epoch);
-    } else {
-        const unsigned long long sw = st & ~kPrefetchMark;
-        const bool evict = mine && !(tag != kNoTag && sw >= protect);
-        const unsigned em = __ballot_sync(0xffffffffu, evict);
-        const unsigned empty = __ballot_sync(0xffffffffu, evict && tag == kNoTag);
-        unsigned long long bv = evict ? sw : ~0ull;
-        int bw = evict ? lane : 32;
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int ow = __shfl_xor_sync(0xffffffffu, bw, o);
-            if (ov < bv || (ov == bv && ow < bw)) {
-                bv = ov;
-                bw = ow;
-            }
-        }
-        const int victim = empty ? 31 - __clz(empty) : (em ? bw : -1);
-        if (victim < 0 || (prefetch && __popc(em) < 3)) {
-            L.slot = -1;
-            L.valid_active = 0;
-            return L;
-        }
-        L.valid_active = 0;
-        rec.way = victim;
-        rec.epoch = whole ? kEpochFull : cur_epoch;
-        way = victim;
-    }
-    L.slot = (long long)set * cv.nways + way;
-    __syncwarp();                     // every lane has read cs.cur
-    if (lane == 0) {
-        cs.cur[ncur] = rec;
-        cs.ncur = ncur + 1;
-    }
-    __syncwarp();
-    return L;
-}
-
-// Mark an already-decided slot as complete (after its tail has been filled).
-__device__ void cache_mark_full(CacheState &cs, const CacheView &cv, long long slot, int local,
-                                unsigned long long clk)
-{
-    CacheRec rec;
-    rec.set = (int)(slot / cv.nways);
-    rec.way = (int)(slot % cv.nways);
-    rec.tag = local;
-    rec.epoch = kEpochFull;
-    rec.stamp = clk;
-    cs.cur[cs.ncur++] = rec;
-}
-
-// --------------------------------------------------------------------------
 // per-block solver context
 // --------------------------------------------------------------------------
+// flags of an active position: label, bound status (ST_*), whole row cached,
+// row evaluated ahead of need and not yet used
+constexpr int kFlagPos = 1, kFlagStatus = 1, kFlagFull = 8, kFlagAhead = 16;   // status at bits 1-2
+__device__ __forceinline__ int flag_y(unsigned f) { return (f & kFlagPos) ? +1 : -1; }
+__device__ __forceinline__ unsigned char flag_s(unsigned f) { return (unsigned char)((f >> kFlagStatus) & 3u); }
+__device__ __forceinline__ unsigned char flags_of(int y, unsigned char s, unsigned slotword)
+{
+    return (unsigned char)((y > 0 ? kFlagPos : 0) | (s << kFlagStatus) | ((slotword >> 13) & (kFlagFull | kFlagAhead)));
+}
+// a slot with its flags, as it travels in records and in D.pos_slot
+constexpr unsigned kSlotFull = 1u << 16, kSlotAhead = 1u << 17;
+__device__ __forceinline__ unsigned slot_word(unsigned slot, unsigned f) { return slot | ((f & (kFlagFull | kFlagAhead)) << 13); }
+// a position and its label as they travel in records
+constexpr unsigned kNoPos = 0xffffffffu;
+__device__ __forceinline__ unsigned pos_code(int p, int y) { return (unsigned)p * 2u + (y > 0 ? 1u : 0u); }
+__device__ __forceinline__ int code_pos(unsigned c) { return c == kNoPos ? -1 : (int)(c >> 1); }
+__device__ __forceinline__ int code_y(unsigned c) { return (c & 1u) ? +1 : -1; }
+
+// work counters of a solve, kept by thread 0
+enum { kCntActive, kCntQ, kCntLook, kCntMiss, kCntFill, kCntAhead, kCntTargets, kCnt };
+
+constexpr int kPollWarps = (kMaxGroupBlocks + 31) / 32;   // each polls the records of 32 blocks
+static_assert(kPollWarps < kWarps, "a warp is left for the prefetch candidates");
+
+// The winning records of a phase as one poll warp saw them.
+//   phase A, track t: words 4t..: {-y G, pos_code} {alpha, column} {QD, slot} {-, row}
+//   phase B:          {decrease, pos_code} {G, column} {alpha, row} {QD, slot} {Gmax2, Q_ij} {Gmax2 of y=-1, Q_ij of track 1}
+// (nu-SVC has two tracks; C-SVC uses track 0 and the first Gmax2)
+struct WinA { double d[2 * kWordsI]; unsigned x[2 * kWordsI]; };
+struct WinB { double d[kWordsJ]; unsigned x[kWordsJ]; };
+// a prefetch candidate: priority, position and label, column, row, slot (kNoSlot: not cached)
+struct Cand { double v; unsigned pc, col, row, slot; };
+
+// what every thread of the block knows about its part of the instance; thread 0
+// writes it, between barriers
+struct Ctx {
+    float *stage;           // source staging area (dynamic smem)
+    float *tile;            // per-warp 32-row transpose tiles (dense rows)
+    int choff;              // my chunk of [0,A): its offset in dynamic shared memory
+    int rank, nb;
+    int A;                  // active size
+    int a0, a1;             // my chunk of [0,A)
+    int t0, t1;             // my chunk of [A,l)
+    int phase;              // exchange counter: selects the record buffer and sequence number
+    uint32_t tcbase;        // FORM_BF16X3: shared address of the operand stages (1024-aligned)
+    long long tc_g;         // tensor-core steps issued so far (mbarrier phase parities)
+    long long fg;           // steps of the fill pipeline so far (its mbarrier phase parities)
+    int fstages;            // operand stages of the fill pipeline (3 or 4, by the stage area)
+};
+
 struct Shared {
+    InstanceDesc D;
+    Ctx c;
     RedScratch red;
-    CacheState cs;
     StageSlots ss;
-    double bd[24];
-    int bi[24];
-    long long bl[8];
+    // warps' partial results of a phase: keys and positions
+    u64 wk[3][kWarps];
+    int wi[2][kWarps], wp[kWarps];
+    WinA wa[kPollWarps];
+    WinB wb[kPollWarps];
+    Cand cand[kPrefetchCand];       // single-block groups: the block's own candidates
+    long long cnt[kCnt], prof[8], tstart;
+    unsigned prof32[8];             // cycles since the last flush
+    unsigned ahead_used;            // rows evaluated ahead of need and used later (every block counts its own)
+    int fail;
+    // slot allocation, replayed identically by every block: the next slot to
+    // look at, whether slots are being reused, and the reference bits
+    int hand, reused;
+    unsigned ref[kRefSlots / 32];
     int srcpos[kSrcBatch];
     int srcrow[kSrcBatch];
     int nsrc;
     int stop_at;
-    Partial lrec[2];
-    double cand_v[kWarps];
-    int cand_p[kWarps];
-    // rows of the current fill pass: row id, label, slot
-    int frow[kPrefetchMax], fy[kPrefetchMax];
-    long long fslot[kPrefetchMax];
+    // rows of the current fill pass: row id, label, slot, position (with how
+    // many of them are evaluated ahead of need)
+    int frow[kPrefetchMax], fy[kPrefetchMax], fslot[kPrefetchMax], fpos[kPrefetchMax], fcol[kPrefetchMax];
+    int nfill, nneed;
     // per source of the fill pass running now: norm, label, destination row
     double fsx[kPrefetchMax];
     int fsy[kPrefetchMax];
     float *fsd[kPrefetchMax];
-    int nfill;
-    int pick[kPrefetchMax];
-    int npick;
-    SetStage sset[kPrefetchMax];    // cache sets of the prefetch picks, read in one round trip
     // tensor-core block products (FORM_BF16X3, FORM_FP16X3): sources of the current pass
     // (row id, position, alpha, norm, C, inverse scale, label, status), the
     // pipeline's mbarriers (one per operand stage) and the TMEM base address
@@ -807,108 +676,88 @@ struct Shared {
     // written / read; fabort is set by a role whose wait ran out
     uint64_t ffull[kFillStagesMax], fempty[kFillStagesMax], faccf[kFillAcc], facce[kFillAcc];
     int fabort;
+    Partial lrec[2];                // single-block groups keep their two exchange records here
 };
 
-// The group's prefetch candidates (kPrefetchCand per block).  They live in
-// the same shared memory as the transpose tiles: candidates are read, chosen
-// and looked up before the fill pass reuses the space.
-struct PrefetchTable {
-    double v[kMaxGroupBlocks * kPrefetchCand];
-    int pos[kMaxGroupBlocks * kPrefetchCand], loc[kMaxGroupBlocks * kPrefetchCand];
-    int row[kMaxGroupBlocks * kPrefetchCand], y[kMaxGroupBlocks * kPrefetchCand];
-};
-
-struct Ctx {
-    const InstanceDesc *D;
-    float *stage;           // source staging area (dynamic smem)
-    float *tile;            // per-warp 32-row transpose tiles (dense rows) ...
-    PrefetchTable *pt;      // ... sharing their space with the prefetch candidates
-    // my chunk of [0,A) held in shared memory
-    double *sG, *sA, *sQD;
-    int *sCol, *sRow;
-    signed char *sY;
-    unsigned char *sS;
-    int rank, nb;
-    int A;                  // active size
-    int a0, a1;             // my chunk of [0,A)
-    int t0, t1;             // my chunk of [A,l)
-    int epoch;
-    int phase;              // exchange counter: selects the record buffer and sequence number
-    Partial *lrec;          // single-block groups keep their two records in shared memory
-    uint32_t tcbase;        // FORM_BF16X3: shared address of the operand stages (1024-aligned)
-    long long tc_g, tc_t;   // tensor-core steps and tiles issued so far (mbarrier phase parities)
-    long long fg;           // steps of the fill pipeline so far (its mbarrier phase parities)
-    int fstages;            // operand stages of the fill pipeline (3 or 4, by the stage area)
-};
-
-__device__ __forceinline__ void set_chunks(Ctx &c)
+// The block's shared state, reachable by its address from every device function
+// (a reference passed to a function that is not inlined would make each
+// access a generic one).
+__device__ __forceinline__ Shared &block_shared()
 {
-    const long long n = c.A;
-    c.a0 = (int)(n * c.rank / c.nb);
-    c.a1 = (int)(n * (c.rank + 1) / c.nb);
-    const long long m = c.D->l - c.A;
-    c.t0 = c.A + (int)(m * c.rank / c.nb);
-    c.t1 = c.A + (int)(m * (c.rank + 1) / c.nb);
+    __shared__ Shared s;
+    return s;
+}
+extern __shared__ __align__(128) unsigned char dyn[];
+
+__device__ __noinline__ float q_of(int yy, double dot, double xsq_a, double xsq_b)
+{
+    return q_value(block_shared().D.kp, yy, dot, xsq_a, xsq_b);
 }
 
-__device__ __forceinline__ Partial *my_partial(const Ctx &c)
+// the block's chunk of the active state, in dynamic shared memory
+struct Chunk {
+    double *G, *A, *QD;
+    int *Col, *Row;
+    unsigned short *Slot;
+    unsigned char *F;       // kFlag*
+};
+__device__ __forceinline__ Chunk chunk_at(int off, int cap)
 {
-    if (c.nb == 1) return c.lrec + (c.phase & 1);
-    return c.D->partials + (long long)(c.phase & 1) * c.nb + c.rank;
-}
-__device__ __forceinline__ const Partial *prev_partials(const Ctx &c)
-{
-    if (c.nb == 1) return c.lrec + ((c.phase - 1) & 1);
-    return c.D->partials + (long long)((c.phase - 1) & 1) * c.nb;
+    Chunk k;
+    k.G = reinterpret_cast<double *>(dyn + off);
+    k.A = k.G + cap;
+    k.QD = k.A + cap;
+    k.Col = reinterpret_cast<int *>(k.QD + cap);
+    k.Row = k.Col + cap;
+    k.Slot = reinterpret_cast<unsigned short *>(k.Row + cap);
+    k.F = reinterpret_cast<unsigned char *>(k.Slot + cap);
+    return k;
 }
 
-// Record fields read by the reductions.  Multi-block records were written by
-// other SMs: read them at L2 (ld.global.cg); single-block records live in
-// shared memory.
-struct RecVals {
-    double v[6];
-    int n[8];
-    float q[2];
-};
-__device__ __forceinline__ void rec_load(const Ctx &c, const Partial *p, RecVals &r, int with_n_hi, int with_q)
+
+// the active size and my chunks of [0,A) and [A,l); called by every thread
+__device__ __forceinline__ void set_active(int A)
 {
-    if (c.nb == 1) {
-        for (int k = 0; k < 6; k++) r.v[k] = p->v[k];
-        for (int k = 0; k < 8; k++) r.n[k] = p->n[k];
-        r.q[0] = p->q[0];
-        r.q[1] = p->q[1];
-        return;
+    Ctx &c = block_shared().c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const long long n = A, m = block_shared().D.l - A;
+        c.A = A;
+        c.a0 = (int)(n * c.rank / c.nb);
+        c.a1 = (int)(n * (c.rank + 1) / c.nb);
+        c.t0 = A + (int)(m * c.rank / c.nb);
+        c.t1 = A + (int)(m * (c.rank + 1) / c.nb);
     }
-    const double2 a = __ldcg(reinterpret_cast<const double2 *>(&p->v[0]));
-    const double2 b = __ldcg(reinterpret_cast<const double2 *>(&p->v[2]));
-    const double2 d = __ldcg(reinterpret_cast<const double2 *>(&p->v[4]));
-    const int4 n0 = __ldcg(reinterpret_cast<const int4 *>(&p->n[0]));
-    r.v[0] = a.x; r.v[1] = a.y; r.v[2] = b.x; r.v[3] = b.y; r.v[4] = d.x; r.v[5] = d.y;
-    r.n[0] = n0.x; r.n[1] = n0.y; r.n[2] = n0.z; r.n[3] = n0.w;
-    if (with_n_hi) {
-        const int4 n1 = __ldcg(reinterpret_cast<const int4 *>(&p->n[4]));
-        r.n[4] = n1.x; r.n[5] = n1.y; r.n[6] = n1.z; r.n[7] = n1.w;
-    }
-    if (with_q) {
-        const float2 q = __ldcg(reinterpret_cast<const float2 *>(&p->q[0]));
-        r.q[0] = q.x;
-        r.q[1] = q.y;
-    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ Partial *my_partial()
+{
+    Ctx &c = block_shared().c;
+    if (c.nb == 1) return block_shared().lrec + (c.phase & 1);
+    return block_shared().D.partials + (long long)(c.phase & 1) * c.nb + c.rank;
+}
+__device__ __forceinline__ const Partial *prev_partials()
+{
+    Ctx &c = block_shared().c;
+    if (c.nb == 1) return block_shared().lrec + ((c.phase - 1) & 1);
+    return block_shared().D.partials + (long long)((c.phase - 1) & 1) * c.nb;
 }
 
 // Publish my record of this phase and wait for everybody's (group barrier).
-__device__ bool exchange(Ctx &c, Shared &sh)
+__device__ bool exchange()
 {
+    Ctx &c = block_shared().c;
     __syncthreads();
     const int want = c.phase + 1;
-    Partial *mine = my_partial(c);
+    Partial *mine = my_partial();
     int ok = 1;
     if (c.nb > 1) {
         // the release store orders this thread's writes and, through the
         // barrier above, the whole block's before the record is seen
         if (threadIdx.x == 0) st_release_i32(&mine->seq, want);
-        const Partial *all = c.D->partials + (long long)(c.phase & 1) * c.nb;
-        const long long limit = c.D->wait_ns > 0 ? c.D->wait_ns : kWaitTimeoutNs;
+        const Partial *all = block_shared().D.partials + (long long)(c.phase & 1) * c.nb;
+        const long long limit = block_shared().D.wait_ns > 0 ? block_shared().D.wait_ns : kWaitTimeoutNs;
         for (int b = threadIdx.x; b < c.nb; b += blockDim.x) {
             const long long t0 = (long long)tc::global_ns();
             long long spins = 0;
@@ -916,8 +765,8 @@ __device__ bool exchange(Ctx &c, Shared &sh)
             // then synchronizes with the record's release store
             while (ld_relaxed_i32(&all[b].seq) != want) {
                 if ((++spins & 63) == 0) {
-                    if (ld_relaxed_i32(&c.D->sync->error) != 0 || (long long)tc::global_ns() - t0 > limit) {
-                        atomicExch(&c.D->sync->error, 1);
+                    if (ld_relaxed_i32(&block_shared().D.sync->error) != 0 || (long long)tc::global_ns() - t0 > limit) {
+                        atomicExch(&block_shared().D.sync->error, 1);
                         ok = 0;
                         break;
                     }
@@ -929,8 +778,7 @@ __device__ bool exchange(Ctx &c, Shared &sh)
     // the pollers' acquire loads, followed by the barrier, order every later
     // read of this block after the other blocks' releases
     ok = __syncthreads_and(ok);
-    if (threadIdx.x == 0) cache_rotate(sh.cs, c.D->cache, c.rank);
-    c.phase++;
+    if (threadIdx.x == 0) c.phase++;
     __syncthreads();
     return ok != 0;
 }
@@ -945,37 +793,45 @@ __device__ __forceinline__ unsigned char status_of(double a, double C)
 }
 
 // chunk state: global -> shared / shared -> global (mutable fields only)
-__device__ void chunk_load(Ctx &c)
+__device__ void chunk_load()
 {
-    const InstanceDesc &D = *c.D;
+    Ctx &c = block_shared().c;
+    const InstanceDesc &D = block_shared().D;
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
     for (int k = threadIdx.x; k < c.a1 - c.a0; k += blockDim.x) {
         const int p = c.a0 + k;
-        c.sG[k] = D.G[p];
-        c.sA[k] = D.alpha[p];
-        c.sQD[k] = D.QD[p];
-        c.sCol[k] = D.pos_local[p];
-        c.sRow[k] = D.pos_row[p];
-        c.sY[k] = D.y[p];
-        c.sS[k] = D.status[p];
+        const unsigned w = (unsigned)D.pos_slot[p];
+        ck.G[k] = D.G[p];
+        ck.A[k] = D.alpha[p];
+        ck.QD[k] = D.QD[p];
+        ck.Col[k] = D.pos_local[p];
+        ck.Row[k] = D.pos_row[p];
+        ck.Slot[k] = (unsigned short)(w & 0xffffu);
+        ck.F[k] = flags_of(D.y[p], D.status[p], w);
     }
     __syncthreads();
 }
-__device__ void chunk_store(Ctx &c)
+__device__ void chunk_store()
 {
-    const InstanceDesc &D = *c.D;
+    Ctx &c = block_shared().c;
+    const InstanceDesc &D = block_shared().D;
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
     __syncthreads();
     for (int k = threadIdx.x; k < c.a1 - c.a0; k += blockDim.x) {
         const int p = c.a0 + k;
-        D.G[p] = c.sG[k];
-        D.alpha[p] = c.sA[k];
-        D.status[p] = c.sS[k];
+        D.G[p] = ck.G[k];
+        D.alpha[p] = ck.A[k];
+        D.status[p] = flag_s(ck.F[k]);
+        D.pos_slot[p] = (int)slot_word(ck.Slot[k], ck.F[k]);
     }
 }
 
 // Sum over the group's blocks of per-block counters of the previous exchange.
-__device__ void group_counts(const Ctx &c, Shared &sh, int slot, int *below, int *above, int *total)
+__device__ void group_counts(int slot, int *below, int *above, int *total)
 {
-    const Partial *all = prev_partials(c);
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const Partial *all = prev_partials();
     int b_lo = 0, b_hi = 0, tot = 0;
     for (int b = threadIdx.x; b < c.nb; b += blockDim.x) {
         const int v = c.nb == 1 ? all[b].n[slot] : __ldcg(&all[b].n[slot]);
@@ -999,9 +855,11 @@ __device__ void group_counts(const Ctx &c, Shared &sh, int slot, int *below, int
 // same order as in the reference.
 // --------------------------------------------------------------------------
 template <int FORM>
-__device__ void accumulate_rows(Ctx &c, Shared &sh, int src_end, int pick_free_only, int with_bar, int lo, int hi)
+__device__ __noinline__ void accumulate_rows(int src_end, int pick_free_only, int with_bar, int lo, int hi)
 {
-    const InstanceDesc &D = *c.D;
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const InstanceDesc &D = block_shared().D;
     const int cap = D.stage_cap > 0 ? D.stage_cap : kSrcBatch;
     int scan = 0;
     while (true) {
@@ -1046,7 +904,7 @@ __device__ void accumulate_rows(Ctx &c, Shared &sh, int src_end, int pick_free_o
                 const int sp = sh.srcpos[k];
                 const int ys = D.y[sp];
                 const double xs = D.x.xsq ? D.x.xsq[sh.srcrow[k]] : 0.0;
-                const float q = q_value(D.kp, ys * ye, dots[k], xs, xe);
+                const float q = q_of(ys * ye, dots[k], xs, xe);
                 g = __dadd_rn(g, __dmul_rn(D.alpha[sp], (double)q));
                 if (with_bar && D.status[sp] == ST_UPPER) gb = __dadd_rn(gb, __dmul_rn(get_C(D, ys), (double)q));
             }
@@ -1085,9 +943,13 @@ __device__ void accumulate_rows(Ctx &c, Shared &sh, int src_end, int pick_free_o
 // from the running step counter c.tc_g.  A wait that times out sets the group's error flag and
 // the product returns false.
 template <class Epi>
-__device__ bool tc_product(Ctx &c, Shared &sh, int ns, int lo, int hi, bool global_targets, Epi &&epi)
+__device__ bool tc_product(int ns, int lo, int hi, bool global_targets, Epi &&epi)
 {
-    const InstanceDesc &D = *c.D;
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const InstanceDesc &D = block_shared().D;
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
+    const long long tcg = c.tc_g;
     const int NK = D.x.nchunk;
     const int ntiles = hi > lo ? (hi - lo + kTcM - 1) / kTcM : 0;
     const int total = ntiles * NK;
@@ -1110,13 +972,13 @@ __device__ bool tc_product(Ctx &c, Shared &sh, int ns, int lo, int hi, bool glob
     auto load = [&](int g) {
         if (warp == issuer) return;
         const int tile = g / NK, kc = g - tile * NK;
-        const uint32_t sa = c.tcbase + (uint32_t)((c.tc_g + g) % kTcStages) * sbytes;
+        const uint32_t sa = c.tcbase + (uint32_t)((tcg + g) % kTcStages) * sbytes;
         const int tb = lo + tile * kTcM;
         for (int i = threadIdx.x; i < kTcM * 16; i += nload) {
             const int r = i >> 4, q = i & 15;
             const int t = tb + r;
             const bool ok = t < hi;
-            const int row = ok ? (global_targets ? D.pos_row[t] : c.sRow[t]) : 0;
+            const int row = ok ? (global_targets ? D.pos_row[t] : ck.Row[t]) : 0;
             tc::cp_async16(sa + (q >= 8 ? a_lo : 0u) + tc::sw128_offset(r, q & 7),
                            Xs + (long long)row * rs + kc * 128 + q * 8, ok ? 16u : 0u);
         }
@@ -1152,7 +1014,7 @@ __device__ bool tc_product(Ctx &c, Shared &sh, int ns, int lo, int hi, bool glob
     }
     bool ok = true;
     for (int g = 0; g < total; g++) {
-        const long long G = c.tc_g + g;
+        const long long G = tcg + g;
         const int tile = g / NK, kc = g - tile * NK;
         // step g has landed: the groups of steps g+1 .. g+kTcStages-2 may still be pending
         tc::cp_async_wait<kTcStages - 2>();
@@ -1208,7 +1070,7 @@ __device__ bool tc_product(Ctx &c, Shared &sh, int ns, int lo, int hi, bool glob
         if (!ok) break;
     }
     if (ok) {
-        const long long G = c.tc_g + total - 1;
+        const long long G = tcg + total - 1;
         ok = __syncthreads_and(tc::mbar_wait(&sh.tbar[G % kTcStages], (unsigned)((G / kTcStages) & 1))) != 0;
         if (ok) {
             absorb(G);
@@ -1217,8 +1079,7 @@ __device__ bool tc_product(Ctx &c, Shared &sh, int ns, int lo, int hi, bool glob
         }
     }
     tc::cp_async_wait<0>();
-    c.tc_g += total;
-    c.tc_t += ntiles;
+    if (threadIdx.x == 0) c.tc_g += total;
     if (!ok && threadIdx.x == 0) atomicExch(&D.sync->error, 1);
     __syncthreads();
     return ok;
@@ -1241,19 +1102,22 @@ __device__ bool tc_product(Ctx &c, Shared &sh, int ns, int lo, int hi, bool glob
 // The MMAs, their order and the fp64 flush are those of tc_product, so the Q
 // values are the same bit for bit.  Every wait is bounded; a role whose wait
 // runs out sets fabort, which ends the other roles' waits.
-__device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, const int *src_y, const long long *slot,
-                             int tail)
+__device__ __noinline__ bool fill_rows_tc(int ns, int tail)
 {
-    const InstanceDesc &D = *c.D;
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const InstanceDesc &D = block_shared().D;
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
+    const long long fg = c.fg;
     if (ns == 0) return true;
     if (threadIdx.x < ns) {
         // the sources' row, norm, inverse scale, label and destination row
         const int k = threadIdx.x;
-        sh.tsrow[k] = src_row[k];
-        sh.fsx[k] = D.x.xsq[src_row[k]];
-        sh.tsi[k] = D.x.xinv ? D.x.xinv[src_row[k]] : 1.0;
-        sh.fsy[k] = src_y[k];
-        sh.fsd[k] = D.cache.data + slot[k] * D.cache.stride;
+        sh.tsrow[k] = sh.frow[k];
+        sh.fsx[k] = D.x.xsq[sh.frow[k]];
+        sh.tsi[k] = D.x.xinv ? D.x.xinv[sh.frow[k]] : 1.0;
+        sh.fsy[k] = sh.fy[k];
+        sh.fsd[k] = D.cache.data + (long long)sh.fslot[k] * D.cache.stride;
     }
     __syncthreads();
     const int lo = tail ? c.t0 : 0, hi = tail ? c.t1 : c.a1 - c.a0;
@@ -1276,8 +1140,8 @@ __device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, con
         double acc[kPrefetchMax];
 #pragma unroll
         for (int k = 0; k < kPrefetchMax; k++) acc[k] = 0.0;
-        int a = (int)(c.fg % kFillAcc);
-        unsigned ph = (unsigned)((c.fg / kFillAcc) & 1);
+        int a = (int)(fg % kFillAcc);
+        unsigned ph = (unsigned)((fg / kFillAcc) & 1);
         int kc = 0, tile = 0;
         int yp = 0, col = 0;
         bool tok = false;
@@ -1293,9 +1157,9 @@ __device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, con
                         yp = D.y[t];
                         col = D.pos_local[t];
                     } else {
-                        r = c.sRow[t];
-                        yp = c.sY[t];
-                        col = c.sCol[t];
+                        r = ck.Row[t];
+                        yp = flag_y(ck.F[t]);
+                        col = ck.Col[t];
                     }
                     xe = D.x.xsq[r];
                     ie = D.x.xinv ? D.x.xinv[r] : 1.0;
@@ -1321,7 +1185,7 @@ __device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, con
 #pragma unroll
                     for (int k = 0; k < kPrefetchMax; k++)
                         if (k < ns)
-                            __stcg(sh.fsd[k] + col, q_value(D.kp, sh.fsy[k] * yp,
+                            __stcg(sh.fsd[k] + col, q_of(sh.fsy[k] * yp,
                                                             __dmul_rn(__dmul_rn(acc[k], ie), sh.tsi[k]), sh.fsx[k], xe));
                 }
 #pragma unroll
@@ -1335,8 +1199,8 @@ __device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, con
         if (lane == 0) {
             const uint32_t idesc = D.form == FORM_TF32 ? tc::idesc_tf32_f32(kTcM, kFillN)
                                                        : tc::idesc_f16_f32(kTcM, kFillN, D.form == FORM_BF16X3);
-            int s = (int)(c.fg % S), a = (int)(c.fg % kFillAcc);
-            unsigned phs = (unsigned)((c.fg / S) & 1), pha = (unsigned)((c.fg / kFillAcc) & 1);
+            int s = (int)(fg % S), a = (int)(fg % kFillAcc);
+            unsigned phs = (unsigned)((fg / S) & 1), pha = (unsigned)((fg / kFillAcc) & 1);
             int issued = 0;
             for (int g = 0; g < total; g++) {
                 if (!tc::mbar_wait_or(&sh.ffull[s], phs, abort) || !tc::mbar_wait_or(&sh.facce[a], pha ^ 1u, abort)) {
@@ -1381,7 +1245,7 @@ __device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, con
             if (issued < total && issued > 0) {
                 // stopped early: let the MMAs already issued finish before the
                 // stages and the accumulators are given up
-                const long long G = c.fg + issued - 1;
+                const long long G = fg + issued - 1;
                 tc::mbar_wait(&sh.fempty[G % S], (unsigned)((G / S) & 1));
             }
         }
@@ -1396,8 +1260,8 @@ __device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, con
         const uint16_t *Xs = D.x.Xs;
         const uint16_t *src[kPieces];
         uint32_t off[kPieces];
-        int s = (int)(c.fg % S), sd = s;
-        unsigned phs = (unsigned)((c.fg / S) & 1);
+        int s = (int)(fg % S), sd = s;
+        unsigned phs = (unsigned)((fg / S) & 1);
         int kc = 0, tile = 0;
         bool run = true;
         // up to S - 1 steps in flight; a landed step is handed to the MMA
@@ -1422,7 +1286,7 @@ __device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, con
                         if (i < 16 * kTcM) {
                             const int r = i >> 4, q = i & 15, t = tb + r;
                             if (t < hi) {
-                                const int row = tail ? D.pos_row[t] : c.sRow[t];
+                                const int row = tail ? D.pos_row[t] : ck.Row[t];
                                 src[j] = Xs + (long long)row * rs + q * 8;
                                 off[j] = (q >= 8 ? a_lo : 0u) + tc::sw128_offset(r, q & 7);
                             }
@@ -1455,11 +1319,13 @@ __device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, con
         }
         tc::cp_async_wait<0>();
     }
-    c.fg += total;
     tc::tc_fence_before();
     __syncthreads();
     const bool ok = *abort == 0;
-    if (!ok && threadIdx.x == 0) atomicExch(&D.sync->error, 1);
+    if (threadIdx.x == 0) {
+        c.fg += total;
+        if (!ok) atomicExch(&D.sync->error, 1);
+    }
     __syncthreads();
     tc::tc_fence_after();
     return ok;
@@ -1468,9 +1334,11 @@ __device__ bool fill_rows_tc(Ctx &c, Shared &sh, int ns, const int *src_row, con
 // tensor-core form of accumulate_rows: sources are taken kTcMaxN (tc_n) at a
 // time; per target the contributions of one pass are summed in source order
 // in four column groups, which are then added in a fixed order
-__device__ bool accumulate_rows_tc(Ctx &c, Shared &sh, int src_end, int pick_free_only, int with_bar, int lo, int hi)
+__device__ __noinline__ bool accumulate_rows_tc(int src_end, int pick_free_only, int with_bar, int lo, int hi)
 {
-    const InstanceDesc &D = *c.D;
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const InstanceDesc &D = block_shared().D;
     const int cap = D.tc_n;
     int scan = 0;
     double *red = reinterpret_cast<double *>(c.tile);   // [2][4][kTcM] partial sums (aux area)
@@ -1516,7 +1384,7 @@ __device__ bool accumulate_rows_tc(Ctx &c, Shared &sh, int src_end, int pick_fre
             sh.tss[threadIdx.x] = D.status[sp];
         }
         __syncthreads();
-        const bool ok = tc_product(c, sh, ns, lo, hi, true, [&](int tlo, const double *acc) {
+        const bool ok = tc_product(ns, lo, hi, true, [&](int tlo, const double *acc) {
             const int t = tlo + lg * 32 + lane;
             double part = 0.0, partb = 0.0;
             if (cg * 16 < ns && t < hi) {
@@ -1529,7 +1397,7 @@ __device__ bool accumulate_rows_tc(Ctx &c, Shared &sh, int src_end, int pick_fre
                     const int s = cg * 16 + k;
                     if (s < ns) {
                         const double dot = __dmul_rn(__dmul_rn(acc[k], ie), sh.tsi[s]);
-                        const float q = q_value(D.kp, sh.tsy[s] * ye, dot, sh.tsx[s], xe);
+                        const float q = q_of(sh.tsy[s] * ye, dot, sh.tsx[s], xe);
                         part = __dadd_rn(part, __dmul_rn(sh.tsa[s], (double)q));
                         if (with_bar && sh.tss[s] == ST_UPPER) partb = __dadd_rn(partb, __dmul_rn(sh.tsc[s], (double)q));
                     }
@@ -1558,12 +1426,12 @@ __device__ bool accumulate_rows_tc(Ctx &c, Shared &sh, int src_end, int pick_fre
 
 // the row-block product of the form: CUDA cores or tensor cores
 template <int FORM>
-__device__ bool accumulate(Ctx &c, Shared &sh, int src_end, int pick_free_only, int with_bar, int lo, int hi)
+__device__ bool accumulate(int src_end, int pick_free_only, int with_bar, int lo, int hi)
 {
     if constexpr (is_tc_form(FORM)) {
-        return accumulate_rows_tc(c, sh, src_end, pick_free_only, with_bar, lo, hi);
+        return accumulate_rows_tc(src_end, pick_free_only, with_bar, lo, hi);
     } else {
-        accumulate_rows<FORM>(c, sh, src_end, pick_free_only, with_bar, lo, hi);
+        accumulate_rows<FORM>(src_end, pick_free_only, with_bar, lo, hi);
         return true;
     }
 }
@@ -1571,21 +1439,22 @@ __device__ bool accumulate(Ctx &c, Shared &sh, int src_end, int pick_free_only, 
 // gradient reconstruction (reference svm.cpp:473-513); group collective on the
 // global state (the caller has stored its chunk)
 template <int FORM>
-__device__ bool reconstruct(Ctx &c, Shared &sh)
+__device__ bool reconstruct()
 {
-    const InstanceDesc &D = *c.D;
+    Ctx &c = block_shared().c;
+    const InstanceDesc &D = block_shared().D;
     if (c.A == D.l) return true;
     if (D.lazy_gbar) {
         // G = p + sum over every alpha > 0 (active or not) of alpha * Q, on the inactive positions
         for (int e = c.t0 + threadIdx.x; e < c.t1; e += blockDim.x) D.G[e] = D.p[e];
         __syncthreads();
-        if (!accumulate<FORM>(c, sh, D.l, 0, 0, c.t0, c.t1)) return false;
-        return exchange(c, sh);
+        if (!accumulate<FORM>(D.l, 0, 0, c.t0, c.t1)) return false;
+        return exchange();
     }
     for (int e = c.t0 + threadIdx.x; e < c.t1; e += blockDim.x) D.G[e] = __dadd_rn(D.G_bar[e], D.p[e]);
     __syncthreads();
-    if (!accumulate<FORM>(c, sh, c.A, 1, 0, c.t0, c.t1)) return false;
-    return exchange(c, sh);
+    if (!accumulate<FORM>(c.A, 1, 0, c.t0, c.t1)) return false;
+    return exchange();
 }
 
 // --------------------------------------------------------------------------
@@ -1615,32 +1484,41 @@ __device__ __forceinline__ void swap_pos(const InstanceDesc &D, int a, int b)
     unsigned char ts = D.status[a]; D.status[a] = D.status[b]; D.status[b] = ts;
     int ti = D.pos_local[a]; D.pos_local[a] = D.pos_local[b]; D.pos_local[b] = ti;
     ti = D.pos_row[a]; D.pos_row[a] = D.pos_row[b]; D.pos_row[b] = ti;
+    ti = D.pos_slot[a]; D.pos_slot[a] = D.pos_slot[b]; D.pos_slot[b] = ti;
 }
 
-// widen the active set to l after a reconstruction (chunk reloaded)
-__device__ void widen(Ctx &c)
+// widen the active set to l after a reconstruction (chunk reloaded).  Only
+// complete rows stay cached, and of an inactive variable's only those whose
+// slot no other row has taken since.
+__device__ void widen()
 {
-    c.A = c.D->l;
-    c.epoch++;
-    set_chunks(c);
-    chunk_load(c);
+    Ctx &c = block_shared().c;
+    const InstanceDesc &D = block_shared().D;
+    set_active(D.l);
+    for (int p = c.a0 + threadIdx.x; p < c.a1; p += blockDim.x) {
+        const unsigned w = (unsigned)D.pos_slot[p], slot = w & 0xffffu;
+        if (slot == kNoSlot) continue;
+        if (!(w & kSlotFull) || __ldcg(&D.cache.tag[slot]) != D.pos_local[p]) D.pos_slot[p] = kNoSlot;
+    }
+    chunk_load();
 }
 
 template <int FORM>
-__device__ bool do_shrinking(Ctx &c, Shared &sh, int &unshrink)
+__device__ __noinline__ bool do_shrinking(int &unshrink)
 {
-    const InstanceDesc &D = *c.D;
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const InstanceDesc &D = block_shared().D;
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
     const int nu = D.nu;
     const int n = c.a1 - c.a0;
     // 1. maximal violations over the active set (C-SVC: Gmax1, Gmax2; nu: Gmax1..4)
     {
         double v[4] = {-SVMB_INF, -SVMB_INF, -SVMB_INF, -SVMB_INF};
-        int ix[4] = {-1, -1, -1, -1};
-        const int kind[4] = {2, 2, 2, 2};
         for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            const unsigned char s = c.sS[k];
-            const double G = c.sG[k];
-            const int y = c.sY[k];
+            const unsigned char s = flag_s(ck.F[k]);
+            const double G = ck.G[k];
+            const int y = flag_y(ck.F[k]);
             if (!nu) {
                 if (y == +1) {
                     if (s != ST_UPPER) v[0] = fmax(v[0], -G);
@@ -1654,47 +1532,42 @@ __device__ bool do_shrinking(Ctx &c, Shared &sh, int &unshrink)
                 if (s != ST_LOWER) { if (y == +1) v[1] = fmax(v[1], G); else v[2] = fmax(v[2], G); }
             }
         }
-        block_reduce<4>(sh.red, v, ix, kind);
+        block_max<4>(sh.red, v);
         if (threadIdx.x == 0) {
-            Partial *pp = my_partial(c);
+            Partial *pp = my_partial();
             for (int k = 0; k < 4; k++) pp->v[k] = v[k];
         }
     }
-    chunk_store(c);     // the swaps and a reconstruction work on the global state
-    if (!exchange(c, sh)) return false;
+    chunk_store();     // the swaps and a reconstruction work on the global state
+    if (!exchange()) return false;
     double g[4];
     {
-        const Partial *all = prev_partials(c);
+        const Partial *all = prev_partials();
         double v[4] = {-SVMB_INF, -SVMB_INF, -SVMB_INF, -SVMB_INF};
-        int ix[4] = {-1, -1, -1, -1};
-        const int kind[4] = {2, 2, 2, 2};
-        for (int b = threadIdx.x; b < c.nb; b += blockDim.x) {
-            RecVals r;
-            rec_load(c, &all[b], r, 0, 0);
-            for (int k = 0; k < 4; k++) v[k] = fmax(v[k], r.v[k]);
-        }
-        block_reduce<4>(sh.red, v, ix, kind);
+        for (int b = threadIdx.x; b < c.nb; b += blockDim.x)
+            for (int k = 0; k < 4; k++) v[k] = fmax(v[k], c.nb == 1 ? all[b].v[k] : __ldcg(&all[b].v[k]));
+        block_max<4>(sh.red, v);
         for (int k = 0; k < 4; k++) g[k] = v[k];
     }
     const double gap = nu ? fmax(__dadd_rn(g[0], g[1]), __dadd_rn(g[2], g[3])) : __dadd_rn(g[0], g[1]);
     if (!unshrink && gap <= __dmul_rn(D.eps, 10.0)) {
         unshrink = 1;
-        if (!reconstruct<FORM>(c, sh)) return false;
-        widen(c);
+        if (!reconstruct<FORM>()) return false;
+        widen();
     }
     // 2. shrunk positions per block -> new active size K
     {
         int cnt = 0;
         for (int k = threadIdx.x; k < c.a1 - c.a0; k += blockDim.x)
-            cnt += be_shrunk(nu, c.sS[k], c.sY[k], c.sG[k], g) ? 1 : 0;
+            cnt += be_shrunk(nu, flag_s(ck.F[k]), flag_y(ck.F[k]), ck.G[k], g) ? 1 : 0;
         cnt = block_sum_i(sh.red, cnt);
-        if (threadIdx.x == 0) my_partial(c)->n[0] = cnt;
+        if (threadIdx.x == 0) my_partial()->n[0] = cnt;
     }
-    if (!exchange(c, sh)) return false;
+    if (!exchange()) return false;
     int K;
     {
         int below, above, tot;
-        group_counts(c, sh, 0, &below, &above, &tot);
+        group_counts(0, &below, &above, &tot);
         K = c.A - tot;
     }
     // 3. holes = shrunk positions in [0,K) ascending, movers = kept positions in [K,A) descending
@@ -1702,18 +1575,18 @@ __device__ bool do_shrinking(Ctx &c, Shared &sh, int &unshrink)
         int h = 0, m = 0;
         for (int k = threadIdx.x; k < c.a1 - c.a0; k += blockDim.x) {
             const int p = c.a0 + k;
-            const bool s = be_shrunk(nu, c.sS[k], c.sY[k], c.sG[k], g);
+            const bool s = be_shrunk(nu, flag_s(ck.F[k]), flag_y(ck.F[k]), ck.G[k], g);
             if (p < K && s) h++;
             if (p >= K && !s) m++;
         }
         h = block_sum_i(sh.red, h);
         m = block_sum_i(sh.red, m);
-        if (threadIdx.x == 0) { Partial *pp = my_partial(c); pp->n[0] = h; pp->n[1] = m; }
+        if (threadIdx.x == 0) { Partial *pp = my_partial(); pp->n[0] = h; pp->n[1] = m; }
     }
-    if (!exchange(c, sh)) return false;
+    if (!exchange()) return false;
     int hole_base, movers_below, movers_above, total_movers, dummy0, dummy1;
-    group_counts(c, sh, 0, &hole_base, &dummy0, &dummy1);
-    group_counts(c, sh, 1, &movers_below, &movers_above, &total_movers);
+    group_counts(0, &hole_base, &dummy0, &dummy1);
+    group_counts(1, &movers_below, &movers_above, &total_movers);
     int *holes = D.scratch;
     int *movers = D.scratch + D.l;
     {
@@ -1722,7 +1595,7 @@ __device__ bool do_shrinking(Ctx &c, Shared &sh, int &unshrink)
             const int k = base + threadIdx.x;
             const int p = c.a0 + k;
             bool s = false;
-            if (p < c.a1) s = be_shrunk(nu, c.sS[k], c.sY[k], c.sG[k], g);
+            if (p < c.a1) s = be_shrunk(nu, flag_s(ck.F[k]), flag_y(ck.F[k]), ck.G[k], g);
             const int isH = (p < c.a1 && p < K && s) ? 1 : 0;
             const int isM = (p < c.a1 && p >= K && !s) ? 1 : 0;
             int totH, totM;
@@ -1737,14 +1610,13 @@ __device__ bool do_shrinking(Ctx &c, Shared &sh, int &unshrink)
             m_run += totM;
         }
     }
-    if (!exchange(c, sh)) return false;
+    if (!exchange()) return false;
     // 4. swap pair r: holes[r] <-> movers[r] (the reference's swap_index loop)
     for (long long r = (long long)c.rank * blockDim.x + threadIdx.x; r < total_movers; r += (long long)c.nb * blockDim.x)
         swap_pos(D, __ldcg(&holes[r]), __ldcg(&movers[r]));
-    if (!exchange(c, sh)) return false;
-    c.A = K;
-    set_chunks(c);
-    chunk_load(c);
+    if (!exchange()) return false;
+    set_active(K);
+    chunk_load();
     return true;
 }
 
@@ -1768,72 +1640,197 @@ __device__ __forceinline__ double prefetch_priority(int y, unsigned char s, doub
     return fmax(up, low);
 }
 
-// Publish the block's I_up maxima (with payload) and its most violating
-// positions (prefetch candidates: the best of each warp, top kPrefetchCand).
-__device__ void iup_publish(const Ctx &c, Shared &sh, double (&v)[2], int (&ix)[2], double pv, int pix)
+// Wait until the W words at p carry sequence number `want`; false when the
+// group's error flag is set or the wait's bound runs out.
+template <int W>
+__device__ __forceinline__ bool poll_words(const InstanceDesc &D, const RecWord *p, unsigned want, RecWord (&w)[W])
 {
-    const int kind[2] = {0, 0};
-    // warp winners of the prefetch priority
-    warp_argmax(pv, pix);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) {
-        sh.cand_v[w] = pv;
-        sh.cand_p[w] = pix;
-    }
-    block_reduce<2>(sh.red, v, ix, kind);   // its barriers also publish cand_*
-    if (threadIdx.x < 32) {
-        double cv = lane < kWarps ? sh.cand_v[lane] : -SVMB_INF;
-        int cp = lane < kWarps ? sh.cand_p[lane] : -1;
-        Partial *pp = my_partial(c);
-        for (int t = 0; t < kPrefetchCand; t++) {
-            double bv = cv;
-            int bp = cp;
-            warp_argmax(bv, bp);
-            if (bp >= 0 && bv > -SVMB_INF) {
-                if (cp == bp) cv = -SVMB_INF;        // remove the winner
-                if (lane == 0) {
-                    const int q = bp - c.a0;
-                    pp->cv[t] = bv;
-                    pp->cpos[t] = bp;
-                    pp->cloc[t] = c.sCol[q];
-                    pp->crow[t] = c.sRow[q];
-                    pp->cy[t] = c.sY[q];
-                }
-            } else if (lane == 0) {
-                pp->cv[t] = -SVMB_INF;
-                pp->cpos[t] = -1;
-            }
-        }
-    }
-    if (threadIdx.x == 0) {
-        Partial *pp = my_partial(c);
-        for (int k = 0; k < 2; k++) {
-            const int p = ix[k];
-            const int q = p - c.a0;
-            pp->v[3 * k + 0] = v[k];
-            pp->n[4 * k + 0] = p;
-            if (p >= 0) {
-                pp->v[3 * k + 1] = c.sA[q];
-                pp->v[3 * k + 2] = c.sQD[q];
-                pp->n[4 * k + 1] = c.sCol[q];
-                pp->n[4 * k + 2] = c.sRow[q];
-                pp->n[4 * k + 3] = c.sY[q];
+    long long t0 = 0;
+    for (unsigned spins = 1;; spins++) {
+        bool all = true;
+#pragma unroll
+        for (int k = 0; k < W; k++) w[k] = ld_word(p + k);
+#pragma unroll
+        for (int k = 0; k < W; k++) all = all && (unsigned)(w[k].hi >> 32) == want;
+        if (all) return true;
+        if ((spins & 255u) == 0) {
+            const long long now = (long long)tc::global_ns();
+            if (t0 == 0) t0 = now;
+            const long long limit = D.wait_ns > 0 ? D.wait_ns : kWaitTimeoutNs;
+            if (ld_relaxed_i32(&D.sync->error) != 0 || now - t0 > limit) {
+                atomicExch(&D.sync->error, 1);
+                return false;
             }
         }
     }
 }
 
-__device__ void scan_iup(Ctx &c, Shared &sh)
+// One poll warp's part of a phase-A exchange: the records of blocks 32 warp ..
+// + 31, the best of each of the T tracks left in sh.wa[warp].
+template <int T>
+__device__ __forceinline__ void poll_iup(unsigned seq, int warp, int lane)
 {
-    const int nu = c.D->nu;
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const int b = warp * 32 + lane;
+    RecWord w[kWordsI * T];
+    bool ok = true;
+    if (b < c.nb) ok = poll_words<kWordsI * T>(sh.D, sh.D.words + (long long)b * kRecWords + kWordA, seq, w);
+    if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) sh.fail = 1;
+        return;
+    }
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+        const int p = b < c.nb ? code_pos((unsigned)w[kWordsI * t].hi) : -1;
+        u64 key = p >= 0 ? key_of(__longlong_as_double((long long)w[kWordsI * t].lo)) : 0;
+        int best = p;
+        warp_best(key, best);
+        if (best >= 0 ? p == best : lane == 0) {
+#pragma unroll
+            for (int e = 0; e < kWordsI; e++) {
+                sh.wa[warp].d[kWordsI * t + e] = __longlong_as_double((long long)w[kWordsI * t + e].lo);
+                sh.wa[warp].x[kWordsI * t + e] = (unsigned)w[kWordsI * t + e].hi;
+            }
+        }
+    }
+}
+
+// Exchange of the block's I_up maxima (per track, with payload) and, with
+// `ahead`, publication of its most violating positions (prefetch candidates:
+// the best of each warp, top kPrefetchCand).  The group's winners are in sh.wa.
+__device__ __forceinline__ bool iup_publish(unsigned seq, int nu, bool ahead, const double (&v)[2],
+                                            const int (&ix)[2], double pv, int pix)
+{
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u64 k0 = ix[0] >= 0 ? key_of(v[0]) : 0, k1 = 0;
+    int p0 = ix[0], p1 = -1;
+    warp_best(k0, p0);
+    if (nu) {
+        k1 = ix[1] >= 0 ? key_of(v[1]) : 0;
+        p1 = ix[1];
+        warp_best(k1, p1);
+    }
+    if (ahead) {
+        u64 kp = pix >= 0 && pv > -SVMB_INF ? key_of(pv) : 0;
+        int pp = kp ? pix : -1;
+        warp_best(kp, pp);
+        if (lane == 0) {
+            sh.wk[2][warp] = kp;
+            sh.wp[warp] = pp;
+        }
+    }
+    if (lane == 0) {
+        sh.wk[0][warp] = k0;
+        sh.wi[0][warp] = p0;
+        sh.wk[1][warp] = k1;
+        sh.wi[1][warp] = p1;
+    }
+    __syncthreads();
+    RecWord *mine = sh.D.words + (long long)c.rank * kRecWords;
+    if (warp < kPollWarps) {
+        if (warp == 0) {
+            k0 = lane < kWarps ? sh.wk[0][lane] : 0;
+            p0 = lane < kWarps ? sh.wi[0][lane] : -1;
+            warp_best(k0, p0);
+            if (nu) {
+                k1 = lane < kWarps ? sh.wk[1][lane] : 0;
+                p1 = lane < kWarps ? sh.wi[1][lane] : -1;
+                warp_best(k1, p1);
+            }
+            if (lane < (nu ? 2 : 1) * kWordsI) {
+                // lane 4t + e builds word e of track t
+                const int p = lane < kWordsI ? p0 : p1, e = lane & (kWordsI - 1);
+                double d = 0.0;
+                unsigned x = 0;
+                if (p >= 0) {
+                    const int q = p - c.a0;
+                    const unsigned f = ck.F[q];
+                    if (e == 0) {
+                        const double G = ck.G[q];
+                        d = flag_y(f) > 0 ? -G : G;
+                        x = pos_code(p, flag_y(f));
+                    } else if (e == 1) {
+                        d = ck.A[q];
+                        x = (unsigned)ck.Col[q];
+                    } else if (e == 2) {
+                        d = ck.QD[q];
+                        x = slot_word(ck.Slot[q], f);
+                    } else {
+                        x = (unsigned)ck.Row[q];
+                    }
+                } else if (e == 0) {
+                    d = -SVMB_INF;
+                    x = kNoPos;
+                }
+                if (c.nb == 1) {
+                    sh.wa[0].d[lane] = d;
+                    sh.wa[0].x[lane] = x;
+                } else {
+                    st_word(mine + kWordA + lane, d, x, seq);
+                }
+            }
+            __syncwarp();
+        }
+        if (c.nb > 1 && warp * 32 < c.nb) {
+            if (nu) poll_iup<2>(seq, warp, lane);
+            else poll_iup<1>(seq, warp, lane);
+        }
+    } else if (warp == kPollWarps && ahead) {
+        // the warps' best by rank: lane w counts the warps ahead of warp w
+        const u64 k = lane < kWarps ? sh.wk[2][lane] : 0;
+        const int p = lane < kWarps ? sh.wp[lane] : -1;
+        int rank = 0;
+#pragma unroll
+        for (int j = 0; j < kWarps; j++) {
+            const u64 kj = __shfl_sync(0xffffffffu, k, j);
+            const int pj = __shfl_sync(0xffffffffu, p, j);
+            rank += kj > k || (kj == k && pj > p) ? 1 : 0;
+        }
+        const int found = __popc(__ballot_sync(0xffffffffu, p >= 0));
+        Cand cd{-SVMB_INF, kNoPos, 0u, 0u, (unsigned)kNoSlot};
+        int at = -1;
+        if (p >= 0) {
+            const int q = p - c.a0;
+            cd.v = key_value(k);
+            cd.pc = pos_code(p, flag_y(ck.F[q]));
+            cd.col = (unsigned)ck.Col[q];
+            cd.row = (unsigned)ck.Row[q];
+            cd.slot = ck.Slot[q];
+            if (rank < kPrefetchCand) at = rank;
+        }
+        // the places no warp takes are marked empty by lanes kWarps ..
+        if (lane >= kWarps && lane < kWarps + kPrefetchCand - found) at = found + lane - kWarps;
+        if (at >= 0) {
+            if (c.nb == 1) {
+                sh.cand[at] = cd;
+            } else {
+                st_word(mine + kWordCand + 2 * at, cd.v, cd.pc, seq);
+                st_word(mine + kWordCand + 2 * at + 1, __longlong_as_double((long long)cd.col | ((long long)cd.row << 32)),
+                        cd.slot, seq);
+            }
+        }
+    }
+    __syncthreads();
+    return sh.fail == 0;
+}
+
+__device__ __noinline__ bool scan_iup(unsigned seq)
+{
+    Ctx &c = block_shared().c;
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
+    const int nu = block_shared().D.nu;
     double v[2] = {-SVMB_INF, -SVMB_INF};
     int ix[2] = {-1, -1};
     double pv = -SVMB_INF;
     int pix = -1;
     for (int k = threadIdx.x; k < c.a1 - c.a0; k += blockDim.x) {
-        const unsigned char s = c.sS[k];
-        const double G = c.sG[k];
-        const int y = c.sY[k];
+        const unsigned char s = flag_s(ck.F[k]);
+        const double G = ck.G[k];
+        const int y = flag_y(ck.F[k]);
         if (y == +1) {
             if (s != ST_UPPER) better_max(v[0], ix[0], -G, c.a0 + k);
         } else {
@@ -1841,7 +1838,138 @@ __device__ void scan_iup(Ctx &c, Shared &sh)
         }
         better_max(pv, pix, prefetch_priority(y, s, G), c.a0 + k);
     }
-    iup_publish(c, sh, v, ix, pv, pix);
+    return iup_publish(seq, nu, block_shared().D.prefetch > 1, v, ix, pv, pix);
+}
+
+// One poll warp's part of a phase-B exchange (W words a record).
+template <int W>
+__device__ __forceinline__ void poll_j(unsigned seq, int warp, int lane)
+{
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const int b = warp * 32 + lane;
+    RecWord w[W];
+    bool ok = true;
+    if (b < c.nb) ok = poll_words<W>(sh.D, sh.D.words + (long long)b * kRecWords + kWordB, seq, w);
+    if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) sh.fail = 1;
+        return;
+    }
+    const int p = b < c.nb ? code_pos((unsigned)w[0].hi) : -1;
+    u64 key = p >= 0 ? key_of(__longlong_as_double((long long)w[0].lo)) : 0;
+    int best = p;
+    warp_best(key, best);
+    const u64 g2 = warp_max_key(b < c.nb ? key_of(__longlong_as_double((long long)w[4].lo)) : 0);
+    u64 g2n = 0;
+    if (W > 5) g2n = warp_max_key(b < c.nb ? key_of(__longlong_as_double((long long)w[W - 1].lo)) : 0);
+    if (best >= 0 ? p == best : lane == 0) {
+#pragma unroll
+        for (int e = 0; e < W; e++) {
+            if (e < 4) sh.wb[warp].d[e] = __longlong_as_double((long long)w[e].lo);
+            sh.wb[warp].x[e] = (unsigned)w[e].hi;
+        }
+    }
+    if (lane == 0) {
+        sh.wb[warp].d[4] = key_value(g2);
+        if (W > 5) sh.wb[warp].d[5] = key_value(g2n);
+    }
+}
+
+// Exchange of the block's second-order j candidate (largest decrease, with
+// payload) and its Gmax2 maxima; the group's are in sh.wb.
+__device__ __forceinline__ bool j_publish(unsigned seq, int nu, double dec, int jx, double g2, double g2n,
+                                          const float *Qi0, const float *Qi1)
+{
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u64 k = jx >= 0 ? key_of(dec) : 0;
+    int p = jx;
+    warp_best(k, p);
+    u64 kg = warp_max_key(key_of(g2)), kn = 0;
+    if (nu) kn = warp_max_key(key_of(g2n));
+    if (lane == 0) {
+        sh.wk[0][warp] = k;
+        sh.wi[0][warp] = p;
+        sh.wk[1][warp] = kg;
+        sh.wk[2][warp] = kn;
+    }
+    __syncthreads();
+    if (warp < kPollWarps) {
+        if (warp == 0) {
+            k = lane < kWarps ? sh.wk[0][lane] : 0;
+            p = lane < kWarps ? sh.wi[0][lane] : -1;
+            warp_best(k, p);
+            kg = warp_max_key(lane < kWarps ? sh.wk[1][lane] : 0);
+            if (nu) kn = warp_max_key(lane < kWarps ? sh.wk[2][lane] : 0);
+            if (lane < kWordsJ) {
+                double d = 0.0;
+                unsigned x = 0;
+                if (lane == 4) d = key_value(kg);
+                if (lane == 5) d = nu ? key_value(kn) : 0.0;
+                if (p >= 0) {
+                    const int q = p - c.a0;
+                    const unsigned f = ck.F[q];
+                    if (lane == 0) {
+                        d = key_value(k);
+                        x = pos_code(p, flag_y(f));
+                    } else if (lane == 1) {
+                        d = ck.G[q];
+                        x = (unsigned)ck.Col[q];
+                    } else if (lane == 2) {
+                        d = ck.A[q];
+                        x = (unsigned)ck.Row[q];
+                    } else if (lane == 3) {
+                        d = ck.QD[q];
+                        x = slot_word(ck.Slot[q], f);
+                    } else {
+                        const float *Q = lane == 4 ? Qi0 : Qi1;
+                        x = __float_as_uint(Q ? Q[ck.Col[q]] : 0.0f);
+                    }
+                } else if (lane == 0) {
+                    x = kNoPos;
+                }
+                if (c.nb == 1) {
+                    sh.wb[0].d[lane] = d;
+                    sh.wb[0].x[lane] = x;
+                } else {
+                    st_word(sh.D.words + (long long)c.rank * kRecWords + kWordB + lane, d, x, seq);
+                }
+            }
+            __syncwarp();
+        }
+        if (c.nb > 1 && warp * 32 < c.nb) {
+            if (nu) poll_j<kWordsJ>(seq, warp, lane);
+            else poll_j<kWordsJ - 1>(seq, warp, lane);
+        }
+    }
+    __syncthreads();
+    return sh.fail == 0;
+}
+
+// which poll warp's record of track t wins (larger value, ties to the larger position)
+__device__ __forceinline__ int win_iup(int np, int t)
+{
+    Shared &sh = block_shared();
+    int e = 0;
+    for (int k = 1; k < np; k++) {
+        const double a = sh.wa[e].d[kWordsI * t], b = sh.wa[k].d[kWordsI * t];
+        const int pa = code_pos(sh.wa[e].x[kWordsI * t]), pb = code_pos(sh.wa[k].x[kWordsI * t]);
+        if (pb >= 0 && (pa < 0 || b > a || (b == a && pb > pa))) e = k;
+    }
+    return e;
+}
+__device__ __forceinline__ int win_j(int np)
+{
+    Shared &sh = block_shared();
+    int e = 0;
+    for (int k = 1; k < np; k++) {
+        const double a = sh.wb[e].d[0], b = sh.wb[k].d[0];
+        const int pa = code_pos(sh.wb[e].x[0]), pb = code_pos(sh.wb[k].x[0]);
+        if (pb >= 0 && (pa < 0 || b > a || (b == a && pb > pa))) e = k;
+    }
+    return e;
 }
 
 // Dot products of the 32 rows of a warp (lane L owns row r) with up to 8
@@ -1873,26 +2001,31 @@ __device__ __forceinline__ D4 src4_at(uint32_t a, double)
     return D4{p.x, p.y, q.x, q.y};
 }
 
+// what a fill pass's warps need of the descriptor, in registers
+struct TileJob {
+    const float *X;
+    int ld;             // multiple of 4
+    int bufs;           // tiles in the warp's ring
+    uint32_t sstride;   // the staged sources lie this many bytes apart
+    uint32_t src0, tile;
+};
+
 template <int FORM, int NS, typename S>
-__device__ __forceinline__ void warp_tile_dots(const InstanceDesc &D, const StageSlots &ss, int ns, int r, float *tile,
-                                               double (&out)[kPrefetchMax])
+__device__ __forceinline__ void warp_tile_dots(const TileJob &J, int ns, int r, double (&out)[kPrefetchMax])
 {
     typedef typename Acc<FORM>::type acc_t;
     const int lane = threadIdx.x & 31;
-    const int ld = D.x.ld;   // multiple of 4
-    const float *X = D.x.X;
+    const int ld = J.ld;
+    const float *X = J.X;
     acc_t acc[NS];
 #pragma unroll
     for (int k = 0; k < NS; k++) acc[k] = acc_t(0);
-    // the staged sources lie D.stage_lds values apart from the first
-    const uint32_t src0 = tc::smem_addr(ss.sp[0]);
-    const uint32_t sstride = (uint32_t)(D.stage_lds * (int)sizeof(S));
+    const uint32_t src0 = J.src0, sstride = J.sstride, tile_s = J.tile;
     // a slice is 32 rows x 4 pieces of 16 bytes; lane L moves pieces L + 32i
     // (i < 4): row (L + 32i) / 4, piece L % 4.  Row t of a tile = the row of lane t.
     const float *prow[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) prow[i] = X + (long long)__shfl_sync(0xffffffffu, r, (lane + 32 * i) >> 2) * ld + 4 * (lane & 3);
-    const uint32_t tile_s = tc::smem_addr(tile);
     auto issue = [&](int c0, int buf) {
         if (c0 < ld) {
 #pragma unroll
@@ -1907,7 +2040,7 @@ __device__ __forceinline__ void warp_tile_dots(const InstanceDesc &D, const Stag
         }
         tc::cp_async_commit();
     };
-    const int nb = D.tile_bufs;
+    const int nb = J.bufs;
     // prologue: slices 0 .. nb-2 in flight
     for (int p = 0; p + 1 < nb; p++) issue(16 * p, p);
     for (int c0 = 0, s = 0; c0 < ld; c0 += 16) {
@@ -1949,39 +2082,42 @@ __device__ __forceinline__ void warp_tile_dots(const InstanceDesc &D, const Stag
 // sources into cache slots on my chunk of [0,A) (tail = 0, from shared
 // memory) or of [A,l) (tail = 1, global state).
 template <int FORM, typename S>
-__device__ __forceinline__ void tile_dots_ns(const InstanceDesc &D, const StageSlots &ss, int ns, int r, float *tile,
-                                             double (&dots)[kPrefetchMax])
+__device__ __forceinline__ void tile_dots_ns(const TileJob &J, int ns, int r, double (&dots)[kPrefetchMax])
 {
     switch (ns) {
-    case 1: warp_tile_dots<FORM, 1, S>(D, ss, ns, r, tile, dots); break;
-    case 2: warp_tile_dots<FORM, 2, S>(D, ss, ns, r, tile, dots); break;
-    case 3: warp_tile_dots<FORM, 3, S>(D, ss, ns, r, tile, dots); break;
-    case 4: warp_tile_dots<FORM, 4, S>(D, ss, ns, r, tile, dots); break;
-    case 5: warp_tile_dots<FORM, 5, S>(D, ss, ns, r, tile, dots); break;
-    case 6: warp_tile_dots<FORM, 6, S>(D, ss, ns, r, tile, dots); break;
-    default: warp_tile_dots<FORM, 8, S>(D, ss, ns, r, tile, dots); break;
+    case 1: warp_tile_dots<FORM, 1, S>(J, ns, r, dots); break;
+    case 2: warp_tile_dots<FORM, 2, S>(J, ns, r, dots); break;
+    case 3: warp_tile_dots<FORM, 3, S>(J, ns, r, dots); break;
+    case 4: warp_tile_dots<FORM, 4, S>(J, ns, r, dots); break;
+    case 5: warp_tile_dots<FORM, 5, S>(J, ns, r, dots); break;
+    case 6: warp_tile_dots<FORM, 6, S>(J, ns, r, dots); break;
+    default: warp_tile_dots<FORM, 8, S>(J, ns, r, dots); break;
     }
 }
 
 template <int FORM>
-__device__ void fill_rows(Ctx &c, Shared &sh, int ns, const int *src_row, const int *src_y, const long long *slot,
-                          int tail)
+__device__ __noinline__ void fill_rows(int ns, int tail)
 {
-    const InstanceDesc &D = *c.D;
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const InstanceDesc &D = block_shared().D;
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
     if (ns == 0) return;
     // per-source constants of this pass, read from shared memory where used
     if (threadIdx.x < ns) {
         const int k = threadIdx.x;
-        sh.fsx[k] = D.x.xsq ? D.x.xsq[src_row[k]] : 0.0;
-        sh.fsy[k] = src_y[k];
-        sh.fsd[k] = D.cache.data + slot[k] * D.cache.stride;
+        sh.fsx[k] = D.x.xsq ? D.x.xsq[sh.frow[k]] : 0.0;
+        sh.fsy[k] = sh.fy[k];
+        sh.fsd[k] = D.cache.data + (long long)sh.fslot[k] * D.cache.stride;
     }
-    stage_sources(D, c.stage, sh.ss, src_row, ns);   // ends with a barrier
+    stage_sources(D, c.stage, sh.ss, sh.frow, ns);   // ends with a barrier
     const int lo = tail ? c.t0 : 0, hi = tail ? c.t1 : c.a1 - c.a0;
+    const double *const xsq = D.x.xsq;
     if (D.x.X && D.stage_cap > 0) {
         // dense rows, staged sources: warp-tiled, whole warps per 32 positions
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        float *tile = c.tile + warp * (D.tile_bufs * 32 * kTileStride);
+        float *const tile = c.tile + warp * (D.tile_bufs * 32 * kTileStride);
+        const TileJob job{D.x.X, D.x.ld, D.tile_bufs, (uint32_t)(D.stage_lds * stage_elem(FORM)), tc::smem_addr(sh.ss.sp[0]), tc::smem_addr(tile)};
         for (int base = lo + warp * 32; base < hi; base += blockDim.x) {
             const int k = base + lane;
             const bool valid = k < hi;
@@ -1992,20 +2128,20 @@ __device__ void fill_rows(Ctx &c, Shared &sh, int ns, const int *src_row, const 
                 yp = D.y[kk];
                 col = D.pos_local[kk];
             } else {
-                r = c.sRow[kk];
-                yp = c.sY[kk];
-                col = c.sCol[kk];
+                r = ck.Row[kk];
+                yp = flag_y(ck.F[kk]);
+                col = ck.Col[kk];
             }
             // the target's norm is loaded before the dots so that its latency hides behind them
-            const double xe = D.x.xsq ? D.x.xsq[r] : 0.0;
+            const double xe = xsq ? xsq[r] : 0.0;
             double dots[kPrefetchMax];
             // staged sources are float64 in the exact form
-            if (FORM == FORM_EXACT) tile_dots_ns<FORM, double>(D, sh.ss, ns, r, tile, dots);
-            else tile_dots_ns<FORM, float>(D, sh.ss, ns, r, tile, dots);
+            if (FORM == FORM_EXACT) tile_dots_ns<FORM, double>(job, ns, r, dots);
+            else tile_dots_ns<FORM, float>(job, ns, r, dots);
             if (valid) {
 #pragma unroll
                 for (int s2 = 0; s2 < kPrefetchMax; s2++)
-                    if (s2 < ns) sh.fsd[s2][col] = q_value(D.kp, sh.fsy[s2] * yp, dots[s2], sh.fsx[s2], xe);
+                    if (s2 < ns) sh.fsd[s2][col] = q_of(sh.fsy[s2] * yp, dots[s2], sh.fsx[s2], xe);
             }
         }
     } else {
@@ -2016,58 +2152,298 @@ __device__ void fill_rows(Ctx &c, Shared &sh, int ns, const int *src_row, const 
                 yp = D.y[k];
                 col = D.pos_local[k];
             } else {
-                r = c.sRow[k];
-                yp = c.sY[k];
-                col = c.sCol[k];
+                r = ck.Row[k];
+                yp = flag_y(ck.F[k]);
+                col = ck.Col[k];
             }
             double dots[kSrcBatch];
             row_dots<FORM>(D, sh.ss, ns, r, dots);
-            const double xe = D.x.xsq ? D.x.xsq[r] : 0.0;
+            const double xe = xsq ? xsq[r] : 0.0;
 #pragma unroll
             for (int s2 = 0; s2 < kPrefetchMax; s2++)
-                if (s2 < ns) sh.fsd[s2][col] = q_value(D.kp, sh.fsy[s2] * yp, dots[s2], sh.fsx[s2], xe);
+                if (s2 < ns) sh.fsd[s2][col] = q_of(sh.fsy[s2] * yp, dots[s2], sh.fsx[s2], xe);
         }
     }
     unstage_sources(D, c.stage, sh.ss);
 }
 
-// the fill pass of the form: CUDA cores or tensor cores
+// the fill pass of the form (the rows listed in sh.f*): CUDA cores or tensor cores
 template <int FORM>
-__device__ bool fill(Ctx &c, Shared &sh, int ns, const int *src_row, const int *src_y, const long long *slot, int tail)
+__device__ __forceinline__ bool fill(int ns, int tail)
 {
     if constexpr (is_tc_form(FORM)) {
-        return fill_rows_tc(c, sh, ns, src_row, src_y, slot, tail);
+        return fill_rows_tc(ns, tail);
     } else {
-        fill_rows<FORM>(c, sh, ns, src_row, src_y, slot, tail);
+        fill_rows<FORM>(ns, tail);
         return true;
     }
 }
 
-// position of the phase-A winner of track k (excluded from prefetching)
-__device__ __forceinline__ int i0_prev_guard(const Shared &sh, int k) { return sh.bi[4 * k]; }
+// --------------------------------------------------------------------------
+// Q-row cache slots
+// --------------------------------------------------------------------------
+// A slot is taken by a hand that goes round the slots and passes over those
+// used since its last visit (it clears their reference bits) and over the two
+// the phase still reads.  Rows evaluated ahead of need get no reference bit
+// until they are used.  With more slots than bits the hand just goes round.
+// Every block takes the same slots in the same order.  The `taken` slots the
+// pass already has in sh.fslot stay its own (a pass takes at most nslots - 2).
+__device__ int take_slot(int keep0, int keep1, int taken, bool used)
+{
+    Shared &sh = block_shared();
+    const int n = sh.D.cache.nslots;
+    int s = sh.hand;
+    while (true) {
+        if (s >= n) {
+            s = 0;
+            sh.reused = 1;
+        }
+        bool free = s != keep0 && s != keep1;
+        for (int t = 0; t < taken; t++) free = free && s != sh.fslot[t];
+        if (free) {
+            if (n > kRefSlots) break;
+            const unsigned m = 1u << (s & 31), w = sh.ref[s >> 5];
+            if (!(w & m)) {
+                if (used) sh.ref[s >> 5] = w | m;
+                break;
+            }
+            sh.ref[s >> 5] = w & ~m;
+        }
+        s++;
+    }
+    sh.hand = s + 1;
+    return s;
+}
+__device__ __forceinline__ void touch_slot(int s)
+{
+    Shared &sh = block_shared();
+    if (sh.D.cache.nslots <= kRefSlots) sh.ref[s >> 5] |= 1u << (s & 31);
+}
+
+// The block's positions learn the fill pass's slots: whoever held one loses
+// it, the variables of the pass get theirs.  Position k belongs to thread
+// k % kThreads here as everywhere; the fill begins with a barrier.
+__device__ __forceinline__ void claim_slots()
+{
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
+    const int n = c.a1 - c.a0, nf = sh.nfill;
+    if (sh.reused) {
+        for (int k = threadIdx.x; k < n; k += kThreads) {
+            const int s = ck.Slot[k];
+            for (int t = 0; t < nf; t++)
+                if (s == sh.fslot[t]) {
+                    ck.Slot[k] = kNoSlot;
+                    ck.F[k] = (unsigned char)(ck.F[k] & ~(kFlagFull | kFlagAhead));
+                }
+        }
+    }
+    for (int t = 0; t < nf; t++) {
+        const int k = sh.fpos[t] - c.a0;
+        if (k >= 0 && k < n && (k & (kThreads - 1)) == (int)threadIdx.x) {
+            ck.Slot[k] = (unsigned short)sh.fslot[t];
+            ck.F[k] = (unsigned char)((ck.F[k] & ~(kFlagFull | kFlagAhead)) | (c.A == sh.D.l ? kFlagFull : 0) |
+                                      (t >= sh.nneed ? kFlagAhead : 0));
+        }
+    }
+    if (c.rank == 0 && threadIdx.x < nf) sh.D.cache.tag[sh.fslot[threadIdx.x]] = sh.fcol[threadIdx.x];
+}
+static_assert((kThreads & (kThreads - 1)) == 0, "a position's thread is found by masking");
+
+// Phase A without the row of track 0 and / or 1 (their records in wa[e0], wa[e1]):
+// the missing rows are evaluated together with the rows of the group's most
+// violating positions (this only fills the cache; it never changes which
+// pair is chosen).
+template <int FORM>
+__device__ __noinline__ bool miss_iup(unsigned seq, int e0, int e1, int need0, int need1)
+{
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    const InstanceDesc &D = sh.D;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        const int nneed = need0 + need1;
+        const int i0 = code_pos(sh.wa[e0].x[0]), i1 = D.nu ? code_pos(sh.wa[e1].x[kWordsI]) : -1;
+        const int held0 = i0 >= 0 && !need0 ? (int)(sh.wa[e0].x[2] & 0xffffu) : -1;
+        const int held1 = i1 >= 0 && !need1 ? (int)(sh.wa[e1].x[kWordsI + 2] & 0xffffu) : -1;
+        if (lane == 0) {
+            int nf = 0;
+            for (int t = 0; t < 2; t++) {
+                if (!(t ? need1 : need0)) continue;
+                const unsigned *x = sh.wa[t ? e1 : e0].x + kWordsI * t;
+                sh.fslot[nf] = take_slot(held0, held1, nf, true);
+                sh.fpos[nf] = code_pos(x[0]);
+                sh.fy[nf] = code_y(x[0]);
+                sh.fcol[nf] = (int)x[1];
+                sh.frow[nf] = (int)x[3];
+                nf++;
+            }
+            sh.nneed = nf;
+        }
+        __syncwarp();
+        int nf = nneed;
+        const int want = D.prefetch - nneed;
+        const int most = min(D.prefetch, D.cache.nslots - 2);
+        if (want > 0 && most > nneed) {
+            // the group's candidates, each lane keeping its best two; then `want`
+            // rounds of the warp's best (the lowest lane on equal priorities)
+            u64 k1 = 0, k2 = 0;
+            Cand c1{}, c2{};
+            bool ok = true;
+            for (int e = lane; e < c.nb * kPrefetchCand; e += 32) {
+                Cand cd;
+                if (c.nb == 1) {
+                    cd = sh.cand[e];
+                } else {
+                    RecWord w[2];
+                    ok = ok && poll_words<2>(D, D.words + (long long)(e / kPrefetchCand) * kRecWords + kWordCand +
+                                                    2 * (e % kPrefetchCand), seq, w);
+                    if (!ok) break;
+                    cd.v = __longlong_as_double((long long)w[0].lo);
+                    cd.pc = (unsigned)w[0].hi;
+                    cd.col = (unsigned)w[1].lo;
+                    cd.row = (unsigned)(w[1].lo >> 32);
+                    cd.slot = (unsigned)w[1].hi;
+                }
+                const int p = code_pos(cd.pc);
+                if (p < 0 || p == i0 || p == i1) continue;
+                const u64 k = key_of(cd.v);
+                if (k > k1) {
+                    k2 = k1;
+                    c2 = c1;
+                    k1 = k;
+                    c1 = cd;
+                } else if (k > k2) {
+                    k2 = k;
+                    c2 = cd;
+                }
+            }
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (lane == 0) sh.fail = 1;
+            } else {
+                for (int r = 0; r < want && nf < most; r++) {
+                    const u64 m = warp_max_key(k1);
+                    if (m == 0) break;
+                    const int who = __ffs(__ballot_sync(0xffffffffu, k1 == m)) - 1;
+                    int took = 0;
+                    if (lane == who) {
+                        if (c1.slot == kNoSlot) {
+                            took = 1;
+                            sh.fslot[nf] = take_slot(held0, held1, nf, false);
+                            sh.fpos[nf] = code_pos(c1.pc);
+                            sh.fy[nf] = code_y(c1.pc);
+                            sh.fcol[nf] = (int)c1.col;
+                            sh.frow[nf] = (int)c1.row;
+                        }
+                        k1 = k2;
+                        c1 = c2;
+                        k2 = 0;
+                    }
+                    nf += __shfl_sync(0xffffffffu, took, who);
+                    __syncwarp();
+                }
+            }
+        }
+        if (lane == 0) sh.nfill = nf;
+    }
+    __syncthreads();
+    if (sh.fail) return false;
+    const int ns = sh.nfill;
+    if (threadIdx.x == 0) {
+        sh.cnt[kCntAhead] += ns - sh.nneed;
+        sh.cnt[kCntMiss] += sh.nneed;
+        sh.cnt[kCntQ] += (long long)ns * c.A;
+        sh.cnt[kCntTargets] += c.A;
+        sh.cnt[kCntFill]++;
+    }
+    claim_slots();
+    return fill<FORM>(ns, 0);
+}
+
+// Phase B without the row of j (its record in wb[e]).
+template <int FORM>
+__device__ __noinline__ bool miss_j(int e, int slot0, int slot1)
+{
+    Ctx &c = block_shared().c;
+    Shared &sh = block_shared();
+    if (threadIdx.x == 0) {
+        const unsigned *x = sh.wb[e].x;
+        sh.fslot[0] = take_slot(slot0, slot1, 0, true);
+        sh.fpos[0] = code_pos(x[0]);
+        sh.fy[0] = code_y(x[0]);
+        sh.fcol[0] = (int)x[1];
+        sh.frow[0] = (int)x[2];
+        sh.nfill = sh.nneed = 1;
+        sh.cnt[kCntMiss]++;
+        sh.cnt[kCntQ] += c.A;
+        sh.cnt[kCntTargets] += c.A;
+        sh.cnt[kCntFill]++;
+    }
+    __syncthreads();
+    claim_slots();
+    return fill<FORM>(1, 0);
+}
+
+// rcp.approx: about 18 good bits, used only to leave out hopeless divisions
+__device__ __forceinline__ double rcp_rough(double x)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    return r;
+}
+
+// an empty staging area: sparse sources are scattered into zeroed dense
+// vectors, or into a table without keys
+template <int FORM>
+__device__ void stage_clear(float *stage)
+{
+    const InstanceDesc &D = block_shared().D;
+    if (!D.x.X && D.stage_cap > 0)
+        for (long long k = threadIdx.x; k < (long long)D.stage_lds * D.stage_cap * (stage_elem(FORM) / 4); k += blockDim.x)
+            stage[k] = 0.0f;
+    if (!D.x.X && D.hash_slots > 0) {
+        int *keys = reinterpret_cast<int *>(stage);
+        for (int k = threadIdx.x; k < kHashSlots; k += blockDim.x) keys[k] = -1;
+        float *vals = reinterpret_cast<float *>(reinterpret_cast<char *>(stage) + kHashSlots * 4);
+        for (int k = threadIdx.x; k < kHashSlots * kSrcBatch * (stage_elem(FORM) / 4); k += blockDim.x) vals[k] = 0.0f;
+    }
+    __syncthreads();
+}
 
 // --------------------------------------------------------------------------
 // the persistent solver
 // --------------------------------------------------------------------------
-template <int FORM>
-__device__ void solve_instance(const InstanceDesc &D, int rank, Shared &sh, unsigned char *dyn)
+__device__ __forceinline__ void put_counters(SolveOut &o)
 {
-    Ctx c;
-    c.D = &D;
-    c.rank = rank;
-    c.nb = D.nblocks;
-    c.A = D.l;
-    c.epoch = 0;
-    c.phase = 0;
-    c.lrec = sh.lrec;
-    {
-        // dynamic shared memory: [tensor-core stages][stage][tiles][G][alpha][QD][col][row][y][status]
-        size_t off = 0;
+    Shared &sh = block_shared();
+    o.sum_active = sh.cnt[kCntActive];
+    o.q_evals = sh.cnt[kCntQ];
+    o.lookups = sh.cnt[kCntLook];
+    o.hits = sh.cnt[kCntLook] - sh.cnt[kCntMiss];
+    o.fills = sh.cnt[kCntFill];
+    o.prefetched = sh.cnt[kCntAhead];
+    o.prefetch_used = (long long)sh.ahead_used;
+    o.fill_targets = sh.cnt[kCntTargets];
+    for (int k = 0; k < 8; k++) o.prof[k] = sh.prof[k];
+}
+
+template <int FORM>
+__device__ void solve_instance(int rank)
+{
+    Shared &sh = block_shared();
+    const InstanceDesc &D = sh.D;
+    Ctx &c = sh.c;
+    if (threadIdx.x == 0) {
+        c.rank = rank;
+        c.nb = D.nblocks;
+        c.phase = 0;
         c.tcbase = 0;
         c.tc_g = 0;
-        c.tc_t = 0;
         c.fg = 0;
         c.fstages = fill_stages(D.tc_n);
+        // dynamic shared memory: [tensor-core stages][stage][tiles][G][alpha][QD][col][row][slot][flags]
+        size_t off = 0;
         if constexpr (is_tc_form(FORM)) {
             const uint32_t raw = tc::smem_addr(dyn);
             c.tcbase = (raw + 1023u) & ~1023u;
@@ -2076,56 +2452,56 @@ __device__ void solve_instance(const InstanceDesc &D, int rank, Shared &sh, unsi
         c.stage = reinterpret_cast<float *>(dyn + off);
         off += (size_t)D.stage_cap * D.stage_lds * stage_elem(FORM);
         if (D.hash_slots > 0) off += (size_t)hash_bytes(FORM);
-        off = (off + 15) & ~(size_t)15;
+        off = (off + 127) & ~(size_t)127;   // 64-byte tile rows: two to a 128-byte line
         c.tile = reinterpret_cast<float *>(dyn + off);
-        c.pt = reinterpret_cast<PrefetchTable *>(dyn + off);
-        off += aux_bytes(FORM, D.tile_bufs);
-        const size_t cap = (size_t)D.chunk_cap;
-        c.sG = reinterpret_cast<double *>(dyn + off); off += cap * 8;
-        c.sA = reinterpret_cast<double *>(dyn + off); off += cap * 8;
-        c.sQD = reinterpret_cast<double *>(dyn + off); off += cap * 8;
-        c.sCol = reinterpret_cast<int *>(dyn + off); off += cap * 4;
-        c.sRow = reinterpret_cast<int *>(dyn + off); off += cap * 4;
-        c.sY = reinterpret_cast<signed char *>(dyn + off); off += cap;
-        c.sS = reinterpret_cast<unsigned char *>(dyn + off);
+        c.choff = (int)(off + aux_bytes(FORM, D.tile_bufs));
     }
-    set_chunks(c);
+    set_active(D.l);
     const int l = D.l;
     const int nu = D.nu;
+    const Chunk ck = chunk_at(c.choff, D.chunk_cap);
+    unsigned seq = 0;       // sequence number of the last record exchange
     long long iter = 0;
     int unshrink = 0;
     int status = 0;
-    // block 0 / thread 0 work counters and section timers
-    long long cnt_active = 0, cnt_q = 0, cnt_look = 0, cnt_hit = 0, cnt_fill = 0, cnt_pf = 0, cnt_pf_used = 0;
-    long long cnt_tgt = 0;   // target positions of the fill passes (one row read each, whatever the sources)
-    long long prof[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    long long tmark = clock64();
-    const long long tstart = tmark;
+    // work counters and section timers of thread 0; the loop adds 32-bit cycle
+    // counts (an add that waits for nothing) and folds them every 1000 iterations
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < kCnt; k++) sh.cnt[k] = 0;
+        for (int k = 0; k < 8; k++) {
+            sh.prof[k] = 0;
+            sh.prof32[k] = 0;
+        }
+        sh.tstart = clock64();
+        sh.ahead_used = 0;
+        sh.fail = 0;
+        sh.hand = 0;
+        sh.reused = 0;
+    }
+    unsigned tmark = (unsigned)clock();
+    for (int k = threadIdx.x; k < kRefSlots / 32; k += blockDim.x) sh.ref[k] = 0;
 #define SVMB_PROF(k)                                   \
     do {                                               \
         if (threadIdx.x == 0) {                        \
-            const long long now_ = clock64();          \
-            prof[k] += now_ - tmark;                   \
+            const unsigned now_ = (unsigned)clock();   \
+            atomicAdd(&sh.prof32[k], now_ - tmark);    \
             tmark = now_;                              \
         }                                              \
     } while (0)
-    if (threadIdx.x == 0) { sh.cs.nprev = 0; sh.cs.ncur = 0; }
-    if (!D.x.X && D.stage_cap > 0)
-        for (long long k = threadIdx.x; k < (long long)D.stage_lds * D.stage_cap * (stage_elem(FORM) / 4); k += blockDim.x)
-            c.stage[k] = 0.0f;
-    if (!D.x.X && D.hash_slots > 0) {
-        // an empty table: keys -1, values zero
-        int *keys = reinterpret_cast<int *>(c.stage);
-        for (int k = threadIdx.x; k < kHashSlots; k += blockDim.x) keys[k] = -1;
-        float *vals = reinterpret_cast<float *>(reinterpret_cast<char *>(c.stage) + kHashSlots * 4);
-        for (int k = threadIdx.x; k < kHashSlots * kSrcBatch * (stage_elem(FORM) / 4); k += blockDim.x) vals[k] = 0.0f;
-    }
-    __syncthreads();
+    auto fold = [&]() {
+        if (threadIdx.x == 0)
+            for (int k = 0; k < 8; k++) {
+                sh.prof[k] += sh.prof32[k];
+                sh.prof32[k] = 0;
+            }
+    };
+    stage_clear<FORM>(c.stage);
 
     // ---- initial state (svm.cpp:525-572, QD svm.cpp:1321-1327) on the global copies ----
     {
         for (int p = c.a0 + threadIdx.x; p < c.a1; p += blockDim.x) {
             D.pos_local[p] = p;      // positions start as local indices
+            D.pos_slot[p] = kNoSlot;
             D.status[p] = status_of(D.alpha[p], get_C(D, D.y[p]));
             const int r = D.pos_row[p];
             const double xs = D.x.xsq ? D.x.xsq[r] : 0.0;
@@ -2134,369 +2510,208 @@ __device__ void solve_instance(const InstanceDesc &D, int rank, Shared &sh, unsi
             D.G[p] = D.p[p];
             D.G_bar[p] = 0.0;
         }
-        if (!exchange(c, sh)) goto fail;
+        if (!exchange()) goto fail;
         int any = 0;
         for (int p = threadIdx.x; p < l; p += blockDim.x) any |= D.alpha[p] > 0 ? 1 : 0;
         any = __syncthreads_or(any);
         if (any) {
-            if (!accumulate<FORM>(c, sh, l, 0, D.lazy_gbar ? 0 : 1, c.a0, c.a1)) goto fail;
-            if (!exchange(c, sh)) goto fail;
+            if (!accumulate<FORM>(l, 0, D.lazy_gbar ? 0 : 1, c.a0, c.a1)) goto fail;
+            if (!exchange()) goto fail;
         }
-        chunk_load(c);
+        chunk_load();
     }
 
     {
         const long long max_iter = D.max_iter;
         int counter = (l < 1000 ? l : 1000) + 1;
-        scan_iup(c, sh);
-        if (!exchange(c, sh)) goto fail;
+        if (!scan_iup(++seq)) goto fail;
+        const int np = (c.nb + 31) >> 5;
+        // slots are never taken back when every variable has one
+        const bool evicts = D.cache.nslots < l;
+        const bool ahead = D.prefetch > 1;
+        long long passes = 0, sum_from = 0;     // phase-A passes; iterations already in the active-size sum
+        auto count_active = [&]() {
+            if (threadIdx.x == 0) sh.cnt[kCntActive] += (iter - sum_from) * c.A;
+            sum_from = iter;
+        };
 
         while (iter < max_iter) {
             if (--counter == 0) {
                 counter = l < 1000 ? l : 1000;
+                fold();
+                count_active();
                 if (D.shrinking) {
                     SVMB_PROF(kProfBUpdate);
-                    if (!do_shrinking<FORM>(c, sh, unshrink)) goto fail;
-                    scan_iup(c, sh);
-                    if (!exchange(c, sh)) goto fail;
+                    if (!do_shrinking<FORM>(unshrink)) goto fail;
+                    if (!scan_iup(++seq)) goto fail;
                     SVMB_PROF(kProfShrink);
                 }
             }
             int widened = 0;
-            double Gmax0, Gmax1;
-            int i0, i1;
         select_again:
             // ======================= phase A =======================
-            const unsigned long long clkA = 4ull * (unsigned long long)iter + 1ull + (unsigned long long)widened;
+            const int n = c.a1 - c.a0;
+            const int e0 = win_iup(np, 0), e1 = nu ? win_iup(np, 1) : 0;
+            const WinA &w0 = sh.wa[e0], &w1 = sh.wa[e1];
+            const int i0 = code_pos(w0.x[0]), i1 = nu ? code_pos(w1.x[kWordsI]) : -1;
+            const double Gmax0 = w0.d[0], Gmax1 = nu ? w1.d[kWordsI] : -SVMB_INF;
+            int slot0 = i0 >= 0 ? (int)(w0.x[2] & 0xffffu) : -1, slot1 = i1 >= 0 ? (int)(w1.x[kWordsI + 2] & 0xffffu) : -1;
             {
-                const Partial *all = prev_partials(c);
-                double v[2] = {-SVMB_INF, -SVMB_INF};
-                int ix[2] = {-1, -1};
-                const int kind[2] = {0, 0};
-                RecVals r;
-                r.n[0] = r.n[4] = -1;
-                if (D.prefetch > 1) {
-                    // the group's prefetch candidates into shared memory, one
-                    // candidate per thread (its five fields loaded together)
-                    const int ncand = c.nb * kPrefetchCand;
-                    for (int e = threadIdx.x; e < ncand; e += blockDim.x) {
-                        const Partial *pr = &all[e / kPrefetchCand];
-                        const int t = e % kPrefetchCand;
-                        double cv;
-                        int cpos, cloc, crow, cy;
-                        if (c.nb == 1) {
-                            cv = pr->cv[t]; cpos = pr->cpos[t]; cloc = pr->cloc[t]; crow = pr->crow[t]; cy = pr->cy[t];
-                        } else {
-                            cv = __ldcg(&pr->cv[t]); cpos = __ldcg(&pr->cpos[t]); cloc = __ldcg(&pr->cloc[t]);
-                            crow = __ldcg(&pr->crow[t]); cy = __ldcg(&pr->cy[t]);
-                        }
-                        c.pt->v[e] = cv; c.pt->pos[e] = cpos; c.pt->loc[e] = cloc; c.pt->row[e] = crow; c.pt->y[e] = cy;
-                    }
+                const int need0 = slot0 == kNoSlot ? 1 : 0, need1 = slot1 == kNoSlot ? 1 : 0;
+                passes++;
+                if (evicts && threadIdx.x == 0) {
+                    if (i0 >= 0 && !need0) touch_slot(slot0);
+                    if (i1 >= 0 && !need1) touch_slot(slot1);
                 }
-                if (threadIdx.x < c.nb) {
-                    rec_load(c, &all[threadIdx.x], r, 1, 0);
-                    better_max(v[0], ix[0], r.v[0], r.n[0]);
-                    better_max(v[1], ix[1], r.v[3], r.n[4]);
-                }
-                block_reduce<2>(sh.red, v, ix, kind);
-                // the thread holding a winning record publishes its payload
-                if (threadIdx.x < c.nb) {
-                    for (int k = 0; k < 2; k++) {
-                        if (ix[k] >= 0 && r.n[4 * k] == ix[k]) {
-                            sh.bd[3 * k + 1] = r.v[3 * k + 1];
-                            sh.bd[3 * k + 2] = r.v[3 * k + 2];
-                            sh.bi[4 * k + 1] = r.n[4 * k + 1];
-                            sh.bi[4 * k + 2] = r.n[4 * k + 2];
-                            sh.bi[4 * k + 3] = r.n[4 * k + 3];
-                        }
-                    }
-                }
-                if (threadIdx.x == 0) {
-                    sh.bd[0] = v[0]; sh.bi[0] = ix[0];
-                    sh.bd[3] = v[1]; sh.bi[4] = ix[1];
-                }
-                __syncthreads();
-                if (threadIdx.x < 32) {
-                    // cache decisions for the row(s) of phase A (warp 0 together; lane 0
-                    // writes them); missing rows go to the fill list
-                    const int whole = c.A == l;
-                    int nf = 0;
-                    for (int k = 0; k < 2; k++) {
-                        long long slot = -1;
-                        int va = 1;
-                        if (sh.bi[4 * k] >= 0 && (k == 0 || nu)) {
-                            const Lookup L = cache_lookup_w(sh.cs, D.cache, sh.bi[4 * k + 1], c.epoch, clkA, whole, clkA, 0);
-                            slot = L.slot;
-                            va = L.valid_active;
-                            cnt_look++;
-                            cnt_hit += L.valid_active;
-                            cnt_pf_used += L.was_prefetched;
-                            if (!va && threadIdx.x == 0) {
-                                sh.frow[nf] = sh.bi[4 * k + 2];
-                                sh.fy[nf] = sh.bi[4 * k + 3];
-                                sh.fslot[nf] = slot;
-                            }
-                            if (!va) nf++;
-                        }
-                        if (threadIdx.x == 0) {
-                            sh.bl[k] = slot;
-                            sh.bi[8 + k] = va;
-                        }
-                    }
-                    if (threadIdx.x == 0) sh.nfill = nf;
-                }
-                __syncthreads();
-                // speculative prefetch: a missing row is evaluated together with
-                // the rows of the group's most violating positions (this only
-                // fills the cache; it never changes which pair is chosen)
-                if (sh.nfill > 0 && D.prefetch > sh.nfill) {
-                    // the `want` highest-priority candidates, chosen by warp 0: every
-                    // lane keeps its own best few, then the lanes' heads are merged
-                    // (the order of prefetched rows affects only what is cached)
-                    const int ncand = c.nb * kPrefetchCand;
-                    const int want = D.prefetch - sh.nfill;
-                    if (threadIdx.x < 32) {
-                        // `want` rounds of a warp argmax over the candidates
-                        // (largest priority, the lowest table index on ties); lane
-                        // L owns entries L + 32j and marks the ones taken in a mask
-                        const int lane = threadIdx.x;
-                        const int g0 = i0_prev_guard(sh, 0), g1 = i0_prev_guard(sh, 1);
-                        unsigned taken = 0;
-                        int got = 0;
-                        for (; got < want; got++) {
-                            double bv = -SVMB_INF;
-                            int be = 0x7fffffff;
-                            for (int e = lane, j = 0; e < ncand; e += 32, j++) {
-                                if ((taken >> j) & 1u) continue;
-                                const int pos = c.pt->pos[e];
-                                const double v = c.pt->v[e];
-                                if (pos < 0 || pos == g0 || pos == g1 || !(v > -SVMB_INF)) continue;
-                                if (v > bv) { bv = v; be = e; }
-                            }
-                            for (int o = 16; o > 0; o >>= 1) {
-                                const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                                const int oe = __shfl_xor_sync(0xffffffffu, be, o);
-                                if (ov > bv || (ov == bv && oe < be)) { bv = ov; be = oe; }
-                            }
-                            if (be == 0x7fffffff) break;
-                            if ((be & 31) == lane) taken |= 1u << (be >> 5);
-                            if (lane == 0) sh.pick[got] = be;
-                        }
-                        if (lane == 0) sh.npick = got;
-                    }
-                    __syncthreads();
-                    // the picks' cache sets, read by one thread per way in a single round trip
-                    if (threadIdx.x < sh.npick * kMaxWays) {
-                        const int t = threadIdx.x / kMaxWays, w = threadIdx.x % kMaxWays;
-                        const int set = c.pt->loc[sh.pick[t]] % D.cache.nsets;
-                        if (w == 0) sh.sset[t].set = set;
-                        if (w < D.cache.nways) {
-                            const long long s = (long long)set * D.cache.nways + w;
-                            sh.sset[t].tag[w] = __ldcg(&D.cache.tag[s]);
-                            sh.sset[t].ep[w] = __ldcg(&D.cache.epoch[s]);
-                            sh.sset[t].st[w] = __ldcg(&D.cache.stamp[s]);
-                        }
-                    }
-                    __syncthreads();
-                    if (threadIdx.x < 32) {
-                        const int whole = c.A == l;
-                        int nf = sh.nfill;
-                        const int npick = sh.npick;
-                        for (int t = 0; t < npick && nf < D.prefetch; t++) {
-                            const int e = sh.pick[t];
-                            const Lookup L = cache_lookup_w(sh.cs, D.cache, c.pt->loc[e], c.epoch, clkA, whole, clkA, 1,
-                                                            &sh.sset[t]);
-                            if (L.slot >= 0 && !L.valid_active) {
-                                if (threadIdx.x == 0) {
-                                    sh.frow[nf] = c.pt->row[e];
-                                    sh.fy[nf] = c.pt->y[e];
-                                    sh.fslot[nf] = L.slot;
-                                }
-                                nf++;
-                                cnt_pf++;
-                            }
-                        }
-                        __syncwarp();
-                        if (threadIdx.x == 0) sh.nfill = nf;
-                    }
-                    __syncthreads();
-                }
-            }
-            Gmax0 = sh.bd[0];
-            Gmax1 = sh.bd[3];
-            i0 = sh.bi[0];
-            i1 = nu ? sh.bi[4] : -1;
-            {
-                // evaluate the missing (and prefetched) rows on my chunk
-                const int ns = sh.nfill;
                 SVMB_PROF(kProfAReduce);
-                if (ns > 0) {
-                    if (!fill<FORM>(c, sh, ns, sh.frow, sh.fy, sh.fslot, 0)) goto fail;
-                    cnt_q += (long long)ns * c.A;
-                    cnt_tgt += c.A;
-                    cnt_fill++;
+                if (need0 | need1) {
+                    if (!miss_iup<FORM>(seq, e0, e1, need0, need1)) goto fail;
+                    if (need0) slot0 = sh.fslot[0];
+                    if (need1) slot1 = sh.fslot[need0];
                 }
                 SVMB_PROF(kProfAFill);
             }
+            const float *const Qi0 = i0 >= 0 ? D.cache.data + (long long)slot0 * D.cache.stride : nullptr;
+            const float *const Qi1 = i1 >= 0 ? D.cache.data + (long long)slot1 * D.cache.stride : nullptr;
             {
-                // second-order j scan on my chunk (svm.cpp:869-924 / :1120-1174)
-                double v[3] = {SVMB_INF, -SVMB_INF, -SVMB_INF};   // obj_min, Gmax2 (C-SVC / nu p), Gmax2 (nu n)
-                int ix[3] = {-1, -1, -1};
-                const int kind[3] = {1, 2, 2};
-                const float *Qi0 = i0 >= 0 ? D.cache.data + sh.bl[0] * D.cache.stride : nullptr;
-                const float *Qi1 = i1 >= 0 ? D.cache.data + sh.bl[1] * D.cache.stride : nullptr;
-                const double QDi0 = sh.bd[2], QDi1 = sh.bd[5];
-                const double two_yi0 = __dmul_rn(2.0, (double)sh.bi[3]);
-                const int n = c.a1 - c.a0;
-                // kScanGroup positions per thread at a time: their Q_i values are
-                // loaded together (one L2 round trip per group, not per position)
-                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * blockDim.x) {
+                // second-order j scan on my chunk (svm.cpp:869-924 / :1120-1174): the
+                // largest decrease (Gmax + y G)^2 / quad, ties to the larger position.
+                // Exact divisions are long, so rough quotients (an approximate
+                // reciprocal, off by 2^-17 at most) come first and only those within
+                // 2^-15 of the warp's best are divided: about one per warp.  A
+                // quotient the estimate is not safe for (quad or the result at the
+                // ends of the exponent range, NaN) counts as infinite.
+                // A thread keeps its best rough quotient (high word + 1) with its
+                // terms, and its second best; it goes over its positions once more
+                // in the rare case that both are in reach.
+                double dec = -SVMB_INF, g2 = -SVMB_INF, g2n = -SVMB_INF;
+                int jx = -1;
+                const double QDi0 = w0.d[2], QDi1 = w1.d[kWordsI + 2];
+                const double two_yi0 = __dmul_rn(2.0, (double)code_y(w0.x[0]));
+                // numerator and denominator of position k; false: not a candidate
+                auto quotient = [&](int k, float q, double &num, double &quad) -> bool {
+                    const unsigned f = ck.F[k];
+                    const unsigned char s = flag_s(f);
+                    const bool pos = (f & kFlagPos) != 0;
+                    if (s == (pos ? ST_LOWER : ST_UPPER)) return false;
+                    const double G = ck.G[k], Gm = pos || !nu ? Gmax0 : Gmax1;
+                    const double yG = pos ? G : -G;
+                    const double grad_diff = __dadd_rn(Gm, yG);
+                    if (pos || !nu) g2 = fmax(g2, yG);
+                    else g2n = fmax(g2n, yG);
+                    if (!(grad_diff > 0)) return false;
+                    const double cross = nu ? (double)__fmul_rn(2.0f, q) : __dmul_rn(pos ? two_yi0 : -two_yi0, (double)q);
+                    quad = __dsub_rn(__dadd_rn(pos || !nu ? QDi0 : QDi1, ck.QD[k]), cross);
+                    num = __dmul_rn(grad_diff, grad_diff);
+                    if (!(quad > 0)) quad = kTau;
+                    return true;
+                };
+                auto rough = [&](double num, double quad) -> unsigned {
+                    const unsigned hq = (unsigned)__double2hiint(quad);
+                    const unsigned h = (unsigned)__double2hiint(__dmul_rn(num, rcp_rough(quad))) & 0x7fffffffu;
+                    return hq - 0x01000000u > 0x7d000000u ? 0x7ff00000u : h + 1u;
+                };
+                unsigned r1 = 0, r2 = 0;
+                int k1 = -1;
+                double num1 = 0.0, quad1 = 1.0;
+                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * kThreads) {
+                    // kScanGroup positions per thread at a time: their Q_i values are
+                    // loaded together (one L2 round trip per group, not per position)
                     float qv[kScanGroup];
 #pragma unroll
                     for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * (int)blockDim.x;
+                        const int k = k0 + u * kThreads;
                         qv[u] = 0.0f;
                         if (k < n) {
-                            const float *Qr = (nu && c.sY[k] != +1) ? Qi1 : Qi0;
-                            if (Qr) qv[u] = Qr[c.sCol[k]];
+                            const float *Qr = (nu && !(ck.F[k] & kFlagPos)) ? Qi1 : Qi0;
+                            if (Qr) qv[u] = Qr[ck.Col[k]];
                         }
                     }
 #pragma unroll
                     for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * (int)blockDim.x;
-                        if (k >= n) continue;
-                        const unsigned char s = c.sS[k];
-                        const double G = c.sG[k];
-                        if (c.sY[k] == +1) {
-                            if (s != ST_LOWER) {
-                                const double grad_diff = __dadd_rn(Gmax0, G);
-                                v[1] = fmax(v[1], G);
-                                if (grad_diff > 0) {
-                                    double quad;
-                                    if (!nu) quad = __dsub_rn(__dadd_rn(QDi0, c.sQD[k]), __dmul_rn(two_yi0, (double)qv[u]));
-                                    else quad = __dsub_rn(__dadd_rn(QDi0, c.sQD[k]), (double)__fmul_rn(2.0f, qv[u]));
-                                    const double num = __dmul_rn(grad_diff, grad_diff);
-                                    const double od = quad > 0 ? -__ddiv_rn(num, quad) : -__ddiv_rn(num, kTau);
-                                    better_min(v[0], ix[0], od, c.a0 + k);
-                                }
-                            }
-                        } else {
-                            if (s != ST_UPPER) {
-                                const double grad_diff = __dsub_rn(nu ? Gmax1 : Gmax0, G);
-                                if (nu) v[2] = fmax(v[2], -G); else v[1] = fmax(v[1], -G);
-                                if (grad_diff > 0) {
-                                    double quad;
-                                    if (!nu) quad = __dadd_rn(__dadd_rn(QDi0, c.sQD[k]), __dmul_rn(two_yi0, (double)qv[u]));
-                                    else quad = __dsub_rn(__dadd_rn(QDi1, c.sQD[k]), (double)__fmul_rn(2.0f, qv[u]));
-                                    const double num = __dmul_rn(grad_diff, grad_diff);
-                                    const double od = quad > 0 ? -__ddiv_rn(num, quad) : -__ddiv_rn(num, kTau);
-                                    better_min(v[0], ix[0], od, c.a0 + k);
-                                }
-                            }
+                        const int k = k0 + u * kThreads;
+                        if (k >= n) break;
+                        double num, quad;
+                        if (!quotient(k, qv[u], num, quad)) continue;
+                        const unsigned r = rough(num, quad);
+                        if (r > r1) {
+                            r2 = r1;
+                            r1 = r;
+                            k1 = k;
+                            num1 = num;
+                            quad1 = quad;
+                        } else if (r > r2) {
+                            r2 = r;
                         }
                     }
                 }
-                block_reduce<3>(sh.red, v, ix, kind);
-                if (threadIdx.x == 0) {
-                    Partial *pp = my_partial(c);
-                    const int j = ix[0];
-                    pp->v[0] = v[0]; pp->n[0] = j;
-                    pp->v[1] = v[1]; pp->v[2] = v[2];
-                    if (j >= 0) {
-                        const int q = j - c.a0;
-                        const int cj = c.sCol[q];
-                        pp->v[3] = c.sG[q]; pp->v[4] = c.sA[q]; pp->v[5] = c.sQD[q];
-                        pp->n[1] = cj; pp->n[2] = c.sRow[q]; pp->n[3] = c.sY[q];
-                        pp->q[0] = Qi0 ? Qi0[cj] : 0.0f;
-                        pp->q[1] = Qi1 ? Qi1[cj] : 0.0f;
+                const unsigned top = __reduce_max_sync(0xffffffffu, r1);
+                const unsigned least = top >= 0x7fe00000u || top <= 64u ? 1u : top - 64u;
+                if (r2 >= least) {
+                    for (int k = threadIdx.x; k < n; k += kThreads) {
+                        const float *Qr = (nu && !(ck.F[k] & kFlagPos)) ? Qi1 : Qi0;
+                        double num, quad;
+                        if (!quotient(k, Qr ? Qr[ck.Col[k]] : 0.0f, num, quad)) continue;
+                        if (rough(num, quad) >= least) better_max(dec, jx, __ddiv_rn(num, quad), c.a0 + k);
                     }
+                } else if (r1 >= least) {
+                    better_max(dec, jx, __ddiv_rn(num1, quad1), c.a0 + k1);
                 }
+                if (!j_publish(++seq, nu, dec, jx, g2, g2n, Qi0, Qi1)) goto fail;
             }
-            if (!exchange(c, sh)) goto fail;
             SVMB_PROF(kProfAScan);
 
             // ======================= phase B =======================
+            const int eb = win_j(np);
+            const WinB &wj = sh.wb[eb];
+            const int j = code_pos(wj.x[0]);
             {
-                const Partial *all = prev_partials(c);
-                double v[3] = {SVMB_INF, -SVMB_INF, -SVMB_INF};
-                int ix[3] = {-1, -1, -1};
-                const int kind[3] = {1, 2, 2};
-                RecVals r;
-                r.n[0] = -1;
-                if (threadIdx.x < c.nb) {
-                    rec_load(c, &all[threadIdx.x], r, 0, 1);
-                    better_min(v[0], ix[0], r.v[0], r.n[0]);
-                    v[1] = r.v[1];
-                    v[2] = r.v[2];
+                double gm = sh.wb[0].d[4], gmn = nu ? sh.wb[0].d[5] : -SVMB_INF;
+                for (int k = 1; k < np; k++) {
+                    gm = fmax(gm, sh.wb[k].d[4]);
+                    if (nu) gmn = fmax(gmn, sh.wb[k].d[5]);
                 }
-                block_reduce<3>(sh.red, v, ix, kind);
-                if (threadIdx.x < c.nb && ix[0] >= 0 && r.n[0] == ix[0]) {
-                    sh.bd[14] = r.v[3]; sh.bd[15] = r.v[4]; sh.bd[16] = r.v[5];
-                    sh.bi[13] = r.n[1]; sh.bi[14] = r.n[2]; sh.bi[15] = r.n[3];
-                    sh.bd[17] = (double)r.q[0]; sh.bd[18] = (double)r.q[1];
-                }
-                if (threadIdx.x == 0) { sh.bi[12] = ix[0]; sh.bd[12] = v[1]; sh.bd[13] = v[2]; }
-                __syncthreads();
-            }
-            const int j = sh.bi[12];
-            {
                 bool stop;
-                if (!nu) stop = __dadd_rn(Gmax0, sh.bd[12]) < D.eps;
-                else stop = fmax(__dadd_rn(Gmax0, sh.bd[12]), __dadd_rn(Gmax1, sh.bd[13])) < D.eps;
+                if (!nu) stop = __dadd_rn(Gmax0, gm) < D.eps;
+                else stop = fmax(__dadd_rn(Gmax0, gm), __dadd_rn(Gmax1, gmn)) < D.eps;
                 if (stop || j < 0) {
                     if (widened) break;
                     // reconstruct the whole gradient, widen, select again (svm.cpp:598-611)
+                    count_active();
                     if (c.A < l) {
-                        chunk_store(c);
-                        if (!exchange(c, sh)) goto fail;
-                        if (!reconstruct<FORM>(c, sh)) goto fail;
-                        widen(c);
+                        chunk_store();
+                        if (!exchange()) goto fail;
+                        if (!reconstruct<FORM>()) goto fail;
+                        widen();
                     }
                     widened = 1;
-                    scan_iup(c, sh);
-                    if (!exchange(c, sh)) goto fail;
+                    if (!scan_iup(++seq)) goto fail;
                     goto select_again;
                 }
                 if (widened) counter = 1;
             }
             ++iter;
-            cnt_active += c.A;
             // the working pair; nu-SVC takes i from the track of y_j (svm.cpp:1179-1182)
-            const int yj = sh.bi[15];
+            const int yj = code_y(wj.x[0]);
             const int tr = (nu && yj != +1) ? 1 : 0;
+            const WinA &wi = tr ? w1 : w0;
             const int i = tr ? i1 : i0;
-            const double Gi = tr ? Gmax1 : ((sh.bi[3] == +1) ? -Gmax0 : Gmax0);
-            const double alpha_i = sh.bd[3 * tr + 1], QDi = sh.bd[3 * tr + 2];
-            const int yi = tr ? -1 : sh.bi[3];
-            const int loc_i = sh.bi[4 * tr + 1], row_i = sh.bi[4 * tr + 2];
-            const long long slot_i = sh.bl[tr];
-            const float Qij = (float)sh.bd[17 + tr];
-            const double Gj = sh.bd[14], alpha_j = sh.bd[15], QDj = sh.bd[16];
-            const int loc_j = sh.bi[13], row_j = sh.bi[14];
+            const int yi = tr ? -1 : code_y(w0.x[0]);
+            const double Gi = tr ? Gmax1 : (yi == +1 ? -Gmax0 : Gmax0);
+            const double alpha_i = wi.d[kWordsI * tr + 1], QDi = wi.d[kWordsI * tr + 2];
+            const int slot_i = tr ? slot1 : slot0;
+            const float Qij = __uint_as_float(wj.x[4 + tr]);
+            const double Gj = wj.d[1], alpha_j = wj.d[2], QDj = wj.d[3];
             // Q_j row
-            // phase-B stamp: above every phase-A stamp of this iteration, below the next
-            const unsigned long long clkB = 4ull * (unsigned long long)iter - 1ull;
-            if (threadIdx.x < 32) {
-                const Lookup L = cache_lookup_w(sh.cs, D.cache, loc_j, c.epoch, clkB, c.A == l, clkA, 0);
-                if (threadIdx.x == 0) {
-                    sh.bl[2] = L.slot;
-                    sh.bi[16] = L.valid_active;
+            int slot_j = (int)(wj.x[3] & 0xffffu);
+            {
+                const bool need = slot_j == kNoSlot;
+                if (evicts && !need && threadIdx.x == 0) touch_slot(slot_j);
+                SVMB_PROF(kProfBReduce);
+                if (need) {
+                    if (!miss_j<FORM>(eb, slot0, slot1)) goto fail;
+                    slot_j = sh.fslot[0];
                 }
-                cnt_look++;
-                cnt_hit += L.valid_active;
-                cnt_pf_used += L.was_prefetched;
-            }
-            __syncthreads();
-            SVMB_PROF(kProfBReduce);
-            const long long slot_j = sh.bl[2];
-            if (!sh.bi[16]) {
-                const int srow[1] = {row_j};
-                const int sy[1] = {yj};
-                const long long ss[1] = {slot_j};
-                if (!fill<FORM>(c, sh, 1, srow, sy, ss, 0)) goto fail;
-                cnt_q += c.A;
-                cnt_tgt += c.A;
-                cnt_fill++;
             }
             // two-variable analytic step (svm.cpp:636-721), identical in every block
             const double C_i = get_C(D, yi), C_j = get_C(D, yj);
@@ -2544,121 +2759,120 @@ __device__ void solve_instance(const InstanceDesc &D, int rank, Shared &sh, unsi
             const bool bar_j = !D.lazy_gbar && (old_sj == ST_UPPER) != (new_sj == ST_UPPER);
             // complete rows for the G_bar update: fill the tail [A,l) where missing
             if ((bar_i || bar_j) && c.A < l) {
+                const bool ti = bar_i && !(wi.x[kWordsI * tr + 2] & kSlotFull), tj = bar_j && !(wj.x[3] & kSlotFull);
+                const int ns = (ti ? 1 : 0) + (tj ? 1 : 0);
+                __syncthreads();    // the last fill's list is no longer read
                 if (threadIdx.x == 0) {
-                    const unsigned long long clk = clkB;
-                    int tg[kMaxWays], ep[kMaxWays];
-                    unsigned long long stp[kMaxWays];
-                    sh.bi[17] = 0;
-                    sh.bi[18] = 0;
-                    if (bar_i) {
-                        cache_read_set(sh.cs, D.cache, (int)(slot_i / D.cache.nways), tg, ep, stp);
-                        sh.bi[17] = ep[slot_i % D.cache.nways] != kEpochFull;
-                        cache_mark_full(sh.cs, D.cache, slot_i, loc_i, clk);
+                    if (ti) {
+                        sh.frow[0] = (int)wi.x[kWordsI * tr + 3];
+                        sh.fy[0] = yi;
+                        sh.fslot[0] = slot_i;
                     }
-                    if (bar_j) {
-                        cache_read_set(sh.cs, D.cache, (int)(slot_j / D.cache.nways), tg, ep, stp);
-                        sh.bi[18] = ep[slot_j % D.cache.nways] != kEpochFull;
-                        cache_mark_full(sh.cs, D.cache, slot_j, loc_j, clk);
+                    if (tj) {
+                        sh.frow[ns - 1] = (int)wj.x[2];
+                        sh.fy[ns - 1] = yj;
+                        sh.fslot[ns - 1] = slot_j;
                     }
+                    sh.cnt[kCntQ] += (long long)ns * (l - c.A);
+                    sh.cnt[kCntTargets] += l - c.A;
                 }
                 __syncthreads();
-                int ns = 0;
-                int srow[2] = {0, 0}, sy[2] = {0, 0};
-                long long sslot[2] = {0, 0};
-                if (sh.bi[17]) { srow[ns] = row_i; sy[ns] = yi; sslot[ns] = slot_i; ns++; }
-                if (sh.bi[18]) { srow[ns] = row_j; sy[ns] = yj; sslot[ns] = slot_j; ns++; }
-                if (!fill<FORM>(c, sh, ns, srow, sy, sslot, 1)) goto fail;
-                cnt_q += (long long)ns * (l - c.A);
-                cnt_tgt += l - c.A;
+                if (!fill<FORM>(ns, 1)) goto fail;
+                const int ki = i - c.a0, kj = j - c.a0;
+                if (ti && i >= c.a0 && i < c.a1 && (ki & (kThreads - 1)) == (int)threadIdx.x) ck.F[ki] |= kFlagFull;
+                if (tj && j >= c.a0 && j < c.a1 && (kj & (kThreads - 1)) == (int)threadIdx.x) ck.F[kj] |= kFlagFull;
             }
             SVMB_PROF(kProfBFill);
-            // owners publish alpha/status of i and j
-            if (threadIdx.x == 0) {
-                if (i >= c.a0 && i < c.a1) { c.sA[i - c.a0] = ai; c.sS[i - c.a0] = new_si; }
-                if (j >= c.a0 && j < c.a1) { c.sA[j - c.a0] = aj; c.sS[j - c.a0] = new_sj; }
+            // the owners of i and j take their new alpha and status (a position is
+            // read and written by its own thread only until the next barrier)
+            {
+                auto take = [&](int p, double a, unsigned char st) {
+                    const int k = p - c.a0;
+                    if (k < 0 || k >= n || (k & (kThreads - 1)) != (int)threadIdx.x) return;
+                    const unsigned f = ck.F[k];
+                    if (f & kFlagAhead) atomicAdd(&sh.ahead_used, 1u);
+                    ck.A[k] = a;
+                    ck.F[k] = (unsigned char)((f & ~((3u << kFlagStatus) | kFlagAhead)) | ((unsigned)st << kFlagStatus));
+                };
+                take(i, ai, new_si);
+                take(j, aj, new_sj);
             }
-            __syncthreads();
             // G update on my chunk (svm.cpp:732-735) + G_bar (svm.cpp:744-769) + next I_up scan
             {
-                const float *Qi = D.cache.data + slot_i * D.cache.stride;
-                const float *Qj = D.cache.data + slot_j * D.cache.stride;
+                const float *Qi = D.cache.data + (long long)slot_i * D.cache.stride;
+                const float *Qj = D.cache.data + (long long)slot_j * D.cache.stride;
                 double v[2] = {-SVMB_INF, -SVMB_INF};
                 int ix[2] = {-1, -1};
                 double pv = -SVMB_INF;
                 int pix = -1;
-                const int n = c.a1 - c.a0;
-                const bool gbar = bar_i || bar_j;
-                // kScanGroup positions per thread at a time, their Q_i, Q_j (and
-                // G_bar) values loaded together before any is used
-                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * blockDim.x) {
+                // kScanGroup positions per thread at a time, their Q_i and Q_j
+                // values loaded together before any is used
+                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * kThreads) {
                     float qi[kScanGroup], qj[kScanGroup];
-                    double gb[kScanGroup];
 #pragma unroll
                     for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * (int)blockDim.x;
+                        const int k = k0 + u * kThreads;
                         qi[u] = 0.0f;
                         qj[u] = 0.0f;
-                        gb[u] = 0.0;
                         if (k < n) {
-                            const int col = c.sCol[k];
+                            const int col = ck.Col[k];
                             qi[u] = Qi[col];
                             qj[u] = Qj[col];
-                            if (gbar) gb[u] = D.G_bar[c.a0 + k];
                         }
                     }
 #pragma unroll
                     for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * (int)blockDim.x;
+                        const int k = k0 + u * kThreads;
                         if (k >= n) continue;
-                        const double G = __dadd_rn(c.sG[k], __dadd_rn(__dmul_rn((double)qi[u], dai), __dmul_rn((double)qj[u], daj)));
-                        c.sG[k] = G;
-                        if (gbar) {
-                            double g = gb[u];
-                            if (bar_i) g = (old_si == ST_UPPER) ? __dsub_rn(g, __dmul_rn(C_i, (double)qi[u])) : __dadd_rn(g, __dmul_rn(C_i, (double)qi[u]));
-                            if (bar_j) g = (old_sj == ST_UPPER) ? __dsub_rn(g, __dmul_rn(C_j, (double)qj[u])) : __dadd_rn(g, __dmul_rn(C_j, (double)qj[u]));
-                            D.G_bar[c.a0 + k] = g;
+                        const double G = __dadd_rn(ck.G[k], __dadd_rn(__dmul_rn((double)qi[u], dai), __dmul_rn((double)qj[u], daj)));
+                        ck.G[k] = G;
+                        const unsigned f = ck.F[k];
+                        const unsigned char s = flag_s(f);
+                        const bool pos = (f & kFlagPos) != 0;
+                        const bool up = s != (pos ? ST_UPPER : ST_LOWER);
+                        const double yG = pos ? -G : G;
+                        if (up) {
+                            if (pos || !nu) better_max(v[0], ix[0], yG, c.a0 + k);
+                            else better_max(v[1], ix[1], yG, c.a0 + k);
                         }
-                        const unsigned char s = c.sS[k];
-                        if (c.sY[k] == +1) {
-                            if (s != ST_UPPER) better_max(v[0], ix[0], -G, c.a0 + k);
-                        } else {
-                            if (s != ST_LOWER) better_max(v[nu], ix[nu], G, c.a0 + k);
-                        }
-                        better_max(pv, pix, prefetch_priority(c.sY[k], s, G), c.a0 + k);
+                        if (ahead) better_max(pv, pix, s == ST_FREE ? fabs(G) : (up ? yG : -yG), c.a0 + k);
                     }
                 }
                 if (bar_i || bar_j) {
-                    for (int p = c.t0 + threadIdx.x; p < c.t1; p += blockDim.x) {
-                        const int col = D.pos_local[p];
-                        double gb = D.G_bar[p];
-                        if (bar_i) { const double q = (double)Qi[col]; gb = (old_si == ST_UPPER) ? __dsub_rn(gb, __dmul_rn(C_i, q)) : __dadd_rn(gb, __dmul_rn(C_i, q)); }
-                        if (bar_j) { const double q = (double)Qj[col]; gb = (old_sj == ST_UPPER) ? __dsub_rn(gb, __dmul_rn(C_j, q)) : __dadd_rn(gb, __dmul_rn(C_j, q)); }
-                        D.G_bar[p] = gb;
-                    }
+                    auto bar = [&](double g, int col) {
+                        if (bar_i) { const double q = (double)Qi[col]; g = (old_si == ST_UPPER) ? __dsub_rn(g, __dmul_rn(C_i, q)) : __dadd_rn(g, __dmul_rn(C_i, q)); }
+                        if (bar_j) { const double q = (double)Qj[col]; g = (old_sj == ST_UPPER) ? __dsub_rn(g, __dmul_rn(C_j, q)) : __dadd_rn(g, __dmul_rn(C_j, q)); }
+                        return g;
+                    };
+                    for (int k = threadIdx.x; k < n; k += kThreads) D.G_bar[c.a0 + k] = bar(D.G_bar[c.a0 + k], ck.Col[k]);
+                    for (int p = c.t0 + threadIdx.x; p < c.t1; p += kThreads) D.G_bar[p] = bar(D.G_bar[p], D.pos_local[p]);
                 }
-                iup_publish(c, sh, v, ix, pv, pix);
+                if (!iup_publish(++seq, nu, ahead, v, ix, pv, pix)) goto fail;
             }
-            if (!exchange(c, sh)) goto fail;
             SVMB_PROF(kProfBUpdate);
         }
 
-        chunk_store(c);
-        if (!exchange(c, sh)) goto fail;
+        count_active();
+        fold();
+        if (threadIdx.x == 0) sh.cnt[kCntLook] = passes * (nu ? 2 : 1) + iter;
+        chunk_store();
+        if (!exchange()) goto fail;
         if (iter >= max_iter) {
             status = 1;
             if (c.A < l) {
-                if (!reconstruct<FORM>(c, sh)) goto fail;
-                c.A = l;
-                set_chunks(c);
+                if (!reconstruct<FORM>()) goto fail;
+                set_active(l);
             }
         }
     }
     // ---- rho (svm.cpp:1013-1049 / 1260-1308), objective (:795-802), alpha out (:805-808) ----
     // The sums run sequentially in position order (bit-exact with the reference), on block 0.
     if (rank == 0) {
-        __shared__ double chv[kThreads], chg[kThreads];
-        __shared__ unsigned char chs[kThreads];
-        __shared__ signed char chy[kThreads];
+        // the staging area is no longer needed
+        double *chv = reinterpret_cast<double *>(dyn), *chg = chv + kThreads;
+        unsigned char *chs = reinterpret_cast<unsigned char *>(chg + kThreads);
+        signed char *chy = reinterpret_cast<signed char *>(chs + kThreads);
+        __syncthreads();
         double ub = SVMB_INF, lb = -SVMB_INF, sum_free = 0;
         int nr_free = 0;
         double ub1 = SVMB_INF, ub2 = SVMB_INF, lb1 = -SVMB_INF, lb2 = -SVMB_INF, sf1 = 0, sf2 = 0;
@@ -2710,16 +2924,8 @@ __device__ void solve_instance(const InstanceDesc &D, int rank, Shared &sh, unsi
             o.unshrink = unshrink;
             o.obj = __ddiv_rn(objv, 2.0);
             o.gap = 0;
-            o.sum_active = cnt_active;
-            o.q_evals = cnt_q;
-            o.lookups = cnt_look;
-            o.hits = cnt_hit;
-            o.fills = cnt_fill;
-            o.prefetched = cnt_pf;
-            o.prefetch_used = cnt_pf_used;
-            o.fill_targets = cnt_tgt;
-            for (int k = 0; k < 7; k++) o.prof[k] = prof[k];
-            o.prof[kProfTotal] = clock64() - tstart;
+            put_counters(o);
+            o.prof[kProfTotal] = clock64() - sh.tstart;
             if (!nu) {
                 o.rho = nr_free > 0 ? __ddiv_rn(sum_free, (double)nr_free) : __ddiv_rn(__dadd_rn(ub, lb), 2.0);
                 o.r = 0;
@@ -2744,9 +2950,7 @@ fail:
         SolveOut o;
         o.iters = iter; o.rho = 0; o.obj = 0; o.r = 0; o.status = -1; o.active_size = c.A;
         o.unshrink = unshrink; o.nr_free = 0; o.gap = 0;
-        o.sum_active = cnt_active; o.q_evals = cnt_q; o.lookups = cnt_look; o.hits = cnt_hit;
-        o.fills = cnt_fill; o.prefetched = cnt_pf; o.prefetch_used = cnt_pf_used; o.fill_targets = cnt_tgt;
-        for (int k = 0; k < 8; k++) o.prof[k] = prof[k];
+        put_counters(o);
         *D.out = o;
     }
 #undef SVMB_PROF
@@ -2772,10 +2976,13 @@ template <int FORM>
 __global__ void __launch_bounds__(kThreads, 1)
 smo_persistent(const InstanceDesc *__restrict__ insts, const int *__restrict__ block_inst)
 {
-    __shared__ Shared sh;
-    extern __shared__ __align__(16) unsigned char dyn[];
+    Shared &sh = block_shared();
     const int inst = block_inst[blockIdx.x];
-    const InstanceDesc &D = insts[inst];
+    // the descriptor is read all through the solve: a copy in shared memory
+    for (int k = threadIdx.x; k < (int)(sizeof(InstanceDesc) / 4); k += blockDim.x)
+        reinterpret_cast<int *>(&sh.D)[k] = reinterpret_cast<const int *>(&insts[inst])[k];
+    __syncthreads();
+    const InstanceDesc &D = sh.D;
     const int rank = blockIdx.x - D.block0;
     if constexpr (is_tc_form(FORM)) {
         // mbarriers of the tensor-core pipeline and the TMEM accumulator (one block per SM)
@@ -2800,7 +3007,7 @@ smo_persistent(const InstanceDesc *__restrict__ insts, const int *__restrict__ b
         __syncthreads();
         tc::tc_fence_after();
     }
-    solve_instance<FORM>(D, rank, sh, dyn);
+    solve_instance<FORM>(rank);
     signal_done(D);
     if constexpr (is_tc_form(FORM)) {
         tc::tc_fence_before();
