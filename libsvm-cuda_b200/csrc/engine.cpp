@@ -827,10 +827,41 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
         w.poff[k + 1] = w.poff[k] + 2 * (size_t)w.nb[k];
         w.coff[k + 1] = w.coff[k] + (size_t)w.lay[k].slots;
     }
+    // Resident instances: a cache that holds every row is filled with the whole
+    // kernel matrix before the solve, by all SMs.  Worth it when that takes
+    // less than what the solves would spend on row passes: their iterations
+    // number about l (0.2 l to 5 l measured) and spend 0.3 to 3 us each on
+    // passes, so the line is the matrices' estimated time against 1 us per
+    // position of the launch's longest instance.  One value costs its dot product
+    // and a kernel function of about 40 operations; dense tiles run at about
+    // 8e12 operations a second, half of the values being copies.  A launch
+    // whose longest instance has no such cache lasts as long without (the 45
+    // pairs of 3,600 to 21,600 positions, the ten smallest resident: 44.1 ms
+    // against 42.6 ms).
+    {
+        double cost = 0.0;
+        long long longest = 0, longest_fit = 0;
+        std::vector<char> fits(count, 0);
+        for (int k = 0; k < count; k++) {
+            const SubProblem &sp = subs[first + k];
+            const DeviceRows &r = rows_of(sp, rows);
+            const double l = (double)sp.rows.size();
+            longest = std::max(longest, (long long)sp.rows.size());
+            if (sp.rows.empty() || w.lay[k].slots < (int)sp.rows.size()) continue;
+            longest_fit = std::max(longest_fit, (long long)sp.rows.size());
+            fits[k] = 1;
+            const double width = is_tc_form(prm.form) ? 0.05 * r.d : r.dense ? (double)r.ld : 8.0 * (double)r.nnz / std::max(r.n, 1);
+            cost += 0.5 * l * l * (width + 40.0);
+        }
+        const bool on = longest_fit == longest && cost <= 8e12 * 1e-6 * (double)longest;
+        w.resident.assign(count, 0);
+        for (int k = 0; k < count; k++) w.resident[k] = on && fits[k];
+    }
     const size_t L = w.loff[count], P = w.poff[count], S = w.coff[count];
     size_t off = 0;
     w.o_desc = off; off = al(off + sizeof(InstanceDesc) * count);
     w.o_bmap = off; off = al(off + sizeof(int) * used);
+    w.o_qmap = off; off = al(off + sizeof(int) * 2 * count);
     w.o_alpha = off; off = al(off + 8 * L);
     w.o_p = off; off = al(off + 8 * L);
     w.o_row = off; off = al(off + 4 * L);
@@ -863,6 +894,23 @@ static cudaError_t wave_issue(Wave &w, InstanceDesc *d_desc, int *d_block_inst, 
     cudaError_t e = xfer_async(dev, host, w.up_bytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(dev + w.o_zero, 0, w.zero_bytes, s);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(w.ev0, s, rec);
+    const int *d_first = (const int *)(dev + w.o_qmap);
+    if (e == cudaSuccess && w.q_total[0] > 0) {
+        e = launch_q_dense(w.form, d_desc, d_first, w.count, w.q_total[0], s);
+        if (!capturing) count_launch();
+    }
+    if (e == cudaSuccess && w.q_total[1] > 0) {
+        e = launch_q_sparse(w.form, d_desc, d_first + w.count, w.count, w.q_total[1], w.q_smem, s);
+        if (!capturing) count_launch();
+    }
+    if (is_tc_form(w.form)) {
+        const InstanceDesc *h = (const InstanceDesc *)(host + w.o_desc);
+        for (int k = 0; k < w.count && e == cudaSuccess; k++) {
+            if (!w.resident[k]) continue;
+            e = launch_q_tensor(w.form, d_desc + k, h[k].l, s);
+            if (!capturing) count_launch();
+        }
+    }
     if (e == cudaSuccess)
         e = launch_smo(w.form, d_desc, d_block_inst, w.used - (w.drop_last_block ? 1 : 0), w.dyn_smem, w.cooperative, s);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(w.ev1, s, rec);
@@ -891,7 +939,10 @@ std::string graph_key(const Wave &w)
     snprintf(buf, sizeof buf, "%p:%p:%zu:%zu:%zu:%zu:%zu:%d:%zu:%d:%d", (void *)w.dev, (void *)w.host, w.up_bytes,
              w.down_bytes, w.zero_bytes, w.o_zero, w.o_out, w.used, w.dyn_smem, w.form,
              (int)w.cooperative);
-    return std::string(buf) + ":" + std::to_string(w.o_desc) + ":" + std::to_string(w.o_bmap);
+    std::string q;      // the resident instances and their launches
+    for (char c : w.resident) q += c ? '1' : '0';
+    q += ":" + std::to_string(w.q_total[0]) + ":" + std::to_string(w.q_total[1]) + ":" + std::to_string(w.q_smem);
+    return std::string(buf) + ":" + q + ":" + std::to_string(w.o_desc) + ":" + std::to_string(w.o_bmap);
 }
 }  // namespace
 
@@ -981,10 +1032,27 @@ int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, cons
     InstanceDesc *d_desc = (InstanceDesc *)(dev + w.o_desc);
     int *d_block_inst = (int *)(dev + w.o_bmap);
     int b0 = 0;
+    int *h_first = (int *)(host + w.o_qmap);
+    w.q_total[0] = w.q_total[1] = 0;
+    w.q_smem = 0;
     for (int k = 0; k < count; k++) {
         const SubProblem &sp = subs[first + k];
         const SolveParams &p = params_of(sp, prm);
         const DeviceRows &r = rows_of(sp, rows);
+        h_first[k] = w.q_total[0];
+        h_first[count + k] = w.q_total[1];
+        if (w.resident[k] && !is_tc_form(prm.form)) {
+            const int l = (int)sp.rows.size();
+            const int cap = w.stage[k][0] > 0 ? w.stage[k][0] : kSrcBatch;
+            if (r.dense) {
+                w.q_total[0] += q_tiles(l);
+            } else {
+                w.q_total[1] += (l + cap - 1) / cap;
+                const size_t elem = prm.form == FORM_EXACT ? 8 : 4;
+                w.q_smem = std::max(w.q_smem, w.stage[k][4] > 0 ? (size_t)hash_bytes(prm.form)
+                                                                : (size_t)w.stage[k][0] * w.stage[k][1] * elem);
+            }
+        }
         const int l = (int)sp.rows.size();
         InstanceDesc &D = h_desc[k];
         memset(&D, 0, sizeof(D));
@@ -1012,6 +1080,8 @@ int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, cons
             const int limit = D.stage_cap > 0 ? std::min(kPrefetchMax, D.stage_cap) : kPrefetchMax;
             const int pf = w.tune_prefetch > 0 ? w.tune_prefetch : p.prefetch;
             D.prefetch = pf > 0 ? std::min(pf, limit) : limit;
+            D.resident = w.resident[k];
+            if (D.resident) D.prefetch = 1;
             D.lazy_gbar = p.lazy_gbar < 0 ? (is_tc_form(prm.form) ? 1 : 0) : p.lazy_gbar;
         }
         for (int b = 0; b < w.nb[k]; b++) h_bmap[b0 + b] = k;

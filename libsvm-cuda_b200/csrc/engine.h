@@ -208,6 +208,7 @@ struct InstanceDesc {
     int stage_cap;              // rows staged at once (1..kSrcBatch); 0: read sources from global memory
     int stage_lds;              // floats per staged row (dense: ld; sparse: d)
     int chunk_cap;              // positions of per-block state held in shared memory (>= ceil(l/nblocks))
+    int resident;               // the cache holds every row from the start (slot = local index)
     int prefetch;               // rows evaluated per fill pass (1 = no prefetch), <= kPrefetchMax
     // 0: G_bar maintained on every bound change, as the reference does (svm.cpp:744-769);
     // 1: no G_bar -- reconstruction recomputes G = p + sum over alpha>0 of alpha*Q on the

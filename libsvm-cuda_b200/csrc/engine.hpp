@@ -97,11 +97,14 @@ struct Wave {
     std::vector<int> nb;                      // blocks per instance
     std::vector<std::array<int, 5>> stage;    // stage_cap, stage_lds, tc_n, chunk_cap, hash_slots per instance
     std::vector<int> fill_path;               // SVMB_FILL_* per instance
+    std::vector<char> resident;               // the instance's kernel matrix is evaluated before the solve
+    int q_total[2] = {0, 0};                  // tiles of the resident dense rows, source groups of the sparse ones
+    size_t q_smem = 0;                        // staging of the source groups
     size_t dyn_smem = 0;
     struct Layout { size_t G, Gb, QD, S, PL, PS, Sc, Data, bytes; int slots; };
     std::vector<Layout> lay;
     std::vector<size_t> loff, poff, coff, inst_off;
-    size_t o_desc = 0, o_bmap = 0, o_alpha = 0, o_p = 0, o_row = 0, o_y = 0, o_out = 0, o_alocal = 0;
+    size_t o_desc = 0, o_bmap = 0, o_qmap = 0, o_alpha = 0, o_p = 0, o_row = 0, o_y = 0, o_out = 0, o_alocal = 0;
     size_t o_zero = 0, o_sync = 0, o_part = 0, o_word = 0, o_tag = 0;
     size_t up_bytes = 0, down_bytes = 0, zero_bytes = 0, dev_bytes = 0;
     char *dev = nullptr, *host = nullptr;
@@ -189,6 +192,14 @@ cudaError_t launch_kernel_block2(const DeviceRows &A, const DeviceRows &B, const
                                  int ma, int nb, double *d_out, long long ldo, int trans, int *d_err, cudaStream_t s);
 cudaError_t launch_smo(int form, const InstanceDesc *d_insts, const int *d_block_inst, int nblocks,
                        size_t dyn_smem, bool cooperative, cudaStream_t s);
+// whole kernel matrices into the caches of an instance's launch (resident
+// instances): dense rows in tiles (d_first[k] = first tile of instance k),
+// sparse rows in groups of sources, tensor forms one instance at a time
+int q_tiles(int l);
+cudaError_t launch_q_dense(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, cudaStream_t s);
+cudaError_t launch_q_sparse(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, size_t dyn_smem,
+                            cudaStream_t s);
+cudaError_t launch_q_tensor(int form, const InstanceDesc *d_inst, int l, cudaStream_t s);
 cudaError_t smo_max_blocks(int form, size_t dyn_smem, int *blocks_per_sm);
 
 }  // namespace svmb

@@ -88,6 +88,10 @@ struct GramArgs {
     long long ldo;
     int trans;
     int *err;
+    // Q matrix of a solver instance: its rows against themselves, written as
+    // the solver's label-signed float32 values into its cache (all of it is read
+    // from the descriptor, so that a captured launch follows the descriptor)
+    const InstanceDesc *inst;
 };
 
 // Persistent CTA: tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the
@@ -97,7 +101,8 @@ struct GramArgs {
 // registers (lanes 32(w%4).., columns 32(w/4)..+31).  Every wait is bounded; a
 // role whose wait runs out sets `abort`, which ends the other roles' waits,
 // and the launch reports the failure through a.err.
-template <int SF>   // the split form: FORM_BF16X3, FORM_FP16X3 or FORM_TF32
+// Q: the solver's Q values (label-signed, float32, transposed) are written.
+template <int SF, bool Q>   // the split form: FORM_BF16X3, FORM_FP16X3 or FORM_TF32
 __global__ void __launch_bounds__(kGThreads, 1) gram_split_kernel(GramArgs a)
 {
     extern __shared__ uint8_t g_smem_raw[];
@@ -105,8 +110,26 @@ __global__ void __launch_bounds__(kGThreads, 1) gram_split_kernel(GramArgs a)
     __shared__ uint32_t tmem_base;
     __shared__ int abort_flag;
     __shared__ double col_xsq[kGColRing][kGN], col_inv[kGColRing][kGN];
+    __shared__ signed char col_y[Q ? kGColRing : 1][kGN];
     __shared__ uint64_t colready[kGColRing];
 
+    float *q_out = nullptr;
+    const signed char *y = nullptr;
+    if (Q) {
+        const InstanceDesc &D = *a.inst;
+        a.xs = a.xs_b = D.x.Xs;
+        a.xinv = a.xinv_b = D.x.xinv;
+        a.xsq = a.xsq_b = D.x.xsq;
+        a.nchunk = D.x.nchunk;
+        a.rs = (long long)D.x.nchunk * 2 * kSplitChunk;
+        a.ia = a.ib = D.pos_row;
+        a.ma = a.nb = D.l;
+        a.kp = D.kp;
+        a.ldo = D.cache.stride;
+        a.err = &D.sync->error;
+        q_out = D.cache.data;
+        y = D.y;
+    }
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t raw = tc::smem_addr(g_smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -152,6 +175,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gram_split_kernel(GramArgs a)
         int ab = 0, kc = 0, t = blockIdx.x, slot = 0;
         unsigned ph = 0, phc = 0;
         double xa = 0.0, sa_inv = 1.0;
+        int y_row = 0;
         for (int g = 0; g < total; g++) {
             if (kc == 0) {
                 const int m0 = (t / ntn) * kGM, n0 = (t % ntn) * kGN;
@@ -160,6 +184,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gram_split_kernel(GramArgs a)
                     const int ra = a.ia ? a.ia[row] : row;
                     xa = a.xsq[ra];
                     sa_inv = a.xinv ? a.xinv[ra] : 1.0;
+                    if (Q) y_row = y[row];
                 }
                 if (rt < kGN) {
                     const int col = n0 + rt;
@@ -171,6 +196,7 @@ __global__ void __launch_bounds__(kGThreads, 1) gram_split_kernel(GramArgs a)
                     }
                     col_xsq[slot][rt] = cx;
                     col_inv[slot][rt] = cs;
+                    if (Q) col_y[slot][rt] = col < a.nb ? y[col] : 0;
                     tc::mbar_arrive(&colready[slot]);
                 }
             }
@@ -206,7 +232,14 @@ __global__ void __launch_bounds__(kGThreads, 1) gram_split_kernel(GramArgs a)
                 for (int k = 0; k < 32; k++)
                     acc[k] = kernel_from_dot(a.kp, __dmul_rn(__dmul_rn(acc[k], sa_inv), col_inv[slot][ch * 32 + k]), xa,
                                              col_xsq[slot][ch * 32 + k]);
-                if (a.trans) {
+                if (Q) {
+                    // the lanes of a warp (consecutive rows) write consecutive words
+#pragma unroll
+                    for (int k = 0; k < 32; k++)
+                        if (c0 + k < a.nb)
+                            q_out[(long long)(c0 + k) * a.ldo + row] =
+                                __double2float_rn(__dmul_rn((double)(y_row * col_y[slot][ch * 32 + k]), acc[k]));
+                } else if (a.trans) {
                     // the lanes of a warp (consecutive rows) write consecutive words
 #pragma unroll
                     for (int k = 0; k < 32; k++)
@@ -511,14 +544,16 @@ __global__ void split_csr_kernel(const long long *__restrict__ rowptr, const int
     }
 }
 
+template <bool Q>
 const void *gram_fn(int form)
 {
-    if (form == FORM_BF16X3) return (const void *)gram_split_kernel<FORM_BF16X3>;
-    if (form == FORM_TF32) return (const void *)gram_split_kernel<FORM_TF32>;
-    return (const void *)gram_split_kernel<FORM_FP16X3>;
+    if (form == FORM_BF16X3) return (const void *)gram_split_kernel<FORM_BF16X3, Q>;
+    if (form == FORM_TF32) return (const void *)gram_split_kernel<FORM_TF32, Q>;
+    return (const void *)gram_split_kernel<FORM_FP16X3, Q>;
 }
 
 // one persistent CTA per SM (or per tile, when there are fewer tiles)
+template <bool Q>
 void launch_gram(int form, const GramArgs &a, cudaStream_t s)
 {
     static int sms = 0;
@@ -530,9 +565,9 @@ void launch_gram(int form, const GramArgs &a, cudaStream_t s)
     }
     const long long tiles = (long long)((a.ma + kGM - 1) / kGM) * ((a.nb + kGN - 1) / kGN);
     const dim3 grid((unsigned)std::max<long long>(1, std::min<long long>(tiles, sms)));
-    if (form == FORM_BF16X3) gram_split_kernel<FORM_BF16X3><<<grid, kGThreads, kGSmem, s>>>(a);
-    else if (form == FORM_TF32) gram_split_kernel<FORM_TF32><<<grid, kGThreads, kGSmem, s>>>(a);
-    else gram_split_kernel<FORM_FP16X3><<<grid, kGThreads, kGSmem, s>>>(a);
+    if (form == FORM_BF16X3) gram_split_kernel<FORM_BF16X3, Q><<<grid, kGThreads, kGSmem, s>>>(a);
+    else if (form == FORM_TF32) gram_split_kernel<FORM_TF32, Q><<<grid, kGThreads, kGSmem, s>>>(a);
+    else gram_split_kernel<FORM_FP16X3, Q><<<grid, kGThreads, kGSmem, s>>>(a);
 }
 
 }  // namespace
@@ -578,7 +613,7 @@ cudaError_t launch_kernel_block(const DeviceRows &rows, const KernelParams &kp, 
 {
     if (ma <= 0 || nb <= 0) return cudaSuccess;
     if (is_tc_form(form)) {
-        const void *fn = gram_fn(form);
+        const void *fn = gram_fn<false>(form);
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem);
         if (e != cudaSuccess) return e;
         GramArgs a;
@@ -595,7 +630,8 @@ cudaError_t launch_kernel_block(const DeviceRows &rows, const KernelParams &kp, 
         a.out = d_out; a.ldo = ldo;
         a.trans = 0;
         a.err = d_err;
-        launch_gram(form, a, s);
+        a.inst = nullptr;
+        launch_gram<false>(form, a, s);
     } else {
         dim3 grid((nb + 15) / 16, (ma + 15) / 16), block(16, 16);
         if (form == FORM_EXACT)
@@ -613,7 +649,7 @@ cudaError_t launch_kernel_block2(const DeviceRows &A, const DeviceRows &B, const
     if (ma <= 0 || nb <= 0) return cudaSuccess;
     if (!is_tc_form(form) || A.split_form != form || B.split_form != form || A.nchunk != B.nchunk)
         return cudaErrorInvalidValue;
-    const void *fn = gram_fn(form);
+    const void *fn = gram_fn<false>(form);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem);
     if (e != cudaSuccess) return e;
     GramArgs a;
@@ -631,8 +667,21 @@ cudaError_t launch_kernel_block2(const DeviceRows &A, const DeviceRows &B, const
     a.out = d_out; a.ldo = ldo;
     a.trans = trans;
     a.err = d_err;
-    launch_gram(form, a, s);
+    a.inst = nullptr;
+    launch_gram<false>(form, a, s);
     count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_q_tensor(int form, const InstanceDesc *d_inst, int l, cudaStream_t s)
+{
+    const void *fn = gram_fn<true>(form);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem);
+    if (e != cudaSuccess) return e;
+    GramArgs a = {};
+    a.ma = a.nb = l;
+    a.inst = d_inst;
+    launch_gram<true>(form, a, s);
     return cudaGetLastError();
 }
 

@@ -4,5 +4,6 @@
 namespace svmb {
 
 const void *smo_entry_exact() { return (const void *)smo_persistent<FORM_EXACT>; }
+const void *smo_rows_exact() { return (const void *)smo_rows<FORM_EXACT>; }
 
 }  // namespace svmb

@@ -4,5 +4,6 @@
 namespace svmb {
 
 const void *smo_entry_fp32() { return (const void *)smo_persistent<FORM_FP32>; }
+const void *smo_rows_fp32() { return (const void *)smo_rows<FORM_FP32>; }
 
 }  // namespace svmb

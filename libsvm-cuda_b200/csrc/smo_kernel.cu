@@ -13,6 +13,8 @@ const void *smo_entry_fp32();
 const void *smo_entry_bf16x3();
 const void *smo_entry_fp16x3();
 const void *smo_entry_tf32();
+const void *smo_rows_exact();
+const void *smo_rows_fp32();
 
 // ---------------------------------------------------------------------------
 // setup kernels
@@ -102,6 +104,16 @@ cudaError_t launch_smo(int form, const InstanceDesc *d_insts, const int *d_block
     if (cooperative)
         return cudaLaunchCooperativeKernel(fn, dim3(nblocks), dim3(kThreads), args, dyn_smem, s);
     return cudaLaunchKernel(fn, dim3(nblocks), dim3(kThreads), args, dyn_smem, s);
+}
+
+cudaError_t launch_q_sparse(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, size_t dyn_smem,
+                            cudaStream_t s)
+{
+    const void *fn = form == FORM_FP32 ? smo_rows_fp32() : smo_rows_exact();
+    cudaError_t e = set_max_dyn_smem(fn);
+    if (e != cudaSuccess) return e;
+    void *args[] = {(void *)&d_insts, (void *)&d_first, (void *)&count, (void *)&total};
+    return cudaLaunchKernel(fn, dim3(total < 148 ? total : 148), dim3(kThreads), args, dyn_smem, s);
 }
 
 cudaError_t smo_max_blocks(int form, size_t dyn_smem, int *blocks_per_sm)

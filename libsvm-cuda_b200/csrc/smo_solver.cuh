@@ -1495,7 +1495,7 @@ __device__ void widen()
     Ctx &c = block_shared().c;
     const InstanceDesc &D = block_shared().D;
     set_active(D.l);
-    for (int p = c.a0 + threadIdx.x; p < c.a1; p += blockDim.x) {
+    for (int p = c.a0 + threadIdx.x; p < c.a1 && !D.resident; p += blockDim.x) {
         const unsigned w = (unsigned)D.pos_slot[p], slot = w & 0xffffu;
         if (slot == kNoSlot) continue;
         if (!(w & kSlotFull) || __ldcg(&D.cache.tag[slot]) != D.pos_local[p]) D.pos_slot[p] = kNoSlot;
@@ -2468,6 +2468,7 @@ __device__ void solve_instance(int rank)
     // counts (an add that waits for nothing) and folds them every 1000 iterations
     if (threadIdx.x == 0) {
         for (int k = 0; k < kCnt; k++) sh.cnt[k] = 0;
+        if (D.resident) sh.cnt[kCntQ] = (long long)D.l * D.l;
         for (int k = 0; k < 8; k++) {
             sh.prof[k] = 0;
             sh.prof32[k] = 0;
@@ -2501,7 +2502,7 @@ __device__ void solve_instance(int rank)
     {
         for (int p = c.a0 + threadIdx.x; p < c.a1; p += blockDim.x) {
             D.pos_local[p] = p;      // positions start as local indices
-            D.pos_slot[p] = kNoSlot;
+            D.pos_slot[p] = D.resident ? (int)((unsigned)p | kSlotFull) : kNoSlot;
             D.status[p] = status_of(D.alpha[p], get_C(D, D.y[p]));
             const int r = D.pos_row[p];
             const double xs = D.x.xsq ? D.x.xsq[r] : 0.0;
@@ -2511,6 +2512,8 @@ __device__ void solve_instance(int rank)
             D.G_bar[p] = 0.0;
         }
         if (!exchange()) goto fail;
+        // a resident matrix whose evaluation gave up leaves the group's error flag
+        if (__syncthreads_or(D.resident && ld_relaxed_i32(&D.sync->error))) goto fail;
         int any = 0;
         for (int p = threadIdx.x; p < l; p += blockDim.x) any |= D.alpha[p] > 0 ? 1 : 0;
         any = __syncthreads_or(any);
@@ -3013,6 +3016,64 @@ smo_persistent(const InstanceDesc *__restrict__ insts, const int *__restrict__ b
         tc::tc_fence_before();
         __syncthreads();
         if (threadIdx.x < 32) tc::tmem_dealloc(sh.tmem, 2 * kTcMaxN);
+    }
+}
+
+// Whole kernel matrices of sparse instances (their caches hold every row):
+// block t takes a group of source variables, stages them as a row pass does
+// and walks the targets from its first source on; the values left of the
+// diagonal are copied from the right.  Bound by the target walks: 8 bytes and
+// one or two table probes per stored value for up to 8 sources.
+template <int FORM>
+__global__ void __launch_bounds__(kThreads, 1)
+smo_rows(const InstanceDesc *__restrict__ insts, const int *__restrict__ first, int count, int total)
+{
+    Shared &sh = block_shared();
+    const InstanceDesc &D = sh.D;
+    int cur = -1;
+    float *const stage = reinterpret_cast<float *>(dyn);
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        int lo = 0, hi = count - 1;
+        while (lo < hi) {
+            const int m = (lo + hi + 1) >> 1;
+            if (first[m] <= t) lo = m;
+            else hi = m - 1;
+        }
+        if (lo != cur) {
+            // another instance: its descriptor, and an empty staging area
+            cur = lo;
+            __syncthreads();
+            for (int k = threadIdx.x; k < (int)(sizeof(InstanceDesc) / 4); k += blockDim.x)
+                reinterpret_cast<int *>(&sh.D)[k] = reinterpret_cast<const int *>(&insts[lo])[k];
+            __syncthreads();
+            stage_clear<FORM>(stage);
+        }
+        const int l = D.l, cap = D.stage_cap > 0 ? D.stage_cap : kSrcBatch;
+        const int p0 = (t - first[lo]) * cap, ns = min(cap, l - p0);
+        if (threadIdx.x < ns) {
+            const int row = D.pos_row[p0 + threadIdx.x];
+            sh.frow[threadIdx.x] = row;
+            sh.fy[threadIdx.x] = D.y[p0 + threadIdx.x];
+            sh.fsx[threadIdx.x] = D.x.xsq ? D.x.xsq[row] : 0.0;
+        }
+        __syncthreads();
+        stage_sources(D, stage, sh.ss, sh.frow, ns);
+        float *const Q = D.cache.data;
+        const long long stride = D.cache.stride;
+        for (int p = p0 + threadIdx.x; p < l; p += blockDim.x) {
+            const int r = D.pos_row[p], yp = D.y[p];
+            double dots[kSrcBatch];
+            row_dots<FORM>(D, sh.ss, ns, r, dots);
+            const double xe = D.x.xsq ? D.x.xsq[r] : 0.0;
+#pragma unroll
+            for (int k = 0; k < kSrcBatch; k++) {
+                if (k >= ns) break;
+                const float q = q_of(sh.fy[k] * yp, dots[k], sh.fsx[k], xe);
+                Q[(long long)(p0 + k) * stride + p] = q;
+                if (p >= p0 + ns) Q[(long long)p * stride + p0 + k] = q;
+            }
+        }
+        unstage_sources(D, stage, sh.ss);
     }
 }
 

@@ -1,0 +1,57 @@
+"""Whole kernel matrices evaluated before the solve (a cache with a slot for
+every variable) against rows evaluated during it (a cache too small for that).
+Both evaluate the same expressions in the same order, so the coefficients and
+the iteration counts must be identical, at tile edges, at widths with a partial
+last slice, and for every kind of rows and form."""
+import numpy as np
+import pytest
+
+from svmb200 import datagen
+from svmb200.lib import FORM_EXACT, FORM_FP16X3, FORM_FP32, FORM_TF32, make_params
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(engine, p, **more):
+    n = p.n * (2 if more.get("svm_type") in (3, 4) else 1)
+    small = make_params(cache_mb=4.0 * n * max(4, n // 3) / (1 << 20), **more)
+    a, sa = engine.solve_binary(p, small)
+    b, sb = engine.solve_binary(p, make_params(cache_mb=100.0, **more))
+    assert sb["fills"] == 0 and (n <= 4 or sa["fills"] > 0)
+    assert sa["iters"] == sb["iters"]
+    np.testing.assert_array_equal(a, b)
+    assert sa["rho"] == sb["rho"] and sa["obj"] == sb["obj"]
+
+
+@pytest.mark.parametrize("form", [FORM_EXACT, FORM_FP32, FORM_FP16X3, FORM_TF32])
+@pytest.mark.parametrize("n,d", [(5, 1), (63, 4), (64, 16), (65, 17), (129, 70), (1030, 33)])
+def test_dense(engine, n, d, form):
+    p, _ = datagen.dense_gauss(n=n, n_test=0, d=d, seed=n + d)
+    _same(engine, p, kernel_type=2, gamma=1.0 / d, C_pos=2.0, form=form)
+
+
+@pytest.mark.parametrize("kernel", [0, 1, 2, 3])
+@pytest.mark.parametrize("d", [150, 20000])
+def test_sparse_rows_and_kernels(engine, d, kernel):
+    p, _ = datagen.sparse_text(n=203, n_test=0, d=d, nnz_mean=12.0, seed=d + kernel)
+    _same(engine, p, kernel_type=kernel, gamma=0.4, coef0=0.5, C_pos=2.0)
+
+
+@pytest.mark.parametrize("svm_type", [1, 2, 3, 4])
+def test_formulations(engine, svm_type):
+    p, _ = (datagen.regression(n=150, n_test=0, d=7, seed=3) if svm_type >= 3 else
+            datagen.dense_gauss(n=300, n_test=0, d=12, seed=4))
+    _same(engine, p, svm_type=svm_type, kernel_type=2, gamma=0.1, nu=0.3, C_pos=2.0)
+
+
+def test_instances_of_one_launch(engine):
+    """Uneven instances over shared rows: tiles of several matrices in one grid."""
+    p, _ = datagen.dense_gauss(n=400, n_test=0, d=20, seed=9)
+    rng = np.random.default_rng(1)
+    rows = [np.sort(rng.choice(p.n, m, replace=False)).astype(np.int32) for m in (70, 64, 301, 9)]
+    ys = [p.y[r] for r in rows]
+    prm = make_params(kernel_type=2, gamma=0.05)
+    got, _ = engine.solve_many(p, rows, ys, [prm] * len(rows))
+    for r, y, a in zip(rows, ys, got):
+        want, _ = engine.solve_binary(p.take(r), make_params(kernel_type=2, gamma=0.05, cache_mb=1e-3), y=y)
+        np.testing.assert_array_equal(a, want)
