@@ -666,12 +666,147 @@ const DeviceRows &rows_of(const SubProblem &sp, const DeviceRows &rows) { return
 
 }  // namespace
 
+// Resident instances: a cache that holds every row is filled with the whole
+// kernel matrix before the solve, by all SMs.  Worth it when that takes less
+// than what the solves would spend on row passes: their iterations number about
+// l (0.2 l to 5 l measured) and spend 0.3 to 3 us each on passes, so the line
+// is the matrices' estimated time against 1 us per position of the launch's
+// longest instance.  One value costs its dot product and a kernel function of
+// about 40 operations; dense tiles run at about 8e12 operations a second, half
+// of the values being copies.  A launch whose longest instance has no such
+// cache lasts as long without (the 45 pairs of 3,600 to 21,600 positions, the
+// ten smallest resident: 44.1 ms against 42.6 ms).
+static std::vector<char> resident_of(const DeviceRows &rows, const std::vector<SubProblem> &subs, const SolveParams &prm,
+                                     int first, int count)
+{
+    double cost = 0.0;
+    long long longest = 0, longest_fit = 0;
+    std::vector<char> fits(count, 0);
+    for (int k = 0; k < count; k++) {
+        const SubProblem &sp = subs[first + k];
+        const DeviceRows &r = rows_of(sp, rows);
+        const long long l = (long long)sp.rows.size();
+        longest = std::max(longest, l);
+        if (l == 0 || instance_layout((int)l, 1, params_of(sp, prm).cache_mb).slots < l) continue;
+        longest_fit = std::max(longest_fit, l);
+        fits[k] = 1;
+        const double width = is_tc_form(prm.form) ? 0.05 * r.d : r.dense ? (double)r.ld : 8.0 * (double)r.nnz / std::max(r.n, 1);
+        cost += 0.5 * (double)l * (double)l * (width + 40.0);
+    }
+    if (longest_fit < longest || cost > 8e12 * 1e-6 * (double)longest) fits.assign(count, 0);
+    return fits;
+}
+
+// Blocks per instance of a launch whose instances are all resident, or 0: then
+// each is one thread-block cluster of that size (smo_resident.cuh).  As many
+// blocks as the longest instance has spans of `span` positions (a power of two, at
+// most kClusterMax), fewer when the instances would not all run at a time.
+static int cluster_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const SolveParams &prm, int first,
+                        int count, long long span, int capacity)
+{
+    long long longest = 0;
+    for (int k = 0; k < count; k++) {
+        if (params_of(subs[first + k], prm).blocks_override > 0) return 0;
+        longest = std::max(longest, (long long)subs[first + k].rows.size());
+    }
+    for (char r : resident_of(rows, subs, prm, first, count))
+        if (!r) return 0;
+    int c = 1;
+    while (c < kClusterMax && c * span < longest) c *= 2;
+    while (c > 1 && (long long)count * c > capacity) c /= 2;
+    return c;
+}
+
+// The staging and the memory of a wave whose instances have nb[k] blocks each.
+static int wave_layout(const DeviceRows &rows, const std::vector<SubProblem> &subs, const SolveParams &prm, Wave &w,
+                       const std::vector<StagePlan> &sp_all, const std::vector<long long> &nb)
+{
+    const int first = w.first, count = (int)sp_all.size();
+    int used = 0;
+    w.count = count;
+    w.nb.assign(nb.begin(), nb.end());
+    for (int k = 0; k < count; k++) used += w.nb[k];
+    w.used = used;
+    w.stage.resize(count);
+    w.fill_path.assign(count, 0);
+    w.tile_bufs = count > 0 ? sp_all[0].tile_bufs : 2;
+    long long dyn = 0;
+    for (int k = 0; k < count; k++) {
+        const long long l = (long long)subs[first + k].rows.size();
+        const long long cap = (l + w.nb[k] - 1) / w.nb[k];
+        w.stage[k][0] = sp_all[k].stage_cap;
+        w.stage[k][1] = sp_all[k].stage_lds;
+        w.stage[k][2] = sp_all[k].tc_n;
+        w.stage[k][3] = (int)cap;
+        w.stage[k][4] = sp_all[k].hash_slots;
+        const bool dense = rows_of(subs[first + k], rows).dense;
+        w.fill_path[k] = is_tc_form(prm.form)           ? SVMB_FILL_TENSOR
+                         : dense                        ? SVMB_FILL_DENSE
+                         : sp_all[k].stage_cap > 0      ? SVMB_FILL_SPARSE_SCATTER
+                         : sp_all[k].hash_slots > 0     ? SVMB_FILL_SPARSE_TABLE
+                                                        : SVMB_FILL_SPARSE_MERGE;
+        dyn = std::max(dyn, sp_all[k].bytes + cap * kChunkBytes);
+    }
+    w.dyn_smem = (size_t)dyn;
+
+    // One device block per wave, laid out so that the host touches it with
+    // one upload, one fill and one download:
+    //   upload   [descriptors][block map][alpha][p][row ids][labels]
+    //   download [outputs][alpha by local index]
+    //   zero     [group syncs][exchange records][record words]
+    //   [cache tags]
+    //   per instance: G, G_bar, QD, status, position->local, position->slot, shrink lists, Q rows
+    auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
+    w.loff.assign(count + 1, 0);
+    w.poff.assign(count + 1, 0);
+    w.coff.assign(count + 1, 0);
+    w.lay.resize(count);
+    for (int k = 0; k < count; k++) {
+        const SubProblem &sp = subs[first + k];
+        const int l = (int)sp.rows.size();
+        w.lay[k] = instance_layout(l, w.nb[k], params_of(sp, prm).cache_mb);
+        w.loff[k + 1] = w.loff[k] + (size_t)l;
+        w.poff[k + 1] = w.poff[k] + 2 * (size_t)w.nb[k];
+        w.coff[k + 1] = w.coff[k] + (size_t)w.lay[k].slots;
+    }
+    if (w.cluster > 0) w.resident.assign(count, 1);
+    else w.resident = resident_of(rows, subs, prm, first, count);
+    const size_t L = w.loff[count], P = w.poff[count], S = w.coff[count];
+    size_t off = 0;
+    w.o_desc = off; off = al(off + sizeof(InstanceDesc) * count);
+    w.o_bmap = off; off = al(off + sizeof(int) * used);
+    w.o_qmap = off; off = al(off + sizeof(int) * 2 * count);
+    w.o_alpha = off; off = al(off + 8 * L);
+    w.o_p = off; off = al(off + 8 * L);
+    w.o_row = off; off = al(off + 4 * L);
+    w.o_y = off; off = al(off + L);
+    w.up_bytes = off;
+    w.o_out = off; off = al(off + sizeof(SolveOut) * count);
+    w.o_alocal = off; off = al(off + 8 * L);
+    w.down_bytes = off - w.o_out;
+    w.o_zero = off;
+    w.o_sync = off; off = al(off + sizeof(GroupSync) * count);
+    w.o_part = off; off = al(off + sizeof(Partial) * P);
+    w.o_word = off; off = al(off + sizeof(RecWord) * kRecWords * (P / 2));
+    w.zero_bytes = off - w.o_zero;
+    w.o_tag = off; off = al(off + 4 * S);
+    w.inst_off.resize(count);
+    for (int k = 0; k < count; k++) {
+        w.inst_off[k] = off;
+        off += w.lay[k].bytes;
+    }
+    w.dev_bytes = off;
+    return 0;
+}
+
 int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const SolveParams &prm, int first,
               int capacity, Wave &w, int limit)
 {
     const int ninst = limit >= 0 && limit < (int)subs.size() ? limit : (int)subs.size();
     const int tune_pf = w.tune_prefetch, tune_rpb = w.tune_rows_per_block;
+    const bool queue = w.queue;
     w = Wave();
+    w.queue = queue;
     w.tune_prefetch = tune_pf;
     w.tune_rows_per_block = tune_rpb;
     w.first = first;
@@ -680,6 +815,41 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
     if (budget <= 0) {
         set_error("cannot query the device's shared memory");
         return -1;
+    }
+    if (!g_drop_block) {
+        // all remaining instances resident: clusters, as many as the memory for
+        // their matrices allows (and, unless they may queue, as many as run at a time)
+        int n = 0;
+        double bytes = 0.0;
+        while (first + n < ninst && (w.queue || n < capacity)) {
+            bytes += (double)instance_layout((int)subs[first + n].rows.size(), 1, params_of(subs[first + n], prm).cache_mb).bytes;
+            if (n > 0 && bytes > 16e9) break;
+            n++;
+        }
+        const int c = n > 0 ? cluster_plan(rows, subs, prm, first, n, w.tune_rows_per_block, capacity) : 0;
+        if (c > 0) {
+            long long need = 0;
+            std::vector<StagePlan> sps;
+            std::vector<long long> nms;
+            bool ok = true;
+            for (int k = 0; k < n && ok; k++) {
+                const SubProblem &sp = subs[first + k];
+                ok = params_of(sp, prm).form == prm.form;
+                const StagePlan st = stage_plan(rows_of(sp, rows), prm.form, budget, 1);
+                const long long cap = ((long long)sp.rows.size() + c - 1) / c;
+                need = std::max(need, st.bytes + cap * kChunkBytes);
+                ok = ok && st.chunk_max >= 64;
+                sps.push_back(st);
+                nms.push_back(c);
+            }
+            int clusters = 0;
+            if (ok && (size_t)need <= smo_cluster_smem(prm.form) &&
+                smo_max_clusters(prm.form, c, (size_t)need, &clusters) == cudaSuccess && clusters > 0) {
+                w.cluster = c;
+                return wave_layout(rows, subs, prm, w, sps, nms);
+            }
+            cudaGetLastError();
+        }
     }
     const int sms = device_sm_count();
     std::vector<StagePlan> sp_all;
@@ -784,105 +954,8 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
             if (w.nb[k] < cap[k]) q.push(k);
         }
     }
-    w.used = used;
-    w.stage.resize(count);
-    w.fill_path.assign(count, 0);
-    w.tile_bufs = count > 0 ? sp_all[0].tile_bufs : 2;
-    long long dyn = 0;
-    for (int k = 0; k < count; k++) {
-        const long long l = (long long)subs[first + k].rows.size();
-        const long long cap = (l + w.nb[k] - 1) / w.nb[k];
-        w.stage[k][0] = sp_all[k].stage_cap;
-        w.stage[k][1] = sp_all[k].stage_lds;
-        w.stage[k][2] = sp_all[k].tc_n;
-        w.stage[k][3] = (int)cap;
-        w.stage[k][4] = sp_all[k].hash_slots;
-        const bool dense = rows_of(subs[first + k], rows).dense;
-        w.fill_path[k] = is_tc_form(prm.form)           ? SVMB_FILL_TENSOR
-                         : dense                        ? SVMB_FILL_DENSE
-                         : sp_all[k].stage_cap > 0      ? SVMB_FILL_SPARSE_SCATTER
-                         : sp_all[k].hash_slots > 0     ? SVMB_FILL_SPARSE_TABLE
-                                                        : SVMB_FILL_SPARSE_MERGE;
-        dyn = std::max(dyn, sp_all[k].bytes + cap * kChunkBytes);
-    }
-    w.dyn_smem = (size_t)dyn;
-
-    // One device block per wave, laid out so that the host touches it with
-    // one upload, one fill and one download:
-    //   upload   [descriptors][block map][alpha][p][row ids][labels]
-    //   download [outputs][alpha by local index]
-    //   zero     [group syncs][exchange records][record words]
-    //   [cache tags]
-    //   per instance: G, G_bar, QD, status, position->local, position->slot, shrink lists, Q rows
-    auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
-    w.loff.assign(count + 1, 0);
-    w.poff.assign(count + 1, 0);
-    w.coff.assign(count + 1, 0);
-    w.lay.resize(count);
-    for (int k = 0; k < count; k++) {
-        const SubProblem &sp = subs[first + k];
-        const int l = (int)sp.rows.size();
-        w.lay[k] = instance_layout(l, w.nb[k], params_of(sp, prm).cache_mb);
-        w.loff[k + 1] = w.loff[k] + (size_t)l;
-        w.poff[k + 1] = w.poff[k] + 2 * (size_t)w.nb[k];
-        w.coff[k + 1] = w.coff[k] + (size_t)w.lay[k].slots;
-    }
-    // Resident instances: a cache that holds every row is filled with the whole
-    // kernel matrix before the solve, by all SMs.  Worth it when that takes
-    // less than what the solves would spend on row passes: their iterations
-    // number about l (0.2 l to 5 l measured) and spend 0.3 to 3 us each on
-    // passes, so the line is the matrices' estimated time against 1 us per
-    // position of the launch's longest instance.  One value costs its dot product
-    // and a kernel function of about 40 operations; dense tiles run at about
-    // 8e12 operations a second, half of the values being copies.  A launch
-    // whose longest instance has no such cache lasts as long without (the 45
-    // pairs of 3,600 to 21,600 positions, the ten smallest resident: 44.1 ms
-    // against 42.6 ms).
-    {
-        double cost = 0.0;
-        long long longest = 0, longest_fit = 0;
-        std::vector<char> fits(count, 0);
-        for (int k = 0; k < count; k++) {
-            const SubProblem &sp = subs[first + k];
-            const DeviceRows &r = rows_of(sp, rows);
-            const double l = (double)sp.rows.size();
-            longest = std::max(longest, (long long)sp.rows.size());
-            if (sp.rows.empty() || w.lay[k].slots < (int)sp.rows.size()) continue;
-            longest_fit = std::max(longest_fit, (long long)sp.rows.size());
-            fits[k] = 1;
-            const double width = is_tc_form(prm.form) ? 0.05 * r.d : r.dense ? (double)r.ld : 8.0 * (double)r.nnz / std::max(r.n, 1);
-            cost += 0.5 * l * l * (width + 40.0);
-        }
-        const bool on = longest_fit == longest && cost <= 8e12 * 1e-6 * (double)longest;
-        w.resident.assign(count, 0);
-        for (int k = 0; k < count; k++) w.resident[k] = on && fits[k];
-    }
-    const size_t L = w.loff[count], P = w.poff[count], S = w.coff[count];
-    size_t off = 0;
-    w.o_desc = off; off = al(off + sizeof(InstanceDesc) * count);
-    w.o_bmap = off; off = al(off + sizeof(int) * used);
-    w.o_qmap = off; off = al(off + sizeof(int) * 2 * count);
-    w.o_alpha = off; off = al(off + 8 * L);
-    w.o_p = off; off = al(off + 8 * L);
-    w.o_row = off; off = al(off + 4 * L);
-    w.o_y = off; off = al(off + L);
-    w.up_bytes = off;
-    w.o_out = off; off = al(off + sizeof(SolveOut) * count);
-    w.o_alocal = off; off = al(off + 8 * L);
-    w.down_bytes = off - w.o_out;
-    w.o_zero = off;
-    w.o_sync = off; off = al(off + sizeof(GroupSync) * count);
-    w.o_part = off; off = al(off + sizeof(Partial) * P);
-    w.o_word = off; off = al(off + sizeof(RecWord) * kRecWords * (P / 2));
-    w.zero_bytes = off - w.o_zero;
-    w.o_tag = off; off = al(off + 4 * S);
-    w.inst_off.resize(count);
-    for (int k = 0; k < count; k++) {
-        w.inst_off[k] = off;
-        off += w.lay[k].bytes;
-    }
-    w.dev_bytes = off;
-    return 0;
+    std::vector<long long> nbs(w.nb.begin(), w.nb.end());
+    return wave_layout(rows, subs, prm, w, sp_all, nbs);
 }
 
 // The stream work of a wave: upload, fills, the launch between two timing
@@ -912,7 +985,9 @@ static cudaError_t wave_issue(Wave &w, InstanceDesc *d_desc, int *d_block_inst, 
         }
     }
     if (e == cudaSuccess)
-        e = launch_smo(w.form, d_desc, d_block_inst, w.used - (w.drop_last_block ? 1 : 0), w.dyn_smem, w.cooperative, s);
+        e = w.cluster > 0 ? launch_smo_cluster(w.form, d_desc, d_block_inst, w.used, w.cluster, w.dyn_smem, s)
+                          : launch_smo(w.form, d_desc, d_block_inst, w.used - (w.drop_last_block ? 1 : 0), w.dyn_smem,
+                                       w.cooperative, s);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(w.ev1, s, rec);
     if (e == cudaSuccess) e = xfer_async(host + w.up_bytes, dev + w.o_out, w.down_bytes, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(w.done, s, rec);
@@ -939,7 +1014,7 @@ std::string graph_key(const Wave &w)
     snprintf(buf, sizeof buf, "%p:%p:%zu:%zu:%zu:%zu:%zu:%d:%zu:%d:%d", (void *)w.dev, (void *)w.host, w.up_bytes,
              w.down_bytes, w.zero_bytes, w.o_zero, w.o_out, w.used, w.dyn_smem, w.form,
              (int)w.cooperative);
-    std::string q;      // the resident instances and their launches
+    std::string q = std::to_string(w.cluster) + ":";    // the resident instances and their launches
     for (char c : w.resident) q += c ? '1' : '0';
     q += ":" + std::to_string(w.q_total[0]) + ":" + std::to_string(w.q_total[1]) + ":" + std::to_string(w.q_smem);
     return std::string(buf) + ":" + q + ":" + std::to_string(w.o_desc) + ":" + std::to_string(w.o_bmap);
@@ -1120,7 +1195,7 @@ int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, cons
         memcpy(h_row + w.loff[k], sp.rows.data(), sizeof(int) * l);
         memcpy(h_y + w.loff[k], sp.y.data(), l);
     }
-    if (g_drop_block.exchange(0)) {
+    if (w.cluster == 0 && g_drop_block.exchange(0)) {
         w.drop_last_block = true;
         w.use_graph = false;
     }
@@ -1416,6 +1491,7 @@ int solve_batch(const DeviceRows &rows, const std::vector<SubProblem> &subs, con
         Wave w;
         w.tune_prefetch = tune.prefetch;
         w.tune_rows_per_block = tune.rows_per_block;
+        w.queue = true;
         if (wave_plan(rows, *plan, prm, first, capacity, w, group_end.empty() ? -1 : group_end[first]) != 0) return -1;
         clk.mark("plan");
         char *arena = arena_reserve(w.dev_bytes);

@@ -97,6 +97,8 @@ struct Wave {
     std::vector<int> nb;                      // blocks per instance
     std::vector<std::array<int, 5>> stage;    // stage_cap, stage_lds, tc_n, chunk_cap, hash_slots per instance
     std::vector<int> fill_path;               // SVMB_FILL_* per instance
+    int cluster = 0;                          // blocks per instance of a launch of clusters (0: general solver)
+    bool queue = false;                       // such a launch may hold more instances than run at a time
     std::vector<char> resident;               // the instance's kernel matrix is evaluated before the solve
     int q_total[2] = {0, 0};                  // tiles of the resident dense rows, source groups of the sparse ones
     size_t q_smem = 0;                        // staging of the source groups
@@ -200,6 +202,11 @@ cudaError_t launch_q_dense(int form, const InstanceDesc *d_insts, const int *d_f
 cudaError_t launch_q_sparse(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, size_t dyn_smem,
                             cudaStream_t s);
 cudaError_t launch_q_tensor(int form, const InstanceDesc *d_inst, int l, cudaStream_t s);
+// resident instances, one cluster each (smo_resident.cuh)
+cudaError_t launch_smo_cluster(int form, const InstanceDesc *d_insts, const int *d_block_inst, int nblocks, int cluster,
+                               size_t dyn_smem, cudaStream_t s);
+cudaError_t smo_max_clusters(int form, int cluster, size_t dyn_smem, int *clusters);
+size_t smo_cluster_smem(int form);
 cudaError_t smo_max_blocks(int form, size_t dyn_smem, int *blocks_per_sm);
 
 }  // namespace svmb

@@ -13,6 +13,11 @@ const void *smo_entry_fp32();
 const void *smo_entry_bf16x3();
 const void *smo_entry_fp16x3();
 const void *smo_entry_tf32();
+const void *smo_cluster_exact();
+const void *smo_cluster_fp32();
+const void *smo_cluster_bf16x3();
+const void *smo_cluster_fp16x3();
+const void *smo_cluster_tf32();
 const void *smo_rows_exact();
 const void *smo_rows_fp32();
 
@@ -104,6 +109,62 @@ cudaError_t launch_smo(int form, const InstanceDesc *d_insts, const int *d_block
     if (cooperative)
         return cudaLaunchCooperativeKernel(fn, dim3(nblocks), dim3(kThreads), args, dyn_smem, s);
     return cudaLaunchKernel(fn, dim3(nblocks), dim3(kThreads), args, dyn_smem, s);
+}
+
+static const void *cluster_fn(int form)
+{
+    if (form == FORM_EXACT) return smo_cluster_exact();
+    if (form == FORM_FP32) return smo_cluster_fp32();
+    if (form == FORM_BF16X3) return smo_cluster_bf16x3();
+    if (form == FORM_TF32) return smo_cluster_tf32();
+    return smo_cluster_fp16x3();
+}
+
+static cudaLaunchConfig_t cluster_config(int nblocks, int cluster, size_t dyn_smem, cudaStream_t s, cudaLaunchAttribute *attr)
+{
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)cluster;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nblocks);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = dyn_smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+cudaError_t launch_smo_cluster(int form, const InstanceDesc *d_insts, const int *d_block_inst, int nblocks, int cluster,
+                               size_t dyn_smem, cudaStream_t s)
+{
+    const void *fn = cluster_fn(form);
+    cudaError_t e = set_max_dyn_smem(fn);
+    if (e != cudaSuccess) return e;
+    void *args[] = {(void *)&d_insts, (void *)&d_block_inst};
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_config(nblocks, cluster, dyn_smem, s, &attr);
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+// clusters of the given size that run at a time, and the dynamic shared memory a block may use
+cudaError_t smo_max_clusters(int form, int cluster, size_t dyn_smem, int *clusters)
+{
+    const void *fn = cluster_fn(form);
+    cudaError_t e = set_max_dyn_smem(fn);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_config(cluster, cluster, dyn_smem, 0, &attr);
+    return cudaOccupancyMaxActiveClusters(clusters, fn, &cfg);
+}
+size_t smo_cluster_smem(int form)
+{
+    int dev = 0, optin = 0;
+    cudaFuncAttributes a;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaFuncGetAttributes(&a, cluster_fn(form)) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return 0;
+    return (size_t)optin - a.sharedSizeBytes - 1024;
 }
 
 cudaError_t launch_q_sparse(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, size_t dyn_smem,

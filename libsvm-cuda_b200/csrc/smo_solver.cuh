@@ -745,7 +745,7 @@ __device__ __forceinline__ const Partial *prev_partials()
 }
 
 // Publish my record of this phase and wait for everybody's (group barrier).
-__device__ bool exchange()
+__device__ __noinline__ bool exchange()
 {
     Ctx &c = block_shared().c;
     __syncthreads();
@@ -793,7 +793,7 @@ __device__ __forceinline__ unsigned char status_of(double a, double C)
 }
 
 // chunk state: global -> shared / shared -> global (mutable fields only)
-__device__ void chunk_load()
+__device__ __noinline__ void chunk_load()
 {
     Ctx &c = block_shared().c;
     const InstanceDesc &D = block_shared().D;
@@ -811,7 +811,7 @@ __device__ void chunk_load()
     }
     __syncthreads();
 }
-__device__ void chunk_store()
+__device__ __noinline__ void chunk_store()
 {
     Ctx &c = block_shared().c;
     const InstanceDesc &D = block_shared().D;
@@ -1424,10 +1424,90 @@ __device__ __noinline__ bool accumulate_rows_tc(int src_end, int pick_free_only,
     return true;
 }
 
+// The same sums for a resident instance: the Q values are read from the cache,
+// consecutive threads on neighbouring columns, instead of evaluated again.
+// Sources go through shared memory a batch at a time: `batch` is a whole block
+// of positions for the CUDA-core forms, whose sums run source by source, and
+// one tensor-core pass for the others, whose sums run in four groups of 16.
+template <int FORM>
+__device__ __noinline__ void accumulate_resident(int src_end, int pick_free_only, int with_bar, int lo, int hi)
+{
+    Shared &sh = block_shared();
+    const InstanceDesc &D = sh.D;
+    constexpr bool tensor = is_tc_form(FORM);
+    const int cap = tensor ? D.tc_n : kThreads;
+    // the staging area holds the batch: alpha, C of the sources at the bound (0: not), column
+    double *const ba = reinterpret_cast<double *>(dyn), *const bc = ba + kThreads;
+    int *const bcol = reinterpret_cast<int *>(bc + kThreads);
+    const float *const Q = D.cache.data;
+    const long long stride = D.cache.stride;
+    int scan = 0;
+    while (true) {
+        if (threadIdx.x == 0) sh.nsrc = 0;
+        __syncthreads();
+        while (scan < src_end) {
+            const int p = scan + threadIdx.x;
+            int sel = 0;
+            unsigned char st = ST_LOWER;
+            if (p < src_end) {
+                st = D.status[p];
+                sel = pick_free_only ? (st == ST_FREE) : (st != ST_LOWER);
+            }
+            int tot;
+            const int pre = block_excl_scan(sh.red, sel, &tot);
+            const int have = sh.nsrc, room = cap - have;
+            if (sel && pre < room) {
+                ba[have + pre] = D.alpha[p];
+                bc[have + pre] = st == ST_UPPER ? get_C(D, D.y[p]) : 0.0;
+                bcol[have + pre] = D.pos_local[p];
+            }
+            const int take = tot < room ? tot : room;
+            if (take < tot && sel && pre == take) sh.stop_at = threadIdx.x;
+            __syncthreads();
+            const int consumed = take == tot ? (int)blockDim.x : sh.stop_at;
+            __syncthreads();
+            if (threadIdx.x == 0) sh.nsrc = have + take;
+            scan += consumed;
+            __syncthreads();
+            if (sh.nsrc == cap) break;
+        }
+        const int ns = sh.nsrc;
+        if (ns == 0) break;
+        for (int e = lo + threadIdx.x; e < hi; e += blockDim.x) {
+            const float *const Qe = Q + D.pos_local[e];
+            double g = D.G[e], gb = with_bar ? D.G_bar[e] : 0.0;
+            constexpr int kGroup = tensor ? 16 : 8;     // loads in flight; a tensor form's partial sum
+            for (int k0 = 0; k0 < ns; k0 += kGroup) {
+                float q[kGroup];
+#pragma unroll
+                for (int u = 0; u < kGroup; u++) q[u] = k0 + u < ns ? Qe[bcol[k0 + u] * stride] : 0.0f;
+                double part = tensor ? 0.0 : g, partb = tensor ? 0.0 : gb;
+#pragma unroll
+                for (int u = 0; u < kGroup; u++) {
+                    if (k0 + u >= ns) break;
+                    part = __dadd_rn(part, __dmul_rn(ba[k0 + u], (double)q[u]));
+                    const double C = bc[k0 + u];
+                    if (with_bar && C != 0.0) partb = __dadd_rn(partb, __dmul_rn(C, (double)q[u]));
+                }
+                g = tensor ? __dadd_rn(g, part) : part;
+                gb = tensor ? __dadd_rn(gb, partb) : partb;
+            }
+            D.G[e] = g;
+            if (with_bar) D.G_bar[e] = gb;
+        }
+        __syncthreads();
+        if (ns < cap) break;
+    }
+}
+
 // the row-block product of the form: CUDA cores or tensor cores
 template <int FORM>
 __device__ bool accumulate(int src_end, int pick_free_only, int with_bar, int lo, int hi)
 {
+    if (block_shared().D.resident) {
+        accumulate_resident<FORM>(src_end, pick_free_only, with_bar, lo, hi);
+        return true;
+    }
     if constexpr (is_tc_form(FORM)) {
         return accumulate_rows_tc(src_end, pick_free_only, with_bar, lo, hi);
     } else {
@@ -1501,6 +1581,17 @@ __device__ void widen()
         if (!(w & kSlotFull) || __ldcg(&D.cache.tag[slot]) != D.pos_local[p]) D.pos_slot[p] = kNoSlot;
     }
     chunk_load();
+}
+
+// the whole gradient reconstructed and the active set widened (svm.cpp:598-611)
+template <int FORM>
+__device__ __noinline__ bool reopen()
+{
+    chunk_store();
+    if (!exchange()) return false;
+    if (!reconstruct<FORM>()) return false;
+    widen();
+    return true;
 }
 
 template <int FORM>
@@ -1699,7 +1790,8 @@ __device__ __forceinline__ void poll_iup(unsigned seq, int warp, int lane)
 // Exchange of the block's I_up maxima (per track, with payload) and, with
 // `ahead`, publication of its most violating positions (prefetch candidates:
 // the best of each warp, top kPrefetchCand).  The group's winners are in sh.wa.
-__device__ __forceinline__ bool iup_publish(unsigned seq, int nu, bool ahead, const double (&v)[2],
+template <int nu>
+__device__ __forceinline__ bool iup_publish(unsigned seq, bool ahead, const double (&v)[2],
                                             const int (&ix)[2], double pv, int pix)
 {
     Ctx &c = block_shared().c;
@@ -1818,11 +1910,11 @@ __device__ __forceinline__ bool iup_publish(unsigned seq, int nu, bool ahead, co
     return sh.fail == 0;
 }
 
+template <int nu>
 __device__ __noinline__ bool scan_iup(unsigned seq)
 {
     Ctx &c = block_shared().c;
     const Chunk ck = chunk_at(c.choff, block_shared().D.chunk_cap);
-    const int nu = block_shared().D.nu;
     double v[2] = {-SVMB_INF, -SVMB_INF};
     int ix[2] = {-1, -1};
     double pv = -SVMB_INF;
@@ -1838,7 +1930,7 @@ __device__ __noinline__ bool scan_iup(unsigned seq)
         }
         better_max(pv, pix, prefetch_priority(y, s, G), c.a0 + k);
     }
-    return iup_publish(seq, nu, block_shared().D.prefetch > 1, v, ix, pv, pix);
+    return iup_publish<nu>(seq, block_shared().D.prefetch > 1, v, ix, pv, pix);
 }
 
 // One poll warp's part of a phase-B exchange (W words a record).
@@ -1877,7 +1969,8 @@ __device__ __forceinline__ void poll_j(unsigned seq, int warp, int lane)
 
 // Exchange of the block's second-order j candidate (largest decrease, with
 // payload) and its Gmax2 maxima; the group's are in sh.wb.
-__device__ __forceinline__ bool j_publish(unsigned seq, int nu, double dec, int jx, double g2, double g2n,
+template <int nu>
+__device__ __forceinline__ bool j_publish(unsigned seq, double dec, int jx, double g2, double g2n,
                                           const float *Qi0, const float *Qi1)
 {
     Ctx &c = block_shared().c;
@@ -1949,7 +2042,7 @@ __device__ __forceinline__ bool j_publish(unsigned seq, int nu, double dec, int 
 }
 
 // which poll warp's record of track t wins (larger value, ties to the larger position)
-__device__ __forceinline__ int win_iup(int np, int t)
+__device__ __noinline__ int win_iup(int np, int t)
 {
     Shared &sh = block_shared();
     int e = 0;
@@ -1960,7 +2053,7 @@ __device__ __forceinline__ int win_iup(int np, int t)
     }
     return e;
 }
-__device__ __forceinline__ int win_j(int np)
+__device__ __noinline__ int win_j(int np)
 {
     Shared &sh = block_shared();
     int e = 0;
@@ -2385,12 +2478,116 @@ __device__ __noinline__ bool miss_j(int e, int slot0, int slot1)
     return fill<FORM>(1, 0);
 }
 
-// rcp.approx: about 18 good bits, used only to leave out hopeless divisions
-__device__ __forceinline__ double rcp_rough(double x)
+// two-variable analytic step with box clipping (svm.cpp:636-721): alpha_i and
+// alpha_j in ai and aj become their new values
+__device__ __forceinline__ void pair_step(int yi, int yj, double QDi, double QDj, float Qij, double Gi, double Gj, double C_i,
+                                          double C_j, double &ai, double &aj)
+{
+    if (yi != yj) {
+        double quad_coef = __dadd_rn(__dadd_rn(QDi, QDj), (double)__fmul_rn(2.0f, Qij));
+        if (quad_coef <= 0) quad_coef = kTau;
+        const double delta = __ddiv_rn(__dsub_rn(-Gi, Gj), quad_coef);
+        const double diff = __dsub_rn(ai, aj);
+        ai = __dadd_rn(ai, delta);
+        aj = __dadd_rn(aj, delta);
+        if (diff > 0) {
+            if (aj < 0) { aj = 0; ai = diff; }
+        } else {
+            if (ai < 0) { ai = 0; aj = -diff; }
+        }
+        if (diff > __dsub_rn(C_i, C_j)) {
+            if (ai > C_i) { ai = C_i; aj = __dsub_rn(C_i, diff); }
+        } else {
+            if (aj > C_j) { aj = C_j; ai = __dadd_rn(C_j, diff); }
+        }
+    } else {
+        double quad_coef = __dsub_rn(__dadd_rn(QDi, QDj), (double)__fmul_rn(2.0f, Qij));
+        if (quad_coef <= 0) quad_coef = kTau;
+        const double delta = __ddiv_rn(__dsub_rn(Gi, Gj), quad_coef);
+        const double sum = __dadd_rn(ai, aj);
+        ai = __dsub_rn(ai, delta);
+        aj = __dadd_rn(aj, delta);
+        if (sum > C_i) {
+            if (ai > C_i) { ai = C_i; aj = __dsub_rn(sum, C_i); }
+        } else {
+            if (aj < 0) { aj = 0; ai = sum; }
+        }
+        if (sum > C_j) {
+            if (aj > C_j) { aj = C_j; ai = __dsub_rn(sum, C_j); }
+        } else {
+            if (ai < 0) { ai = 0; aj = sum; }
+        }
+    }
+}
+
+// Row i and / or j completed over the inactive positions.
+template <int FORM>
+__device__ __noinline__ bool fill_tail(bool ti, bool tj, int i, int yi, int row_i, int slot_i, int j, int yj, int row_j,
+                                       int slot_j)
+{
+    Shared &sh = block_shared();
+    Ctx &c = sh.c;
+    const Chunk ck = chunk_at(c.choff, sh.D.chunk_cap);
+    const int ns = (ti ? 1 : 0) + (tj ? 1 : 0);
+    __syncthreads();    // the last fill's list is no longer read
+    if (threadIdx.x == 0) {
+        if (ti) {
+            sh.frow[0] = row_i;
+            sh.fy[0] = yi;
+            sh.fslot[0] = slot_i;
+        }
+        if (tj) {
+            sh.frow[ns - 1] = row_j;
+            sh.fy[ns - 1] = yj;
+            sh.fslot[ns - 1] = slot_j;
+        }
+        sh.cnt[kCntQ] += (long long)ns * (sh.D.l - c.A);
+        sh.cnt[kCntTargets] += sh.D.l - c.A;
+    }
+    __syncthreads();
+    if (!fill<FORM>(ns, 1)) return false;
+    const int ki = i - c.a0, kj = j - c.a0;
+    if (ti && i >= c.a0 && i < c.a1 && (ki & (kThreads - 1)) == (int)threadIdx.x) ck.F[ki] |= kFlagFull;
+    if (tj && j >= c.a0 && j < c.a1 && (kj & (kThreads - 1)) == (int)threadIdx.x) ck.F[kj] |= kFlagFull;
+    return true;
+}
+
+// G_bar of all my positions after i and / or j reached or left their bound
+// (svm.cpp:744-769): G_bar -+ C Q for each of the two that did.
+__device__ __noinline__ void update_gbar(const float *Qi, bool bar_i, bool sub_i, double C_i, const float *Qj, bool bar_j,
+                                         bool sub_j, double C_j)
+{
+    Shared &sh = block_shared();
+    const InstanceDesc &D = sh.D;
+    Ctx &c = sh.c;
+    const Chunk ck = chunk_at(c.choff, D.chunk_cap);
+    auto bar = [&](double g, int col) {
+        if (bar_i) { const double q = (double)Qi[col]; g = sub_i ? __dsub_rn(g, __dmul_rn(C_i, q)) : __dadd_rn(g, __dmul_rn(C_i, q)); }
+        if (bar_j) { const double q = (double)Qj[col]; g = sub_j ? __dsub_rn(g, __dmul_rn(C_j, q)) : __dadd_rn(g, __dmul_rn(C_j, q)); }
+        return g;
+    };
+    const int n = c.a1 - c.a0;
+    for (int k = threadIdx.x; k < n; k += kThreads) D.G_bar[c.a0 + k] = bar(D.G_bar[c.a0 + k], ck.Col[k]);
+    for (int p = c.t0 + threadIdx.x; p < c.t1; p += kThreads) D.G_bar[p] = bar(D.G_bar[p], D.pos_local[p]);
+}
+
+// num / quad roughly, as an integer that orders like it (high word + 1): an
+// approximate reciprocal, off by 2^-17 at most.  A quotient that is not safe
+// to estimate (quad or the result at the ends of the exponent range, NaN) is
+// given the value of an infinite one.
+__device__ __forceinline__ unsigned rough_quotient(double num, double quad)
 {
     double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    return r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(quad));
+    const unsigned hq = (unsigned)__double2hiint(quad);
+    const unsigned h = (unsigned)__double2hiint(__dmul_rn(num, r)) & 0x7fffffffu;
+    return hq - 0x01000000u > 0x7d000000u ? 0x7ff00000u : h + 1u;
+}
+// what a rough quotient must reach to be divided exactly when the best one is
+// `top`: 2^-15 below it, or everything when the best is not a safe estimate
+__device__ __forceinline__ unsigned rough_least(unsigned top)
+{
+    return top >= 0x7fe00000u || top <= 64u ? 1u : top - 64u;
 }
 
 // an empty staging area: sparse sources are scattered into zeroed dense
@@ -2428,8 +2625,10 @@ __device__ __forceinline__ void put_counters(SolveOut &o)
     for (int k = 0; k < 8; k++) o.prof[k] = sh.prof[k];
 }
 
+// A block's context, its work counters and the initial state (svm.cpp:525-572,
+// QD svm.cpp:1321-1327) on the global copies; the block's chunk is loaded.
 template <int FORM>
-__device__ void solve_instance(int rank)
+__device__ __noinline__ bool start_solve(int rank)
 {
     Shared &sh = block_shared();
     const InstanceDesc &D = sh.D;
@@ -2457,15 +2656,6 @@ __device__ void solve_instance(int rank)
         c.choff = (int)(off + aux_bytes(FORM, D.tile_bufs));
     }
     set_active(D.l);
-    const int l = D.l;
-    const int nu = D.nu;
-    const Chunk ck = chunk_at(c.choff, D.chunk_cap);
-    unsigned seq = 0;       // sequence number of the last record exchange
-    long long iter = 0;
-    int unshrink = 0;
-    int status = 0;
-    // work counters and section timers of thread 0; the loop adds 32-bit cycle
-    // counts (an add that waits for nothing) and folds them every 1000 iterations
     if (threadIdx.x == 0) {
         for (int k = 0; k < kCnt; k++) sh.cnt[k] = 0;
         if (D.resident) sh.cnt[kCntQ] = (long long)D.l * D.l;
@@ -2479,396 +2669,41 @@ __device__ void solve_instance(int rank)
         sh.hand = 0;
         sh.reused = 0;
     }
-    unsigned tmark = (unsigned)clock();
     for (int k = threadIdx.x; k < kRefSlots / 32; k += blockDim.x) sh.ref[k] = 0;
-#define SVMB_PROF(k)                                   \
-    do {                                               \
-        if (threadIdx.x == 0) {                        \
-            const unsigned now_ = (unsigned)clock();   \
-            atomicAdd(&sh.prof32[k], now_ - tmark);    \
-            tmark = now_;                              \
-        }                                              \
-    } while (0)
-    auto fold = [&]() {
-        if (threadIdx.x == 0)
-            for (int k = 0; k < 8; k++) {
-                sh.prof[k] += sh.prof32[k];
-                sh.prof32[k] = 0;
-            }
-    };
     stage_clear<FORM>(c.stage);
-
-    // ---- initial state (svm.cpp:525-572, QD svm.cpp:1321-1327) on the global copies ----
-    {
-        for (int p = c.a0 + threadIdx.x; p < c.a1; p += blockDim.x) {
-            D.pos_local[p] = p;      // positions start as local indices
-            D.pos_slot[p] = D.resident ? (int)((unsigned)p | kSlotFull) : kNoSlot;
-            D.status[p] = status_of(D.alpha[p], get_C(D, D.y[p]));
-            const int r = D.pos_row[p];
-            const double xs = D.x.xsq ? D.x.xsq[r] : 0.0;
-            // dot(x,x) in feature order is exactly what xsq holds
-            D.QD[p] = kernel_from_dot(D.kp, xs, xs, xs);
-            D.G[p] = D.p[p];
-            D.G_bar[p] = 0.0;
-        }
-        if (!exchange()) goto fail;
-        // a resident matrix whose evaluation gave up leaves the group's error flag
-        if (__syncthreads_or(D.resident && ld_relaxed_i32(&D.sync->error))) goto fail;
-        int any = 0;
-        for (int p = threadIdx.x; p < l; p += blockDim.x) any |= D.alpha[p] > 0 ? 1 : 0;
-        any = __syncthreads_or(any);
-        if (any) {
-            if (!accumulate<FORM>(l, 0, D.lazy_gbar ? 0 : 1, c.a0, c.a1)) goto fail;
-            if (!exchange()) goto fail;
-        }
-        chunk_load();
+    const int l = D.l;
+    for (int p = c.a0 + threadIdx.x; p < c.a1; p += blockDim.x) {
+        D.pos_local[p] = p;      // positions start as local indices
+        D.pos_slot[p] = D.resident ? (int)((unsigned)p | kSlotFull) : kNoSlot;
+        D.status[p] = status_of(D.alpha[p], get_C(D, D.y[p]));
+        const int r = D.pos_row[p];
+        const double xs = D.x.xsq ? D.x.xsq[r] : 0.0;
+        // dot(x,x) in feature order is exactly what xsq holds
+        D.QD[p] = kernel_from_dot(D.kp, xs, xs, xs);
+        D.G[p] = D.p[p];
+        D.G_bar[p] = 0.0;
     }
-
-    {
-        const long long max_iter = D.max_iter;
-        int counter = (l < 1000 ? l : 1000) + 1;
-        if (!scan_iup(++seq)) goto fail;
-        const int np = (c.nb + 31) >> 5;
-        // slots are never taken back when every variable has one
-        const bool evicts = D.cache.nslots < l;
-        const bool ahead = D.prefetch > 1;
-        long long passes = 0, sum_from = 0;     // phase-A passes; iterations already in the active-size sum
-        auto count_active = [&]() {
-            if (threadIdx.x == 0) sh.cnt[kCntActive] += (iter - sum_from) * c.A;
-            sum_from = iter;
-        };
-
-        while (iter < max_iter) {
-            if (--counter == 0) {
-                counter = l < 1000 ? l : 1000;
-                fold();
-                count_active();
-                if (D.shrinking) {
-                    SVMB_PROF(kProfBUpdate);
-                    if (!do_shrinking<FORM>(unshrink)) goto fail;
-                    if (!scan_iup(++seq)) goto fail;
-                    SVMB_PROF(kProfShrink);
-                }
-            }
-            int widened = 0;
-        select_again:
-            // ======================= phase A =======================
-            const int n = c.a1 - c.a0;
-            const int e0 = win_iup(np, 0), e1 = nu ? win_iup(np, 1) : 0;
-            const WinA &w0 = sh.wa[e0], &w1 = sh.wa[e1];
-            const int i0 = code_pos(w0.x[0]), i1 = nu ? code_pos(w1.x[kWordsI]) : -1;
-            const double Gmax0 = w0.d[0], Gmax1 = nu ? w1.d[kWordsI] : -SVMB_INF;
-            int slot0 = i0 >= 0 ? (int)(w0.x[2] & 0xffffu) : -1, slot1 = i1 >= 0 ? (int)(w1.x[kWordsI + 2] & 0xffffu) : -1;
-            {
-                const int need0 = slot0 == kNoSlot ? 1 : 0, need1 = slot1 == kNoSlot ? 1 : 0;
-                passes++;
-                if (evicts && threadIdx.x == 0) {
-                    if (i0 >= 0 && !need0) touch_slot(slot0);
-                    if (i1 >= 0 && !need1) touch_slot(slot1);
-                }
-                SVMB_PROF(kProfAReduce);
-                if (need0 | need1) {
-                    if (!miss_iup<FORM>(seq, e0, e1, need0, need1)) goto fail;
-                    if (need0) slot0 = sh.fslot[0];
-                    if (need1) slot1 = sh.fslot[need0];
-                }
-                SVMB_PROF(kProfAFill);
-            }
-            const float *const Qi0 = i0 >= 0 ? D.cache.data + (long long)slot0 * D.cache.stride : nullptr;
-            const float *const Qi1 = i1 >= 0 ? D.cache.data + (long long)slot1 * D.cache.stride : nullptr;
-            {
-                // second-order j scan on my chunk (svm.cpp:869-924 / :1120-1174): the
-                // largest decrease (Gmax + y G)^2 / quad, ties to the larger position.
-                // Exact divisions are long, so rough quotients (an approximate
-                // reciprocal, off by 2^-17 at most) come first and only those within
-                // 2^-15 of the warp's best are divided: about one per warp.  A
-                // quotient the estimate is not safe for (quad or the result at the
-                // ends of the exponent range, NaN) counts as infinite.
-                // A thread keeps its best rough quotient (high word + 1) with its
-                // terms, and its second best; it goes over its positions once more
-                // in the rare case that both are in reach.
-                double dec = -SVMB_INF, g2 = -SVMB_INF, g2n = -SVMB_INF;
-                int jx = -1;
-                const double QDi0 = w0.d[2], QDi1 = w1.d[kWordsI + 2];
-                const double two_yi0 = __dmul_rn(2.0, (double)code_y(w0.x[0]));
-                // numerator and denominator of position k; false: not a candidate
-                auto quotient = [&](int k, float q, double &num, double &quad) -> bool {
-                    const unsigned f = ck.F[k];
-                    const unsigned char s = flag_s(f);
-                    const bool pos = (f & kFlagPos) != 0;
-                    if (s == (pos ? ST_LOWER : ST_UPPER)) return false;
-                    const double G = ck.G[k], Gm = pos || !nu ? Gmax0 : Gmax1;
-                    const double yG = pos ? G : -G;
-                    const double grad_diff = __dadd_rn(Gm, yG);
-                    if (pos || !nu) g2 = fmax(g2, yG);
-                    else g2n = fmax(g2n, yG);
-                    if (!(grad_diff > 0)) return false;
-                    const double cross = nu ? (double)__fmul_rn(2.0f, q) : __dmul_rn(pos ? two_yi0 : -two_yi0, (double)q);
-                    quad = __dsub_rn(__dadd_rn(pos || !nu ? QDi0 : QDi1, ck.QD[k]), cross);
-                    num = __dmul_rn(grad_diff, grad_diff);
-                    if (!(quad > 0)) quad = kTau;
-                    return true;
-                };
-                auto rough = [&](double num, double quad) -> unsigned {
-                    const unsigned hq = (unsigned)__double2hiint(quad);
-                    const unsigned h = (unsigned)__double2hiint(__dmul_rn(num, rcp_rough(quad))) & 0x7fffffffu;
-                    return hq - 0x01000000u > 0x7d000000u ? 0x7ff00000u : h + 1u;
-                };
-                unsigned r1 = 0, r2 = 0;
-                int k1 = -1;
-                double num1 = 0.0, quad1 = 1.0;
-                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * kThreads) {
-                    // kScanGroup positions per thread at a time: their Q_i values are
-                    // loaded together (one L2 round trip per group, not per position)
-                    float qv[kScanGroup];
-#pragma unroll
-                    for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * kThreads;
-                        qv[u] = 0.0f;
-                        if (k < n) {
-                            const float *Qr = (nu && !(ck.F[k] & kFlagPos)) ? Qi1 : Qi0;
-                            if (Qr) qv[u] = Qr[ck.Col[k]];
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * kThreads;
-                        if (k >= n) break;
-                        double num, quad;
-                        if (!quotient(k, qv[u], num, quad)) continue;
-                        const unsigned r = rough(num, quad);
-                        if (r > r1) {
-                            r2 = r1;
-                            r1 = r;
-                            k1 = k;
-                            num1 = num;
-                            quad1 = quad;
-                        } else if (r > r2) {
-                            r2 = r;
-                        }
-                    }
-                }
-                const unsigned top = __reduce_max_sync(0xffffffffu, r1);
-                const unsigned least = top >= 0x7fe00000u || top <= 64u ? 1u : top - 64u;
-                if (r2 >= least) {
-                    for (int k = threadIdx.x; k < n; k += kThreads) {
-                        const float *Qr = (nu && !(ck.F[k] & kFlagPos)) ? Qi1 : Qi0;
-                        double num, quad;
-                        if (!quotient(k, Qr ? Qr[ck.Col[k]] : 0.0f, num, quad)) continue;
-                        if (rough(num, quad) >= least) better_max(dec, jx, __ddiv_rn(num, quad), c.a0 + k);
-                    }
-                } else if (r1 >= least) {
-                    better_max(dec, jx, __ddiv_rn(num1, quad1), c.a0 + k1);
-                }
-                if (!j_publish(++seq, nu, dec, jx, g2, g2n, Qi0, Qi1)) goto fail;
-            }
-            SVMB_PROF(kProfAScan);
-
-            // ======================= phase B =======================
-            const int eb = win_j(np);
-            const WinB &wj = sh.wb[eb];
-            const int j = code_pos(wj.x[0]);
-            {
-                double gm = sh.wb[0].d[4], gmn = nu ? sh.wb[0].d[5] : -SVMB_INF;
-                for (int k = 1; k < np; k++) {
-                    gm = fmax(gm, sh.wb[k].d[4]);
-                    if (nu) gmn = fmax(gmn, sh.wb[k].d[5]);
-                }
-                bool stop;
-                if (!nu) stop = __dadd_rn(Gmax0, gm) < D.eps;
-                else stop = fmax(__dadd_rn(Gmax0, gm), __dadd_rn(Gmax1, gmn)) < D.eps;
-                if (stop || j < 0) {
-                    if (widened) break;
-                    // reconstruct the whole gradient, widen, select again (svm.cpp:598-611)
-                    count_active();
-                    if (c.A < l) {
-                        chunk_store();
-                        if (!exchange()) goto fail;
-                        if (!reconstruct<FORM>()) goto fail;
-                        widen();
-                    }
-                    widened = 1;
-                    if (!scan_iup(++seq)) goto fail;
-                    goto select_again;
-                }
-                if (widened) counter = 1;
-            }
-            ++iter;
-            // the working pair; nu-SVC takes i from the track of y_j (svm.cpp:1179-1182)
-            const int yj = code_y(wj.x[0]);
-            const int tr = (nu && yj != +1) ? 1 : 0;
-            const WinA &wi = tr ? w1 : w0;
-            const int i = tr ? i1 : i0;
-            const int yi = tr ? -1 : code_y(w0.x[0]);
-            const double Gi = tr ? Gmax1 : (yi == +1 ? -Gmax0 : Gmax0);
-            const double alpha_i = wi.d[kWordsI * tr + 1], QDi = wi.d[kWordsI * tr + 2];
-            const int slot_i = tr ? slot1 : slot0;
-            const float Qij = __uint_as_float(wj.x[4 + tr]);
-            const double Gj = wj.d[1], alpha_j = wj.d[2], QDj = wj.d[3];
-            // Q_j row
-            int slot_j = (int)(wj.x[3] & 0xffffu);
-            {
-                const bool need = slot_j == kNoSlot;
-                if (evicts && !need && threadIdx.x == 0) touch_slot(slot_j);
-                SVMB_PROF(kProfBReduce);
-                if (need) {
-                    if (!miss_j<FORM>(eb, slot0, slot1)) goto fail;
-                    slot_j = sh.fslot[0];
-                }
-            }
-            // two-variable analytic step (svm.cpp:636-721), identical in every block
-            const double C_i = get_C(D, yi), C_j = get_C(D, yj);
-            double ai = alpha_i, aj = alpha_j;
-            if (yi != yj) {
-                double quad_coef = __dadd_rn(__dadd_rn(QDi, QDj), (double)__fmul_rn(2.0f, Qij));
-                if (quad_coef <= 0) quad_coef = kTau;
-                const double delta = __ddiv_rn(__dsub_rn(-Gi, Gj), quad_coef);
-                const double diff = __dsub_rn(ai, aj);
-                ai = __dadd_rn(ai, delta);
-                aj = __dadd_rn(aj, delta);
-                if (diff > 0) {
-                    if (aj < 0) { aj = 0; ai = diff; }
-                } else {
-                    if (ai < 0) { ai = 0; aj = -diff; }
-                }
-                if (diff > __dsub_rn(C_i, C_j)) {
-                    if (ai > C_i) { ai = C_i; aj = __dsub_rn(C_i, diff); }
-                } else {
-                    if (aj > C_j) { aj = C_j; ai = __dadd_rn(C_j, diff); }
-                }
-            } else {
-                double quad_coef = __dsub_rn(__dadd_rn(QDi, QDj), (double)__fmul_rn(2.0f, Qij));
-                if (quad_coef <= 0) quad_coef = kTau;
-                const double delta = __ddiv_rn(__dsub_rn(Gi, Gj), quad_coef);
-                const double sum = __dadd_rn(ai, aj);
-                ai = __dsub_rn(ai, delta);
-                aj = __dadd_rn(aj, delta);
-                if (sum > C_i) {
-                    if (ai > C_i) { ai = C_i; aj = __dsub_rn(sum, C_i); }
-                } else {
-                    if (aj < 0) { aj = 0; ai = sum; }
-                }
-                if (sum > C_j) {
-                    if (aj > C_j) { aj = C_j; ai = __dsub_rn(sum, C_j); }
-                } else {
-                    if (ai < 0) { ai = 0; aj = sum; }
-                }
-            }
-            const double dai = __dsub_rn(ai, alpha_i);
-            const double daj = __dsub_rn(aj, alpha_j);
-            const unsigned char old_si = status_of(alpha_i, C_i), old_sj = status_of(alpha_j, C_j);
-            const unsigned char new_si = status_of(ai, C_i), new_sj = status_of(aj, C_j);
-            const bool bar_i = !D.lazy_gbar && (old_si == ST_UPPER) != (new_si == ST_UPPER);
-            const bool bar_j = !D.lazy_gbar && (old_sj == ST_UPPER) != (new_sj == ST_UPPER);
-            // complete rows for the G_bar update: fill the tail [A,l) where missing
-            if ((bar_i || bar_j) && c.A < l) {
-                const bool ti = bar_i && !(wi.x[kWordsI * tr + 2] & kSlotFull), tj = bar_j && !(wj.x[3] & kSlotFull);
-                const int ns = (ti ? 1 : 0) + (tj ? 1 : 0);
-                __syncthreads();    // the last fill's list is no longer read
-                if (threadIdx.x == 0) {
-                    if (ti) {
-                        sh.frow[0] = (int)wi.x[kWordsI * tr + 3];
-                        sh.fy[0] = yi;
-                        sh.fslot[0] = slot_i;
-                    }
-                    if (tj) {
-                        sh.frow[ns - 1] = (int)wj.x[2];
-                        sh.fy[ns - 1] = yj;
-                        sh.fslot[ns - 1] = slot_j;
-                    }
-                    sh.cnt[kCntQ] += (long long)ns * (l - c.A);
-                    sh.cnt[kCntTargets] += l - c.A;
-                }
-                __syncthreads();
-                if (!fill<FORM>(ns, 1)) goto fail;
-                const int ki = i - c.a0, kj = j - c.a0;
-                if (ti && i >= c.a0 && i < c.a1 && (ki & (kThreads - 1)) == (int)threadIdx.x) ck.F[ki] |= kFlagFull;
-                if (tj && j >= c.a0 && j < c.a1 && (kj & (kThreads - 1)) == (int)threadIdx.x) ck.F[kj] |= kFlagFull;
-            }
-            SVMB_PROF(kProfBFill);
-            // the owners of i and j take their new alpha and status (a position is
-            // read and written by its own thread only until the next barrier)
-            {
-                auto take = [&](int p, double a, unsigned char st) {
-                    const int k = p - c.a0;
-                    if (k < 0 || k >= n || (k & (kThreads - 1)) != (int)threadIdx.x) return;
-                    const unsigned f = ck.F[k];
-                    if (f & kFlagAhead) atomicAdd(&sh.ahead_used, 1u);
-                    ck.A[k] = a;
-                    ck.F[k] = (unsigned char)((f & ~((3u << kFlagStatus) | kFlagAhead)) | ((unsigned)st << kFlagStatus));
-                };
-                take(i, ai, new_si);
-                take(j, aj, new_sj);
-            }
-            // G update on my chunk (svm.cpp:732-735) + G_bar (svm.cpp:744-769) + next I_up scan
-            {
-                const float *Qi = D.cache.data + (long long)slot_i * D.cache.stride;
-                const float *Qj = D.cache.data + (long long)slot_j * D.cache.stride;
-                double v[2] = {-SVMB_INF, -SVMB_INF};
-                int ix[2] = {-1, -1};
-                double pv = -SVMB_INF;
-                int pix = -1;
-                // kScanGroup positions per thread at a time, their Q_i and Q_j
-                // values loaded together before any is used
-                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * kThreads) {
-                    float qi[kScanGroup], qj[kScanGroup];
-#pragma unroll
-                    for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * kThreads;
-                        qi[u] = 0.0f;
-                        qj[u] = 0.0f;
-                        if (k < n) {
-                            const int col = ck.Col[k];
-                            qi[u] = Qi[col];
-                            qj[u] = Qj[col];
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * kThreads;
-                        if (k >= n) continue;
-                        const double G = __dadd_rn(ck.G[k], __dadd_rn(__dmul_rn((double)qi[u], dai), __dmul_rn((double)qj[u], daj)));
-                        ck.G[k] = G;
-                        const unsigned f = ck.F[k];
-                        const unsigned char s = flag_s(f);
-                        const bool pos = (f & kFlagPos) != 0;
-                        const bool up = s != (pos ? ST_UPPER : ST_LOWER);
-                        const double yG = pos ? -G : G;
-                        if (up) {
-                            if (pos || !nu) better_max(v[0], ix[0], yG, c.a0 + k);
-                            else better_max(v[1], ix[1], yG, c.a0 + k);
-                        }
-                        if (ahead) better_max(pv, pix, s == ST_FREE ? fabs(G) : (up ? yG : -yG), c.a0 + k);
-                    }
-                }
-                if (bar_i || bar_j) {
-                    auto bar = [&](double g, int col) {
-                        if (bar_i) { const double q = (double)Qi[col]; g = (old_si == ST_UPPER) ? __dsub_rn(g, __dmul_rn(C_i, q)) : __dadd_rn(g, __dmul_rn(C_i, q)); }
-                        if (bar_j) { const double q = (double)Qj[col]; g = (old_sj == ST_UPPER) ? __dsub_rn(g, __dmul_rn(C_j, q)) : __dadd_rn(g, __dmul_rn(C_j, q)); }
-                        return g;
-                    };
-                    for (int k = threadIdx.x; k < n; k += kThreads) D.G_bar[c.a0 + k] = bar(D.G_bar[c.a0 + k], ck.Col[k]);
-                    for (int p = c.t0 + threadIdx.x; p < c.t1; p += kThreads) D.G_bar[p] = bar(D.G_bar[p], D.pos_local[p]);
-                }
-                if (!iup_publish(++seq, nu, ahead, v, ix, pv, pix)) goto fail;
-            }
-            SVMB_PROF(kProfBUpdate);
-        }
-
-        count_active();
-        fold();
-        if (threadIdx.x == 0) sh.cnt[kCntLook] = passes * (nu ? 2 : 1) + iter;
-        chunk_store();
-        if (!exchange()) goto fail;
-        if (iter >= max_iter) {
-            status = 1;
-            if (c.A < l) {
-                if (!reconstruct<FORM>()) goto fail;
-                set_active(l);
-            }
-        }
+    if (!exchange()) return false;
+    // a resident matrix whose evaluation gave up leaves the group's error flag
+    if (__syncthreads_or(D.resident && ld_relaxed_i32(&D.sync->error))) return false;
+    int any = 0;
+    for (int p = threadIdx.x; p < l; p += blockDim.x) any |= D.alpha[p] > 0 ? 1 : 0;
+    any = __syncthreads_or(any);
+    if (any) {
+        if (!accumulate<FORM>(l, 0, D.lazy_gbar ? 0 : 1, c.a0, c.a1)) return false;
+        if (!exchange()) return false;
     }
-    // ---- rho (svm.cpp:1013-1049 / 1260-1308), objective (:795-802), alpha out (:805-808) ----
+    chunk_load();
+    return true;
+}
+
+// rho (svm.cpp:1013-1049 / 1260-1308), objective (:795-802), alpha out (:805-808)
+__device__ __noinline__ void finish_solve(int nu, long long iter, int status, int unshrink)
+{
+    Shared &sh = block_shared();
+    const InstanceDesc &D = sh.D;
+    Ctx &c = sh.c;
+    const int l = D.l, rank = c.rank;
     // The sums run sequentially in position order (bit-exact with the reference), on block 0.
     if (rank == 0) {
         // the staging area is no longer needed
@@ -2947,8 +2782,15 @@ __device__ void solve_instance(int rank)
         const int lo = (int)((long long)l * rank / c.nb), hi = (int)((long long)l * (rank + 1) / c.nb);
         for (int p = lo + threadIdx.x; p < hi; p += blockDim.x) D.alpha_local[D.pos_local[p]] = D.alpha[p];
     }
-    return;
-fail:
+}
+
+// a wait ran out: the group's error
+__device__ __noinline__ void fail_solve(long long iter, int unshrink)
+{
+    Shared &sh = block_shared();
+    const InstanceDesc &D = sh.D;
+    Ctx &c = sh.c;
+    const int rank = c.rank;
     if (threadIdx.x == 0 && rank == 0) {
         SolveOut o;
         o.iters = iter; o.rho = 0; o.obj = 0; o.r = 0; o.status = -1; o.active_size = c.A;
@@ -2956,6 +2798,319 @@ fail:
         put_counters(o);
         *D.out = o;
     }
+}
+
+// NU: Solver_NU (two tracks) or Solver
+template <int FORM, bool NU>
+__device__ __noinline__ void solve_instance(int rank)
+{
+    Shared &sh = block_shared();
+    const InstanceDesc &D = sh.D;
+    Ctx &c = sh.c;
+    if (!start_solve<FORM>(rank)) {
+        fail_solve(0, 0);
+        return;
+    }
+    const int l = D.l;
+    constexpr int nu = NU ? 1 : 0;
+    const Chunk ck = chunk_at(c.choff, D.chunk_cap);
+    unsigned seq = 0;       // sequence number of the last record exchange
+    long long iter = 0;
+    int unshrink = 0;
+    int status = 0;
+    // section timers of thread 0: the loop adds 32-bit cycle counts (an add that
+    // waits for nothing) and folds them every 1000 iterations
+    unsigned tmark = (unsigned)clock();
+#define SVMB_PROF(k)                                   \
+    do {                                               \
+        if (threadIdx.x == 0) {                        \
+            const unsigned now_ = (unsigned)clock();   \
+            atomicAdd(&sh.prof32[k], now_ - tmark);    \
+            tmark = now_;                              \
+        }                                              \
+    } while (0)
+    auto fold = [&]() {
+        if (threadIdx.x == 0)
+            for (int k = 0; k < 8; k++) {
+                sh.prof[k] += sh.prof32[k];
+                sh.prof32[k] = 0;
+            }
+    };
+    {
+        const long long max_iter = D.max_iter;
+        int counter = (l < 1000 ? l : 1000) + 1;
+        if (!scan_iup<nu>(++seq)) goto fail;
+        const int np = (c.nb + 31) >> 5;
+        // slots are never taken back when every variable has one
+        const bool evicts = D.cache.nslots < l;
+        const bool ahead = D.prefetch > 1;
+        long long passes = 0, sum_from = 0;     // phase-A passes; iterations already in the active-size sum
+        auto count_active = [&]() {
+            if (threadIdx.x == 0) sh.cnt[kCntActive] += (iter - sum_from) * c.A;
+            sum_from = iter;
+        };
+
+        while (iter < max_iter) {
+            if (--counter == 0) {
+                counter = l < 1000 ? l : 1000;
+                fold();
+                count_active();
+                if (D.shrinking) {
+                    SVMB_PROF(kProfBUpdate);
+                    if (!do_shrinking<FORM>(unshrink)) goto fail;
+                    if (!scan_iup<nu>(++seq)) goto fail;
+                    SVMB_PROF(kProfShrink);
+                }
+            }
+            int widened = 0;
+        select_again:
+            // ======================= phase A =======================
+            const int n = c.a1 - c.a0;
+            const int e0 = np > 1 ? win_iup(np, 0) : 0, e1 = nu && np > 1 ? win_iup(np, 1) : 0;
+            const WinA &w0 = sh.wa[e0], &w1 = sh.wa[e1];
+            const int i0 = code_pos(w0.x[0]), i1 = nu ? code_pos(w1.x[kWordsI]) : -1;
+            const double Gmax0 = w0.d[0], Gmax1 = nu ? w1.d[kWordsI] : -SVMB_INF;
+            int slot0 = i0 >= 0 ? (int)(w0.x[2] & 0xffffu) : -1, slot1 = i1 >= 0 ? (int)(w1.x[kWordsI + 2] & 0xffffu) : -1;
+            {
+                const int need0 = slot0 == kNoSlot ? 1 : 0, need1 = slot1 == kNoSlot ? 1 : 0;
+                passes++;
+                if (evicts && threadIdx.x == 0) {
+                    if (i0 >= 0 && !need0) touch_slot(slot0);
+                    if (i1 >= 0 && !need1) touch_slot(slot1);
+                }
+                SVMB_PROF(kProfAReduce);
+                if (need0 | need1) {
+                    if (!miss_iup<FORM>(seq, e0, e1, need0, need1)) goto fail;
+                    if (need0) slot0 = sh.fslot[0];
+                    if (need1) slot1 = sh.fslot[need0];
+                }
+                SVMB_PROF(kProfAFill);
+            }
+            const float *const Qi0 = i0 >= 0 ? D.cache.data + (long long)slot0 * D.cache.stride : nullptr;
+            const float *const Qi1 = i1 >= 0 ? D.cache.data + (long long)slot1 * D.cache.stride : nullptr;
+            {
+                // second-order j scan on my chunk (svm.cpp:869-924 / :1120-1174): the
+                // largest decrease (Gmax + y G)^2 / quad, ties to the larger position.
+                // Exact divisions are long, so rough quotients (an approximate
+                // reciprocal, off by 2^-17 at most) come first and only those within
+                // 2^-15 of the warp's best are divided: about one per warp.  A
+                // quotient the estimate is not safe for (quad or the result at the
+                // ends of the exponent range, NaN) counts as infinite.
+                // A thread keeps its best rough quotient (high word + 1) with its
+                // terms, and its second best; it goes over its positions once more
+                // in the rare case that both are in reach.
+                double dec = -SVMB_INF, g2 = -SVMB_INF, g2n = -SVMB_INF;
+                int jx = -1;
+                const double QDi0 = w0.d[2], QDi1 = w1.d[kWordsI + 2];
+                const double two_yi0 = __dmul_rn(2.0, (double)code_y(w0.x[0]));
+                // numerator and denominator of position k; false: not a candidate
+                auto quotient = [&](int k, float q, double &num, double &quad) -> bool {
+                    const unsigned f = ck.F[k];
+                    const unsigned char s = flag_s(f);
+                    const bool pos = (f & kFlagPos) != 0;
+                    if (s == (pos ? ST_LOWER : ST_UPPER)) return false;
+                    const double G = ck.G[k], Gm = pos || !nu ? Gmax0 : Gmax1;
+                    const double yG = pos ? G : -G;
+                    const double grad_diff = __dadd_rn(Gm, yG);
+                    if (pos || !nu) g2 = fmax(g2, yG);
+                    else g2n = fmax(g2n, yG);
+                    if (!(grad_diff > 0)) return false;
+                    const double cross = nu ? (double)__fmul_rn(2.0f, q) : __dmul_rn(pos ? two_yi0 : -two_yi0, (double)q);
+                    quad = __dsub_rn(__dadd_rn(pos || !nu ? QDi0 : QDi1, ck.QD[k]), cross);
+                    num = __dmul_rn(grad_diff, grad_diff);
+                    if (!(quad > 0)) quad = kTau;
+                    return true;
+                };
+                unsigned r1 = 0, r2 = 0;
+                int k1 = -1;
+                double num1 = 0.0, quad1 = 1.0;
+                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * kThreads) {
+                    // kScanGroup positions per thread at a time: their Q_i values are
+                    // loaded together (one L2 round trip per group, not per position)
+                    float qv[kScanGroup];
+#pragma unroll
+                    for (int u = 0; u < kScanGroup; u++) {
+                        const int k = k0 + u * kThreads;
+                        qv[u] = 0.0f;
+                        if (k < n) {
+                            const float *Qr = (nu && !(ck.F[k] & kFlagPos)) ? Qi1 : Qi0;
+                            if (Qr) qv[u] = Qr[ck.Col[k]];
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < kScanGroup; u++) {
+                        const int k = k0 + u * kThreads;
+                        if (k >= n) break;
+                        double num, quad;
+                        if (!quotient(k, qv[u], num, quad)) continue;
+                        const unsigned r = rough_quotient(num, quad);
+                        if (r > r1) {
+                            r2 = r1;
+                            r1 = r;
+                            k1 = k;
+                            num1 = num;
+                            quad1 = quad;
+                        } else if (r > r2) {
+                            r2 = r;
+                        }
+                    }
+                }
+                const unsigned least = rough_least(__reduce_max_sync(0xffffffffu, r1));
+                if (r2 >= least) {
+                    for (int k = threadIdx.x; k < n; k += kThreads) {
+                        const float *Qr = (nu && !(ck.F[k] & kFlagPos)) ? Qi1 : Qi0;
+                        double num, quad;
+                        if (!quotient(k, Qr ? Qr[ck.Col[k]] : 0.0f, num, quad)) continue;
+                        if (rough_quotient(num, quad) >= least) better_max(dec, jx, __ddiv_rn(num, quad), c.a0 + k);
+                    }
+                } else if (r1 >= least) {
+                    better_max(dec, jx, __ddiv_rn(num1, quad1), c.a0 + k1);
+                }
+                if (!j_publish<nu>(++seq, dec, jx, g2, g2n, Qi0, Qi1)) goto fail;
+            }
+            SVMB_PROF(kProfAScan);
+
+            // ======================= phase B =======================
+            const int eb = np > 1 ? win_j(np) : 0;
+            const WinB &wj = sh.wb[eb];
+            const int j = code_pos(wj.x[0]);
+            {
+                double gm = sh.wb[0].d[4], gmn = nu ? sh.wb[0].d[5] : -SVMB_INF;
+                for (int k = 1; k < np; k++) {
+                    gm = fmax(gm, sh.wb[k].d[4]);
+                    if (nu) gmn = fmax(gmn, sh.wb[k].d[5]);
+                }
+                bool stop;
+                if (!nu) stop = __dadd_rn(Gmax0, gm) < D.eps;
+                else stop = fmax(__dadd_rn(Gmax0, gm), __dadd_rn(Gmax1, gmn)) < D.eps;
+                if (stop || j < 0) {
+                    if (widened) break;
+                    // reconstruct the whole gradient, widen, select again (svm.cpp:598-611)
+                    count_active();
+                    if (c.A < l && !reopen<FORM>()) goto fail;
+                    widened = 1;
+                    if (!scan_iup<nu>(++seq)) goto fail;
+                    goto select_again;
+                }
+                if (widened) counter = 1;
+            }
+            ++iter;
+            // the working pair; nu-SVC takes i from the track of y_j (svm.cpp:1179-1182)
+            const int yj = code_y(wj.x[0]);
+            const int tr = (nu && yj != +1) ? 1 : 0;
+            const WinA &wi = tr ? w1 : w0;
+            const int i = tr ? i1 : i0;
+            const int yi = tr ? -1 : code_y(w0.x[0]);
+            const double Gi = tr ? Gmax1 : (yi == +1 ? -Gmax0 : Gmax0);
+            const double alpha_i = wi.d[kWordsI * tr + 1], QDi = wi.d[kWordsI * tr + 2];
+            const int slot_i = tr ? slot1 : slot0;
+            const float Qij = __uint_as_float(wj.x[4 + tr]);
+            const double Gj = wj.d[1], alpha_j = wj.d[2], QDj = wj.d[3];
+            // Q_j row
+            int slot_j = (int)(wj.x[3] & 0xffffu);
+            {
+                const bool need = slot_j == kNoSlot;
+                if (evicts && !need && threadIdx.x == 0) touch_slot(slot_j);
+                SVMB_PROF(kProfBReduce);
+                if (need) {
+                    if (!miss_j<FORM>(eb, slot0, slot1)) goto fail;
+                    slot_j = sh.fslot[0];
+                }
+            }
+            // identical in every block
+            const double C_i = get_C(D, yi), C_j = get_C(D, yj);
+            double ai = alpha_i, aj = alpha_j;
+            pair_step(yi, yj, QDi, QDj, Qij, Gi, Gj, C_i, C_j, ai, aj);
+            const double dai = __dsub_rn(ai, alpha_i);
+            const double daj = __dsub_rn(aj, alpha_j);
+            const unsigned char old_si = status_of(alpha_i, C_i), old_sj = status_of(alpha_j, C_j);
+            const unsigned char new_si = status_of(ai, C_i), new_sj = status_of(aj, C_j);
+            const bool bar_i = !D.lazy_gbar && (old_si == ST_UPPER) != (new_si == ST_UPPER);
+            const bool bar_j = !D.lazy_gbar && (old_sj == ST_UPPER) != (new_sj == ST_UPPER);
+            // complete rows for the G_bar update: fill the tail [A,l) where missing
+            if ((bar_i || bar_j) && c.A < l) {
+                const bool ti = bar_i && !(wi.x[kWordsI * tr + 2] & kSlotFull), tj = bar_j && !(wj.x[3] & kSlotFull);
+                if (!fill_tail<FORM>(ti, tj, i, yi, (int)wi.x[kWordsI * tr + 3], slot_i, j, yj, (int)wj.x[2], slot_j)) goto fail;
+            }
+            SVMB_PROF(kProfBFill);
+            // the owners of i and j take their new alpha and status (a position is
+            // read and written by its own thread only until the next barrier)
+            {
+                auto take = [&](int p, double a, unsigned char st) {
+                    const int k = p - c.a0;
+                    if (k < 0 || k >= n || (k & (kThreads - 1)) != (int)threadIdx.x) return;
+                    const unsigned f = ck.F[k];
+                    if (f & kFlagAhead) atomicAdd(&sh.ahead_used, 1u);
+                    ck.A[k] = a;
+                    ck.F[k] = (unsigned char)((f & ~((3u << kFlagStatus) | kFlagAhead)) | ((unsigned)st << kFlagStatus));
+                };
+                take(i, ai, new_si);
+                take(j, aj, new_sj);
+            }
+            // G update on my chunk (svm.cpp:732-735) + G_bar (svm.cpp:744-769) + next I_up scan
+            {
+                const float *Qi = D.cache.data + (long long)slot_i * D.cache.stride;
+                const float *Qj = D.cache.data + (long long)slot_j * D.cache.stride;
+                double v[2] = {-SVMB_INF, -SVMB_INF};
+                int ix[2] = {-1, -1};
+                double pv = -SVMB_INF;
+                int pix = -1;
+                // kScanGroup positions per thread at a time, their Q_i and Q_j
+                // values loaded together before any is used
+                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * kThreads) {
+                    float qi[kScanGroup], qj[kScanGroup];
+#pragma unroll
+                    for (int u = 0; u < kScanGroup; u++) {
+                        const int k = k0 + u * kThreads;
+                        qi[u] = 0.0f;
+                        qj[u] = 0.0f;
+                        if (k < n) {
+                            const int col = ck.Col[k];
+                            qi[u] = Qi[col];
+                            qj[u] = Qj[col];
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < kScanGroup; u++) {
+                        const int k = k0 + u * kThreads;
+                        if (k >= n) continue;
+                        const double G = __dadd_rn(ck.G[k], __dadd_rn(__dmul_rn((double)qi[u], dai), __dmul_rn((double)qj[u], daj)));
+                        ck.G[k] = G;
+                        const unsigned f = ck.F[k];
+                        const unsigned char s = flag_s(f);
+                        const bool pos = (f & kFlagPos) != 0;
+                        const bool up = s != (pos ? ST_UPPER : ST_LOWER);
+                        const double yG = pos ? -G : G;
+                        if (up) {
+                            if (pos || !nu) better_max(v[0], ix[0], yG, c.a0 + k);
+                            else better_max(v[1], ix[1], yG, c.a0 + k);
+                        }
+                        if (ahead) better_max(pv, pix, s == ST_FREE ? fabs(G) : (up ? yG : -yG), c.a0 + k);
+                    }
+                }
+                if (bar_i || bar_j) update_gbar(Qi, bar_i, old_si == ST_UPPER, C_i, Qj, bar_j, old_sj == ST_UPPER, C_j);
+                if (!iup_publish<nu>(++seq, ahead, v, ix, pv, pix)) goto fail;
+            }
+            SVMB_PROF(kProfBUpdate);
+        }
+
+        count_active();
+        fold();
+        if (threadIdx.x == 0) sh.cnt[kCntLook] = passes * (nu ? 2 : 1) + iter;
+        chunk_store();
+        if (!exchange()) goto fail;
+        if (iter >= max_iter) {
+            status = 1;
+            if (c.A < l) {
+                if (!reconstruct<FORM>()) goto fail;
+                set_active(l);
+            }
+        }
+    }
+    finish_solve(nu, iter, status, unshrink);
+    return;
+fail:
+    fail_solve(iter, unshrink);
 #undef SVMB_PROF
 }
 
@@ -3010,7 +3165,8 @@ smo_persistent(const InstanceDesc *__restrict__ insts, const int *__restrict__ b
         __syncthreads();
         tc::tc_fence_after();
     }
-    solve_instance<FORM>(rank);
+    if (D.nu) solve_instance<FORM, true>(rank);
+    else solve_instance<FORM, false>(rank);
     signal_done(D);
     if constexpr (is_tc_form(FORM)) {
         tc::tc_fence_before();
