@@ -10,8 +10,8 @@
 // The file is compiled with -fmad=false.
 //
 // Kernel values are kept SV-major, kv[s][t] for the t-th test row of a chunk,
-// so that the pair sums (one thread per test row and pair, each walking the
-// SVs in model order) read consecutive words across a warp.  Dense rows take
+// so that the pair sums (each in model order over the two classes' SVs)
+// read consecutive words across a warp.  Dense rows take
 // a tiled kernel: a block computes 64 test rows x 64 SVs, 16 features at a
 // time staged in shared memory, 4 x 4 values per thread.  With a
 // tensor-core predict form the values come from the split-product kernel
@@ -210,31 +210,205 @@ __global__ void kvalue_csr(KP kp, Rows T, Rows S, double *__restrict__ out)
     }
 }
 
-// one thread per (test row, pair): sequential sums in model order (svm.cpp:2606-2631)
-__global__ void pair_sums(const double *__restrict__ kv, int nt, int ns, int nr_class, const int *__restrict__ start,
-                          const int *__restrict__ nsv, const double *__restrict__ coef, const double *__restrict__ rho,
-                          double *__restrict__ dec)
+// Pair sums, each sequential over the two classes' SVs in model order
+// (svm.cpp:2606-2631).  A sum is one chain of dependent additions, so a thread
+// that also fetches and multiplies each term waits out a memory round trip per
+// few terms (a single row against 1,500 SVs: 125 us); and with a thread per
+// row and pair every kernel value is read once per pair its class is in (9 times
+// with 10 classes: 3.6 ms for 6,000 rows x 20,000 SVs).  Two kernels:
+//   few sums   a block per (row, pair): all threads form the products of the
+//              next piece in shared memory while one adds up the previous one;
+//   many rows  a thread per row walks all SVs once and keeps every pair's sum:
+//              classes come in order, so a pair's first class is added before its
+//              second, as the reference does.
+constexpr int kPiece = 1024;     // products per piece of a sum
+
+__device__ __forceinline__ void pair_classes(int p, int nr_class, int &i, int &j)
 {
+    i = 0;
+    int rem = p;
+    while (rem >= nr_class - 1 - i) { rem -= nr_class - 1 - i; ++i; }
+    j = i + 1 + rem;
+}
+
+__global__ void __launch_bounds__(256) pair_sums_few(const double *__restrict__ kv, int nt, int ns, int nr_class,
+                                                     const int *__restrict__ start, const int *__restrict__ nsv,
+                                                     const double *__restrict__ coef, const double *__restrict__ rho,
+                                                     double *__restrict__ dec)
+{
+    __shared__ __align__(16) double prod[2][kPiece];
     const int npair = nr_class * (nr_class - 1) / 2;
     const long long total = (long long)nt * npair;
-    for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < total; id += (long long)gridDim.x * blockDim.x) {
-        // consecutive threads on consecutive test rows of one pair
-        const int p = (int)(id / nt);
-        const int t = (int)(id % nt);
-        // pair index -> (i,j)
-        int i = 0, rem = p;
-        while (rem >= nr_class - 1 - i) { rem -= nr_class - 1 - i; ++i; }
-        const int j = i + 1 + rem;
-        const double *k = kv + t;                // kv[s][t]: SV s of test row t at s * nt
-        const double *coef1 = coef + (long long)(j - 1) * ns;
-        const double *coef2 = coef + (long long)i * ns;
+    for (long long id = blockIdx.x; id < total; id += gridDim.x) {
+        const int p = (int)(id / nt), t = (int)(id % nt);
+        int i, j;
+        pair_classes(p, nr_class, i, j);
+        const double *coef1 = coef + (long long)(j - 1) * ns, *coef2 = coef + (long long)i * ns;
+        const int ni = nsv[i], n = ni + nsv[j], s1 = start[i], s2 = start[j] - ni;
+        const int pieces = (n + kPiece - 1) / kPiece;
         double sum = 0;
-        for (int q = 0; q < nsv[i]; q++)
-            sum = __dadd_rn(sum, __dmul_rn(coef1[start[i] + q], k[(long long)(start[i] + q) * nt]));
-        for (int q = 0; q < nsv[j]; q++)
-            sum = __dadd_rn(sum, __dmul_rn(coef2[start[j] + q], k[(long long)(start[j] + q) * nt]));
-        dec[(long long)t * npair + p] = __dsub_rn(sum, rho[p]);
+        // threads 32.. form piece q + 1 while thread 0 adds piece q
+        auto form = [&](int q, int from, int step) {
+            const int hi = min(n, (q + 1) * kPiece);
+            for (int e = q * kPiece + from; e < hi; e += step) {
+                const bool one = e < ni;
+                const int s = e + (one ? s1 : s2);
+                prod[q & 1][e - q * kPiece] = __dmul_rn(one ? coef1[s] : coef2[s], kv[(long long)s * nt + t]);
+            }
+        };
+        form(0, threadIdx.x, blockDim.x);
+        __syncthreads();
+        for (int q = 0; q < pieces; q++) {
+            if (threadIdx.x >= 32) {
+                if (q + 1 < pieces) form(q + 1, threadIdx.x - 32, blockDim.x - 32);
+            } else if (threadIdx.x == 0) {
+                const double *v = prod[q & 1];
+                const int m = min(kPiece, n - q * kPiece);
+                int e = 0;
+                for (; e + 16 <= m; e += 16) {
+                    double2 w[8];
+#pragma unroll
+                    for (int u = 0; u < 8; u++) w[u] = reinterpret_cast<const double2 *>(v + e)[u];
+#pragma unroll
+                    for (int u = 0; u < 8; u++) sum = __dadd_rn(__dadd_rn(sum, w[u].x), w[u].y);
+                }
+                for (; e < m; e++) sum = __dadd_rn(sum, v[e]);
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) dec[(long long)t * npair + p] = __dsub_rn(sum, rho[p]);
+        __syncthreads();
     }
+}
+
+constexpr int kSumRows = 64;     // test rows per block
+constexpr int kSumGroups = 4;    // threads per row, each with a share of a class's partners
+constexpr int kSumSv = 32;       // SVs per staged tile
+constexpr int kSumStages = 5;
+constexpr int kSumMost = 3;      // partners per thread and walk, at most
+constexpr int kSumStage = kSumSv * (kSumRows + kSumGroups * kSumMost);       // doubles per stage
+constexpr int kSumSmem = kSumStages * kSumStage * 8;
+
+__device__ __forceinline__ void cp_async8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// N: partners per thread (a class of k has k - 1; its SVs are walked again when
+// they are more than kSumGroups * kSumMost).  Bound by HBM: the
+// kernel values come from there once, four staged tiles ahead (8-byte copies: an odd
+// number of rows leaves no wider alignment).  With plain loads, eight ahead
+// per thread, 6,000 rows x 20,000 SVs x 10 classes took 4.5 ms.
+template <int N>
+__global__ void __launch_bounds__(kSumRows *kSumGroups) pair_sums_many(const double *__restrict__ kv, int nt, int ns,
+                                                                        int nr_class, const int *__restrict__ start,
+                                                                        const int *__restrict__ nsv,
+                                                                        const double *__restrict__ coef,
+                                                                        const double *__restrict__ rho,
+                                                                        double *__restrict__ dec)
+{
+    extern __shared__ __align__(16) double stages[];
+    const int npair = nr_class * (nr_class - 1) / 2;
+    const int tid = threadIdx.x, row = tid % kSumRows, grp = tid / kSumRows;
+    const int t0 = blockIdx.x * kSumRows, t = t0 + row;
+    const bool in = t < nt;
+    double *const mine = dec + (long long)(in ? t : 0) * npair;     // the row's running sums, one per pair
+    // the tile the next copies take: class lc, partners from lr, SVs from ls
+    int lc = 0, lr = 0, ls = 0;
+    auto next_class = [&]() {
+        while (lc < nr_class && nsv[lc] == 0) lc++;
+        lr = 0;
+        if (lc < nr_class) ls = start[lc];
+    };
+    next_class();
+    int to = 0, from = 0;       // stages to copy into / to use
+    auto copy = [&]() {
+        if (lc < nr_class) {
+            double *const kt = stages + to * kSumStage, *const ct = kt + kSumSv * kSumRows;
+            const int end = start[lc] + nsv[lc];
+            for (int e = tid; e < kSumSv * kSumRows; e += kSumRows * kSumGroups) {
+                const int s = ls + e / kSumRows, tt = t0 + e % kSumRows;
+                if (s < end && tt < nt) cp_async8(kt + e, kv + (long long)s * nt + tt);
+            }
+            for (int e = tid; e < kSumSv * kSumGroups * N; e += kSumRows * kSumGroups) {
+                const int r = lr + e / kSumSv, s = ls + e % kSumSv;
+                if (s < end && r < nr_class - 1) cp_async8(ct + e, coef + (long long)r * ns + s);
+            }
+            ls += kSumSv;
+            if (ls >= end) {
+                lr += kSumGroups * N;
+                ls = start[lc];
+                if (lr >= nr_class - 1) {
+                    lc++;
+                    next_class();
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        to = to + 1 == kSumStages ? 0 : to + 1;
+    };
+    for (int q = 0; q < kSumStages - 1; q++) copy();
+    for (int c = 0; c < nr_class; c++) {
+        const int end = start[c] + nsv[c];
+        for (int r0 = 0; r0 < nr_class - 1; r0 += kSumGroups * N) {
+            // partner r of class c is class r (r < c) or r + 1, its coefficients row r of coef
+            double sum[N];
+            int pair[N];
+            bool second[N];
+#pragma unroll
+            for (int u = 0; u < N; u++) {
+                const int r = r0 + grp * N + u, o = r < c ? r : r + 1, i = min(c, o), j = max(c, o);
+                pair[u] = r < nr_class - 1 && in ? i * (nr_class - 1) - i * (i - 1) / 2 + j - i - 1 : -1;
+                second[u] = o < c;
+                sum[u] = pair[u] >= 0 && second[u] ? mine[pair[u]] : 0.0;
+            }
+            for (int sb = start[c]; sb < end; sb += kSumSv) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kSumStages - 2) : "memory");
+                __syncthreads();        // the tile has landed, and everyone is done with the one before
+                copy();
+                const double *const kt = stages + from * kSumStage + row;
+                const double *const ct = stages + from * kSumStage + kSumSv * kSumRows + grp * N * kSumSv;
+                const int m = min(kSumSv, end - sb);
+#pragma unroll 4
+                for (int e = 0; e < m; e++) {
+                    const double k = kt[e * kSumRows];
+#pragma unroll
+                    for (int u = 0; u < N; u++) sum[u] = __dadd_rn(sum[u], __dmul_rn(ct[u * kSumSv + e], k));
+                }
+                from = from + 1 == kSumStages ? 0 : from + 1;
+            }
+#pragma unroll
+            for (int u = 0; u < N; u++)     // a pair is complete after its second class
+                if (pair[u] >= 0) mine[pair[u]] = second[u] ? __dsub_rn(sum[u], rho[pair[u]]) : sum[u];
+        }
+        __syncthreads();        // another thread of the row may hold the pair next
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// The kernel for nt rows: the estimated time of both, in additions of one
+// chain (about 10 cycles).  Few: the sums go round the GPU's block places (8
+// per SM), each the length of its pair.  Many: a block of 64 rows takes about 30
+// cycles per SV.  One row, 1,500 SVs, 2 classes: few.  6,000 rows, 20,000
+// SVs, 10 classes: many.
+cudaError_t launch_pair_sums(const double *kv, int nt, int ns, int nr_class, const int *start, const int *nsv,
+                             const double *coef, const double *rho, double *dec)
+{
+    const double npair = 0.5 * nr_class * (nr_class - 1);
+    const double pair_len = 2.0 * ns / nr_class;
+    const int blocks = (nt + kSumRows - 1) / kSumRows;
+    const double few = std::ceil(nt * npair / (148.0 * 8)) * (pair_len + 200.0);
+    const double many = std::ceil(blocks / (148.0 * 2)) * (ns + 500.0 * nr_class) * 3.0;
+    if (few <= many) {
+        pair_sums_few<<<(int)std::min<double>(nt * npair, 148.0 * 8), 256>>>(kv, nt, ns, nr_class, start, nsv, coef, rho, dec);
+        return cudaGetLastError();
+    }
+    const int r = nr_class - 1;
+    auto *const fn = r <= kSumGroups ? pair_sums_many<1> : r <= 2 * kSumGroups ? pair_sums_many<2> : pair_sums_many<3>;
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSumSmem);
+    if (e != cudaSuccess) return e;
+    fn<<<blocks, kSumRows * kSumGroups, kSumSmem>>>(kv, nt, ns, nr_class, start, nsv, coef, rho, dec);
+    return cudaGetLastError();
 }
 
 // Tensor forms: kv[t][s] row-major; one warp per (test row, pair), the lanes
@@ -553,7 +727,7 @@ int predict_batch(const svm_model *m, const svm_node *const *rows, int n, double
                 pair_sums_rows<<<(int)std::min<long long>(((long long)tn * npair * 32 + 255) / 256, 148 * 16), 256>>>(
                     kv, tn, m->l, k, s->start, s->nsv, s->coef, s->rho, d_dec);
             else
-                pair_sums<<<std::min<long long>(((long long)tn * npair + 127) / 128, 148 * 8), 128>>>(kv, tn, m->l, k, s->start, s->nsv, s->coef, s->rho, d_dec);
+                PK(launch_pair_sums(kv, tn, m->l, k, s->start, s->nsv, s->coef, s->rho, d_dec));
             count_launch();
             cudaError_t e = cudaDeviceSynchronize();
             if (e != cudaSuccess) {
