@@ -475,7 +475,46 @@ struct Workspace {
     int *err = nullptr;
     size_t cap_kv = 0, cap_dec = 0, cap_err = 0;
     Rows T;                     // test rows of the current chunk
+    // test rows of a tensor form: CSR with float32 values, norms, split copy
+    char *t_block = nullptr;
+    uint16_t *t_Xs = nullptr;
+    double *t_xinv = nullptr;
+    size_t cap_t = 0, cap_Xs = 0, cap_xinv = 0;
+    char *pin = nullptr;        // page-locked staging of test rows and decision values (at most kPinMost)
+    size_t cap_pin = 0;
+    void release()
+    {
+        cudaFree(kv); cudaFree(dec); cudaFree(err); cudaFree(t_block); cudaFree(t_Xs); cudaFree(t_xinv);
+        T.release();
+        if (pin) cudaFreeHost(pin);
+        *this = Workspace();
+    }
 } g_ws;
+constexpr size_t kPinMost = 512u << 20;
+
+// host staging of at least `bytes`: page-locked and kept, or for very large
+// calls ordinary memory of the call
+char *staging(size_t bytes, std::vector<char> &fallback)
+{
+    if (bytes <= g_ws.cap_pin) return g_ws.pin;
+    if (bytes <= kPinMost) {
+        if (g_ws.pin) cudaFreeHost(g_ws.pin);
+        g_ws.pin = nullptr;
+        g_ws.cap_pin = 0;
+        const size_t want = std::min(kPinMost, std::max<size_t>(bytes + bytes / 4, 1 << 20));
+        if (cudaHostAlloc((void **)&g_ws.pin, want, cudaHostAllocDefault) == cudaSuccess) {
+            g_ws.cap_pin = want;
+            return g_ws.pin;
+        }
+        cudaGetLastError();
+        g_ws.pin = nullptr;
+    }
+    fallback.resize(bytes);
+    return fallback.data();
+}
+// host loops over fewer rows than this stay on the calling thread (waking the
+// others takes longer)
+[[maybe_unused]] constexpr int kParallelRows = 128;
 
 #define PK(call)                                                                  \
     do {                                                                          \
@@ -486,34 +525,58 @@ struct Workspace {
         }                                                                         \
     } while (0)
 
+// the nodes of every row counted: rp[r + 1] - rp[r]
+void count_nodes(const svm_node *const *x, int n, long long *rp)
+{
+    rp[0] = 0;
+#pragma omp parallel for schedule(static) if (n > kParallelRows)
+    for (int r = 0; r < n; r++) {
+        long long c = 0;
+        for (const svm_node *p = x[r]; p->index != -1; ++p) c++;
+        rp[(size_t)r + 1] = c;
+    }
+    for (int r = 0; r < n; r++) rp[(size_t)r + 1] += rp[r];
+}
+
+// The copies are queued on the default stream; the caller waits for it before
+// the next use of the staging.
 int upload_nodes(const svm_node *const *x, int n, int d, int base, bool dense, Rows &out)
 {
     out.n = n;
     out.dense = dense;
     out.ld = (d + 3) & ~3;
     if (out.ld == 0) out.ld = 4;
+    std::vector<char> fallback;
     if (dense) {
-        std::vector<double> h((size_t)std::max(n, 1) * out.ld, 0.0);
-#pragma omp parallel for schedule(static)
-        for (int r = 0; r < n; r++)
+        const size_t bytes = (size_t)std::max(n, 1) * out.ld * sizeof(double);
+        double *h = (double *)staging(bytes, fallback);
+        if (n == 0) memset(h, 0, bytes);
+#pragma omp parallel for schedule(static) if (n > kParallelRows)
+        for (int r = 0; r < n; r++) {
+            double *row = h + (size_t)r * out.ld;
+            memset(row, 0, sizeof(double) * out.ld);
             for (const svm_node *p = x[r]; p->index != -1; ++p) {
                 const int c = p->index - base;
-                if (c >= 0 && c < out.ld) h[(size_t)r * out.ld + c] = p->value;
+                if (c >= 0 && c < out.ld) row[c] = p->value;
             }
-        PK(grow(out.X, out.capX, h.size() * sizeof(double)));
-        PK(xfer(out.X, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+        }
+        PK(grow(out.X, out.capX, bytes));
+        PK(xfer_async(out.X, h, bytes, cudaMemcpyHostToDevice, 0));
+        if (!fallback.empty()) PK(cudaStreamSynchronize(0));
     } else {
         std::vector<long long> rp((size_t)n + 1, 0);
-#pragma omp parallel for schedule(static)
-        for (int r = 0; r < n; r++) {
-            long long c = 0;
-            for (const svm_node *p = x[r]; p->index != -1; ++p) c++;
-            rp[(size_t)r + 1] = c;
+        count_nodes(x, n, rp.data());
+        const size_t nnz = (size_t)std::max<long long>(rp[n], 1);
+        const size_t b_val = ((size_t)n + 1) * sizeof(long long), b_col = b_val + nnz * sizeof(double);
+        char *h = staging(b_col + nnz * sizeof(int), fallback);
+        memcpy(h, rp.data(), b_val);
+        double *val = (double *)(h + b_val);
+        int *col = (int *)(h + b_col);
+        if (rp[n] == 0) {
+            val[0] = 0.0;
+            col[0] = 0;
         }
-        for (int r = 0; r < n; r++) rp[(size_t)r + 1] += rp[r];
-        std::vector<int> col((size_t)std::max<long long>(rp[n], 1), 0);
-        std::vector<double> val(col.size(), 0.0);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (n > kParallelRows)
         for (int r = 0; r < n; r++) {
             long long k = rp[r];
             for (const svm_node *p = x[r]; p->index != -1; ++p, ++k) {
@@ -521,12 +584,13 @@ int upload_nodes(const svm_node *const *x, int n, int d, int base, bool dense, R
                 val[k] = p->value;
             }
         }
-        PK(grow(out.rowptr, out.capRp, rp.size() * sizeof(long long)));
-        PK(grow(out.col, out.capCol, col.size() * sizeof(int)));
-        PK(grow(out.val, out.capVal, val.size() * sizeof(double)));
-        PK(xfer(out.rowptr, rp.data(), rp.size() * sizeof(long long), cudaMemcpyHostToDevice));
-        PK(xfer(out.col, col.data(), col.size() * sizeof(int), cudaMemcpyHostToDevice));
-        PK(xfer(out.val, val.data(), val.size() * sizeof(double), cudaMemcpyHostToDevice));
+        PK(grow(out.rowptr, out.capRp, b_val));
+        PK(grow(out.col, out.capCol, nnz * sizeof(int)));
+        PK(grow(out.val, out.capVal, nnz * sizeof(double)));
+        PK(xfer_async(out.rowptr, h, b_val, cudaMemcpyHostToDevice, 0));
+        PK(xfer_async(out.col, col, nnz * sizeof(int), cudaMemcpyHostToDevice, 0));
+        PK(xfer_async(out.val, val, nnz * sizeof(double), cudaMemcpyHostToDevice, 0));
+        if (!fallback.empty()) PK(cudaStreamSynchronize(0));
     }
     return 0;
 }
@@ -556,6 +620,10 @@ Session *get_session(const svm_model *m)
     s->d = maxi + 1;
     const bool dense = m->l == 0 || (double)nnz >= 0.25 * (double)m->l * s->d || (double)m->l * s->d * 4 < 32e6;
     if (upload_nodes(m->SV, m->l, s->d, s->base, dense, s->sv) != 0) return nullptr;
+    if (cudaStreamSynchronize(0) != cudaSuccess) {      // the staging is used again
+        set_error("upload of the support vectors failed");
+        return nullptr;
+    }
     const int k = m->nr_class, npair = k * (k - 1) / 2;
     std::vector<double> coef((size_t)std::max(k - 1, 1) * std::max(m->l, 1), 0.0);
     for (int j = 0; j < k - 1; j++)
@@ -609,6 +677,62 @@ int rows_to_device(const svm_node *const *x, int n, int d, int form, DeviceRows 
     return out.prepare_form(form, 0);
 }
 
+// The test rows of a call in a tensor form: CSR in the kept workspace, its
+// norms and split copy.  `out` borrows the buffers (see BorrowedRows).
+int tensor_rows(const svm_node *const *x, int n, int d, int form, DeviceRows &out)
+{
+    std::vector<long long> rp((size_t)n + 1, 0);
+    count_nodes(x, n, rp.data());
+    const size_t nnz = (size_t)std::max<long long>(rp[n], 1);
+    auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
+    const size_t b_col = al(((size_t)n + 1) * 8), b_val = al(b_col + nnz * 4), up = b_val + nnz * 4;
+    const size_t b_sq = al(up), total = b_sq + (size_t)n * 8;
+    std::vector<char> fallback;
+    char *h = staging(up, fallback);
+    memcpy(h, rp.data(), ((size_t)n + 1) * 8);
+    int *col = (int *)(h + b_col);
+    float *val = (float *)(h + b_val);
+#pragma omp parallel for schedule(static) if (n > kParallelRows)
+    for (int r = 0; r < n; r++) {
+        long long k = rp[r];
+        for (const svm_node *p = x[r]; p->index != -1; ++p, ++k) {
+            col[k] = p->index;
+            val[k] = (float)p->value;
+        }
+    }
+    out.n = n;
+    out.d = d > 0 ? d : 1;
+    out.ld = (out.d + 3) & ~3;
+    out.nnz = rp[n];
+    out.nchunk = std::max(1, (out.d + kSplitChunk - 1) / kSplitChunk);
+    const size_t b_Xs = (size_t)n * out.nchunk * 2 * kSplitChunk * sizeof(uint16_t);
+    PK(grow(g_ws.t_block, g_ws.cap_t, total));
+    PK(grow(g_ws.t_Xs, g_ws.cap_Xs, b_Xs));
+    if (form == FORM_FP16X3) PK(grow(g_ws.t_xinv, g_ws.cap_xinv, (size_t)n * 8));
+    out.rowptr = (long long *)g_ws.t_block;
+    out.col = (int *)(g_ws.t_block + b_col);
+    out.val = (float *)(g_ws.t_block + b_val);
+    out.xsq[FORM_EXACT] = (double *)(g_ws.t_block + b_sq);
+    PK(xfer_async(g_ws.t_block, h, up, cudaMemcpyHostToDevice, 0));
+    if (!fallback.empty()) PK(cudaStreamSynchronize(0));
+    PK(launch_xsq(out.view(FORM_EXACT), n, out.xsq[FORM_EXACT], FORM_EXACT, 0));
+    count_launch();
+    PK(cudaMemsetAsync(g_ws.t_Xs, 0, b_Xs, 0));
+    PK(launch_split(out, form, out.nchunk, g_ws.t_Xs, form == FORM_FP16X3 ? g_ws.t_xinv : nullptr, 0));
+    out.Xs = g_ws.t_Xs;
+    out.xinv = form == FORM_FP16X3 ? g_ws.t_xinv : nullptr;
+    out.split_form = form;
+    return 0;
+}
+// a DeviceRows frees its split copy: one that borrows it lets go first
+struct BorrowedRows : DeviceRows {
+    ~BorrowedRows()
+    {
+        Xs = nullptr;
+        xinv = nullptr;
+    }
+};
+
 // The SVs' split (or tf32) copy for tensor-core kernel values, made once per
 // model, form and width: both row sets of the block product need the same
 // split width, and test rows wider than the SVs widen it (their extra
@@ -642,6 +766,7 @@ void predict_forget(const svm_model *model)
     if (it != g_sessions.end()) {
         it->second->release();
         g_sessions.erase(it);
+        if (g_sessions.empty()) g_ws.release();     // the last model: nothing is kept
     }
 }
 
@@ -670,10 +795,15 @@ int predict_batch(const svm_model *m, const svm_node *const *rows, int n, double
         // device memory (at most 4 GB)
         const bool trace = getenv("SVMB_TRACE") && *getenv("SVMB_TRACE") == '1';
         const auto c0 = std::chrono::steady_clock::now();
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 1ull << 32;
+        // (asking for the free memory takes longer than a small call's kernels:
+        // not when the block in hand, or the least one allowed, will do)
         const long long per_row = (long long)m->l * 8;
-        const long long budget = std::min<long long>(4LL << 30, std::max<long long>((long long)free_b / 4, 64LL << 20));
+        long long budget = std::max<long long>((long long)g_ws.cap_kv, 64LL << 20);
+        if (n * per_row > budget) {
+            size_t free_b = 0, total_b = 0;
+            if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 1ull << 32;
+            budget = std::max(budget, std::min<long long>(4LL << 30, (long long)(free_b / 4)));
+        }
         const int chunk = (int)std::max<long long>(1, std::min<long long>(n, budget / per_row));
         PK(grow(g_ws.kv, g_ws.cap_kv, (size_t)chunk * per_row));
         PK(grow(g_ws.dec, g_ws.cap_dec, (size_t)chunk * npair * 8));
@@ -681,29 +811,31 @@ int predict_batch(const svm_model *m, const svm_node *const *rows, int n, double
         // test rows: features beyond the SVs' width cannot meet an SV feature in a
         // dot product but still count in the RBF distance, so widen to cover them
         int maxi = s->d - 1;
-#pragma omp parallel for schedule(static) reduction(max : maxi)
+#pragma omp parallel for schedule(static) reduction(max : maxi) if (n > kParallelRows)
         for (int r = 0; r < n; r++)
             for (const svm_node *p = rows[r]; p->index != -1; ++p) maxi = std::max(maxi, p->index);
         const bool wider = maxi + 1 > s->d;
         const bool tensor = is_tc_form(g_predict_form);
         const bool dense = !tensor && s->sv.dense && !wider;
         Rows &T = g_ws.T;
-        DeviceRows Ttc;
+        BorrowedRows Ttc;
         if (tensor) {
             if (prepare_tensor_svs(m, s, maxi + 1, g_predict_form) != 0) return -1;
-            if (rows_to_device(rows, n, s->sv_tc->d, g_predict_form, Ttc) != 0) return -1;
+            if (tensor_rows(rows, n, s->sv_tc->d, g_predict_form, Ttc) != 0) return -1;
         } else if (dense) {
             if (upload_nodes(rows, n, s->d, s->base, true, T) != 0) return -1;
         } else {
-            if (s->sv.dense && !s->sv_csr.rowptr && upload_nodes(m->SV, m->l, s->d, s->base, false, s->sv_csr) != 0)
-                return -1;
+            if (s->sv.dense && !s->sv_csr.rowptr) {
+                if (upload_nodes(m->SV, m->l, s->d, s->base, false, s->sv_csr) != 0) return -1;
+                PK(cudaStreamSynchronize(0));       // the staging is used again
+            }
             if (upload_nodes(rows, n, maxi + 1, s->base, false, T) != 0) return -1;
         }
         int *d_err = nullptr;
         if (tensor) {
             PK(grow(g_ws.err, g_ws.cap_err, sizeof(int)));
             d_err = g_ws.err;
-            PK(cudaMemset(d_err, 0, sizeof(int)));
+            PK(cudaMemsetAsync(d_err, 0, sizeof(int), 0));
         }
         const auto c1 = std::chrono::steady_clock::now();
         KernelParams kpk{m->param.kernel_type, m->param.degree, m->param.gamma, m->param.coef0};
@@ -729,12 +861,19 @@ int predict_batch(const svm_model *m, const svm_node *const *rows, int n, double
             else
                 PK(launch_pair_sums(kv, tn, m->l, k, s->start, s->nsv, s->coef, s->rho, d_dec));
             count_launch();
-            cudaError_t e = cudaDeviceSynchronize();
+            // (the test rows have left the staging once these kernels have run)
+            std::vector<char> fallback;
+            const size_t bytes = (size_t)tn * npair * 8;
+            cudaError_t e = cudaSuccess;
+            if (t0 == 0) e = cudaStreamSynchronize(0);
+            char *h = staging(bytes, fallback);
+            if (e == cudaSuccess) e = xfer_async(h, d_dec, bytes, cudaMemcpyDeviceToHost, 0);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(0);
             if (e != cudaSuccess) {
                 set_error(std::string("prediction kernels failed: ") + cudaGetErrorString(e));
                 return -1;
             }
-            PK(xfer(dec.data() + (size_t)t0 * npair, d_dec, (size_t)tn * npair * 8, cudaMemcpyDeviceToHost));
+            memcpy(dec.data() + (size_t)t0 * npair, h, bytes);
         }
         if (tensor) {
             int herr = 0;
@@ -756,6 +895,7 @@ int predict_batch(const svm_model *m, const svm_node *const *rows, int n, double
         for (int t = 0; t < n; t++)
             for (int p = 0; p < npair; p++) dec[(size_t)t * npair + p] = -m->rho[p];
     }
+#pragma omp parallel for schedule(static) if (n > kParallelRows)
     for (int t = 0; t < n; t++) {
         if (!classify) {
             // one-class: the side of the boundary; SVR: the value (svm.cpp:2585-2587)
