@@ -676,8 +676,11 @@ const DeviceRows &rows_of(const SubProblem &sp, const DeviceRows &rows) { return
 // of the values being copies.  A launch whose longest instance has no such
 // cache lasts as long without (the 45 pairs of 3,600 to 21,600 positions, the
 // ten smallest resident: 44.1 ms against 42.6 ms).
+// A cache with room for half of the matrix keeps its lower triangle, in the
+// clusters' loop only (`triangles`): half of a row's values then lie a column
+// apart, which a loop bound by latency does not feel.
 static std::vector<char> resident_of(const DeviceRows &rows, const std::vector<SubProblem> &subs, const SolveParams &prm,
-                                     int first, int count)
+                                     int first, int count, bool triangles)
 {
     double cost = 0.0;
     long long longest = 0, longest_fit = 0;
@@ -687,9 +690,11 @@ static std::vector<char> resident_of(const DeviceRows &rows, const std::vector<S
         const DeviceRows &r = rows_of(sp, rows);
         const long long l = (long long)sp.rows.size();
         longest = std::max(longest, l);
-        if (l == 0 || instance_layout((int)l, 1, params_of(sp, prm).cache_mb).slots < l) continue;
+        const long long slots = l > 0 ? instance_layout((int)l, 1, params_of(sp, prm).cache_mb).slots : 0;
+        if (l > 0 && slots >= l) fits[k] = kResidentFull;
+        else if (l > 0 && triangles && !is_tc_form(prm.form) && 2 * slots >= l + 1 && l <= kMaxSlots) fits[k] = kResidentTri;
+        if (!fits[k]) continue;
         longest_fit = std::max(longest_fit, l);
-        fits[k] = 1;
         const double width = is_tc_form(prm.form) ? 0.05 * r.d : r.dense ? (double)r.ld : 8.0 * (double)r.nnz / std::max(r.n, 1);
         cost += 0.5 * (double)l * (double)l * (width + 40.0);
     }
@@ -702,14 +707,15 @@ static std::vector<char> resident_of(const DeviceRows &rows, const std::vector<S
 // blocks as the longest instance has spans of `span` positions (a power of two, at
 // most kClusterMax), fewer when the instances would not all run at a time.
 static int cluster_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const SolveParams &prm, int first,
-                        int count, long long span, int capacity)
+                        int count, long long span, int capacity, std::vector<char> &resident)
 {
     long long longest = 0;
     for (int k = 0; k < count; k++) {
         if (params_of(subs[first + k], prm).blocks_override > 0) return 0;
         longest = std::max(longest, (long long)subs[first + k].rows.size());
     }
-    for (char r : resident_of(rows, subs, prm, first, count))
+    resident = resident_of(rows, subs, prm, first, count, true);
+    for (char r : resident)
         if (!r) return 0;
     int c = 1;
     while (c < kClusterMax && c * span < longest) c *= 2;
@@ -769,8 +775,7 @@ static int wave_layout(const DeviceRows &rows, const std::vector<SubProblem> &su
         w.poff[k + 1] = w.poff[k] + 2 * (size_t)w.nb[k];
         w.coff[k + 1] = w.coff[k] + (size_t)w.lay[k].slots;
     }
-    if (w.cluster > 0) w.resident.assign(count, 1);
-    else w.resident = resident_of(rows, subs, prm, first, count);
+    if (w.cluster == 0) w.resident = resident_of(rows, subs, prm, first, count, false);
     const size_t L = w.loff[count], P = w.poff[count], S = w.coff[count];
     size_t off = 0;
     w.o_desc = off; off = al(off + sizeof(InstanceDesc) * count);
@@ -826,7 +831,8 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
             if (n > 0 && bytes > 16e9) break;
             n++;
         }
-        const int c = n > 0 ? cluster_plan(rows, subs, prm, first, n, w.tune_rows_per_block, capacity) : 0;
+        std::vector<char> resident;
+        const int c = n > 0 ? cluster_plan(rows, subs, prm, first, n, w.tune_rows_per_block, capacity, resident) : 0;
         if (c > 0) {
             long long need = 0;
             std::vector<StagePlan> sps;
@@ -846,6 +852,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
             if (ok && (size_t)need <= smo_cluster_smem(prm.form) &&
                 smo_max_clusters(prm.form, c, (size_t)need, &clusters) == cudaSuccess && clusters > 0) {
                 w.cluster = c;
+                w.resident = resident;
                 return wave_layout(rows, subs, prm, w, sps, nms);
             }
             cudaGetLastError();
@@ -1015,7 +1022,7 @@ std::string graph_key(const Wave &w)
              w.down_bytes, w.zero_bytes, w.o_zero, w.o_out, w.used, w.dyn_smem, w.form,
              (int)w.cooperative);
     std::string q = std::to_string(w.cluster) + ":";    // the resident instances and their launches
-    for (char c : w.resident) q += c ? '1' : '0';
+    for (char c : w.resident) q += (char)('0' + c);
     q += ":" + std::to_string(w.q_total[0]) + ":" + std::to_string(w.q_total[1]) + ":" + std::to_string(w.q_smem);
     return std::string(buf) + ":" + q + ":" + std::to_string(w.o_desc) + ":" + std::to_string(w.o_bmap);
 }

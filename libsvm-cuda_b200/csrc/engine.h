@@ -179,6 +179,13 @@ struct SolveOut {
 };
 enum { kProfAReduce = 0, kProfAFill, kProfAScan, kProfBReduce, kProfBFill, kProfBUpdate, kProfShrink, kProfTotal };
 
+// kResidentFull: variable v's row is in slot v.  kResidentTri: the lower
+// triangle only, row by row (the cache has room for half of the matrix).
+enum { kResidentNone = 0, kResidentFull = 1, kResidentTri = 2 };
+// where value (a, b) of a triangle is; a (a + 1) fits for the 65,534 variables a
+// resident instance may have
+SVMB_HD constexpr unsigned tri_at(unsigned a, unsigned b) { return a >= b ? a * (a + 1u) / 2u + b : b * (b + 1u) / 2u + a; }
+
 struct InstanceDesc {
     int l;
     int nu;                     // 0: Solver (C-SVC), 1: Solver_NU
@@ -209,7 +216,7 @@ struct InstanceDesc {
     int stage_cap;              // rows staged at once (1..kSrcBatch); 0: read sources from global memory
     int stage_lds;              // floats per staged row (dense: ld; sparse: d)
     int chunk_cap;              // positions of per-block state held in shared memory (>= ceil(l/nblocks))
-    int resident;               // the cache holds every row from the start (slot = local index)
+    int resident;               // kResident*: the whole kernel matrix is in the cache from the start
     int prefetch;               // rows evaluated per fill pass (1 = no prefetch), <= kPrefetchMax
     // 0: G_bar maintained on every bound change, as the reference does (svm.cpp:744-769);
     // 1: no G_bar -- reconstruction recomputes G = p + sum over alpha>0 of alpha*Q on the

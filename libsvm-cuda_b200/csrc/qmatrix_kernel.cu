@@ -3,7 +3,8 @@
 //
 // When an instance's Q-row cache has a slot for every variable, its rows are
 // evaluated here, tile by tile, straight into the cache (variable v's row in
-// slot v), and the solver then never evaluates a row.  The values are those of
+// slot v), and the solver then never evaluates a row.  With room for half of the
+// matrix the lower triangle alone is kept.  The values are those of
 // the solver's own row passes bit for bit: every dot product accumulates in
 // feature order (float64, or float32 in the plain form), and K(a, b) is the
 // same number as K(b, a), so only the tiles on and below the diagonal are
@@ -134,10 +135,13 @@ __global__ void __launch_bounds__(kQThreads) q_dense_kernel(const InstanceDesc *
         for (int e = tid; e < kQT * kQT; e += kQThreads) {
             const int r = e >> 6, c = e & (kQT - 1);
             const float q = q_value(kp, ya[r] * yb[c], dots[r * kQDots + c], xa[r], xb[c]);
-            if (p0 + r < l && q0 + c < l) Q[(p0 + r) * stride + q0 + c] = q;
+            if (p0 + r < l && q0 + c < l) {
+                if (D.resident == kResidentFull) Q[(p0 + r) * stride + q0 + c] = q;
+                else if (p0 + r >= q0 + c) Q[tri_at(p0 + r, q0 + c)] = q;
+            }
             dots[r * kQDots + c] = (double)q;
         }
-        if (bi == bj) continue;
+        if (bi == bj || D.resident == kResidentTri) continue;
         __syncthreads();
         // the transposed tile: consecutive threads on consecutive rows
         for (int e = tid; e < kQT * kQT; e += kQThreads) {

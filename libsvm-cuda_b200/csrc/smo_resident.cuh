@@ -91,6 +91,23 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, unsigned parity
     return mbar_wait_long(bar, parity);
 }
 
+// Row i of a resident matrix: a row of its own, or a row and a column of the triangle.
+struct TriRow {
+    const float *Q;
+    unsigned i;
+    __device__ __forceinline__ float operator[](int c) const { return Q[tri_at(i, (unsigned)c)]; }
+};
+template <bool TRI>
+struct RowOf {
+    typedef const float *type;
+    static __device__ __forceinline__ type at(const float *Q, long long stride, int i) { return Q + (long long)i * stride; }
+};
+template <>
+struct RowOf<true> {
+    typedef TriRow type;
+    static __device__ __forceinline__ type at(const float *Q, long long, int i) { return TriRow{Q, (unsigned)i}; }
+};
+
 // The block's I_up maxima (per track) to every block of the cluster, then the
 // group's.  ok: this warp's last wait did not run out.  Returns 1 when the
 // records are in buffer (count - 1) & 1, 0 when this warp's wait ran out (its
@@ -159,9 +176,9 @@ __device__ __forceinline__ int res_exchange_iup(unsigned &count, bool ok, const 
 }
 
 // The same for the block's second-order j candidate and its Gmax2 maxima.
-template <int nu>
+template <int nu, class Row>
 __device__ __forceinline__ int res_exchange_j(unsigned &count, bool ok, double dec, int jx, double g2, double g2n,
-                                              const float *Qi0, const float *Qi1)
+                                              bool has0, Row Qi0, bool has1, Row Qi1)
 {
     Shared &sh = block_shared();
     ResRecords &R = res_records();
@@ -205,8 +222,9 @@ __device__ __forceinline__ int res_exchange_j(unsigned &count, bool ok, double d
             } else if (e == 3) {
                 d = ck.QD[q];
             } else {
-                const float *Q = nu && e == 5 ? Qi1 : Qi0;
-                x = __float_as_uint(!nu || Q ? Q[ck.Col[q]] : 0.0f);
+                const bool second = nu && e == 5;
+                const Row Q = second ? Qi1 : Qi0;
+                x = __float_as_uint((second ? has1 : has0) ? Q[ck.Col[q]] : 0.0f);
             }
         }
         if (lane == 0) mbar_expect(&R.bar_b, (unsigned)(c.nb * W * 16));
@@ -249,7 +267,7 @@ __device__ __noinline__ int res_scan_iup(unsigned &count)
     return res_exchange_iup<nu>(count, true, v, ix);
 }
 
-template <int FORM, bool NU>
+template <int FORM, bool NU, bool TRI>
 __device__ __noinline__ void solve_resident(int rank)
 {
     constexpr int nu = NU ? 1 : 0;
@@ -263,6 +281,7 @@ __device__ __noinline__ void solve_resident(int rank)
     }
     const Chunk ck = chunk_at(c.choff, D.chunk_cap);
     const int l = D.l, nb = D.nblocks;
+    typedef typename RowOf<TRI>::type Row;
     const float *const Q = D.cache.data;
     const long long stride = D.cache.stride;
     unsigned ka = 0, kb = 0;        // exchanges so far
@@ -309,15 +328,15 @@ __device__ __noinline__ void solve_resident(int rank)
         const int e0 = ok ? res_win(R.a[pa], 0, nb) : 0, e1 = nu && ok ? res_win(R.a[pa], kWordsI, nb) : 0;
         const ResWord *const w0 = R.a[pa][e0], *const w1 = R.a[pa][e1] + kWordsI;
         int i0 = -1, i1 = -1;
-        const float *Qi0 = nullptr, *Qi1 = nullptr;
+        Row Qi0 = RowOf<TRI>::at(Q, stride, 0), Qi1 = Qi0;
         double dec = -SVMB_INF, g2 = -SVMB_INF, g2n = -SVMB_INF;
         int jx = -1;
         if (ok) {
             i0 = code_pos(w0[0].x);
-            Qi0 = i0 >= 0 ? Q + (long long)w0[1].x * stride : nullptr;
+            if (i0 >= 0) Qi0 = RowOf<TRI>::at(Q, stride, (int)w0[1].x);
             if (nu) {
                 i1 = code_pos(w1[0].x);
-                Qi1 = i1 >= 0 ? Q + (long long)w1[1].x * stride : nullptr;
+                if (i1 >= 0) Qi1 = RowOf<TRI>::at(Q, stride, (int)w1[1].x);
             }
         }
         if (i0 >= 0 || (nu && i1 >= 0)) {
@@ -327,8 +346,8 @@ __device__ __noinline__ void solve_resident(int rank)
             // the general loop's scan: rough quotients first, see there
             auto row_at = [&](int k) -> float {
                 if (!nu) return Qi0[ck.Col[k]];
-                const float *Qr = (ck.F[k] & kFlagPos) ? Qi0 : Qi1;
-                return Qr ? Qr[ck.Col[k]] : 0.0f;
+                if (ck.F[k] & kFlagPos) return i0 >= 0 ? Qi0[ck.Col[k]] : 0.0f;
+                return i1 >= 0 ? Qi1[ck.Col[k]] : 0.0f;
             };
             auto quotient = [&](int k, float q, double &num, double &quad) -> bool {
                 const unsigned f = ck.F[k];
@@ -389,7 +408,7 @@ __device__ __noinline__ void solve_resident(int rank)
             }
         }
         __syncwarp();
-        if ((ok = res_exchange_j<nu>(kb, ok != 0, dec, jx, g2, g2n, Qi0, Qi1)) < 0) goto fail;
+        if ((ok = res_exchange_j<nu>(kb, ok != 0, dec, jx, g2, g2n, i0 >= 0, Qi0, nu && i1 >= 0, Qi1)) < 0) goto fail;
         mark(kProfAScan);
 
         // ======================= phase B: step and update =======================
@@ -423,7 +442,7 @@ __device__ __noinline__ void solve_resident(int rank)
             const int tr = nu && yj != +1 ? 1 : 0;
             const ResWord *const wi = tr ? w1 : w0;
             const int i = tr ? i1 : i0, yi = tr ? -1 : code_y(w0[0].x);
-            const float *const Qi = tr ? Qi1 : Qi0, *const Qj = Q + (long long)wj[1].x * stride;
+            const Row Qi = tr ? Qi1 : Qi0, Qj = RowOf<TRI>::at(Q, stride, (int)wj[1].x);
             int k = threadIdx.x;
             float qin = 0.0f, qjn = 0.0f;
             if (k < n) {        // on their way during the step
@@ -516,8 +535,18 @@ smo_cluster(const InstanceDesc *__restrict__ insts, const int *__restrict__ bloc
     __syncthreads();
     cluster_sync();     // no block sends before every block's mbarriers exist
     const int rank = blockIdx.x - sh.D.block0;
-    if (sh.D.nu) solve_resident<FORM, true>(rank);
-    else solve_resident<FORM, false>(rank);
+    // (the tensor forms' values differ in the last bits with the operands swapped:
+    // their matrices are whole)
+    if constexpr (!is_tc_form(FORM)) {
+        if (sh.D.resident == kResidentTri) {
+            if (sh.D.nu) solve_resident<FORM, true, true>(rank);
+            else solve_resident<FORM, false, true>(rank);
+        }
+    }
+    if (sh.D.resident == kResidentFull) {
+        if (sh.D.nu) solve_resident<FORM, true, false>(rank);
+        else solve_resident<FORM, false, false>(rank);
+    }
     signal_done(sh.D);
     __syncthreads();
     cluster_sync();     // no block leaves while another may still send to it

@@ -1441,6 +1441,7 @@ __device__ __noinline__ void accumulate_resident(int src_end, int pick_free_only
     int *const bcol = reinterpret_cast<int *>(bc + kThreads);
     const float *const Q = D.cache.data;
     const long long stride = D.cache.stride;
+    const bool tri = D.resident == kResidentTri;
     int scan = 0;
     while (true) {
         if (threadIdx.x == 0) sh.nsrc = 0;
@@ -1474,13 +1475,14 @@ __device__ __noinline__ void accumulate_resident(int src_end, int pick_free_only
         const int ns = sh.nsrc;
         if (ns == 0) break;
         for (int e = lo + threadIdx.x; e < hi; e += blockDim.x) {
-            const float *const Qe = Q + D.pos_local[e];
+            const int ecol = D.pos_local[e];
+            const float *const Qe = Q + ecol;
             double g = D.G[e], gb = with_bar ? D.G_bar[e] : 0.0;
             constexpr int kGroup = tensor ? 16 : 8;     // loads in flight; a tensor form's partial sum
             for (int k0 = 0; k0 < ns; k0 += kGroup) {
                 float q[kGroup];
 #pragma unroll
-                for (int u = 0; u < kGroup; u++) q[u] = k0 + u < ns ? Qe[bcol[k0 + u] * stride] : 0.0f;
+                for (int u = 0; u < kGroup; u++) q[u] = k0 + u >= ns ? 0.0f : tri ? Q[tri_at(bcol[k0 + u], ecol)] : Qe[bcol[k0 + u] * stride];
                 double part = tensor ? 0.0 : g, partb = tensor ? 0.0 : gb;
 #pragma unroll
                 for (int u = 0; u < kGroup; u++) {
@@ -2554,8 +2556,9 @@ __device__ __noinline__ bool fill_tail(bool ti, bool tj, int i, int yi, int row_
 
 // G_bar of all my positions after i and / or j reached or left their bound
 // (svm.cpp:744-769): G_bar -+ C Q for each of the two that did.
-__device__ __noinline__ void update_gbar(const float *Qi, bool bar_i, bool sub_i, double C_i, const float *Qj, bool bar_j,
-                                         bool sub_j, double C_j)
+// Row: const float * or TriRow.
+template <class Row>
+__device__ __noinline__ void update_gbar(Row Qi, bool bar_i, bool sub_i, double C_i, Row Qj, bool bar_j, bool sub_j, double C_j)
 {
     Shared &sh = block_shared();
     const InstanceDesc &D = sh.D;
@@ -3225,6 +3228,10 @@ smo_rows(const InstanceDesc *__restrict__ insts, const int *__restrict__ first, 
             for (int k = 0; k < kSrcBatch; k++) {
                 if (k >= ns) break;
                 const float q = q_of(sh.fy[k] * yp, dots[k], sh.fsx[k], xe);
+                if (D.resident == kResidentTri) {
+                    if (p >= p0 + k) Q[tri_at(p, p0 + k)] = q;
+                    continue;
+                }
                 Q[(long long)(p0 + k) * stride + p] = q;
                 if (p >= p0 + ns) Q[(long long)p * stride + p0 + k] = q;
             }

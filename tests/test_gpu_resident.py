@@ -17,14 +17,14 @@ def _same(engine, p, **more):
     small = make_params(cache_mb=4.0 * n * max(4, n // 3) / (1 << 20), **more)
     a, sa = engine.solve_binary(p, small)
     b, sb = engine.solve_binary(p, make_params(cache_mb=100.0, **more))
-    assert sb["fills"] == 0 and (n <= 4 or sa["fills"] > 0)
+    assert sb["fills"] == 0 and sa["fills"] > 0
     assert sa["iters"] == sb["iters"]
     np.testing.assert_array_equal(a, b)
     assert sa["rho"] == sb["rho"] and sa["obj"] == sb["obj"]
 
 
 @pytest.mark.parametrize("form", [FORM_EXACT, FORM_FP32, FORM_FP16X3, FORM_TF32])
-@pytest.mark.parametrize("n,d", [(5, 1), (63, 4), (64, 16), (65, 17), (129, 70), (1030, 33)])
+@pytest.mark.parametrize("n,d", [(9, 1), (63, 4), (64, 16), (65, 17), (129, 70), (1030, 33)])
 def test_dense(engine, n, d, form):
     p, _ = datagen.dense_gauss(n=n, n_test=0, d=d, seed=n + d)
     _same(engine, p, kernel_type=2, gamma=1.0 / d, C_pos=2.0, form=form)
@@ -42,6 +42,29 @@ def test_formulations(engine, svm_type):
     p, _ = (datagen.regression(n=150, n_test=0, d=7, seed=3) if svm_type >= 3 else
             datagen.dense_gauss(n=300, n_test=0, d=12, seed=4))
     _same(engine, p, svm_type=svm_type, kernel_type=2, gamma=0.1, nu=0.3, C_pos=2.0)
+
+
+@pytest.mark.parametrize("n,kind,more", [
+    (65, "dense", {}), (130, "dense", dict(form=FORM_FP32)), (1301, "dense", {}), (1024, "dense", dict(svm_type=1, nu=0.3)),
+    (260, "sparse", dict(kernel_type=1)), (777, "wide", {}), (301, "wide", dict(svm_type=1, nu=0.2)), (90, "regression", dict(svm_type=3))])
+def test_triangles(engine, n, kind, more):
+    """A cache with room for half of the matrix: its lower triangle, against rows evaluated during the solve."""
+    if kind == "dense":
+        p, _ = datagen.dense_gauss(n=n, n_test=0, d=19, seed=n)
+    elif kind == "regression":
+        p, _ = datagen.regression(n=n, n_test=0, d=5, seed=n)
+    else:
+        p, _ = datagen.sparse_text(n=n, n_test=0, d=120 if kind == "sparse" else 20000, nnz_mean=15.0, seed=n)
+    l = 2 * n if more.get("svm_type") == 3 else n
+    prm = dict(kernel_type=2, gamma=0.2, C_pos=2.0)
+    prm.update(more)
+    mb = lambda rows: 4.0 * l * (rows + 0.5) / (1 << 20)
+    a, sa = engine.solve_binary(p, make_params(cache_mb=mb(l // 3), **prm))
+    b, sb = engine.solve_binary(p, make_params(cache_mb=mb((l + 2) // 2), **prm))
+    assert sa["fills"] > 0 and sb["fills"] == 0
+    assert sa["iters"] == sb["iters"]
+    np.testing.assert_array_equal(a, b)
+    assert sa["rho"] == sb["rho"] and sa["obj"] == sb["obj"]
 
 
 def test_instances_of_one_launch(engine):
