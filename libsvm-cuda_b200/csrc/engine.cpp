@@ -710,15 +710,18 @@ static int cluster_plan(const DeviceRows &rows, const std::vector<SubProblem> &s
                         int count, long long span, int capacity, std::vector<char> &resident)
 {
     long long longest = 0;
+    int hint = 0;
     for (int k = 0; k < count; k++) {
-        if (params_of(subs[first + k], prm).blocks_override > 0) return 0;
+        const SolveParams &p = params_of(subs[first + k], prm);
+        if (p.blocks_override > 0) return 0;
+        hint = std::max(hint, p.blocks_hint);
         longest = std::max(longest, (long long)subs[first + k].rows.size());
     }
     resident = resident_of(rows, subs, prm, first, count, true);
     for (char r : resident)
         if (!r) return 0;
     int c = 1;
-    while (c < kClusterMax && c * span < longest) c *= 2;
+    while (c < kClusterMax && (hint > 0 ? c < hint + 1 && longest > 1000 : c * span < longest)) c *= 2;
     while (c > 1 && (long long)count * c > capacity) c /= 2;
     return c;
 }
@@ -832,28 +835,25 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
             n++;
         }
         std::vector<char> resident;
-        const int c = n > 0 ? cluster_plan(rows, subs, prm, first, n, w.tune_rows_per_block, capacity, resident) : 0;
-        if (c > 0) {
+        int c = n > 0 ? cluster_plan(rows, subs, prm, first, n, w.tune_rows_per_block, capacity, resident) : 0;
+        for (; c > 0; c /= 2) {
             long long need = 0;
             std::vector<StagePlan> sps;
-            std::vector<long long> nms;
             bool ok = true;
             for (int k = 0; k < n && ok; k++) {
                 const SubProblem &sp = subs[first + k];
-                ok = params_of(sp, prm).form == prm.form;
                 const StagePlan st = stage_plan(rows_of(sp, rows), prm.form, budget, 1);
                 const long long cap = ((long long)sp.rows.size() + c - 1) / c;
                 need = std::max(need, st.bytes + cap * kChunkBytes);
-                ok = ok && st.chunk_max >= 64;
+                ok = params_of(sp, prm).form == prm.form && st.chunk_max >= 64;
                 sps.push_back(st);
-                nms.push_back(c);
             }
+            if (!ok || (size_t)need > smo_cluster_smem(prm.form)) break;
             int clusters = 0;
-            if (ok && (size_t)need <= smo_cluster_smem(prm.form) &&
-                smo_max_clusters(prm.form, c, (size_t)need, &clusters) == cudaSuccess && clusters > 0) {
+            if (smo_max_clusters(prm.form, c, (size_t)need, &clusters) == cudaSuccess && clusters > 0) {
                 w.cluster = c;
                 w.resident = resident;
-                return wave_layout(rows, subs, prm, w, sps, nms);
+                return wave_layout(rows, subs, prm, w, sps, std::vector<long long>(n, c));
             }
             cudaGetLastError();
         }
@@ -938,7 +938,8 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
     for (int k = 0; k < count; k++) {
         const SubProblem &sp = subs[first + k];
         const long long l = (long long)sp.rows.size();
-        const int bo = params_of(sp, prm).blocks_override;
+        const int bo = params_of(sp, prm).blocks_override > 0 ? params_of(sp, prm).blocks_override
+                                                               : params_of(sp, prm).blocks_hint;
         const long long rpb = std::max(1, w.tune_rows_per_block);
         long long want = bo > 0 ? bo : std::max<long long>(1, std::min<long long>(sms, (l + rpb - 1) / rpb));
         want = std::min<long long>(want, std::max<long long>(1, l));

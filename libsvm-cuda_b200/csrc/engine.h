@@ -31,7 +31,10 @@ constexpr int kMaxSlots = 65534;
 constexpr int kRefSlots = 8192;
 constexpr int kPrefetchCand = 4;        // prefetch candidates published per block and phase
 constexpr int kPrefetchMax = 8;         // rows evaluated per fill pass (the missing row + prefetched)
-constexpr int kClusterMax = 8;          // blocks of a resident instance (one cluster)
+// blocks of a resident instance (one cluster; more than 8 is a size the device
+// may refuse, the plan then takes fewer).  16 against 8: 750 positions a block
+// took 11.0k cycles an iteration, 375 8.5k.
+constexpr int kClusterMax = 16;
 constexpr int kMaxGroupBlocks = 160;     // blocks per instance (one per SM)
 constexpr int kTileStride = 16;         // floats per row of a warp's 32x16 transpose tile (16-byte pieces swizzled)
 // shared memory of the transpose tiles (two per warp: the next column slice

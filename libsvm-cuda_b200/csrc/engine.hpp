@@ -78,6 +78,7 @@ struct SolveParams {
     double cache_mb = 100;
     int form = FORM_EXACT;
     int blocks_override = 0;        // 0: heuristic
+    int blocks_hint = 0;            // a request loop's share (0: none); clusters take the power of two above it
     int prefetch = 0;               // rows per fill pass; 0: automatic (as many as can be staged)
     int lazy_gbar = -1;             // -1: by form (recomputed for FORM_BF16X3), 0: incremental, 1: recomputed
 };

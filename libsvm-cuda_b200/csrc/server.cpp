@@ -458,7 +458,7 @@ long long svmb_server_submit(svmb_server *h, int n, int d, const long long *rowp
     j->y.assign(y, y + n);
     j->prm = svmb::capi::to_solve_params(*params);
     if (j->prm.blocks_override <= 0)
-        j->prm.blocks_override = std::max(1, std::min(svmb::device_sm_count(), n / h->s.cfg.rows_per_block));
+        j->prm.blocks_hint = std::max(1, std::min(svmb::device_sm_count(), n / h->s.cfg.rows_per_block));
     std::vector<int> idx(n);
     for (int i = 0; i < n; i++) idx[i] = i;
     if (svmb::capi::make_subproblem(*params, n, idx.data(), y, n, j->sub) != 0) return -1;

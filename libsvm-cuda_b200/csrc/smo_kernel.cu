@@ -140,6 +140,7 @@ cudaError_t launch_smo_cluster(int form, const InstanceDesc *d_insts, const int 
 {
     const void *fn = cluster_fn(form);
     cudaError_t e = set_max_dyn_smem(fn);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     void *args[] = {(void *)&d_insts, (void *)&d_block_inst};
     cudaLaunchAttribute attr;
@@ -152,6 +153,7 @@ cudaError_t smo_max_clusters(int form, int cluster, size_t dyn_smem, int *cluste
 {
     const void *fn = cluster_fn(form);
     cudaError_t e = set_max_dyn_smem(fn);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = cluster_config(cluster, cluster, dyn_smem, 0, &attr);

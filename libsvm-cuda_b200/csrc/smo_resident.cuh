@@ -119,6 +119,8 @@ __device__ __forceinline__ int res_exchange_iup(unsigned &count, bool ok, const 
     ResRecords &R = res_records();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned par = count & 1u;
+    const Ctx &c = sh.c;
+    const Chunk ck = chunk_at(c.choff, sh.D.chunk_cap);
     u64 k0 = ix[0] >= 0 ? key_of(v[0]) : 0, k1 = 0;
     int p0 = ix[0], p1 = -1;
     warp_best(k0, p0);
@@ -137,34 +139,27 @@ __device__ __forceinline__ int res_exchange_iup(unsigned &count, bool ok, const 
     }
     if (__syncthreads_or(!ok)) return -1;
     if (warp == 0) {
-        const Ctx &c = sh.c;
-        const Chunk ck = chunk_at(c.choff, sh.D.chunk_cap);
         constexpr int W = (nu ? 2 : 1) * kWordsI;
-        k0 = lane < kWarps ? sh.wk[0][lane] : 0;
-        p0 = lane < kWarps ? sh.wi[0][lane] : -1;
+        const int m = lane & (kWarps - 1);      // (both halves of the warp see every warp's result)
+        k0 = sh.wk[0][m];
+        p0 = sh.wi[0][m];
         warp_best(k0, p0);
         if (nu) {
-            k1 = lane < kWarps ? sh.wk[1][lane] : 0;
-            p1 = lane < kWarps ? sh.wi[1][lane] : -1;
+            k1 = sh.wk[1][m];
+            p1 = sh.wi[1][m];
             warp_best(k1, p1);
         }
         // a lane builds word e of the record and sends it to blocks lane / W, + 32 / W ..
+        // (without branches: word w of a track is the w-th of G, alpha and QD)
         const int e = lane & (W - 1), w = e & (kWordsI - 1), p = nu && e >= kWordsI ? p1 : p0;
-        double d = w == 0 ? -SVMB_INF : 0.0;
-        unsigned x = kNoPos;
-        if (p >= 0) {
-            const int q = p - c.a0;
-            if (w == 0) {
-                const unsigned f = ck.F[q];
-                const double G = ck.G[q];
-                d = flag_y(f) > 0 ? -G : G;
-                x = pos_code(p, flag_y(f));
-            } else if (w == 1) {
-                d = ck.A[q];
-                x = (unsigned)ck.Col[q];
-            } else if (w == 2) {
-                d = ck.QD[q];
-            }
+        const int q = p >= 0 ? p - c.a0 : 0;
+        double d = ck.G[min(w, 2) * sh.D.chunk_cap + q];
+        const unsigned f = ck.F[q], col = (unsigned)ck.Col[q];
+        if (w == 0 && flag_y(f) > 0) d = -d;
+        unsigned x = w == 0 ? pos_code(p, flag_y(f)) : col;
+        if (p < 0) {
+            d = -SVMB_INF;
+            x = kNoPos;
         }
         if (lane == 0) mbar_expect(&R.bar_a, (unsigned)(c.nb * W * 16));
         const uint32_t dst = tc::smem_addr(&R.a[par][c.rank][e]), bar = tc::smem_addr(&R.bar_a);
@@ -176,19 +171,21 @@ __device__ __forceinline__ int res_exchange_iup(unsigned &count, bool ok, const 
 }
 
 // The same for the block's second-order j candidate and its Gmax2 maxima.
-template <int nu, class Row>
-__device__ __forceinline__ int res_exchange_j(unsigned &count, bool ok, double dec, int jx, double g2, double g2n,
-                                              bool has0, Row Qi0, bool has1, Row Qi1)
+template <int nu>
+__device__ __forceinline__ int res_exchange_j(unsigned &count, bool ok, double dec, int jx, float jq, double g2, double g2n)
 {
     Shared &sh = block_shared();
     ResRecords &R = res_records();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned par = count & 1u;
+    const Ctx &c = sh.c;
+    const Chunk ck = chunk_at(c.choff, sh.D.chunk_cap);
     u64 k = jx >= 0 ? key_of(dec) : 0;
     int p = jx;
     warp_best(k, p);
     u64 kg = warp_max_key(key_of(g2)), kn = 0;
     if (nu) kn = warp_max_key(key_of(g2n));
+    if (jx == p && p >= 0) sh.wq[warp] = jq;
     if (lane == 0) {
         sh.wk[0][warp] = k;
         sh.wi[0][warp] = p;
@@ -197,36 +194,22 @@ __device__ __forceinline__ int res_exchange_j(unsigned &count, bool ok, double d
     }
     if (__syncthreads_or(!ok)) return -1;
     if (warp == 0) {
-        const Ctx &c = sh.c;
-        const Chunk ck = chunk_at(c.choff, sh.D.chunk_cap);
         constexpr int W = nu ? kWordsJ : kWordsJ - 1;
-        k = lane < kWarps ? sh.wk[0][lane] : 0;
-        p = lane < kWarps ? sh.wi[0][lane] : -1;
+        const int m = lane & (kWarps - 1), mi = sh.wi[0][m];
+        const float mq = sh.wq[m];
+        k = sh.wk[0][m];
+        p = mi;
         warp_best(k, p);
-        kg = warp_max_key(lane < kWarps ? sh.wk[1][lane] : 0);
-        if (nu) kn = warp_max_key(lane < kWarps ? sh.wk[2][lane] : 0);
-        const int e = lane & 7;
-        double d = e == 4 ? key_value(kg) : 0.0;
-        if (nu && e == 5) d = key_value(kn);
-        unsigned x = kNoPos;
-        if (p >= 0 && e < W) {
-            const int q = p - c.a0;
-            if (e == 0) {
-                d = key_value(k);
-                x = pos_code(p, flag_y(ck.F[q]));
-            } else if (e == 1) {
-                d = ck.G[q];
-                x = (unsigned)ck.Col[q];
-            } else if (e == 2) {
-                d = ck.A[q];
-            } else if (e == 3) {
-                d = ck.QD[q];
-            } else {
-                const bool second = nu && e == 5;
-                const Row Q = second ? Qi1 : Qi0;
-                x = __float_as_uint((second ? has1 : has0) ? Q[ck.Col[q]] : 0.0f);
-            }
-        }
+        kg = warp_max_key(sh.wk[1][m]);
+        if (nu) kn = warp_max_key(sh.wk[2][m]);
+        // (without branches: words 1 to 3 are the 1st to 3rd of G, alpha and QD)
+        const int e = lane & 7, q = p >= 0 ? p - c.a0 : 0;
+        const double g = ck.G[min(max(e - 1, 0), 2) * sh.D.chunk_cap + q];
+        const unsigned f = ck.F[q], col = (unsigned)ck.Col[q];
+        const u64 kd = e == 0 ? k : e == 4 ? kg : kn;
+        const double d = e >= 1 && e <= 3 ? g : key_value(kd);
+        const float jqv = __shfl_sync(0xffffffffu, mq, __ffs(__ballot_sync(0xffffffffu, mi == p)) - 1);
+        const unsigned x = p < 0 ? kNoPos : e == 0 ? pos_code(p, flag_y(f)) : e == 1 ? col : __float_as_uint(jqv);
         if (lane == 0) mbar_expect(&R.bar_b, (unsigned)(c.nb * W * 16));
         const uint32_t dst = tc::smem_addr(&R.b[par][c.rank][e]), bar = tc::smem_addr(&R.bar_b);
         if (e < W)
@@ -247,6 +230,13 @@ __device__ __forceinline__ int res_win(const ResWord (&r)[kClusterMax][kResWords
     int best = p;
     warp_best(key, best);
     return best < 0 ? 0 : __ffs(__ballot_sync(0xffffffffu, p == best)) - 1;
+}
+// the largest d of a word over the blocks
+__device__ __forceinline__ double res_max(const ResWord (&r)[kClusterMax][kResWords], int word, int nb)
+{
+    if (nb == 1) return r[0][word].d;
+    const int lane = threadIdx.x & 31;
+    return key_value(warp_max_key(lane < nb ? key_of(r[lane][word].d) : 0));
 }
 
 template <int nu>
@@ -331,6 +321,7 @@ __device__ __noinline__ void solve_resident(int rank)
         Row Qi0 = RowOf<TRI>::at(Q, stride, 0), Qi1 = Qi0;
         double dec = -SVMB_INF, g2 = -SVMB_INF, g2n = -SVMB_INF;
         int jx = -1;
+        float jq = 0.0f;
         if (ok) {
             i0 = code_pos(w0[0].x);
             if (i0 >= 0) Qi0 = RowOf<TRI>::at(Q, stride, (int)w0[1].x);
@@ -367,6 +358,7 @@ __device__ __noinline__ void solve_resident(int rank)
             unsigned r1 = 0, r2 = 0;
             int k1 = -1;
             double num1 = 0.0, quad1 = 1.0;
+            float q1 = 0.0f;
             float qn = threadIdx.x < n ? row_at(threadIdx.x) : 0.0f;
 #pragma unroll 1
             for (int k = threadIdx.x; k < n; k += kThreads) {
@@ -381,6 +373,7 @@ __device__ __noinline__ void solve_resident(int rank)
                     k1 = k;
                     num1 = num;
                     quad1 = quad;
+                    q1 = q;
                 } else if (r > r2) {
                     r2 = r;
                 }
@@ -391,11 +384,14 @@ __device__ __noinline__ void solve_resident(int rank)
 #pragma unroll 1
                 for (int k = threadIdx.x; k < n; k += kThreads) {
                     double num, quad;
-                    if (!quotient(k, row_at(k), num, quad)) continue;
-                    if (rough_quotient(num, quad) >= least) better_max(dec, jx, __ddiv_rn(num, quad), a0 + k);
+                    const float q = row_at(k);
+                    if (!quotient(k, q, num, quad) || rough_quotient(num, quad) < least) continue;
+                    better_max(dec, jx, __ddiv_rn(num, quad), a0 + k);
+                    if (jx == a0 + k) jq = q;
                 }
             } else if (r1 >= least) {
                 better_max(dec, jx, __ddiv_rn(num1, quad1), a0 + k1);
+                jq = q1;
             }
         } else if (ok) {
             // no candidate i at all: only the Gmax2 maxima matter
@@ -408,7 +404,7 @@ __device__ __noinline__ void solve_resident(int rank)
             }
         }
         __syncwarp();
-        if ((ok = res_exchange_j<nu>(kb, ok != 0, dec, jx, g2, g2n, i0 >= 0, Qi0, nu && i1 >= 0, Qi1)) < 0) goto fail;
+        if ((ok = res_exchange_j<nu>(kb, ok != 0, dec, jx, jq, g2, g2n)) < 0) goto fail;
         mark(kProfAScan);
 
         // ======================= phase B: step and update =======================
@@ -419,12 +415,20 @@ __device__ __noinline__ void solve_resident(int rank)
         int ix[2] = {-1, -1};
         if (ok) {
             const int j = code_pos(wj[0].x);
-            const double Gmax0 = w0[0].d, Gmax1 = nu ? w1[0].d : 0.0;
-            double gm = R.b[pb][0][4].d, gmn = nu ? R.b[pb][0][5].d : 0.0;
-            for (int b = 1; b < nb; b++) {
-                gm = fmax(gm, R.b[pb][b][4].d);
-                if (nu) gmn = fmax(gmn, R.b[pb][b][5].d);
+            // the working pair; nu-SVC takes i from the track of y_j (svm.cpp:1179-1182)
+            const int yj = code_y(wj[0].x);
+            const int tr = nu && j >= 0 && yj != +1 ? 1 : 0;
+            const ResWord *const wi = tr ? w1 : w0;
+            const int i = tr ? i1 : i0, yi = tr ? -1 : code_y(w0[0].x);
+            const Row Qi = tr ? Qi1 : Qi0, Qj = RowOf<TRI>::at(Q, stride, j >= 0 ? (int)wj[1].x : 0);
+            int k = threadIdx.x;
+            float qin = 0.0f, qjn = 0.0f;
+            if (j >= 0 && k < n) {      // on their way during the stopping test and the step
+                qin = Qi[ck.Col[k]];
+                qjn = Qj[ck.Col[k]];
             }
+            const double Gmax0 = w0[0].d, Gmax1 = nu ? w1[0].d : 0.0;
+            const double gm = res_max(R.b[pb], 4, nb), gmn = nu ? res_max(R.b[pb], 5, nb) : 0.0;
             const bool stop = (!nu ? __dadd_rn(Gmax0, gm) : fmax(__dadd_rn(Gmax0, gm), __dadd_rn(Gmax1, gmn))) < D.eps;
             if (stop || j < 0) {
                 if (__syncthreads_or(0)) goto fail;
@@ -437,22 +441,10 @@ __device__ __noinline__ void solve_resident(int rank)
             }
             if (widened) counter = 1;
             ++iter;
-            // the working pair; nu-SVC takes i from the track of y_j (svm.cpp:1179-1182)
-            const int yj = code_y(wj[0].x);
-            const int tr = nu && yj != +1 ? 1 : 0;
-            const ResWord *const wi = tr ? w1 : w0;
-            const int i = tr ? i1 : i0, yi = tr ? -1 : code_y(w0[0].x);
-            const Row Qi = tr ? Qi1 : Qi0, Qj = RowOf<TRI>::at(Q, stride, (int)wj[1].x);
-            int k = threadIdx.x;
-            float qin = 0.0f, qjn = 0.0f;
-            if (k < n) {        // on their way during the step
-                qin = Qi[ck.Col[k]];
-                qjn = Qj[ck.Col[k]];
-            }
             const double alpha_i = wi[1].d, alpha_j = wj[2].d;
             const double C_i = get_C(D, yi), C_j = get_C(D, yj);
             double ai = alpha_i, aj = alpha_j;
-            pair_step(yi, yj, wi[2].d, wj[3].d, __uint_as_float(wj[4 + tr].x),
+            pair_step(yi, yj, wi[2].d, wj[3].d, __uint_as_float(wj[4].x),
                       tr ? Gmax1 : (yi == +1 ? -Gmax0 : Gmax0), wj[1].d, C_i, C_j, ai, aj);
             const double dai = __dsub_rn(ai, alpha_i), daj = __dsub_rn(aj, alpha_j);
             const unsigned char new_si = status_of(ai, C_i), new_sj = status_of(aj, C_j);

@@ -502,7 +502,9 @@ __device__ __forceinline__ u64 warp_max_key(u64 k)
     return ((u64)mh << 32) | ml;
 }
 // the largest key of the warp and, among the lanes that hold it, the largest
-// index (ties go to the larger index); every lane gets both
+// index (ties go to the larger index); every lane gets both.  (Stopping after
+// the high words when one lane holds the maximum, by a vote, was slower: the
+// reductions are short, the branch is not.)
 __device__ __forceinline__ void warp_best(u64 &k, int &i)
 {
     const u64 m = warp_max_key(k);
@@ -640,6 +642,7 @@ struct Shared {
     // warps' partial results of a phase: keys and positions
     u64 wk[3][kWarps];
     int wi[2][kWarps], wp[kWarps];
+    float wq[kWarps];               // the Q value of a warp's j candidate
     WinA wa[kPollWarps];
     WinB wb[kPollWarps];
     Cand cand[kPrefetchCand];       // single-block groups: the block's own candidates
