@@ -70,9 +70,9 @@ namespace {
 #define SVMB_INF __longlong_as_double(0x7ff0000000000000ULL)
 constexpr double kTau = 1e-12;                     // reference svm.cpp:42
 constexpr long long kWaitTimeoutNs = 30000000000LL;  // default bound of a cross-block wait: 30 s
-// positions a thread takes at a time in the chunk scans that read Q rows from
-// global memory: their loads are issued together
-constexpr int kScanGroup = 4;
+// positions ahead of the one in hand whose Q values a thread of the chunk scans
+// has on their way
+constexpr int kScanAhead = 3;
 
 // --------------------------------------------------------------------------
 // memory-model helpers
@@ -610,7 +610,7 @@ static_assert(kPollWarps < kWarps, "a warp is left for the prefetch candidates")
 
 // The winning records of a phase as one poll warp saw them.
 //   phase A, track t: words 4t..: {-y G, pos_code} {alpha, column} {QD, slot} {-, row}
-//   phase B:          {decrease, pos_code} {G, column} {alpha, row} {QD, slot} {Gmax2, Q_ij} {Gmax2 of y=-1, Q_ij of track 1}
+//   phase B:          {decrease, pos_code} {G, column} {alpha, row} {QD, slot} {Gmax2, Q_ij} {Gmax2 of y=-1, -}
 // (nu-SVC has two tracks; C-SVC uses track 0 and the first Gmax2)
 struct WinA { double d[2 * kWordsI]; unsigned x[2 * kWordsI]; };
 struct WinB { double d[kWordsJ]; unsigned x[kWordsJ]; };
@@ -1839,27 +1839,15 @@ __device__ __forceinline__ bool iup_publish(unsigned seq, bool ahead, const doub
                 warp_best(k1, p1);
             }
             if (lane < (nu ? 2 : 1) * kWordsI) {
-                // lane 4t + e builds word e of track t
-                const int p = lane < kWordsI ? p0 : p1, e = lane & (kWordsI - 1);
-                double d = 0.0;
-                unsigned x = 0;
-                if (p >= 0) {
-                    const int q = p - c.a0;
-                    const unsigned f = ck.F[q];
-                    if (e == 0) {
-                        const double G = ck.G[q];
-                        d = flag_y(f) > 0 ? -G : G;
-                        x = pos_code(p, flag_y(f));
-                    } else if (e == 1) {
-                        d = ck.A[q];
-                        x = (unsigned)ck.Col[q];
-                    } else if (e == 2) {
-                        d = ck.QD[q];
-                        x = slot_word(ck.Slot[q], f);
-                    } else {
-                        x = (unsigned)ck.Row[q];
-                    }
-                } else if (e == 0) {
+                // lane 4t + e builds word e of track t, without branches: words 0 to
+                // 2 carry the 1st to 3rd of G, alpha and QD
+                const int p = lane < kWordsI ? p0 : p1, e = lane & (kWordsI - 1), q = p >= 0 ? p - c.a0 : 0;
+                double d = ck.G[min(e, 2) * sh.D.chunk_cap + q];
+                const unsigned f = ck.F[q];
+                if (e == 0 && flag_y(f) > 0) d = -d;
+                const unsigned col = (unsigned)ck.Col[q], row = (unsigned)ck.Row[q], slot = slot_word(ck.Slot[q], f);
+                unsigned x = e == 0 ? pos_code(p, flag_y(f)) : e == 1 ? col : e == 2 ? slot : row;
+                if (p < 0) {
                     d = -SVMB_INF;
                     x = kNoPos;
                 }
@@ -1975,8 +1963,8 @@ __device__ __forceinline__ void poll_j(unsigned seq, int warp, int lane)
 // Exchange of the block's second-order j candidate (largest decrease, with
 // payload) and its Gmax2 maxima; the group's are in sh.wb.
 template <int nu>
-__device__ __forceinline__ bool j_publish(unsigned seq, double dec, int jx, double g2, double g2n,
-                                          const float *Qi0, const float *Qi1)
+__device__ __forceinline__ bool j_publish(unsigned seq, double dec, int jx, float jq, double g2,
+                                          double g2n)
 {
     Ctx &c = block_shared().c;
     Shared &sh = block_shared();
@@ -1987,6 +1975,7 @@ __device__ __forceinline__ bool j_publish(unsigned seq, double dec, int jx, doub
     warp_best(k, p);
     u64 kg = warp_max_key(key_of(g2)), kn = 0;
     if (nu) kn = warp_max_key(key_of(g2n));
+    if (jx == p && p >= 0) sh.wq[warp] = jq;
     if (lane == 0) {
         sh.wk[0][warp] = k;
         sh.wi[0][warp] = p;
@@ -1996,38 +1985,23 @@ __device__ __forceinline__ bool j_publish(unsigned seq, double dec, int jx, doub
     __syncthreads();
     if (warp < kPollWarps) {
         if (warp == 0) {
-            k = lane < kWarps ? sh.wk[0][lane] : 0;
-            p = lane < kWarps ? sh.wi[0][lane] : -1;
+            const int m = lane & (kWarps - 1), mi = sh.wi[0][m];
+            const float mq = sh.wq[m];
+            k = sh.wk[0][m];
+            p = mi;
             warp_best(k, p);
-            kg = warp_max_key(lane < kWarps ? sh.wk[1][lane] : 0);
-            if (nu) kn = warp_max_key(lane < kWarps ? sh.wk[2][lane] : 0);
+            kg = warp_max_key(sh.wk[1][m]);
+            if (nu) kn = warp_max_key(sh.wk[2][m]);
+            const float jqv = __shfl_sync(0xffffffffu, mq, __ffs(__ballot_sync(0xffffffffu, mi == p)) - 1);
             if (lane < kWordsJ) {
-                double d = 0.0;
-                unsigned x = 0;
-                if (lane == 4) d = key_value(kg);
-                if (lane == 5) d = nu ? key_value(kn) : 0.0;
-                if (p >= 0) {
-                    const int q = p - c.a0;
-                    const unsigned f = ck.F[q];
-                    if (lane == 0) {
-                        d = key_value(k);
-                        x = pos_code(p, flag_y(f));
-                    } else if (lane == 1) {
-                        d = ck.G[q];
-                        x = (unsigned)ck.Col[q];
-                    } else if (lane == 2) {
-                        d = ck.A[q];
-                        x = (unsigned)ck.Row[q];
-                    } else if (lane == 3) {
-                        d = ck.QD[q];
-                        x = slot_word(ck.Slot[q], f);
-                    } else {
-                        const float *Q = lane == 4 ? Qi0 : Qi1;
-                        x = __float_as_uint(Q ? Q[ck.Col[q]] : 0.0f);
-                    }
-                } else if (lane == 0) {
-                    x = kNoPos;
-                }
+                // without branches: words 1 to 3 carry the 1st to 3rd of G, alpha and QD
+                const int q = p >= 0 ? p - c.a0 : 0;
+                const double g = ck.G[min(max(lane - 1, 0), 2) * sh.D.chunk_cap + q];
+                const unsigned f = ck.F[q], col = (unsigned)ck.Col[q], row = (unsigned)ck.Row[q], slot = slot_word(ck.Slot[q], f);
+                const u64 kd = lane == 0 ? k : lane == 4 ? kg : kn;
+                const double d = lane >= 1 && lane <= 3 ? g : nu || lane < 5 ? key_value(kd) : 0.0;
+                const unsigned x = p < 0 ? kNoPos : lane == 0 ? pos_code(p, flag_y(f)) : lane == 1 ? col : lane == 2 ? row :
+                                   lane == 3 ? slot : __float_as_uint(jqv);
                 if (c.nb == 1) {
                     sh.wb[0].d[lane] = d;
                     sh.wb[0].x[lane] = x;
@@ -2577,23 +2551,28 @@ __device__ __noinline__ void update_gbar(Row Qi, bool bar_i, bool sub_i, double 
     for (int p = c.t0 + threadIdx.x; p < c.t1; p += kThreads) D.G_bar[p] = bar(D.G_bar[p], D.pos_local[p]);
 }
 
-// num / quad roughly, as an integer that orders like it (high word + 1): an
-// approximate reciprocal, off by 2^-17 at most.  A quotient that is not safe
-// to estimate (quad or the result at the ends of the exponent range, NaN) is
-// given the value of an infinite one.
+// num / quad roughly, as an integer that orders like it: the high word (20 bits
+// of mantissa) + 1 of num times an approximate reciprocal with one Newton step,
+// which together are off by less than 2^-30.  A quotient that is not safe to estimate
+// (quad or the result at the ends of the exponent range, NaN) is given the
+// value of an infinite one.
 __device__ __forceinline__ unsigned rough_quotient(double num, double quad)
 {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(quad));
+    r = fma(r, fma(-quad, r, 1.0), r);
     const unsigned hq = (unsigned)__double2hiint(quad);
     const unsigned h = (unsigned)__double2hiint(__dmul_rn(num, r)) & 0x7fffffffu;
     return hq - 0x01000000u > 0x7d000000u ? 0x7ff00000u : h + 1u;
 }
 // what a rough quotient must reach to be divided exactly when the best one is
-// `top`: 2^-15 below it, or everything when the best is not a safe estimate
+// `top`: two below it (one is what truncation can cost), or everything when the
+// best is not a safe estimate.  Without the Newton step the line had to lie
+// 64 below, which let in most of a one-vs-one pair's untouched positions (equal
+// gradients, kernel values near 0) and sent every warp through its positions again.
 __device__ __forceinline__ unsigned rough_least(unsigned top)
 {
-    return top >= 0x7fe00000u || top <= 64u ? 1u : top - 64u;
+    return top >= 0x7fe00000u || top <= 0x00200000u ? 1u : top - 2u;
 }
 
 // an empty staging area: sparse sources are scattered into zeroed dense
@@ -2897,12 +2876,9 @@ __device__ __noinline__ void solve_instance(int rank)
             {
                 // second-order j scan on my chunk (svm.cpp:869-924 / :1120-1174): the
                 // largest decrease (Gmax + y G)^2 / quad, ties to the larger position.
-                // Exact divisions are long, so rough quotients (an approximate
-                // reciprocal, off by 2^-17 at most) come first and only those within
-                // 2^-15 of the warp's best are divided: about one per warp.  A
-                // quotient the estimate is not safe for (quad or the result at the
-                // ends of the exponent range, NaN) counts as infinite.
-                // A thread keeps its best rough quotient (high word + 1) with its
+                // Exact divisions are long, so rough quotients come first and only
+                // those that may be the warp's best are divided: about one per warp.
+                // A thread keeps its best rough quotient with its
                 // terms, and its second best; it goes over its positions once more
                 // in the rare case that both are in reach.
                 double dec = -SVMB_INF, g2 = -SVMB_INF, g2n = -SVMB_INF;
@@ -2930,49 +2906,55 @@ __device__ __noinline__ void solve_instance(int rank)
                 unsigned r1 = 0, r2 = 0;
                 int k1 = -1;
                 double num1 = 0.0, quad1 = 1.0;
-                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * kThreads) {
-                    // kScanGroup positions per thread at a time: their Q_i values are
-                    // loaded together (one L2 round trip per group, not per position)
-                    float qv[kScanGroup];
+                float q1 = 0.0f, jq = 0.0f;
+                auto row_at = [&](int k) -> float {
+                    const float *Qr = (nu && !(ck.F[k] & kFlagPos)) ? Qi1 : Qi0;
+                    return Qr ? Qr[ck.Col[k]] : 0.0f;
+                };
+                // a rolled loop, its Q_i values kScanAhead positions ahead
+                float qn[kScanAhead];
 #pragma unroll
-                    for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * kThreads;
-                        qv[u] = 0.0f;
-                        if (k < n) {
-                            const float *Qr = (nu && !(ck.F[k] & kFlagPos)) ? Qi1 : Qi0;
-                            if (Qr) qv[u] = Qr[ck.Col[k]];
-                        }
-                    }
+                for (int u = 0; u < kScanAhead; u++) {
+                    const int k = threadIdx.x + u * kThreads;
+                    qn[u] = k < n ? row_at(k) : 0.0f;
+                }
+#pragma unroll 1
+                for (int k = threadIdx.x; k < n; k += kThreads) {
+                    const float q = qn[0];
 #pragma unroll
-                    for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * kThreads;
-                        if (k >= n) break;
-                        double num, quad;
-                        if (!quotient(k, qv[u], num, quad)) continue;
-                        const unsigned r = rough_quotient(num, quad);
-                        if (r > r1) {
-                            r2 = r1;
-                            r1 = r;
-                            k1 = k;
-                            num1 = num;
-                            quad1 = quad;
-                        } else if (r > r2) {
-                            r2 = r;
-                        }
+                    for (int u = 0; u + 1 < kScanAhead; u++) qn[u] = qn[u + 1];
+                    if (k + kScanAhead * kThreads < n) qn[kScanAhead - 1] = row_at(k + kScanAhead * kThreads);
+                    double num, quad;
+                    if (!quotient(k, q, num, quad)) continue;
+                    const unsigned r = rough_quotient(num, quad);
+                    if (r > r1) {
+                        r2 = r1;
+                        r1 = r;
+                        k1 = k;
+                        num1 = num;
+                        quad1 = quad;
+                        q1 = q;
+                    } else if (r > r2) {
+                        r2 = r;
                     }
                 }
+                __syncwarp();
                 const unsigned least = rough_least(__reduce_max_sync(0xffffffffu, r1));
                 if (r2 >= least) {
+#pragma unroll 1
                     for (int k = threadIdx.x; k < n; k += kThreads) {
-                        const float *Qr = (nu && !(ck.F[k] & kFlagPos)) ? Qi1 : Qi0;
+                        const float q = row_at(k);
                         double num, quad;
-                        if (!quotient(k, Qr ? Qr[ck.Col[k]] : 0.0f, num, quad)) continue;
-                        if (rough_quotient(num, quad) >= least) better_max(dec, jx, __ddiv_rn(num, quad), c.a0 + k);
+                        if (!quotient(k, q, num, quad) || rough_quotient(num, quad) < least) continue;
+                        better_max(dec, jx, __ddiv_rn(num, quad), c.a0 + k);
+                        if (jx == c.a0 + k) jq = q;
                     }
                 } else if (r1 >= least) {
                     better_max(dec, jx, __ddiv_rn(num1, quad1), c.a0 + k1);
+                    jq = q1;
                 }
-                if (!j_publish<nu>(++seq, dec, jx, g2, g2n, Qi0, Qi1)) goto fail;
+                __syncwarp();
+                if (!j_publish<nu>(++seq, dec, jx, jq, g2, g2n)) goto fail;
             }
             SVMB_PROF(kProfAScan);
 
@@ -3010,7 +2992,7 @@ __device__ __noinline__ void solve_instance(int rank)
             const double Gi = tr ? Gmax1 : (yi == +1 ? -Gmax0 : Gmax0);
             const double alpha_i = wi.d[kWordsI * tr + 1], QDi = wi.d[kWordsI * tr + 2];
             const int slot_i = tr ? slot1 : slot0;
-            const float Qij = __uint_as_float(wj.x[4 + tr]);
+            const float Qij = __uint_as_float(wj.x[4]);     // (of the track of y_j)
             const double Gj = wj.d[1], alpha_j = wj.d[2], QDj = wj.d[3];
             // Q_j row
             int slot_j = (int)(wj.x[3] & 0xffffu);
@@ -3061,39 +3043,42 @@ __device__ __noinline__ void solve_instance(int rank)
                 int ix[2] = {-1, -1};
                 double pv = -SVMB_INF;
                 int pix = -1;
-                // kScanGroup positions per thread at a time, their Q_i and Q_j
-                // values loaded together before any is used
-                for (int k0 = threadIdx.x; k0 < n; k0 += kScanGroup * kThreads) {
-                    float qi[kScanGroup], qj[kScanGroup];
+                // rolled like the j scan, Q_i and Q_j kScanAhead positions ahead
+                float qi[kScanAhead], qj[kScanAhead];
 #pragma unroll
-                    for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * kThreads;
-                        qi[u] = 0.0f;
-                        qj[u] = 0.0f;
-                        if (k < n) {
-                            const int col = ck.Col[k];
-                            qi[u] = Qi[col];
-                            qj[u] = Qj[col];
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < kScanGroup; u++) {
-                        const int k = k0 + u * kThreads;
-                        if (k >= n) continue;
-                        const double G = __dadd_rn(ck.G[k], __dadd_rn(__dmul_rn((double)qi[u], dai), __dmul_rn((double)qj[u], daj)));
-                        ck.G[k] = G;
-                        const unsigned f = ck.F[k];
-                        const unsigned char s = flag_s(f);
-                        const bool pos = (f & kFlagPos) != 0;
-                        const bool up = s != (pos ? ST_UPPER : ST_LOWER);
-                        const double yG = pos ? -G : G;
-                        if (up) {
-                            if (pos || !nu) better_max(v[0], ix[0], yG, c.a0 + k);
-                            else better_max(v[1], ix[1], yG, c.a0 + k);
-                        }
-                        if (ahead) better_max(pv, pix, s == ST_FREE ? fabs(G) : (up ? yG : -yG), c.a0 + k);
-                    }
+                for (int u = 0; u < kScanAhead; u++) {
+                    const int k = threadIdx.x + u * kThreads;
+                    const int col = k < n ? ck.Col[k] : 0;
+                    qi[u] = k < n ? Qi[col] : 0.0f;
+                    qj[u] = k < n ? Qj[col] : 0.0f;
                 }
+#pragma unroll 1
+                for (int k = threadIdx.x; k < n; k += kThreads) {
+                    const double qid = (double)qi[0], qjd = (double)qj[0];
+#pragma unroll
+                    for (int u = 0; u + 1 < kScanAhead; u++) {
+                        qi[u] = qi[u + 1];
+                        qj[u] = qj[u + 1];
+                    }
+                    if (k + kScanAhead * kThreads < n) {
+                        const int col = ck.Col[k + kScanAhead * kThreads];
+                        qi[kScanAhead - 1] = Qi[col];
+                        qj[kScanAhead - 1] = Qj[col];
+                    }
+                    const double G = __dadd_rn(ck.G[k], __dadd_rn(__dmul_rn(qid, dai), __dmul_rn(qjd, daj)));
+                    ck.G[k] = G;
+                    const unsigned f = ck.F[k];
+                    const unsigned char s = flag_s(f);
+                    const bool pos = (f & kFlagPos) != 0;
+                    const bool up = s != (pos ? ST_UPPER : ST_LOWER);
+                    const double yG = pos ? -G : G;
+                    if (up) {
+                        if (pos || !nu) better_max(v[0], ix[0], yG, c.a0 + k);
+                        else better_max(v[1], ix[1], yG, c.a0 + k);
+                    }
+                    if (ahead) better_max(pv, pix, s == ST_FREE ? fabs(G) : (up ? yG : -yG), c.a0 + k);
+                }
+                __syncwarp();
                 if (bar_i || bar_j) update_gbar(Qi, bar_i, old_si == ST_UPPER, C_i, Qj, bar_j, old_sj == ST_UPPER, C_j);
                 if (!iup_publish<nu>(++seq, ahead, v, ix, pv, pix)) goto fail;
             }
