@@ -30,9 +30,20 @@
 // 128B-swizzled K-major shared-memory tiles, four stages deep.  The warps are
 // specialised and meet only at mbarriers: loader warps fill free stages (and
 // run on into the next tile), one thread issues the 12 MMAs of a chunk (4
-// K-steps x 3 products, M=128 N=64 K=16) into one of four TMEM accumulators,
-// and eight reader warps add each finished chunk into float64 registers and
-// write the tile's kernel values while the next tile's chunks are loaded.
+// K-steps x 3 products, M=128 N=64 K=16) into one of eight TMEM accumulators,
+// and sixteen reader warps add each finished chunk into float64 registers and
+// write the tile's kernel values while the next tile's chunks are loaded and
+// multiplied.
+//
+// What bounds it: the readers.  For 10000 x 30011 RBF values of 784 features
+// (fp16 split) a tile takes ~30k cycles: the readers' 13 chunks and float64
+// kernel function ~21k by themselves, the 156 MMAs ~16k, and the two do not
+// overlap fully.  With eight reader warps of 32 columns, the kernel function
+// unrolled 32 times (it missed the instruction cache, and two warps per
+// scheduler do not hide its latency) and four accumulators, the tile took 39k
+// cycles: 5.34 ms against 4.0 ms.  Tiles
+// of 128 columns would halve the MMA count, but their float64 sums do not fit
+// the registers left beside the loaders'.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -50,13 +61,14 @@ namespace {
 
 constexpr int kGM = 128;                                // rows of a tile (TMEM lanes)
 constexpr int kGN = 64;                                 // columns of a tile
-constexpr int kGReaders = 8;                            // warps 0-7: 4 lane quarters x 2 column halves
-constexpr int kGIssuer = 8;                             // warp 8 issues the MMAs
-constexpr int kGLoad0 = 9;                              // warps 9-15 load the operands
-constexpr int kGThreads = 512;
+constexpr int kGReaders = 16;                           // warps 0-15: 4 lane quarters x 4 column quarters
+constexpr int kGCols = 16;                              // columns of a reader thread
+constexpr int kGIssuer = 16;                            // warp 16 issues the MMAs
+constexpr int kGLoad0 = 17;                             // warps 17-23 load the operands
+constexpr int kGThreads = 768;
 constexpr int kGLoaders = kGThreads - kGLoad0 * 32;
 constexpr int kGStages = 4;
-constexpr int kGAcc = 4;                                // TMEM accumulators of kGN columns, used in turn
+constexpr int kGAcc = 8;                                // TMEM accumulators of kGN columns, used in turn
 constexpr int kGTileA = kGM * 128;                      // bytes of a 128-row x 64-bf16 operand tile
 constexpr int kGTileB = kGN * 128;                      // bytes of a 64-row x 64-bf16 operand tile
 constexpr int kGStageBytes = 2 * kGTileA + 2 * kGTileB; // A hi, A lo, B hi, B lo
@@ -66,8 +78,8 @@ static_assert(kGSmem <= 227 * 1024, "stages exceed the shared memory of a CTA");
 // Column norms and scales of a tile, written by reader threads 0-63 when the
 // tile starts and read by all readers at its end.  Reader warps stay within
 // kGAcc steps of each other, so a slot is rewritten at the earliest
-// 1 + ceil((kGAcc + 1) / nchunk) tiles later: 8 slots cover nchunk = 1.
-constexpr int kGColRing = 8;
+// 1 + ceil((kGAcc + 1) / nchunk) tiles later: 10 slots cover nchunk = 1.
+constexpr int kGColRing = 10;
 static_assert(kGColRing >= 2 + kGAcc, "column ring too short for one-chunk rows");
 
 struct GramArgs {
@@ -98,7 +110,7 @@ struct GramArgs {
 // ceil(ma/128) x ceil(nb/64) tiles, tile t = (t / ntn, t % ntn).  Each 64-feature
 // chunk's 12 MMAs start a fresh float32 accumulator, so the tensor core's
 // float32 accumulation spans 64 features; reader warp w adds it into float64
-// registers (lanes 32(w%4).., columns 32(w/4)..+31).  Every wait is bounded; a
+// registers (lanes 32(w%4).., columns 16(w/4)..+15).  Every wait is bounded; a
 // role whose wait runs out sets `abort`, which ends the other roles' waits,
 // and the launch reports the failure through a.err.
 // Q: the solver's Q values (label-signed, float32, transposed) are written.
@@ -169,9 +181,9 @@ __global__ void __launch_bounds__(kGThreads, 1) gram_split_kernel(GramArgs a)
         // scales (shared memory, one buffer per tile parity) are loaded when the
         // tile starts, so the epilogue waits on no global load.
         const int lq = warp & 3, ch = warp >> 2, rt = warp * 32 + lane;
-        double acc[32];
+        double acc[kGCols];
 #pragma unroll
-        for (int k = 0; k < 32; k++) acc[k] = 0.0;
+        for (int k = 0; k < kGCols; k++) acc[k] = 0.0;
         int ab = 0, kc = 0, t = blockIdx.x, slot = 0;
         unsigned ph = 0, phc = 0;
         double xa = 0.0, sa_inv = 1.0;
@@ -205,13 +217,10 @@ __global__ void __launch_bounds__(kGThreads, 1) gram_split_kernel(GramArgs a)
                 break;
             }
             tc::tc_fence_after();
-            float v[16];
+            float v[kGCols];
+            tc::tmem_ld16(tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(ab * kGN + ch * kGCols), v);
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                tc::tmem_ld16(tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(ab * kGN + ch * 32 + h * 16), v);
-#pragma unroll
-                for (int k = 0; k < 16; k++) acc[h * 16 + k] = __dadd_rn(acc[h * 16 + k], (double)v[k]);
-            }
+            for (int k = 0; k < kGCols; k++) acc[k] = __dadd_rn(acc[k], (double)v[k]);
             tc::tc_fence_before();
             tc::mbar_arrive(&acce[ab]);
             if (++ab == kGAcc) {
@@ -219,45 +228,55 @@ __global__ void __launch_bounds__(kGThreads, 1) gram_split_kernel(GramArgs a)
                 ph ^= 1u;
             }
             if (++kc < nk) continue;
-            // epilogue of tile t: this thread's row and 32 columns, once the
+            // epilogue of tile t: this thread's row and 16 columns, once the
             // tile's column data are in place
             if (!tc::mbar_wait_or(&colready[slot], phc, abort)) {
                 *abort = 1;
                 break;
             }
             const int m0 = (t / ntn) * kGM, n0 = (t % ntn) * kGN;
-            const int row = m0 + lq * 32 + lane, c0 = n0 + ch * 32;
-            if (row < a.ma) {
+            const int row = m0 + lq * 32 + lane, c0 = n0 + ch * kGCols;
+            // four columns at a time in a rolled loop (the sums move down by four):
+            // unrolled, the kernel function's code misses the instruction cache
+#pragma unroll 1
+            for (int q = 0; q < kGCols; q += 4) {
+                if (row < a.ma && c0 + q < a.nb) {
+                    double kv[4];
 #pragma unroll
-                for (int k = 0; k < 32; k++)
-                    acc[k] = kernel_from_dot(a.kp, __dmul_rn(__dmul_rn(acc[k], sa_inv), col_inv[slot][ch * 32 + k]), xa,
-                                             col_xsq[slot][ch * 32 + k]);
-                if (Q) {
-                    // the lanes of a warp (consecutive rows) write consecutive words
+                    for (int u = 0; u < 4; u++) {
+                        const int cl = ch * kGCols + q + u;
+                        kv[u] = kernel_from_dot(a.kp, __dmul_rn(__dmul_rn(acc[u], sa_inv), col_inv[slot][cl]), xa, col_xsq[slot][cl]);
+                    }
+                    const int col = c0 + q;
+                    if (Q) {
+                        // the lanes of a warp (consecutive rows) write consecutive words
 #pragma unroll
-                    for (int k = 0; k < 32; k++)
-                        if (c0 + k < a.nb)
-                            q_out[(long long)(c0 + k) * a.ldo + row] =
-                                __double2float_rn(__dmul_rn((double)(y_row * col_y[slot][ch * 32 + k]), acc[k]));
-                } else if (a.trans) {
-                    // the lanes of a warp (consecutive rows) write consecutive words
+                        for (int u = 0; u < 4; u++)
+                            if (col + u < a.nb)
+                                q_out[(long long)(col + u) * a.ldo + row] =
+                                    __double2float_rn(__dmul_rn((double)(y_row * col_y[slot][ch * kGCols + q + u]), kv[u]));
+                    } else if (a.trans) {
+                        // the lanes of a warp (consecutive rows) write consecutive words
 #pragma unroll
-                    for (int k = 0; k < 32; k++)
-                        if (c0 + k < a.nb) a.out[(long long)(c0 + k) * a.ldo + row] = acc[k];
-                } else {
-                    double *o = a.out + (long long)row * a.ldo + c0;
-                    if (c0 + 32 <= a.nb && ((uintptr_t)o & 15u) == 0) {
-#pragma unroll
-                        for (int k = 0; k < 32; k += 2) *reinterpret_cast<double2 *>(o + k) = make_double2(acc[k], acc[k + 1]);
+                        for (int u = 0; u < 4; u++)
+                            if (col + u < a.nb) a.out[(long long)(col + u) * a.ldo + row] = kv[u];
                     } else {
+                        double *o = a.out + (long long)row * a.ldo + col;
+                        if (col + 4 <= a.nb && ((uintptr_t)o & 15u) == 0) {
+                            *reinterpret_cast<double2 *>(o) = make_double2(kv[0], kv[1]);
+                            *reinterpret_cast<double2 *>(o + 2) = make_double2(kv[2], kv[3]);
+                        } else {
 #pragma unroll
-                        for (int k = 0; k < 32; k++)
-                            if (c0 + k < a.nb) o[k] = acc[k];
+                            for (int u = 0; u < 4; u++)
+                                if (col + u < a.nb) o[u] = kv[u];
+                        }
                     }
                 }
+#pragma unroll
+                for (int k = 0; k + 4 < kGCols; k++) acc[k] = acc[k + 4];
             }
 #pragma unroll
-            for (int k = 0; k < 32; k++) acc[k] = 0.0;
+            for (int k = 0; k < kGCols; k++) acc[k] = 0.0;
             kc = 0;
             t += gridDim.x;
             if (++slot == kGColRing) {

@@ -124,3 +124,27 @@ def test_many_tiles_per_cta_one_chunk(engine, form):
     else:
         bound = (2.0 ** -10 + 2 * d * u) * S
     assert np.all(np.abs(got - want) <= bound + 1e-30)
+
+
+@pytest.mark.parametrize("ma,nb,d", [(1, 15, 40), (33, 17, 130), (129, 63, 64), (127, 65, 200), (128, 129, 65),
+                                     (2000, 20011, 40)])
+def test_tile_edges_fp16x3(engine, ma, nb, d):
+    """Edges of the 128 x 64 tiles and of their readers' 16-column parts (four
+    columns at a time), one to four 64-feature chunks, and with 20011 columns of
+    one chunk ~34 tiles per CTA, which wraps the ring of column data three
+    times.  Linear and RBF values, the bounds of the tests above."""
+    n, gamma = 2500, 1.0 / d
+    p, X = _dense_rows(n, d, seed=ma + nb)
+    rows = ResidentRows(engine, p)
+    ia, ib = _blocks(n, ma, nb, seed=d)
+    A, B = X[ia], X[ib]
+    dot = A @ B.T
+    M = d * np.abs(A).max(1)[:, None] * np.abs(B).max(1)[None, :]
+    bound = (2.0 ** -19 + 2 * d * 2.0 ** -24) * M
+    got = rows.kernel_block(ia, ib, make_params(kernel_type=0, form=FORM_FP16X3))
+    assert np.all(np.abs(got - dot) <= bound + 1e-30)
+    norms = (A * A).sum(1)[:, None] + (B * B).sum(1)[None, :]
+    want = np.exp(-gamma * (norms - 2 * dot))
+    got = rows.kernel_block(ia, ib, make_params(kernel_type=2, gamma=gamma, form=FORM_FP16X3))
+    # |e^x - 1| <= 2|x| for |x| <= 1, which the bound on the exponent stays below
+    assert np.all(np.abs(got - want) <= 2 * want * gamma * 2 * (bound + 1e-12 * norms) + 1e-12)
