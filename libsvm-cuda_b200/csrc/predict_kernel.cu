@@ -53,6 +53,7 @@ struct Rows {
         X = nullptr; rowptr = nullptr; col = nullptr; val = nullptr;
         capX = capRp = capCol = capVal = 0;
     }
+    size_t held() const { return capX + capRp + capCol + capVal; }
 };
 
 // device buffer of at least `bytes`, reallocated only when it must grow
@@ -482,6 +483,7 @@ struct Workspace {
     size_t cap_t = 0, cap_Xs = 0, cap_xinv = 0;
     char *pin = nullptr;        // page-locked staging of test rows and decision values (at most kPinMost)
     size_t cap_pin = 0;
+    size_t held() const { return cap_kv + cap_dec + cap_t + cap_Xs + cap_xinv + cap_pin + T.held(); }
     void release()
     {
         cudaFree(kv); cudaFree(dec); cudaFree(err); cudaFree(t_block); cudaFree(t_Xs); cudaFree(t_xinv);
@@ -491,6 +493,11 @@ struct Workspace {
     }
 } g_ws;
 constexpr size_t kPinMost = 512u << 20;
+// With no model left, buffers above this are given back.  Smaller ones stay:
+// a cross-validation makes and frees a model per fold, and allocating (the
+// page-locked staging above all) anew for each took 15 to 40 ms of a call
+// whose solves take 1.3 ms, on hosts where such calls are slow.
+constexpr size_t kKeepMost = 64u << 20;
 
 // host staging of at least `bytes`: page-locked and kept, or for very large
 // calls ordinary memory of the call
@@ -766,7 +773,7 @@ void predict_forget(const svm_model *model)
     if (it != g_sessions.end()) {
         it->second->release();
         g_sessions.erase(it);
-        if (g_sessions.empty()) g_ws.release();     // the last model: nothing is kept
+        if (g_sessions.empty() && g_ws.held() > kKeepMost) g_ws.release();
     }
 }
 
