@@ -864,7 +864,8 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
     int last = first;
     // the instances from `first` that one launch holds with `bufs` transpose
     // tiles per warp.  Returns -1 on an error that no depth avoids, -2 when the
-    // first instance does not fit at this depth (reported only at depth 1).
+    // first instance does not fit at this depth (reported only at depth 1:
+    // kNoRoom when `capacity` blocks are too few for its positions).
     auto fit = [&](int bufs, std::vector<StagePlan> &sps, std::vector<long long> &nms, int &end) -> int {
         sps.clear();
         nms.clear();
@@ -889,7 +890,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
                 if (end == first) {
                     if (bufs > 1) return -2;
                     set_error("problem too large: more positions than the device's blocks can hold in shared memory");
-                    return -1;
+                    return kNoRoom;
                 }
                 break;
             }
@@ -903,7 +904,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
     };
     if (is_tc_form(prm.form)) {
         // the tensor forms have no transpose tiles
-        if (fit(2, sp_all, nmin, last) != 0) return -1;
+        if (const int rc = fit(2, sp_all, nmin, last)) return rc == kNoRoom ? rc : -1;
     } else {
         // the deepest ring (deeper rings keep more of a fill in flight) among
         // those that put the most instances into this launch
@@ -913,7 +914,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
         for (int bufs = fill_depth(); bufs >= 1; bufs--) {
             int end = first;
             const int rc = fit(bufs, spb, nmb, end);
-            if (rc == -1) return -1;
+            if (rc == -1 || rc == kNoRoom) return rc;
             if (rc == 0 && end > best) {
                 best = end;
                 sp_all.swap(spb);

@@ -692,6 +692,12 @@ cudaError_t launch_kernel_block2(const DeviceRows &A, const DeviceRows &B, const
     return cudaGetLastError();
 }
 
+cudaError_t load_q_tensor(int form)
+{
+    cudaFuncAttributes at;
+    return cudaFuncGetAttributes(&at, gram_fn<true>(form));
+}
+
 cudaError_t launch_q_tensor(int form, const InstanceDesc *d_inst, int l, cudaStream_t s)
 {
     const void *fn = gram_fn<true>(form);

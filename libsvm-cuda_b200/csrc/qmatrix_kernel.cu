@@ -159,6 +159,13 @@ int q_tiles(int l)
     return (int)(t * (t + 1) / 2);
 }
 
+cudaError_t load_q_dense(int form)
+{
+    cudaFuncAttributes at;
+    return form == FORM_FP32 ? cudaFuncGetAttributes(&at, (const void *)q_dense_kernel<float>)
+                             : cudaFuncGetAttributes(&at, (const void *)q_dense_kernel<double>);
+}
+
 cudaError_t launch_q_dense(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, cudaStream_t s)
 {
     const int blocks = total < 148 * 4 ? total : 148 * 4;

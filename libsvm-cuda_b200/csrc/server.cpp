@@ -126,6 +126,7 @@ struct Server {
     bool any_submit = false;
 
     cudaStream_t copy_stream = nullptr;
+    int no_room = 0;            // free blocks that were too few for the leading request (0: none waits)
 
     void loop();
     void admit(Slot &slot, std::unique_lock<std::mutex> &lk);
@@ -217,7 +218,8 @@ void Server::reap(Slot &slot)
 void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
 {
     const int free_blocks = capacity - blocks_used;
-    if (free_blocks <= 0 || pending.empty()) return;
+    if (free_blocks <= no_room || pending.empty()) return;
+    no_room = 0;
     std::vector<Job *> take;
     size_t mem = 0;
     // A leading request, then pending requests whose size is within a factor
@@ -271,7 +273,7 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
     const auto now = Clock::now();
     slot.jobs = take;
     slot.subs.clear();
-    bool ok = true;
+    bool ok = true, wait_room = false;
     std::string err;
     std::vector<Job *> back;
     for (Job *j : take) {
@@ -288,7 +290,11 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
         slot.subs.push_back(j->sub);
     }
     if (ok) {
-        if (wave_plan(empty_rows(), slot.subs, take[0]->prm, 0, free_blocks, slot.w) != 0) {
+        const int rc = wave_plan(empty_rows(), slot.subs, take[0]->prm, 0, free_blocks, slot.w);
+        if (rc != 0) {
+            // the leader's state needs more blocks than the running launches
+            // leave free: it waits for them
+            wait_room = rc == kNoRoom && free_blocks < capacity;
             ok = false;
             err = last_error();
         } else if (slot.w.count < (int)take.size()) {
@@ -333,6 +339,16 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
         pending.push_front(*it);
     }
     mem_used -= [&] { size_t b = 0; for (Job *j : back) b += j->mem; return b; }();
+    if (wait_room) {
+        no_room = free_blocks;
+        for (auto it = take.rbegin(); it != take.rend(); ++it) {
+            (*it)->rows->release_async(slot.stream);
+            (*it)->rows.reset();
+            (*it)->state = 0;
+            pending.push_front(*it);
+        }
+        slot.jobs.clear();
+    }
     if (!ok) {
         for (Job *j : slot.jobs) {
             if (j->rows) j->rows->release_async(slot.stream);
@@ -416,6 +432,7 @@ int svmb_server_create(const svmb_server_config *cfg, svmb_server **out)
     if (S.cfg.policy != SVMB_SERVE_ARRIVAL_ORDER) S.cfg.policy = SVMB_SERVE_SMALLEST_FIRST;
     S.capacity = svmb::device_sm_count();     // one solver block per SM at its largest shared memory
     if (S.capacity <= 0) { svmb::set_error("no CUDA device"); return -1; }
+    if (svmb::load_solver_kernels(S.cfg.form) != cudaSuccess) { svmb::set_error("loading the kernels failed"); return -1; }
     S.slots.resize(S.cfg.max_inflight);
     if (cudaStreamCreateWithFlags(&S.copy_stream, cudaStreamNonBlocking) != cudaSuccess) {
         svmb::set_error("stream creation failed");

@@ -7,6 +7,8 @@
 
 namespace svmb {
 
+cudaError_t load_q_dense(int form);     // qmatrix_kernel.cu
+cudaError_t load_q_tensor(int form);    // gram_kernel.cu
 // the solver kernel of each form (smo_form_*.cu)
 const void *smo_entry_exact();
 const void *smo_entry_fp32();
@@ -167,6 +169,16 @@ size_t smo_cluster_smem(int form)
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
         return 0;
     return (size_t)optin - a.sharedSizeBytes - 1024;
+}
+
+cudaError_t load_solver_kernels(int form)
+{
+    cudaFuncAttributes at;
+    cudaError_t e = cudaFuncGetAttributes(&at, smo_fn(form));
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, cluster_fn(form));
+    if (is_tc_form(form)) return e == cudaSuccess ? load_q_tensor(form) : e;
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, form == FORM_FP32 ? smo_rows_fp32() : smo_rows_exact());
+    return e == cudaSuccess ? load_q_dense(form) : e;
 }
 
 cudaError_t launch_q_sparse(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, size_t dyn_smem,

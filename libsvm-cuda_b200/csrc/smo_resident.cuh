@@ -22,6 +22,13 @@
 // buffer two exchanges of the same kind later, when every block's warps have
 // gone through a barrier after their last read of it.
 //
+// Measured (whole svm_train calls; the general loop as it was before this one,
+// with its fence-and-flag records and row passes, then this loop): 500 x 16 8.0
+// and 1.5 ms, 4000 x 64 66.5 and 11.1 ms (8 blocks), epsilon-SVR 2500 x 8 450
+// and 90 ms, 6000 sparse rows of 20000 columns (a triangle, 16 blocks) 484 and
+// 52 ms.  An iteration takes 3.3 to 4.4 us; instruction-cache misses fell
+// from 225 to 13 per iteration.
+//
 // Choices, arithmetic and tie rules are the general loop's; the collective
 // sections (shrinking, reconstruction, start and end) are the same functions.
 #pragma once

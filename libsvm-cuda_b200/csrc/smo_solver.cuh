@@ -37,6 +37,11 @@
 //     in the record, so a phase knows a hit or a miss as soon as it knows the
 //     variable; every block replays the same slot allocation.
 //
+// Measured, 45 one-vs-one pairs of 3,600 to 21,600 rows, d = 256: kernel 55.7 ms
+// with fence-and-flag records, per-set LRU cache lookups and 64-bit shuffles,
+// 44.0 ms with the above; 100,000 x 784 exact form 9.27 and 6.87 s.  Row passes
+// (see warp_tile_dots) are then two thirds of an iteration there.
+//
 // Shrinking (svm.cpp:932-1011), gradient reconstruction (:473-513) and the
 // initial gradient (:545-572) run inside the same launch as group-collective
 // sections on the global copies of the state.  The position permutation of

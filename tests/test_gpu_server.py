@@ -58,3 +58,25 @@ def test_rejects_a_request_larger_than_the_budget(engine):
             srv.wait(t)
     finally:
         srv.close()
+
+
+def test_a_request_waits_for_the_blocks_its_state_needs(engine):
+    """A request whose positions need more blocks than the running launches
+    leave free waits for them: 140 of the blocks are taken by the first, and the
+    second's 60000 positions need more than the other 8."""
+    long, _ = datagen.dense_gauss(n=14000, n_test=0, d=32, seed=21, flip=0.05)
+    long_prm = make_params(svm_type=0, kernel_type=2, gamma=1.0 / 32, C_pos=10.0, cache_mb=40.0)
+    wide, _ = datagen.dense_gauss(n=60000, n_test=0, d=4, seed=22, flip=0.05)
+    wide_prm = make_params(svm_type=0, kernel_type=2, gamma=0.25, C_pos=0.01, eps=0.5, cache_mb=40.0)
+    srv = Server(engine, max_inflight=4, rows_per_block=100)
+    try:
+        t_long = srv.submit(long, long_prm)
+        time.sleep(0.1)
+        t_wide = srv.submit(wide, wide_prm)
+        got = srv.wait(t_wide), srv.wait(t_long)
+        st = srv.stats()
+    finally:
+        srv.close()
+    assert st["completed"] == 2 and st["failed"] == 0, st
+    assert np.array_equal(got[0][0], engine.solve_binary(wide, wide_prm)[0])
+    assert np.array_equal(got[1][0], engine.solve_binary(long, long_prm)[0])
