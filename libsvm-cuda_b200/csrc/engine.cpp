@@ -13,6 +13,7 @@
 #include <chrono>
 #include <climits>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
 #include <atomic>
@@ -157,6 +158,53 @@ int device_sm_count()
         sms = p.multiProcessorCount;
     }
     return sms;
+}
+
+namespace {
+// solver blocks at work per device, and the calls that wait for theirs
+struct BlockCount {
+    std::mutex mu;
+    std::condition_variable cv;
+    std::map<int, int> used, waiting;
+} g_blocks;
+int current_device()
+{
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess ? dev : 0;
+}
+}  // namespace
+
+int blocks_take(int count)
+{
+    const int dev = current_device(), sms = device_sm_count();
+    count = std::min(count, sms);
+    std::unique_lock<std::mutex> lk(g_blocks.mu);
+    int &used = g_blocks.used[dev], &waiting = g_blocks.waiting[dev];
+    waiting++;
+    g_blocks.cv.wait(lk, [&] { return used + count <= sms; });
+    waiting--;
+    used += count;
+    return count;
+}
+
+int blocks_take_free()
+{
+    const int dev = current_device(), sms = device_sm_count();
+    std::lock_guard<std::mutex> g(g_blocks.mu);
+    int &used = g_blocks.used[dev];
+    if (g_blocks.waiting[dev] > 0) return 0;
+    const int n = std::max(0, sms - used);
+    used += n;
+    return n;
+}
+
+void blocks_give(int count)
+{
+    if (count <= 0) return;
+    const int dev = current_device();
+    std::lock_guard<std::mutex> g(g_blocks.mu);
+    g_blocks.used[dev] -= count;
+    g_blocks.cv.notify_all();
 }
 
 // One grow-only device block reused by the row uploads of svm_train and
@@ -1516,6 +1564,7 @@ int solve_batch(const DeviceRows &rows, const std::vector<SubProblem> &subs, con
         }
         clk.mark("arena");
         w.use_graph = g_graphs_on && host != host_fallback.data();
+        const BlockShare share((w.used + per_sm - 1) / per_sm);
         if (wave_start(rows, *plan, prm, w, arena, host, ws) != 0) return -1;
         clk.mark("launch");
         if (wave_finish(w, out) != 0) return -1;

@@ -125,6 +125,21 @@ struct Wave {
 };
 
 constexpr int kNoRoom = -3;     // wave_plan: the first instance needs more than `capacity` blocks
+// The solver blocks at work on the current device, of this process's request
+// loops and solve calls together.  A launch's blocks may wait for one another
+// (the general loop), so they must all find an SM: blocks that are waiting for
+// room while others of two launches spin would hold each other up until the
+// wait limit.  blocks_take waits until `count` SMs (at most the device's) are
+// free; blocks_take_free takes what is free, nothing while a call waits.
+int blocks_take(int count);
+int blocks_take_free();
+void blocks_give(int count);
+struct BlockShare {             // what a call holds until it returns
+    int count;
+    explicit BlockShare(int n) : count(blocks_take(n)) {}
+    BlockShare(const BlockShare &) = delete;
+    ~BlockShare() { blocks_give(count); }
+};
 // Plan the wave that starts at instance `first` within `capacity` co-resident
 // blocks (as many instances before `limit` as fit; limit < 0: up to the end).
 // Needs w.dev_bytes of device memory and w.up_bytes + w.down_bytes of

@@ -228,6 +228,7 @@ extern "C" int svmb_solve_dense_noalloc(int n, int ld, const float *X, const dou
     count_launch();
     NA_CK(launch_xsq(D.x, n, xsq, params->form, s));
     count_launch();
+    const BlockShare share(nb);
     NA_CK(launch_smo(params->form, d_desc, d_block_inst, nb, dyn_smem, true, s));
     count_launch();
     noalloc_finish<<<(n + 255) / 256, 256, 0, s>>>(alpha_local, y, n, alpha_out);

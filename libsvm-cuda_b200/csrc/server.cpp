@@ -10,8 +10,8 @@
 // similar size (within a factor of 4 in rows) are admitted while
 //   - the device memory of the admitted work (rows + solver state with its
 //     Q-row cache budget) stays within the server's budget, and
-//   - the thread blocks their state needs fit in the SMs that no running wave
-//     holds,
+//   - the thread blocks their state needs fit in the SMs that no running wave,
+//     of any loop or solve call of the process, holds,
 // then uploaded (stream-ordered allocations, no device-wide synchronisation)
 // and launched together as one new wave next to the waves already running.
 // Requests get fewer blocks than a solve alone (rows / rows_per_block): a
@@ -115,7 +115,6 @@ struct Server {
     std::map<long long, std::unique_ptr<Job>> jobs;
     std::vector<Slot> slots;
     size_t mem_used = 0, mem_peak = 0;
-    int blocks_used = 0;
     long long next_ticket = 0;
     bool stop = false;
     std::thread worker;
@@ -172,7 +171,7 @@ void Server::collect(Slot &slot)
         slot.jobs[k] = nullptr;                 // a waiter may free the request once it is complete
         std::lock_guard<std::mutex> g(mu);
         complete_locked(j, rc == 0, err);
-        blocks_used -= slot.w.nb[k];
+        blocks_give(slot.w.nb[k]);
         slot.blocks -= slot.w.nb[k];
     }
 }
@@ -206,7 +205,7 @@ void Server::reap(Slot &slot)
         complete_locked(slot.jobs[k], ok[k] != 0, ok[k] ? std::string() : (err.empty() ? "solve failed" : err));
     }
     mem_used -= slot.mem;
-    blocks_used -= slot.blocks;
+    blocks_give(slot.blocks);
     slot.jobs.clear();
     slot.subs.clear();
     slot.busy = false;
@@ -217,8 +216,13 @@ void Server::reap(Slot &slot)
 // drops it while uploading and launching).
 void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
 {
-    const int free_blocks = capacity - blocks_used;
-    if (free_blocks <= no_room || pending.empty()) return;
+    if (pending.empty()) return;
+    // all free blocks, until the wave's plan fixes how many it needs
+    const int free_blocks = blocks_take_free();
+    if (free_blocks <= no_room) {
+        blocks_give(free_blocks);
+        return;
+    }
     no_room = 0;
     std::vector<Job *> take;
     size_t mem = 0;
@@ -243,7 +247,7 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
         }
         if (mem_used + mem + j->mem > (size_t)cfg.mem_bytes) {
             // nothing running and nothing taken: this request can never fit
-            if (take.empty() && blocks_used == 0 && j->mem > (size_t)cfg.mem_bytes) {
+            if (take.empty() && mem_used == 0 && j->mem > (size_t)cfg.mem_bytes) {
                 j->state = -1;
                 j->error = "request exceeds the server's device memory budget";
                 j->t_done = Clock::now();
@@ -261,11 +265,13 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
         mem += j->mem;
         it = pending.erase(it);
     }
-    if (take.empty()) return;
+    if (take.empty()) {
+        blocks_give(free_blocks);
+        return;
+    }
     for (Job *j : take) j->state = 1;
     mem_used += mem;
     mem_peak = std::max(mem_peak, mem_used);
-    blocks_used += free_blocks;     // provisional: the wave's plan fixes the real count
     slot.busy = true;
     lk.unlock();
 
@@ -361,7 +367,7 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
         if (slot.dev) cudaFreeAsync(slot.dev, slot.stream);
         slot.dev = nullptr;
         mem_used -= mem;
-        blocks_used -= free_blocks;
+        blocks_give(free_blocks);
         slot.jobs.clear();
         slot.subs.clear();
         slot.busy = false;
@@ -370,7 +376,7 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
     }
     slot.mem = mem;
     slot.blocks = slot.w.used;
-    blocks_used += slot.w.used - free_blocks;
+    blocks_give(free_blocks - slot.w.used);
     waves++;
     int running = 0;
     for (const Slot &s : slots) running += s.busy ? 1 : 0;
@@ -399,7 +405,8 @@ void Server::loop()
             else break;     // nothing admissible now
         }
         if (stop && pending.empty() && !any_busy) break;
-        if (any_busy) cv_work.wait_for(lk, std::chrono::microseconds(50));
+        // (requests may also wait for blocks that another loop or call holds)
+        if (any_busy || !pending.empty()) cv_work.wait_for(lk, std::chrono::microseconds(50));
         else cv_work.wait(lk, [&] { return stop || !pending.empty(); });
     }
 }
