@@ -312,25 +312,37 @@ DevX DeviceRows::view(int form) const
     return v;
 }
 
+// The layout rule: dense rows only when they are not much larger than the CSR
+// arrays.  A kernel row streams the whole stored row of every active position,
+// so the byte count is what matters.
+static bool dense_layout(int force, int n, int ld, long long nnz, double *dense_bytes, double *csr_bytes)
+{
+    *dense_bytes = (double)n * ld * 4.0;
+    *csr_bytes = (double)(n + 1) * 8.0 + (double)nnz * 8.0;
+    bool dense = force == 1 || (force < 0 && *dense_bytes <= 1.2 * *csr_bytes);
+    if (dense && *dense_bytes > 60e9) dense = false;
+    return dense;
+}
+
+void rows_shape(int n, int d, long long nnz, int force, DeviceRows &out)
+{
+    double dense_bytes, csr_bytes;
+    out.n = n;
+    out.d = d > 0 ? d : 1;
+    out.ld = (out.d + 3) & ~3;
+    out.nnz = nnz;
+    out.dense = dense_layout(force, n, out.ld, nnz, &dense_bytes, &csr_bytes);
+}
+
 int upload_csr(const long long *rowptr, const int *col, const float *val, int n, int d, DeviceRows &out,
                int force, cudaStream_t s, int alloc)
 {
     const bool async_alloc = alloc == kAllocAsync;
-    out.n = n;
-    out.d = d > 0 ? d : 1;
     const long long nnz = rowptr[n];
-    out.ld = (out.d + 3) & ~3;
-    // Dense rows only when they are not larger than the CSR arrays: a kernel
-    // row streams the whole stored row of every active position, so the byte
-    // count is what matters.
-    const double dense_bytes = (double)n * out.ld * 4.0;
-    const double csr_bytes = (double)(n + 1) * 8.0 + (double)nnz * 8.0;
-    bool dense = force == 1 || (force < 0 && dense_bytes <= 1.2 * csr_bytes);
-    if (dense && dense_bytes > 60e9) dense = false;
-    out.dense = dense;
+    rows_shape(n, d, nnz, force, out);
+    const bool dense = out.dense;
     // the CSR arrays always travel; dense rows are scattered on the device.
     // One device block holds [rowptr][col][val][dense rows][norms x 2].
-    out.nnz = nnz;
     auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
     const size_t b_rp = 0;
     const size_t b_col = al(b_rp + (size_t)(n + 1) * sizeof(long long));
@@ -447,16 +459,6 @@ static long long dense_row(const svm_node *row_nodes, int base, int d, int ld, f
         for (const svm_node *p = row_nodes; p->index != -1; ++p) row[p->index - base] = (float)p->value;
     }
     return c;
-}
-
-// upload_csr's layout rule: dense rows when they are not much larger than the CSR arrays
-static bool dense_layout(int force, int n, int ld, long long nnz, double *dense_bytes, double *csr_bytes)
-{
-    *dense_bytes = (double)n * ld * 4.0;
-    *csr_bytes = (double)(n + 1) * 8.0 + (double)nnz * 8.0;
-    bool dense = force == 1 || (force < 0 && *dense_bytes <= 1.2 * *csr_bytes);
-    if (dense && *dense_bytes > 60e9) dense = false;
-    return dense;
 }
 
 int upload_rows(const svm_node *const *x, int n, DeviceRows &out, int force, cudaStream_t s, int alloc)
@@ -938,6 +940,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
                 if (end == first) {
                     if (bufs > 1) return -2;
                     set_error("problem too large: more positions than the device's blocks can hold in shared memory");
+                    w.used = (int)std::min<long long>(nm, INT_MAX);
                     return kNoRoom;
                 }
                 break;

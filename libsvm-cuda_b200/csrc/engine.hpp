@@ -55,6 +55,8 @@ int upload_rows(const svm_node *const *x, int n, DeviceRows &out, int force, cud
 enum { kAllocPlain = 0, kAllocAsync = 1, kAllocPooled = 2 };
 int upload_csr(const long long *rowptr, const int *col, const float *val, int n, int d, DeviceRows &out,
                int force, cudaStream_t s, int alloc = kAllocPlain);
+// what upload_csr makes of n rows of d columns with nnz nonzeros: their shape and layout, without device memory
+void rows_shape(int n, int d, long long nnz, int force, DeviceRows &out);
 // device bytes of one instance's solver state (gradient, status, shrink lists, Q-row cache)
 size_t instance_bytes(int l, double cache_mb);
 
@@ -124,7 +126,7 @@ struct Wave {
     float ms = 0;
 };
 
-constexpr int kNoRoom = -3;     // wave_plan: the first instance needs more than `capacity` blocks
+constexpr int kNoRoom = -3;     // wave_plan: the first instance needs w.used blocks, more than `capacity`
 // The solver blocks at work on the current device, of this process's request
 // loops and solve calls together.  A launch's blocks may wait for one another
 // (the general loop), so they must all find an SM: blocks that are waiting for

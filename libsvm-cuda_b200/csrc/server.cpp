@@ -62,6 +62,7 @@ struct Job {
     SubProblem sub;
     std::unique_ptr<DeviceRows> rows;
     size_t mem = 0;             // device bytes reserved while the request runs
+    int need_blocks = 0;        // blocks that a plan found too few free for (0: none has)
     // result
     int state = 0;              // 0 queued, 1 running, 2 done, -1 failed (written under the server lock)
     std::string error;
@@ -125,7 +126,6 @@ struct Server {
     bool any_submit = false;
 
     cudaStream_t copy_stream = nullptr;
-    int no_room = 0;            // free blocks that were too few for the leading request (0: none waits)
 
     void loop();
     void admit(Slot &slot, std::unique_lock<std::mutex> &lk);
@@ -219,29 +219,35 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
     if (pending.empty()) return;
     // all free blocks, until the wave's plan fixes how many it needs
     const int free_blocks = blocks_take_free();
-    if (free_blocks <= no_room) {
-        blocks_give(free_blocks);
-        return;
-    }
-    no_room = 0;
     std::vector<Job *> take;
     size_t mem = 0;
     // A leading request, then pending requests whose size is within a factor
     // of 4 of the leader's: a launch keeps its device memory until its
     // longest solve ends, so similar sizes free it sooner.
     // the leader: the oldest request, or (smallest-first policy) the smallest
-    // one unless the oldest has waited longer than kMaxWait
-    if (cfg.policy == SVMB_SERVE_SMALLEST_FIRST &&
-        std::chrono::duration<double>(Clock::now() - pending.front()->t_submit).count() < kMaxWait) {
-        auto best = std::min_element(pending.begin(), pending.end(), [](const Job *a, const Job *b) { return a->n < b->n; });
-        Job *lead = *best;
-        pending.erase(best);
-        pending.push_front(lead);
+    // one unless the oldest has waited longer than kMaxWait.  A request whose
+    // state needs more blocks than are free is passed by others until it leads
+    // by its age; then all wait for it.
+    auto lead = std::min_element(pending.begin(), pending.end(), [](const Job *a, const Job *b) { return a->ticket < b->ticket; });
+    const bool by_age = cfg.policy != SVMB_SERVE_SMALLEST_FIRST ||
+                        std::chrono::duration<double>(Clock::now() - (*lead)->t_submit).count() >= kMaxWait;
+    const auto fits = [&](const Job *j) { return free_blocks > 0 && j->need_blocks <= free_blocks; };
+    if (!by_age)
+        for (auto it = pending.begin(); it != pending.end(); ++it)
+            if (fits(*it) && (!fits(*lead) || (*it)->n < (*lead)->n)) lead = it;
+    if (!fits(*lead)) {
+        blocks_give(free_blocks);
+        return;
+    }
+    if (lead != pending.begin()) {
+        Job *const j = *lead;
+        pending.erase(lead);
+        pending.push_front(j);
     }
     double lead_rows = 0;
     for (auto it = pending.begin(); it != pending.end() && (int)take.size() < std::min(cfg.max_batch, free_blocks);) {
         Job *j = *it;
-        if (!take.empty() && ((double)j->n > 4.0 * lead_rows || 4.0 * (double)j->n < lead_rows)) {
+        if (!take.empty() && (!fits(j) || (double)j->n > 4.0 * lead_rows || 4.0 * (double)j->n < lead_rows)) {
             ++it;
             continue;
         }
@@ -277,43 +283,37 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
 
     cudaSetDevice(device);
     const auto now = Clock::now();
-    slot.jobs = take;
     slot.subs.clear();
-    bool ok = true, wait_room = false;
     std::string err;
     std::vector<Job *> back;
     for (Job *j : take) {
         j->t_start = now;
-        j->rows.reset(new DeviceRows());
-        if (upload_csr(j->rowptr.data(), j->col.data(), j->val.data(), j->n, j->d, *j->rows, -1, slot.stream, kAllocAsync) != 0 ||
-            j->rows->prepare_form(j->prm.form, slot.stream) != 0) {
-            ok = false;
-            err = last_error();
-            break;
-        }
         j->sub.rows_dev = j->rows.get();
         j->sub.own = &j->prm;
         slot.subs.push_back(j->sub);
     }
+    // the plan needs the rows' shapes only: what it does not take stays on the host
+    const int rc = wave_plan(empty_rows(), slot.subs, take[0]->prm, 0, free_blocks, slot.w);
+    bool ok = rc == 0;
     if (ok) {
-        const int rc = wave_plan(empty_rows(), slot.subs, take[0]->prm, 0, free_blocks, slot.w);
-        if (rc != 0) {
-            // the leader's state needs more blocks than the running launches
-            // leave free: it waits for them
-            wait_room = rc == kNoRoom && free_blocks < capacity;
+        back.assign(take.begin() + slot.w.count, take.end());
+    } else if (rc == kNoRoom && free_blocks < capacity) {
+        // the leader's state needs more blocks than are free now
+        take[0]->need_blocks = slot.w.used;
+        back = take;
+    } else {
+        err = last_error();
+        back.assign(take.begin() + 1, take.end());      // the leader fails
+    }
+    take.resize(take.size() - back.size());
+    for (Job *j : back) mem -= j->mem;
+    slot.jobs = take;
+    slot.subs.resize(take.size());
+    for (Job *j : take) {
+        if (ok && (upload_csr(j->rowptr.data(), j->col.data(), j->val.data(), j->n, j->d, *j->rows, -1, slot.stream, kAllocAsync) != 0 ||
+                   j->rows->prepare_form(j->prm.form, slot.stream) != 0)) {
             ok = false;
             err = last_error();
-        } else if (slot.w.count < (int)take.size()) {
-            // the plan holds fewer requests than admitted: the rest go back to the queue head
-            back.assign(take.begin() + slot.w.count, take.end());
-            take.resize(slot.w.count);
-            slot.jobs = take;
-            slot.subs.resize(slot.w.count);
-            for (Job *j : back) {
-                j->rows->release_async(slot.stream);
-                j->rows.reset();
-                mem -= j->mem;
-            }
         }
     }
     if (ok && slot.host_bytes < slot.w.up_bytes + slot.w.down_bytes) {
@@ -342,22 +342,12 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
     lk.lock();
     for (auto it = back.rbegin(); it != back.rend(); ++it) {
         (*it)->state = 0;
+        mem_used -= (*it)->mem;
         pending.push_front(*it);
-    }
-    mem_used -= [&] { size_t b = 0; for (Job *j : back) b += j->mem; return b; }();
-    if (wait_room) {
-        no_room = free_blocks;
-        for (auto it = take.rbegin(); it != take.rend(); ++it) {
-            (*it)->rows->release_async(slot.stream);
-            (*it)->rows.reset();
-            (*it)->state = 0;
-            pending.push_front(*it);
-        }
-        slot.jobs.clear();
     }
     if (!ok) {
         for (Job *j : slot.jobs) {
-            if (j->rows) j->rows->release_async(slot.stream);
+            j->rows->release_async(slot.stream);
             j->rows.reset();
             j->state = -1;
             j->error = err;
@@ -487,6 +477,8 @@ long long svmb_server_submit(svmb_server *h, int n, int d, const long long *rowp
     for (int i = 0; i < n; i++) idx[i] = i;
     if (svmb::capi::make_subproblem(*params, n, idx.data(), y, n, j->sub) != 0) return -1;
     j->mem = svmb::request_bytes(n, d, rowptr[n], params->cache_mb);
+    j->rows.reset(new svmb::DeviceRows());
+    svmb::rows_shape(n, d, rowptr[n], -1, *j->rows);
     j->t_submit = svmb::Clock::now();
     Server &S = h->s;
     std::lock_guard<std::mutex> g(S.mu);

@@ -6,12 +6,13 @@ import glob
 import os
 import subprocess
 import threading
+import time
 
 import numpy as np
 import pytest
 
 from svmb200.datagen import CSR
-from svmb200.lib import Engine, Server, make_params
+from svmb200.lib import Engine, EngineError, Server, make_params
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.join(os.path.dirname(HERE), "libsvm-cuda_b200")
@@ -58,3 +59,53 @@ def test_launches_of_two_loops_and_a_call_fit_the_device(host):
     assert [st["iters"] for _, st, _ in got] == [14000, 14000]
     assert host.lib.fake_general_launches() == 3
     assert host.lib.fake_peak_blocks() <= 148
+
+
+def test_a_request_that_waits_for_blocks_is_passed_and_uploaded_once(host):
+    """140 of 148 blocks are at work; the next request's 60000 positions need
+    more than the other 8.  A small request that comes later does not wait for
+    it, and the waiting one's rows go to the device once."""
+    long, wide, small = _rows(14000), _rows(60000), _rows(500)
+    prm = make_params(gamma=1.0, cache_mb=10.0)
+    host.lib.fake_us_per_row(30)
+    loop = Server(host, max_inflight=4, rows_per_block=100)
+    try:
+        alone = 0
+        for p in (long, wide, small):
+            host.lib.fake_us_per_row(0)
+            host.lib.fake_h2d_bytes()
+            loop.wait(loop.submit(p, prm))
+            alone += host.lib.fake_h2d_bytes()
+        host.lib.fake_us_per_row(30)
+        t_long = loop.submit(long, prm)
+        while not host.lib.fake_h2d_bytes():
+            time.sleep(0.001)
+        t_wide = loop.submit(wide, prm)
+        time.sleep(0.02)
+        t_small = loop.submit(small, prm)
+        loop.wait(t_small)
+        assert not loop.done(t_long) and not loop.done(t_wide)
+        host.lib.fake_us_per_row(0)
+        assert loop.wait(t_wide)[1]["iters"] == 60000 and loop.done(t_long)
+        loop.wait(t_long)
+    finally:
+        host.lib.fake_us_per_row(1)
+        loop.close()
+    assert host.lib.fake_h2d_bytes() <= alone
+
+
+def test_a_request_too_large_for_the_device_fails_alone(host):
+    first, huge, large = _rows(500), _rows(900000, 1), _rows(300000, 1)
+    prm = make_params(gamma=1.0, cache_mb=10.0)
+    host.lib.fake_us_per_row(100)
+    loop = Server(host, max_inflight=1, policy=1)       # arrival order: the two that wait are taken together
+    try:
+        tickets = [loop.submit(p, prm) for p in (first, huge, large)]
+        loop.wait(tickets[0])
+        host.lib.fake_us_per_row(0)
+        with pytest.raises(EngineError, match="too large"):
+            loop.wait(tickets[1])
+        assert loop.wait(tickets[2])[1]["iters"] == 300000
+    finally:
+        host.lib.fake_us_per_row(1)
+        loop.close()
