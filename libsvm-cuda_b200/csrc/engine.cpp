@@ -1049,7 +1049,8 @@ static cudaError_t wave_issue(Wave &w, InstanceDesc *d_desc, int *d_block_inst, 
                           : launch_smo(w.form, d_desc, d_block_inst, w.used - (w.drop_last_block ? 1 : 0), w.dyn_smem,
                                        w.cooperative, s);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(w.ev1, s, rec);
-    if (e == cudaSuccess) e = xfer_async(host + w.up_bytes, dev + w.o_out, w.down_bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && !w.host_dev)
+        e = xfer_async(host + w.up_bytes, dev + w.o_out, w.down_bytes, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(w.done, s, rec);
     return e;
 }
@@ -1236,8 +1237,10 @@ int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, cons
         D.p = (double *)(dev + w.o_p) + w.loff[k];
         D.pos_row = (int *)(dev + w.o_row) + w.loff[k];
         D.y = (signed char *)(dev + w.o_y) + w.loff[k];
-        D.out = (SolveOut *)(dev + w.o_out) + k;
-        D.alpha_local = (double *)(dev + w.o_alocal) + w.loff[k];
+        char *const res = w.host_dev ? w.host_dev + w.up_bytes : dev + w.o_out;
+        D.out = (SolveOut *)res + k;
+        D.alpha_local = (double *)(res + (w.o_alocal - w.o_out)) + w.loff[k];
+        if (w.host_dev) ((SolveOut *)(host + w.up_bytes))[k].status = -1;   // until the solve has ended
         D.sync = (GroupSync *)(dev + w.o_sync) + k;
         D.partials = (Partial *)(dev + w.o_part) + w.poff[k];
         D.words = (RecWord *)(dev + w.o_word) + kRecWords * (w.poff[k] / 2);
@@ -1275,15 +1278,14 @@ int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, cons
 
 bool wave_ready(const Wave &w) { return w.done && cudaEventQuery(w.done) != cudaErrorNotReady; }
 
-int wave_fetch(const Wave &w, int k, SolveResult &r, cudaStream_t s)
+int wave_fetch(const Wave &w, int k, SolveResult &r)
 {
-    const size_t l = w.loff[k + 1] - w.loff[k];
-    r.alpha.resize(l);
-    CK(xfer_async(&r.out, w.dev + w.o_out + sizeof(SolveOut) * k, sizeof(SolveOut), cudaMemcpyDeviceToHost, s));
-    if (l) CK(xfer_async(r.alpha.data(), w.dev + w.o_alocal + 8 * w.loff[k], 8 * l, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    const double *h_alocal = (const double *)(w.host + w.up_bytes + (w.o_alocal - w.o_out));
+    r.alpha.assign(h_alocal + w.loff[k], h_alocal + w.loff[k + 1]);
+    r.out = ((const SolveOut *)(w.host + w.up_bytes))[k];
     r.seconds = 0;
     r.fill_path = w.fill_path[k];
+    count_transfer(0, (long long)(sizeof(SolveOut) + 8 * r.alpha.size()));
     if (r.out.status < 0) {
         set_error("solver group barrier timed out");
         return -1;

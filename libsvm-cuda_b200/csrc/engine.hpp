@@ -122,6 +122,7 @@ struct Wave {
     int tune_rows_per_block = 500;   // autotuner: positions per block a solve aims at (caps its blocks)
     int tile_bufs = 2;         // transpose tiles per warp of the CUDA-core fills
     int *done_flags = nullptr; // device view of host-mapped words, one per instance (nullptr: none)
+    char *host_dev = nullptr;  // device view of `host`: the blocks write their results there (nullptr: a copy brings them)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, done = nullptr;
     float ms = 0;
 };
@@ -153,7 +154,7 @@ int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, cons
                char *dev, char *host, cudaStream_t s);
 bool wave_ready(const Wave &w);
 // Copy instance k's results (once its done flag is set) with a copy on stream s.
-int wave_fetch(const Wave &w, int k, SolveResult &r, cudaStream_t s);
+int wave_fetch(const Wave &w, int k, SolveResult &r);
 // Wait for the wave and unpack results[first .. first+count).
 int wave_finish(Wave &w, std::vector<SolveResult> &res);
 

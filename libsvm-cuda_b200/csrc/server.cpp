@@ -19,10 +19,10 @@
 // more throughput than more blocks per request.
 // A wave's blocks are planned within the free SMs, so all of them are
 // resident at once; launches are therefore plain (not cooperative) and
-// several run concurrently.  When every block of one request has finished,
-// the kernel sets that request's word in host-mapped memory; the scheduler
-// then copies its result out and hands its SMs to the next wave while the
-// rest of the launch runs on.  Rows and solver state stay on the device
+// several run concurrently.  The blocks write a request's result into host-mapped
+// memory (a copy would wait in a hardware queue that other streams' launches may
+// fill) and, when all have finished, set its word there; the scheduler then hands
+// the result out and its SMs to the next wave while the rest of the launch runs on.  Rows and solver state stay on the device
 // until the launch ends.  Results equal a solve of the same request
 // alone: the solver's arithmetic does not depend on the number of blocks or
 // on the other instances of a launch.
@@ -81,7 +81,7 @@ struct Slot {
     std::vector<Job *> jobs;
     std::vector<SubProblem> subs;
     char *dev = nullptr;
-    char *host = nullptr;
+    char *host = nullptr, *host_dev = nullptr;
     size_t host_bytes = 0;
     size_t mem = 0;
     int blocks = 0;
@@ -125,8 +125,6 @@ struct Server {
     Clock::time_point t_first, t_last;
     bool any_submit = false;
 
-    cudaStream_t copy_stream = nullptr;
-
     void loop();
     void admit(Slot &slot, std::unique_lock<std::mutex> &lk);
     void collect(Slot &slot);
@@ -156,10 +154,10 @@ void Server::complete_locked(Job *j, bool ok, const std::string &err)
 void Server::collect(Slot &slot)
 {
     for (int k = 0; k < slot.w.count; k++) {
-        if (slot.delivered[k] || *(volatile int *)(slot.flags_host + k) == 0) continue;
+        if (slot.delivered[k] || __atomic_load_n(slot.flags_host + k, __ATOMIC_ACQUIRE) == 0) continue;
         Job *j = slot.jobs[k];
         SolveResult r;
-        const int rc = wave_fetch(slot.w, k, r, copy_stream);
+        const int rc = wave_fetch(slot.w, k, r);
         if (rc == 0) {
             j->alpha.assign(j->n, 0.0);
             capi::finish_instance(j->params, j->sub, r, j->y.data(), j->n, j->alpha.data(), &j->stats);
@@ -321,7 +319,8 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
         slot.host = nullptr;
         slot.host_bytes = 0;
         const size_t want = (slot.w.up_bytes + slot.w.down_bytes) * 2;
-        if (cudaHostAlloc((void **)&slot.host, want, cudaHostAllocDefault) == cudaSuccess) slot.host_bytes = want;
+        if (cudaHostAlloc((void **)&slot.host, want, cudaHostAllocMapped) == cudaSuccess &&
+            cudaHostGetDevicePointer((void **)&slot.host_dev, slot.host, 0) == cudaSuccess) slot.host_bytes = want;
         else { ok = false; err = "page-locked staging allocation failed"; }
     }
     if (ok && cudaMallocAsync((void **)&slot.dev, slot.w.dev_bytes, slot.stream) != cudaSuccess) {
@@ -333,6 +332,7 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
         slot.w.cooperative = false;
         memset(slot.flags_host, 0, sizeof(int) * (size_t)cfg.max_batch);
         slot.w.done_flags = slot.flags_dev;
+        slot.w.host_dev = slot.host_dev;
         slot.delivered.assign(slot.w.count, 0);
         if (wave_start(empty_rows(), slot.subs, take[0]->prm, slot.w, slot.dev, slot.host, slot.stream) != 0) {
             ok = false;
@@ -431,10 +431,6 @@ int svmb_server_create(const svmb_server_config *cfg, svmb_server **out)
     if (S.capacity <= 0) { svmb::set_error("no CUDA device"); return -1; }
     if (svmb::load_solver_kernels(S.cfg.form) != cudaSuccess) { svmb::set_error("loading the kernels failed"); return -1; }
     S.slots.resize(S.cfg.max_inflight);
-    if (cudaStreamCreateWithFlags(&S.copy_stream, cudaStreamNonBlocking) != cudaSuccess) {
-        svmb::set_error("stream creation failed");
-        return -1;
-    }
     for (auto &sl : S.slots) {
         if (cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking) != cudaSuccess) {
             svmb::set_error("stream creation failed");
@@ -565,7 +561,6 @@ void svmb_server_destroy(svmb_server *h)
         if (sl.host) cudaFreeHost(sl.host);
         if (sl.flags_host) cudaFreeHost(sl.flags_host);
     }
-    if (h->s.copy_stream) cudaStreamDestroy(h->s.copy_stream);
     delete h;
 }
 

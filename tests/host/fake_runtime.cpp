@@ -85,6 +85,7 @@ cudaError_t got(void **p, size_t n)
 
 std::atomic<int> blocks_now{0}, blocks_peak{0}, cluster_launches{0}, general_launches{0};
 std::atomic<long long> us_per_row{1}, h2d_bytes{0};
+std::atomic<int> waits{0};           // calls that wait for the device
 
 void solve(const svmb::InstanceDesc *insts, const int *map, int blocks)
 {
@@ -119,6 +120,7 @@ int fake_peak_blocks() { return blocks_peak.exchange(0); }
 int fake_cluster_launches() { return cluster_launches.exchange(0); }
 int fake_general_launches() { return general_launches.exchange(0); }
 long long fake_h2d_bytes() { return h2d_bytes.exchange(0); }
+int fake_waits() { return waits.exchange(0); }
 void fake_us_per_row(long long us) { us_per_row = us; }
 
 int omp_get_max_threads() { return 1; }
@@ -128,7 +130,7 @@ cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int)
     *v = a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 232448 : a == cudaDevAttrMaxSharedMemoryPerMultiprocessor ? 233472 : 148;
     return cudaSuccess;
 }
-cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { return waits++, cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int *n) { return *n = 1, cudaSuccess; }
@@ -177,15 +179,19 @@ cudaError_t cudaEventRecordWithFlags(cudaEvent_t ev, cudaStream_t s, unsigned)
     });
     return cudaSuccess;
 }
-cudaError_t cudaMalloc(void **p, size_t n) { return got(p, n); }
+cudaError_t cudaMalloc(void **p, size_t n) { return waits++, got(p, n); }
 cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { return got(p, n); }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return got(p, n); }
 cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned) { return *d = h, cudaSuccess; }
-cudaError_t cudaFree(void *p) { return free(p), cudaSuccess; }
+cudaError_t cudaFree(void *p)
+{
+    if (p) waits++;
+    return free(p), cudaSuccess;
+}
 cudaError_t cudaFreeHost(void *p) { return free(p), cudaSuccess; }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t s) { return stream(s).push([p] { free(p); }), cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t *f, size_t *t) { return *f = *t = size_t(64) << 30, cudaSuccess; }
-cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { return memcpy(d, s, n), cudaSuccess; }
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { return waits++, memcpy(d, s, n), cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind kind, cudaStream_t st)
 {
     if (kind == cudaMemcpyHostToDevice) h2d_bytes += (long long)n;
@@ -194,7 +200,7 @@ cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind kin
 cudaError_t cudaMemset(void *d, int v, size_t n) { return memset(d, v, n), cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t s) { return stream(s).push([=] { memset(d, v, n); }), cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return *s = (cudaStream_t) new Stream, cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { return stream(s).sync(), cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { return waits++, stream(s).sync(), cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t s)
 {
     ((Stream *)s)->sync();

@@ -109,3 +109,20 @@ def test_a_request_too_large_for_the_device_fails_alone(host):
     finally:
         host.lib.fake_us_per_row(1)
         loop.close()
+
+
+@pytest.mark.parametrize("form", [0])
+def test_the_loop_does_not_wait_for_the_device(host, form):
+    """A call that waits (a synchronisation, or an allocation or a release that
+    is not stream-ordered) would hold every request up behind whatever runs."""
+    prm = make_params(gamma=1.0, cache_mb=10.0, form=form)
+    loop = Server(host, max_inflight=4, form=form)
+    try:
+        host.lib.fake_waits()
+        tickets = [(n, loop.submit(_rows(n), prm)) for n in (500, 3000, 700, 9000, 500, 12000)]
+        for n, t in tickets:
+            alpha, st, _ = loop.wait(t)
+            assert st["iters"] == n and np.array_equal(np.abs(alpha), np.ones(n))
+        assert host.lib.fake_waits() == 0
+    finally:
+        loop.close()
