@@ -256,6 +256,13 @@ void DeviceRows::release_async(cudaStream_t s)
         else if (block_async) cudaFreeAsync(block, s);
         else cudaFree(block);
     }
+    if (block_async) {          // the split copy came from the stream's allocator too
+        if (Xs) cudaFreeAsync(Xs, s);
+        if (xinv) cudaFreeAsync(xinv, s);
+        Xs = nullptr;
+        xinv = nullptr;
+        split_form = -1;
+    }
     block = nullptr;
     X = nullptr; rowptr = nullptr; col = nullptr; val = nullptr;
     xsq[0] = xsq[1] = nullptr;
@@ -275,11 +282,13 @@ int DeviceRows::prepare_form(int form, cudaStream_t s)
     const size_t b = (size_t)n * nc * 2 * kSplitChunk * sizeof(uint16_t);
     uint16_t *p = nullptr;
     double *q = nullptr;
-    cudaError_t e = cudaMalloc(&p, b);
-    if (e == cudaSuccess && form == FORM_FP16X3) e = cudaMalloc(&q, (size_t)n * sizeof(double));
+    // (rows of a request loop: stream-ordered, without waiting for the device)
+    auto alloc = [&](void **ptr, size_t bytes) { return block_async ? cudaMallocAsync(ptr, bytes, s) : cudaMalloc(ptr, bytes); };
+    cudaError_t e = alloc((void **)&p, b);
+    if (e == cudaSuccess && form == FORM_FP16X3) e = alloc((void **)&q, (size_t)n * sizeof(double));
     if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, b, s);
     if (e == cudaSuccess) e = launch_split(*this, form, nc, p, q, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && !block_async) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         cudaFree(p);
         cudaFree(q);

@@ -111,7 +111,7 @@ def test_a_request_too_large_for_the_device_fails_alone(host):
         loop.close()
 
 
-@pytest.mark.parametrize("form", [0])
+@pytest.mark.parametrize("form", [0, 3, 4])
 def test_the_loop_does_not_wait_for_the_device(host, form):
     """A call that waits (a synchronisation, or an allocation or a release that
     is not stream-ordered) would hold every request up behind whatever runs."""
