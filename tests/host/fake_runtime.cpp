@@ -189,7 +189,11 @@ cudaError_t cudaFree(void *p)
     return free(p), cudaSuccess;
 }
 cudaError_t cudaFreeHost(void *p) { return free(p), cudaSuccess; }
-cudaError_t cudaFreeAsync(void *p, cudaStream_t s) { return p == nullptr ? cudaErrorInvalidValue : stream(s).push([p] { free(p); }), cudaSuccess; }
+cudaError_t cudaFreeAsync(void *p, cudaStream_t s)
+{
+    if (!p) return cudaErrorInvalidValue;
+    return stream(s).push([p] { free(p); }), cudaSuccess;
+}
 cudaError_t cudaMemGetInfo(size_t *f, size_t *t) { return *f = *t = size_t(64) << 30, cudaSuccess; }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { return waits++, memcpy(d, s, n), cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind kind, cudaStream_t st)
