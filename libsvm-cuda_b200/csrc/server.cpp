@@ -80,6 +80,7 @@ struct Slot {
     std::vector<char> delivered;    // instance results already handed out
     std::vector<Job *> jobs;
     std::vector<SubProblem> subs;
+    std::vector<std::unique_ptr<DeviceRows>> done_rows;     // of the instances handed out
     char *dev = nullptr;
     char *host = nullptr, *host_dev = nullptr;
     size_t host_bytes = 0;
@@ -164,8 +165,10 @@ void Server::collect(Slot &slot)
         }
         const std::string err = rc ? std::string(last_error()) : std::string();
         slot.delivered[k] = 1;
-        j->rows->release_async(slot.stream);    // ordered after the launch on its stream
-        j->rows.reset();
+        // The rows stay until the launch ends.  Freed now, in its stream's order,
+        // their memory could go to another stream's request, which would then
+        // wait for this launch.
+        slot.done_rows.push_back(std::move(j->rows));
         slot.jobs[k] = nullptr;                 // a waiter may free the request once it is complete
         std::lock_guard<std::mutex> g(mu);
         complete_locked(j, rc == 0, err);
@@ -183,6 +186,8 @@ void Server::reap(Slot &slot)
     const std::string err = rc ? std::string(last_error()) : std::string();
     cudaFreeAsync(slot.dev, slot.stream);
     slot.dev = nullptr;
+    for (auto &r : slot.done_rows) r->release_async(slot.stream);
+    slot.done_rows.clear();
     // each request by its own outcome: one instance whose group timed out
     // fails alone; a launch that failed leaves every result unfilled
     std::vector<char> ok(slot.jobs.size(), 0);

@@ -27,6 +27,7 @@ struct Stream {
     std::condition_variable cv, idle;
     std::deque<std::function<void()>> queue;
     bool busy = false, stop = false;
+    std::atomic<int> solving{0};        // launches of the solver queued or at work
     std::thread worker;
     Stream()
     {
@@ -86,6 +87,8 @@ cudaError_t got(void **p, size_t n)
 std::atomic<int> blocks_now{0}, blocks_peak{0}, cluster_launches{0}, general_launches{0};
 std::atomic<long long> us_per_row{1}, h2d_bytes{0};
 std::atomic<int> waits{0};           // calls that wait for the device
+std::atomic<int> frees_behind{0};    // memory given back behind a launch at work: who gets it waits for that launch
+
 
 void solve(const svmb::InstanceDesc *insts, const int *map, int blocks)
 {
@@ -111,6 +114,16 @@ void solve(const svmb::InstanceDesc *insts, const int *map, int blocks)
         if (D.done_flag) __atomic_store_n(D.done_flag, 1, __ATOMIC_RELEASE);
     }
 }
+cudaError_t launch(const svmb::InstanceDesc *insts, const int *map, int blocks, cudaStream_t s)
+{
+    Stream *const st = &stream(s);
+    st->solving++;
+    st->push([=] {
+        solve(insts, map, blocks);
+        st->solving--;
+    });
+    return cudaSuccess;
+}
 cudaError_t nothing() { return cudaSuccess; }
 
 }  // namespace
@@ -120,6 +133,7 @@ int fake_peak_blocks() { return blocks_peak.exchange(0); }
 int fake_cluster_launches() { return cluster_launches.exchange(0); }
 int fake_general_launches() { return general_launches.exchange(0); }
 long long fake_h2d_bytes() { return h2d_bytes.exchange(0); }
+int fake_frees_behind_a_launch() { return frees_behind.exchange(0); }
 int fake_waits() { return waits.exchange(0); }
 void fake_us_per_row(long long us) { us_per_row = us; }
 
@@ -192,6 +206,7 @@ cudaError_t cudaFreeHost(void *p) { return free(p), cudaSuccess; }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t s)
 {
     if (!p) return cudaErrorInvalidValue;
+    if (stream(s).solving) frees_behind++;
     return stream(s).push([p] { free(p); }), cudaSuccess;
 }
 cudaError_t cudaMemGetInfo(size_t *f, size_t *t) { return *f = *t = size_t(64) << 30, cudaSuccess; }
@@ -238,12 +253,12 @@ cudaError_t launch_kernel_block(const DeviceRows &, const KernelParams &, int, c
 cudaError_t launch_smo(int, const InstanceDesc *d, const int *map, int n, size_t, bool, cudaStream_t s)
 {
     general_launches++;
-    return stream(s).push([=] { solve(d, map, n); }), cudaSuccess;
+    return launch(d, map, n, s);
 }
 cudaError_t launch_smo_cluster(int, const InstanceDesc *d, const int *map, int n, int, size_t, cudaStream_t s)
 {
     cluster_launches++;
-    return stream(s).push([=] { solve(d, map, n); }), cudaSuccess;
+    return launch(d, map, n, s);
 }
 int predict_batch(const svm_model *, const svm_node *const *, int, double *, double *) { return -1; }
 void predict_forget(const svm_model *) {}

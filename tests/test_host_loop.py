@@ -111,18 +111,23 @@ def test_a_request_too_large_for_the_device_fails_alone(host):
         loop.close()
 
 
-@pytest.mark.parametrize("form", [0, 3, 4])
-def test_the_loop_does_not_wait_for_the_device(host, form):
+@pytest.mark.parametrize("form,inflight", [(0, 4), (0, 1), (3, 4), (4, 1)])
+def test_the_loop_does_not_wait_for_the_device(host, form, inflight):
     """A call that waits (a synchronisation, or an allocation or a release that
-    is not stream-ordered) would hold every request up behind whatever runs."""
+    is not stream-ordered) would hold every request up behind whatever runs, and
+    so would memory that becomes another request's only when a launch ends."""
     prm = make_params(gamma=1.0, cache_mb=10.0, form=form)
-    loop = Server(host, max_inflight=4, form=form)
+    loop = Server(host, max_inflight=inflight, form=form)
+    host.lib.fake_us_per_row(5)
     try:
         host.lib.fake_waits()
-        tickets = [(n, loop.submit(_rows(n), prm)) for n in (500, 3000, 700, 9000, 500, 12000)]
+        host.lib.fake_frees_behind_a_launch()
+        tickets = [(n, loop.submit(_rows(n), prm)) for n in (500, 3000, 700, 9000, 1900, 12000)]
         for n, t in tickets:
             alpha, st, _ = loop.wait(t)
             assert st["iters"] == n and np.array_equal(np.abs(alpha), np.ones(n))
         assert host.lib.fake_waits() == 0
+        assert host.lib.fake_frees_behind_a_launch() == 0
     finally:
+        host.lib.fake_us_per_row(1)
         loop.close()
