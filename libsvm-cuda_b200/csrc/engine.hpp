@@ -218,12 +218,11 @@ cudaError_t launch_smo(int form, const InstanceDesc *d_insts, const int *d_block
 // instances): dense rows in tiles (d_first[k] = first tile of instance k),
 // sparse rows in groups of sources, tensor forms one instance at a time
 int q_tiles(int l);
-// Load the kernels that solves of the form may launch.  (A kernel's first use
+// Load the kernels that a request of the form may launch, its rows' upload
+// included.  (A kernel's first use
 // otherwise loads it, and that waits for the kernels already running: the request
 // loop would stand still until its longest solve ends.)
 cudaError_t load_solver_kernels(int form);
-cudaError_t load_q_dense(int form);
-cudaError_t load_q_tensor(int form);
 cudaError_t launch_q_dense(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, cudaStream_t s);
 cudaError_t launch_q_sparse(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, size_t dyn_smem,
                             cudaStream_t s);

@@ -692,6 +692,22 @@ cudaError_t launch_kernel_block2(const DeviceRows &A, const DeviceRows &B, const
     return cudaGetLastError();
 }
 
+cudaError_t load_split(int form)
+{
+    const void *const fns[] = {(const void *)row_scale_kernel,
+                               form == FORM_TF32     ? (const void *)tf32_dense_kernel
+                               : form == FORM_BF16X3 ? (const void *)split_dense_kernel<true>
+                                                     : (const void *)split_dense_kernel<false>,
+                               form == FORM_TF32     ? (const void *)tf32_csr_kernel
+                               : form == FORM_BF16X3 ? (const void *)split_csr_kernel<true>
+                                                     : (const void *)split_csr_kernel<false>};
+    cudaFuncAttributes at;
+    cudaError_t e = cudaSuccess;
+    for (const void *fn : fns)
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, fn);
+    return e;
+}
+
 cudaError_t load_q_tensor(int form)
 {
     cudaFuncAttributes at;

@@ -9,6 +9,7 @@ namespace svmb {
 
 cudaError_t load_q_dense(int form);     // qmatrix_kernel.cu
 cudaError_t load_q_tensor(int form);    // gram_kernel.cu
+cudaError_t load_split(int form);
 // the solver kernel of each form (smo_form_*.cu)
 const void *smo_entry_exact();
 const void *smo_entry_fp32();
@@ -176,7 +177,13 @@ cudaError_t load_solver_kernels(int form)
     cudaFuncAttributes at;
     cudaError_t e = cudaFuncGetAttributes(&at, smo_fn(form));
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, cluster_fn(form));
-    if (is_tc_form(form)) return e == cudaSuccess ? load_q_tensor(form) : e;
+    // the upload's kernels: norms, dense rows, split copies
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, (const void *)xsq_kernel);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, (const void *)scatter_dense_kernel);
+    if (is_tc_form(form)) {
+        if (e == cudaSuccess) e = load_split(form);
+        return e == cudaSuccess ? load_q_tensor(form) : e;
+    }
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, form == FORM_FP32 ? smo_rows_fp32() : smo_rows_exact());
     return e == cudaSuccess ? load_q_dense(form) : e;
 }

@@ -2,13 +2,15 @@
 binary solves.  Requests submitted while others run are admitted next to
 them (concurrent launches); every result must equal the same request solved
 alone (the exact form is bit-reproducible, so the check is equality)."""
+import subprocess
+import sys
 import time
 
 import numpy as np
 import pytest
 
 from svmb200 import datagen
-from svmb200.lib import EngineError, Server, make_params
+from svmb200.lib import PKG_DIR, EngineError, Server, make_params
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +82,33 @@ def test_a_request_waits_for_the_blocks_its_state_needs(engine):
     assert st["completed"] == 2 and st["failed"] == 0, st
     assert np.array_equal(got[0][0], engine.solve_binary(wide, wide_prm)[0])
     assert np.array_equal(got[1][0], engine.solve_binary(long, long_prm)[0])
+
+
+FIRST_DENSE = """
+import sys, time
+sys.path.insert(0, sys.argv[1])
+from svmb200 import datagen
+from svmb200.lib import Engine, Server, make_params
+eng = Engine()
+form = int(sys.argv[2])
+long, _ = datagen.sparse_text(n=8000, n_test=0, d=2000, seed=31)
+small, _ = datagen.dense_gauss(n=500, n_test=0, d=16, seed=32)
+srv = Server(eng, form=form)
+t_long = srv.submit(long, make_params(gamma=0.5, C_pos=4.0, cache_mb=0.5, form=form))
+while srv.stats()["waves"] < 1:
+    time.sleep(0.001)
+time.sleep(0.02)
+srv.wait(srv.submit(small, make_params(gamma=1.0 / 16, form=form)))
+print("long one done:", srv.done(t_long))
+srv.wait(t_long)
+srv.close()
+"""
+
+
+@pytest.mark.parametrize("form", [0, 3])
+def test_the_first_dense_request_does_not_wait_for_a_running_solve(engine, form):
+    """In a new process: the kernels of the dense rows' upload are loaded when the
+    loop is made, not by its first dense request (a load waits for what runs)."""
+    out = subprocess.run([sys.executable, "-c", FIRST_DENSE, PKG_DIR, str(form)], capture_output=True, text=True, timeout=250)
+    assert out.returncode == 0, out.stderr
+    assert "long one done: False" in out.stdout
