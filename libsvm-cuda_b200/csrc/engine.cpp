@@ -689,6 +689,9 @@ struct StagePlan {
     long long chunk_max = 0;    // positions of state one block can hold
 };
 
+// positions a block must be able to hold beside its staging
+constexpr int kChunkLeast = 64;
+
 StagePlan stage_plan(const DeviceRows &rows, int form, long long budget, int tile_bufs)
 {
     StagePlan p;
@@ -705,9 +708,13 @@ StagePlan stage_plan(const DeviceRows &rows, int form, long long budget, int til
             p.stage_lds = rows.d;
             p.stage_cap = (int)std::min<long long>(kSrcBatch, (budget / 2) / ((long long)std::max(rows.d, 1) * 4));
         }
-        if (p.stage_cap < 2) p.stage_cap = 0;
         // the exact form stages its source values as float64
         const long long elem = form == FORM_EXACT ? 8 : 4;
+        // (sparse sources that, so staged, leave a block no room for its positions
+        // get half of the memory)
+        if (!rows.dense && (budget - p.stage_cap * p.stage_lds * elem - aux_bytes(form, 1)) / kChunkBytes < kChunkLeast + 4)
+            p.stage_cap = (int)((budget / 2) / (p.stage_lds * elem));
+        if (p.stage_cap < 2) p.stage_cap = 0;
         p.bytes = (((long long)p.stage_cap * p.stage_lds * elem) + 127) & ~127LL;
         if (!rows.dense && p.stage_cap == 0) {
             // too wide to scatter: the sources go into a column-keyed table
@@ -904,7 +911,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
                 const StagePlan st = stage_plan(rows_of(sp, rows), prm.form, budget, 1);
                 const long long cap = ((long long)sp.rows.size() + c - 1) / c;
                 need = std::max(need, st.bytes + cap * kChunkBytes);
-                ok = params_of(sp, prm).form == prm.form && st.chunk_max >= 64;
+                ok = params_of(sp, prm).form == prm.form && st.chunk_max >= kChunkLeast;
                 sps.push_back(st);
             }
             if (!ok || (size_t)need > smo_cluster_smem(prm.form)) break;
@@ -938,7 +945,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
                 return -1;
             }
             const StagePlan st = stage_plan(rows_of(sp, rows), prm.form, budget, bufs);
-            if (st.chunk_max < 64) {
+            if (st.chunk_max < kChunkLeast) {
                 if (bufs > 1) return -2;
                 set_error("not enough shared memory for the solver state");
                 return -1;

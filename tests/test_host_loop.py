@@ -131,3 +131,18 @@ def test_the_loop_does_not_wait_for_the_device(host, form, inflight):
     finally:
         host.lib.fake_us_per_row(1)
         loop.close()
+
+
+@pytest.mark.parametrize("form", [0, 1, 3])
+def test_sparse_rows_of_every_width_are_taken(host, form):
+    """The staging of sparse sources leaves room for a block's positions at every
+    width between the ones that are scattered eight at a time and the table's."""
+    refused = []
+    for d in range(500, 30000, 250):
+        p = CSR(np.arange(101, dtype=np.int64) * 2, np.tile(np.array([1, d]), 100), np.ones(200), np.where(np.arange(100) % 2, 1.0, -1.0), d)
+        for cache_mb in (100.0, 0.001):     # evaluated ahead, and by row passes
+            try:
+                host.solve_binary(p, make_params(gamma=1.0, cache_mb=cache_mb, form=form))
+            except EngineError as e:
+                refused.append((d, cache_mb, str(e)))
+    assert not refused
