@@ -130,7 +130,11 @@ void svmb_print_nothing(const char *s);
  *            the whole group return and the call report an error
  *   "test_drop_block" 1: the next solver launch leaves out its last thread
  *            block (one shot), so that its group's waits run out; for testing
- *            the timeout path (the instance must have two or more blocks) */
+ *            the timeout path (the instance must have two or more blocks; the
+ *            launch is one of the general loop)
+ *   "test_mute_block" the same for a launch of thread-block clusters (instances
+ *            whose kernel matrix is resident): the last block falls silent, 1:
+ *            before its first record, k > 1: after k - 2 iterations */
 int svmb_set_option(const char *name, long long value);
 
 /* The autotuner's configuration of the last batched solve of this process:

@@ -43,6 +43,9 @@ int set_blocks_per_sm(int b)
     return 0;
 }
 void arm_drop_block() { g_drop_block = 1; }
+// one-shot: a block of the next launch of clusters falls silent (InstanceDesc::mute)
+static std::atomic<int> g_mute_block{0};
+void arm_mute_block(int how) { g_mute_block = how; }
 
 
 static thread_local std::string g_last_error;
@@ -1274,6 +1277,7 @@ int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, cons
         memcpy(h_row + w.loff[k], sp.rows.data(), sizeof(int) * l);
         memcpy(h_y + w.loff[k], sp.y.data(), l);
     }
+    if (w.cluster > 1) h_desc[count - 1].mute = g_mute_block.exchange(0);
     if (w.cluster == 0 && g_drop_block.exchange(0)) {
         w.drop_last_block = true;
         w.use_graph = false;

@@ -220,6 +220,7 @@ struct InstanceDesc {
     int stage_lds;              // floats per staged row (dense: ld; sparse: d)
     int chunk_cap;              // positions of per-block state held in shared memory (>= ceil(l/nblocks))
     int resident;               // kResident*: the whole kernel matrix is in the cache from the start
+    int mute;                   // test hook, clusters: 1: the last block sends no record; k > 1: it leaves after k - 2 iterations
     int prefetch;               // rows evaluated per fill pass (1 = no prefetch), <= kPrefetchMax
     // 0: G_bar maintained on every bound change, as the reference does (svm.cpp:744-769);
     // 1: no G_bar -- reconstruction recomputes G = p + sum over alpha>0 of alpha*Q on the

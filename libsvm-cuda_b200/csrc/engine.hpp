@@ -153,7 +153,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
 int wave_start(const DeviceRows &rows, const std::vector<SubProblem> &subs, const SolveParams &prm, Wave &w,
                char *dev, char *host, cudaStream_t s);
 bool wave_ready(const Wave &w);
-// Copy instance k's results (once its done flag is set) with a copy on stream s.
+// Instance k's results, once its done flag is set (a wave with host_dev).
 int wave_fetch(const Wave &w, int k, SolveResult &r);
 // Wait for the wave and unpack results[first .. first+count).
 int wave_finish(Wave &w, std::vector<SolveResult> &res);
@@ -182,6 +182,7 @@ void set_wait_limit_ms(long long ms);
 // waits run out after the wait bound, the group returns with an error and
 // the call reports it.  The instance must have two or more blocks.
 void arm_drop_block();
+void arm_mute_block(int how);
 // solver blocks placed on one SM (1 to 4, default 1): the shared memory a
 // block may use is the SM's divided among them; a launch then holds up to
 // that many blocks per SM where registers allow it.  Speed only.

@@ -276,6 +276,7 @@ __device__ __noinline__ void solve_resident(int rank)
         fail_solve(0, 0);
         return;
     }
+    if (D.mute == 1 && rank == D.nblocks - 1) return;
     const Chunk ck = chunk_at(c.choff, D.chunk_cap);
     const int l = D.l, nb = D.nblocks;
     typedef typename RowOf<TRI>::type Row;
@@ -507,6 +508,9 @@ __device__ __noinline__ void solve_resident(int rank)
     finish_solve(nu, iter, status, unshrink);
     return;
 fail:
+    // Nobody waits for the records this block sent last: they land (well within
+    // this pause) before it lets the others leave.
+    __nanosleep(100000);
     fail_solve(iter, unshrink);
 }
 
@@ -532,8 +536,9 @@ smo_cluster(const InstanceDesc *__restrict__ insts, const int *__restrict__ bloc
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    cluster_sync();     // no block sends before every block's mbarriers exist
     const int rank = blockIdx.x - sh.D.block0;
+    if (threadIdx.x == 0 && sh.D.mute > 1 && rank == sh.D.nblocks - 1) sh.D.max_iter = sh.D.mute - 2;
+    cluster_sync();     // no block sends before every block's mbarriers exist
     // (the tensor forms' values differ in the last bits with the operands swapped:
     // their matrices are whole)
     if constexpr (!is_tc_form(FORM)) {

@@ -232,6 +232,9 @@ int api_set_option(const char *name, long long value)
     } else if (!strcmp(name, "test_drop_block")) {
         if (value != 1) return -1;
         arm_drop_block();
+    } else if (!strcmp(name, "test_mute_block")) {
+        if (value < 1 || value > 1000000) return -1;
+        arm_mute_block((int)value);
     } else if (!strcmp(name, "prefetch")) {
         if (value < 0 || value > kPrefetchMax) return -1;
         g_opt.prefetch = (int)value;

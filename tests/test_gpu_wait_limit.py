@@ -42,6 +42,44 @@ def test_solve_reports_a_group_that_never_completes(short_waits):
     assert st["iters"] == st_want["iters"]
 
 
+@pytest.mark.parametrize("n,svm_type", [(600, 0), (2000, 0), (2000, 1), (5000, 0)])     # clusters of 2, 4, 4 and 16 blocks
+@pytest.mark.parametrize("mute", [1, 2, 7])
+def test_cluster_reports_a_block_that_falls_silent(short_waits, n, svm_type, mute):
+    """Resident instances: the last block sends no record (mute 1) or leaves after
+    mute - 2 iterations.  The other blocks' waits run out, all return, and the
+    next solve gives the usual result."""
+    eng = short_waits
+    tr, _ = datagen.dense_gauss(n=n, n_test=0, d=16, seed=n)
+    params = make_params(svm_type=svm_type, kernel_type=2, gamma=1.0 / 16, nu=0.3)
+    want, st_want = eng.solve_binary(tr, params)
+    assert st_want["fills"] == 0 and st_want["iters"] > 7
+    eng.set_option("test_mute_block", mute)
+    t0 = time.perf_counter()
+    with pytest.raises(EngineError, match="timed out"):
+        eng.solve_binary(tr, params)
+    assert 0.4 < time.perf_counter() - t0 < 20.0
+    got, st = eng.solve_binary(tr, params)
+    np.testing.assert_array_equal(got, want)
+    assert st["iters"] == st_want["iters"]
+
+
+def test_request_loop_fails_only_the_cluster_with_the_silent_block(short_waits):
+    eng = short_waits
+    tr, _ = datagen.dense_gauss(n=1500, n_test=0, d=16, seed=9)
+    params = make_params(svm_type=0, kernel_type=2, gamma=1.0 / 16)
+    want, _ = eng.solve_binary(tr, params)
+    srv = Server(eng)
+    try:
+        eng.set_option("test_mute_block", 1)
+        with pytest.raises(EngineError, match="timed out"):
+            srv.wait(srv.submit(tr, params))
+        got, _, _ = srv.wait(srv.submit(tr, params))
+        np.testing.assert_array_equal(got, want)
+        assert srv.stats()["failed"] == 1
+    finally:
+        srv.close()
+
+
 def test_svm_train_returns_null_and_recovers(short_waits):
     eng = short_waits
     tr, _ = datagen.dense_gauss(n=2000, n_test=0, d=16, seed=6)
