@@ -78,3 +78,29 @@ def test_instances_of_one_launch(engine):
     for r, y, a in zip(rows, ys, got):
         want, _ = engine.solve_binary(p.take(r), make_params(kernel_type=2, gamma=0.05, cache_mb=1e-3), y=y)
         np.testing.assert_array_equal(a, want)
+
+
+@pytest.mark.parametrize("n,more", [(3001, dict(svm_type=1, nu=0.3)), (4001, {}), (5117, dict(svm_type=1, nu=0.2)),
+                                    (4100, dict(form=FORM_FP16X3)), (2100, dict(svm_type=3, C_pos=1.0))])
+def test_clusters_of_8_and_16_blocks(engine, n, more):
+    p, _ = (datagen.regression(n=n, n_test=0, d=5, seed=n) if more.get("svm_type") == 3 else
+            datagen.dense_gauss(n=n, n_test=0, d=10, seed=n))
+    _same(engine, p, **dict(dict(kernel_type=2, gamma=0.1, C_pos=2.0), **more))
+
+
+@pytest.mark.parametrize("n,more", [(7300, {}), (7001, dict(svm_type=1, nu=0.2))])
+def test_triangles_on_16_blocks(engine, n, more):
+    test_triangles(engine, n, "dense", more)
+
+
+def test_more_blocks_than_positions(engine):
+    """9 rows launched beside 5,000, on 16 blocks as these."""
+    p, _ = datagen.dense_gauss(n=5000, n_test=0, d=20, seed=9)
+    rows = [np.sort(np.random.default_rng(1).choice(p.n, 9, replace=False)).astype(np.int32), np.arange(p.n, dtype=np.int32)]
+    ys = [p.y[r] for r in rows]
+    prm = make_params(kernel_type=2, gamma=0.05)
+    got, st = engine.solve_many(p, rows, ys, [prm] * 2)
+    assert [s["launch"] for s in st] == [0, 0]
+    for r, y, a in zip(rows, ys, got):
+        want, _ = engine.solve_binary(p.take(r), make_params(kernel_type=2, gamma=0.05, cache_mb=0.1), y=y)
+        np.testing.assert_array_equal(a, want)

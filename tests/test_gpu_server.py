@@ -112,3 +112,26 @@ def test_the_first_dense_request_does_not_wait_for_a_running_solve(engine, form)
     out = subprocess.run([sys.executable, "-c", FIRST_DENSE, PKG_DIR, str(form)], capture_output=True, text=True, timeout=250)
     assert out.returncode == 0, out.stderr
     assert "long one done: False" in out.stdout
+
+
+def test_dense_and_sparse_requests_of_both_formulations_in_one_launch(engine):
+    """At the default cache size every one of these is resident; with one launch
+    at a time, those that come during the first are taken into the second."""
+    ps = [datagen.dense_gauss(n=900 + 37 * k, n_test=0, d=24, seed=50 + k)[0] if k % 2 else
+          datagen.sparse_text(n=950 + 61 * k, n_test=0, d=300, nnz_mean=15.0, seed=60 + k)[0] for k in range(8)]
+    prm = [make_params(svm_type=k // 2 % 2, kernel_type=1 + k // 4 % 2, gamma=0.3, nu=0.2) for k in range(8)]
+    first, _ = datagen.dense_gauss(n=9000, n_test=0, d=64, seed=70)
+    srv = Server(engine, max_inflight=1)
+    try:
+        t_first = srv.submit(first, make_params(gamma=1.0 / 64, C_pos=10.0, cache_mb=40.0))
+        while srv.stats()["waves"] < 1:
+            time.sleep(0.0005)
+        got = [srv.wait(t) for t in [srv.submit(p, q) for p, q in zip(ps, prm)]]
+        srv.wait(t_first)
+        assert srv.stats()["waves"] == 2
+    finally:
+        srv.close()
+    for p, q, (alpha, st, _) in zip(ps, prm, got):
+        want, st_want = engine.solve_binary(p, q)
+        assert np.array_equal(alpha, want) and st["iters"] == st_want["iters"] and st["rho"] == st_want["rho"]
+        assert st["fills"] == 0
