@@ -739,8 +739,11 @@ const DeviceRows &rows_of(const SubProblem &sp, const DeviceRows &rows) { return
 // kernel matrix before the solve, by all SMs.  Worth it when that takes less
 // than what the solves would spend on row passes: their iterations number about
 // l (0.2 l to 5 l measured) and spend 0.3 to 3 us each on passes, so the line
-// is the matrices' estimated time against 1 us per position of the launch's
-// longest instance.  One value costs its dot product and a kernel function of
+// is the matrices' estimated time against 1 us per position of the launch: of its
+// longest instance, or of one of the `at_a_time` queues when the instances wait
+// for room (450 x 1000 positions of 64 features and one of 2000: one launch of
+// clusters 23 ms; against the longest alone, four launches, three of them of the
+// general loop, 39 ms).  One value costs its dot product and a kernel function of
 // about 40 operations; dense tiles run at about 8e12 operations a second, half
 // of the values being copies.  A launch whose longest instance has no such
 // cache lasts as long without (the 45 pairs of 3,600 to 21,600 positions, the
@@ -749,16 +752,17 @@ const DeviceRows &rows_of(const SubProblem &sp, const DeviceRows &rows) { return
 // clusters' loop only (`triangles`): half of a row's values then lie a column
 // apart, which a loop bound by latency does not feel.
 static std::vector<char> resident_of(const DeviceRows &rows, const std::vector<SubProblem> &subs, const SolveParams &prm,
-                                     int first, int count, bool triangles)
+                                     int first, int count, bool triangles, double at_a_time)
 {
     double cost = 0.0;
-    long long longest = 0, longest_fit = 0;
+    long long longest = 0, longest_fit = 0, sum = 0;
     std::vector<char> fits(count, 0);
     for (int k = 0; k < count; k++) {
         const SubProblem &sp = subs[first + k];
         const DeviceRows &r = rows_of(sp, rows);
         const long long l = (long long)sp.rows.size();
         longest = std::max(longest, l);
+        sum += l;
         const long long slots = l > 0 ? instance_layout((int)l, 1, params_of(sp, prm).cache_mb).slots : 0;
         if (l > 0 && slots >= l) fits[k] = kResidentFull;
         else if (l > 0 && triangles && !is_tc_form(prm.form) && 2 * slots >= l + 1 && l <= kMaxSlots) fits[k] = kResidentTri;
@@ -767,7 +771,8 @@ static std::vector<char> resident_of(const DeviceRows &rows, const std::vector<S
         const double width = is_tc_form(prm.form) ? 0.05 * r.d : r.dense ? (double)r.ld : 8.0 * (double)r.nnz / std::max(r.n, 1);
         cost += 0.5 * (double)l * (double)l * (width + 40.0);
     }
-    if (longest_fit < longest || cost > 8e12 * 1e-6 * (double)longest) fits.assign(count, 0);
+    const double span = std::max((double)longest, (double)sum / at_a_time);
+    if (longest_fit < longest || cost > 8e12 * 1e-6 * span) fits.assign(count, 0);
     return fits;
 }
 
@@ -786,12 +791,12 @@ static int cluster_plan(const DeviceRows &rows, const std::vector<SubProblem> &s
         hint = std::max(hint, p.blocks_hint);
         longest = std::max(longest, (long long)subs[first + k].rows.size());
     }
-    resident = resident_of(rows, subs, prm, first, count, true);
-    for (char r : resident)
-        if (!r) return 0;
     int c = 1;
     while (c < kClusterMax && (hint > 0 ? c < hint + 1 && longest > 1000 : c * span < longest)) c *= 2;
     while (c > 1 && (long long)count * c > capacity) c /= 2;
+    resident = resident_of(rows, subs, prm, first, count, true, (double)capacity / c);
+    for (char r : resident)
+        if (!r) return 0;
     return c;
 }
 
@@ -847,7 +852,7 @@ static int wave_layout(const DeviceRows &rows, const std::vector<SubProblem> &su
         w.poff[k + 1] = w.poff[k] + 2 * (size_t)w.nb[k];
         w.coff[k + 1] = w.coff[k] + (size_t)w.lay[k].slots;
     }
-    if (w.cluster == 0) w.resident = resident_of(rows, subs, prm, first, count, false);
+    if (w.cluster == 0) w.resident = resident_of(rows, subs, prm, first, count, false, count);
     const size_t L = w.loff[count], P = w.poff[count], S = w.coff[count];
     size_t off = 0;
     w.o_desc = off; off = al(off + sizeof(InstanceDesc) * count);
@@ -895,7 +900,7 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
     }
     if (!g_drop_block) {
         // all remaining instances resident: clusters, as many as the memory for
-        // their matrices allows (and, unless they may queue, as many as run at a time)
+        // their matrices allows (and, unless they may queue, as the blocks free)
         int n = 0;
         double bytes = 0.0;
         while (first + n < ninst && (w.queue || n < capacity)) {

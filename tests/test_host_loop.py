@@ -146,3 +146,17 @@ def test_sparse_rows_of_every_width_are_taken(host, form):
             except EngineError as e:
                 refused.append((d, cache_mb, str(e)))
     assert not refused
+
+
+def test_instances_that_queue_stay_one_launch_of_clusters(host):
+    """The matrices of 330 instances are weighed against the whole launch, in which
+    they wait for room, not against the longest of them."""
+    host.lib.fake_us_per_row(0)
+    p = _rows(500, 64)
+    inst = [np.arange(500, dtype=np.int32)] * 330
+    host.lib.fake_cluster_launches()
+    host.lib.fake_general_launches()
+    _, st = host.solve_many(p, inst, [p.y] * 330, [make_params(gamma=1.0 / 64)] * 330)
+    host.lib.fake_us_per_row(1)
+    assert host.lib.fake_cluster_launches() == 1 and host.lib.fake_general_launches() == 0
+    assert {s["launch"] for s in st} == {0}
