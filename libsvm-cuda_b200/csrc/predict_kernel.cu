@@ -482,7 +482,7 @@ struct Workspace {
     double *t_xinv = nullptr;
     size_t cap_t = 0, cap_Xs = 0, cap_xinv = 0;
     char *pin = nullptr;        // page-locked staging of test rows and decision values (at most kPinMost)
-    size_t cap_pin = 0;
+    size_t cap_pin = 0, asked_pin[2] = {0, 0};      // what there is; the most that each use asked for without getting it
     size_t held() const { return cap_kv + cap_dec + cap_t + cap_Xs + cap_xinv + cap_pin + T.held(); }
     void release()
     {
@@ -492,23 +492,29 @@ struct Workspace {
         *this = Workspace();
     }
 } g_ws;
-constexpr size_t kPinMost = 512u << 20;
+constexpr size_t kPinMost = 512u << 20, kPinLeast = 1u << 20;
 // With no model left, buffers above this are given back.  Smaller ones stay:
 // a cross-validation makes and frees a model per fold, and allocating (the
 // page-locked staging above all) anew for each took 15 to 40 ms of a call
 // whose solves take 1.3 ms, on hosts where such calls are slow.
 constexpr size_t kKeepMost = 64u << 20;
 
-// host staging of at least `bytes`: page-locked and kept, or for very large
-// calls ordinary memory of the call
-char *staging(size_t bytes, std::vector<char> &fallback)
+// Host staging of at least `bytes`: page-locked and kept, or ordinary memory of
+// the call.  Page-locking costs 1 to 5 ms per MB, more than it saves in one call: it
+// waits for the second use that needs more than there is, of test rows and of
+// models' support vectors each (a model's are staged once).  8,192 rows x 64 after a
+// small call: 7 to 28 ms locked at once, 2.8 ms in ordinary memory; later calls
+// 0.55 and 1.3 ms.
+enum StagingUse { kStageRows, kStageModel };
+char *staging(size_t bytes, std::unique_ptr<char[]> &fallback, StagingUse use)
 {
+    size_t &asked = g_ws.asked_pin[use];
     if (bytes <= g_ws.cap_pin) return g_ws.pin;
-    if (bytes <= kPinMost) {
+    if (bytes <= asked) {
         if (g_ws.pin) cudaFreeHost(g_ws.pin);
         g_ws.pin = nullptr;
         g_ws.cap_pin = 0;
-        const size_t want = std::min(kPinMost, std::max<size_t>(bytes + bytes / 4, 1 << 20));
+        const size_t want = std::min(kPinMost, std::max(bytes + bytes / 4, kPinLeast));
         if (cudaHostAlloc((void **)&g_ws.pin, want, cudaHostAllocDefault) == cudaSuccess) {
             g_ws.cap_pin = want;
             return g_ws.pin;
@@ -516,8 +522,9 @@ char *staging(size_t bytes, std::vector<char> &fallback)
         cudaGetLastError();
         g_ws.pin = nullptr;
     }
-    fallback.resize(bytes);
-    return fallback.data();
+    if (bytes <= kPinMost) asked = std::max(asked, std::max(bytes, kPinLeast));
+    fallback.reset(new char[bytes]);
+    return fallback.get();
 }
 // host loops over fewer rows than this stay on the calling thread (waking the
 // others takes longer)
@@ -547,16 +554,16 @@ void count_nodes(const svm_node *const *x, int n, long long *rp)
 
 // The copies are queued on the default stream; the caller waits for it before
 // the next use of the staging.
-int upload_nodes(const svm_node *const *x, int n, int d, int base, bool dense, Rows &out)
+int upload_nodes(const svm_node *const *x, int n, int d, int base, bool dense, Rows &out, StagingUse use)
 {
     out.n = n;
     out.dense = dense;
     out.ld = (d + 3) & ~3;
     if (out.ld == 0) out.ld = 4;
-    std::vector<char> fallback;
+    std::unique_ptr<char[]> fallback;
     if (dense) {
         const size_t bytes = (size_t)std::max(n, 1) * out.ld * sizeof(double);
-        double *h = (double *)staging(bytes, fallback);
+        double *h = (double *)staging(bytes, fallback, use);
         if (n == 0) memset(h, 0, bytes);
 #pragma omp parallel for schedule(static) if (n > kParallelRows)
         for (int r = 0; r < n; r++) {
@@ -569,13 +576,13 @@ int upload_nodes(const svm_node *const *x, int n, int d, int base, bool dense, R
         }
         PK(grow(out.X, out.capX, bytes));
         PK(xfer_async(out.X, h, bytes, cudaMemcpyHostToDevice, 0));
-        if (!fallback.empty()) PK(cudaStreamSynchronize(0));
+        if (fallback) PK(cudaStreamSynchronize(0));
     } else {
         std::vector<long long> rp((size_t)n + 1, 0);
         count_nodes(x, n, rp.data());
         const size_t nnz = (size_t)std::max<long long>(rp[n], 1);
         const size_t b_val = ((size_t)n + 1) * sizeof(long long), b_col = b_val + nnz * sizeof(double);
-        char *h = staging(b_col + nnz * sizeof(int), fallback);
+        char *h = staging(b_col + nnz * sizeof(int), fallback, use);
         memcpy(h, rp.data(), b_val);
         double *val = (double *)(h + b_val);
         int *col = (int *)(h + b_col);
@@ -597,7 +604,7 @@ int upload_nodes(const svm_node *const *x, int n, int d, int base, bool dense, R
         PK(xfer_async(out.rowptr, h, b_val, cudaMemcpyHostToDevice, 0));
         PK(xfer_async(out.col, col, nnz * sizeof(int), cudaMemcpyHostToDevice, 0));
         PK(xfer_async(out.val, val, nnz * sizeof(double), cudaMemcpyHostToDevice, 0));
-        if (!fallback.empty()) PK(cudaStreamSynchronize(0));
+        if (fallback) PK(cudaStreamSynchronize(0));
     }
     return 0;
 }
@@ -626,7 +633,7 @@ Session *get_session(const svm_model *m)
     s->base = 0;
     s->d = maxi + 1;
     const bool dense = m->l == 0 || (double)nnz >= 0.25 * (double)m->l * s->d || (double)m->l * s->d * 4 < 32e6;
-    if (upload_nodes(m->SV, m->l, s->d, s->base, dense, s->sv) != 0) return nullptr;
+    if (upload_nodes(m->SV, m->l, s->d, s->base, dense, s->sv, kStageModel) != 0) return nullptr;
     if (cudaStreamSynchronize(0) != cudaSuccess) {      // the staging is used again
         set_error("upload of the support vectors failed");
         return nullptr;
@@ -694,8 +701,8 @@ int tensor_rows(const svm_node *const *x, int n, int d, int form, DeviceRows &ou
     auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
     const size_t b_col = al(((size_t)n + 1) * 8), b_val = al(b_col + nnz * 4), up = b_val + nnz * 4;
     const size_t b_sq = al(up), total = b_sq + (size_t)n * 8;
-    std::vector<char> fallback;
-    char *h = staging(up, fallback);
+    std::unique_ptr<char[]> fallback;
+    char *h = staging(up, fallback, kStageRows);
     memcpy(h, rp.data(), ((size_t)n + 1) * 8);
     int *col = (int *)(h + b_col);
     float *val = (float *)(h + b_val);
@@ -721,7 +728,7 @@ int tensor_rows(const svm_node *const *x, int n, int d, int form, DeviceRows &ou
     out.val = (float *)(g_ws.t_block + b_val);
     out.xsq[FORM_EXACT] = (double *)(g_ws.t_block + b_sq);
     PK(xfer_async(g_ws.t_block, h, up, cudaMemcpyHostToDevice, 0));
-    if (!fallback.empty()) PK(cudaStreamSynchronize(0));
+    if (fallback) PK(cudaStreamSynchronize(0));
     PK(launch_xsq(out.view(FORM_EXACT), n, out.xsq[FORM_EXACT], FORM_EXACT, 0));
     count_launch();
     PK(cudaMemsetAsync(g_ws.t_Xs, 0, b_Xs, 0));
@@ -830,13 +837,13 @@ int predict_batch(const svm_model *m, const svm_node *const *rows, int n, double
             if (prepare_tensor_svs(m, s, maxi + 1, g_predict_form) != 0) return -1;
             if (tensor_rows(rows, n, s->sv_tc->d, g_predict_form, Ttc) != 0) return -1;
         } else if (dense) {
-            if (upload_nodes(rows, n, s->d, s->base, true, T) != 0) return -1;
+            if (upload_nodes(rows, n, s->d, s->base, true, T, kStageRows) != 0) return -1;
         } else {
             if (s->sv.dense && !s->sv_csr.rowptr) {
-                if (upload_nodes(m->SV, m->l, s->d, s->base, false, s->sv_csr) != 0) return -1;
+                if (upload_nodes(m->SV, m->l, s->d, s->base, false, s->sv_csr, kStageModel) != 0) return -1;
                 PK(cudaStreamSynchronize(0));       // the staging is used again
             }
-            if (upload_nodes(rows, n, maxi + 1, s->base, false, T) != 0) return -1;
+            if (upload_nodes(rows, n, maxi + 1, s->base, false, T, kStageRows) != 0) return -1;
         }
         int *d_err = nullptr;
         if (tensor) {
@@ -869,18 +876,17 @@ int predict_batch(const svm_model *m, const svm_node *const *rows, int n, double
                 PK(launch_pair_sums(kv, tn, m->l, k, s->start, s->nsv, s->coef, s->rho, d_dec));
             count_launch();
             // (the test rows have left the staging once these kernels have run)
-            std::vector<char> fallback;
             const size_t bytes = (size_t)tn * npair * 8;
+            char *const to = (char *)(dec.data() + (size_t)t0 * npair), *const h = bytes <= g_ws.cap_pin ? g_ws.pin : to;
             cudaError_t e = cudaSuccess;
             if (t0 == 0) e = cudaStreamSynchronize(0);
-            char *h = staging(bytes, fallback);
             if (e == cudaSuccess) e = xfer_async(h, d_dec, bytes, cudaMemcpyDeviceToHost, 0);
             if (e == cudaSuccess) e = cudaStreamSynchronize(0);
             if (e != cudaSuccess) {
                 set_error(std::string("prediction kernels failed: ") + cudaGetErrorString(e));
                 return -1;
             }
-            memcpy(dec.data() + (size_t)t0 * npair, h, bytes);
+            if (h != to) memcpy(to, h, bytes);
         }
         if (tensor) {
             int herr = 0;
