@@ -181,6 +181,10 @@ def max_over_ranks(value, world, device):
 def run_reference(args, world, rank):
     if rank != 0:
         return 0
+    # (a worker pool whose initializer raises would start workers for ever)
+    if _reference_lib() is None:
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libsvm_ref.so is not built"}), flush=True)
+        return 0
     cores = os.cpu_count() or 1
     npairs = 45
     ctx = mp.get_context("spawn")

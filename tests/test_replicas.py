@@ -66,3 +66,16 @@ def test_reference_arm_runs_on_rank_zero_only(rank):
                         "--warmup", "3"], env=env, capture_output=True, text=True, timeout=120)
     assert r.returncode == 0
     assert r.stdout.strip() == ""
+
+
+def test_reference_arm_without_its_library_says_so(monkeypatch, capsys):
+    sys.path.insert(0, ROOT)
+    import argparse
+    import json
+
+    import bench
+    monkeypatch.setattr(bench, "_reference_lib", lambda: None)
+    monkeypatch.setattr(bench.mp, "get_context", lambda kind: pytest.fail("no workers are started"))
+    assert bench.run_reference(argparse.Namespace(steps=1, warmup=3), 1, 0) == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"]
