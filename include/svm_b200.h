@@ -48,7 +48,9 @@ typedef struct svmb_solve_stats {
     long long prof_cycles[8];   /* SM cycles per loop section (diagnostics) */
     long long fill_targets;     /* target positions of all row-evaluation passes: each pass reads
                                    every target row once, whatever the number of its source rows */
-    int fill_path;              /* SVMB_FILL_*: how the solve evaluated its kernel rows */
+    int fill_path;              /* SVMB_FILL_*: how the solve evaluated its kernel rows; with fills == 0
+                                   all of them at once, before it started (its cache holds the whole
+                                   kernel matrix, or half of it) */
     int reserved;
 } svmb_solve_stats;
 
@@ -71,7 +73,8 @@ typedef struct svmb_params {
     double C_neg;        /* C-SVC: C for y<=0 (Cn) */
     double nu;           /* nu-SVC, one-class, nu-SVR */
     double eps;
-    double cache_mb;     /* Q-row cache budget per solve, MB (svm_parameter.cache_size) */
+    double cache_mb;     /* Q-row cache budget per solve, MB (svm_parameter.cache_size); a solve
+                            keeps at most 65,534 rows, whatever the budget */
     int form;            /* SVMB_FORM_* */
     int blocks;          /* thread blocks per solve; 0 = automatic */
     int prefetch;        /* kernel rows evaluated per cache-miss pass (1 = only the missing row); 0 = automatic */
@@ -251,9 +254,11 @@ int svmb_rows_kernel_block(const svmb_rows *rows, const svmb_params *params, int
  * scheduler thread picks a leading request (the policy), adds pending
  * requests of a similar size while their device memory (rows + solver state
  * with the Q-row cache budget) fits the server's budget and the thread blocks
- * they need fit the SMs that no running launch holds, and launches them
- * together next to the launches already running (up to max_inflight at a
- * time).  A request's result equals its solve alone. */
+ * they need fit the SMs that no running launch of the process holds, and
+ * launches them together next to the launches already running (up to
+ * max_inflight at a time).  A request that needs more blocks than are free
+ * waits, and others may pass it until it is the oldest and has waited 2 s.  A
+ * request's result equals its solve alone. */
 typedef struct svmb_server svmb_server;
 typedef struct svmb_server_config {
     long long mem_bytes;     /* device memory for admitted requests; 0 = 80% of the free memory */

@@ -725,7 +725,7 @@ StagePlan stage_plan(const DeviceRows &rows, int form, long long budget, int til
             p.bytes = hash_bytes(form);
         }
     }
-    p.bytes += aux_bytes(form, tile_bufs);   // transpose tiles / prefetch candidates / block-product partial sums
+    p.bytes += aux_bytes(form, tile_bufs);   // transpose tiles / block-product partial sums
     p.chunk_max = (budget - p.bytes) / kChunkBytes;
     return p;
 }

@@ -122,7 +122,7 @@ extern "C" int svmb_solve_dense_noalloc(int n, int ld, const float *X, const dou
     // staged source values are float64 in the exact form
     const int elem = params->form == SVMB_FORM_EXACT ? 8 : 4;
     long long stage_bytes = (((long long)stage_cap * ld * elem) + 127) & ~127LL;
-    stage_bytes += kAuxBytes;   // transpose tiles (two per warp) / prefetch candidates
+    stage_bytes += kAuxBytes;   // transpose tiles (two per warp)
     const long long chunk_max = (budget - stage_bytes) / kChunkBytes;
     if (chunk_max < 64) { set_error("not enough shared memory for the solver state"); return -1; }
     int nb = (int)std::max<long long>(1, std::min<long long>(sms, (n + 1499) / 1500));

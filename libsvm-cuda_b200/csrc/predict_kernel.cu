@@ -398,10 +398,11 @@ cudaError_t launch_pair_sums(const double *kv, int nt, int ns, int nr_class, con
     const double npair = 0.5 * nr_class * (nr_class - 1);
     const double pair_len = 2.0 * ns / nr_class;
     const int blocks = (nt + kSumRows - 1) / kSumRows;
-    const double few = std::ceil(nt * npair / (148.0 * 8)) * (pair_len + 200.0);
-    const double many = std::ceil(blocks / (148.0 * 2)) * (ns + 500.0 * nr_class) * 3.0;
+    const double sms = device_sm_count();
+    const double few = std::ceil(nt * npair / (sms * 8)) * (pair_len + 200.0);
+    const double many = std::ceil(blocks / (sms * 2)) * (ns + 500.0 * nr_class) * 3.0;
     if (few <= many) {
-        pair_sums_few<<<(int)std::min<double>(nt * npair, 148.0 * 8), 256>>>(kv, nt, ns, nr_class, start, nsv, coef, rho, dec);
+        pair_sums_few<<<(int)std::min<double>(nt * npair, sms * 8), 256>>>(kv, nt, ns, nr_class, start, nsv, coef, rho, dec);
         return cudaGetLastError();
     }
     const int r = nr_class - 1;

@@ -168,7 +168,7 @@ cudaError_t load_q_dense(int form)
 
 cudaError_t launch_q_dense(int form, const InstanceDesc *d_insts, const int *d_first, int count, int total, cudaStream_t s)
 {
-    const int blocks = total < 148 * 4 ? total : 148 * 4;
+    const int most = device_sm_count() * 4, blocks = total < most ? total : most;
     if (form == FORM_FP32) q_dense_kernel<float><<<blocks, kQThreads, 0, s>>>(d_insts, d_first, count, total);
     else q_dense_kernel<double><<<blocks, kQThreads, 0, s>>>(d_insts, d_first, count, total);
     return cudaGetLastError();

@@ -7,6 +7,7 @@
 
 namespace svmb {
 
+int device_sm_count();                  // engine.cpp
 cudaError_t load_q_dense(int form);     // qmatrix_kernel.cu
 cudaError_t load_q_tensor(int form);    // gram_kernel.cu
 cudaError_t load_split(int form);
@@ -195,7 +196,8 @@ cudaError_t launch_q_sparse(int form, const InstanceDesc *d_insts, const int *d_
     cudaError_t e = set_max_dyn_smem(fn);
     if (e != cudaSuccess) return e;
     void *args[] = {(void *)&d_insts, (void *)&d_first, (void *)&count, (void *)&total};
-    return cudaLaunchKernel(fn, dim3(total < 148 ? total : 148), dim3(kThreads), args, dyn_smem, s);
+    const int most = device_sm_count();
+    return cudaLaunchKernel(fn, dim3(total < most ? total : most), dim3(kThreads), args, dyn_smem, s);
 }
 
 cudaError_t smo_max_blocks(int form, size_t dyn_smem, int *blocks_per_sm)
