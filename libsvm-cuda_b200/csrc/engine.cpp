@@ -978,8 +978,8 @@ int wave_plan(const DeviceRows &rows, const std::vector<SubProblem> &subs, const
         return 0;
     };
     if (is_tc_form(prm.form)) {
-        // the tensor forms have no transpose tiles
-        if (const int rc = fit(2, sp_all, nmin, last)) return rc == kNoRoom ? rc : -1;
+        // the tensor forms have no transpose tiles: one depth
+        if (const int rc = fit(1, sp_all, nmin, last)) return rc;
     } else {
         // the deepest ring (deeper rings keep more of a fill in flight) among
         // those that put the most instances into this launch

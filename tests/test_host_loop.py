@@ -61,14 +61,15 @@ def test_launches_of_two_loops_and_a_call_fit_the_device(host):
     assert host.lib.fake_peak_blocks() <= 148
 
 
-def test_a_request_that_waits_for_blocks_is_passed_and_uploaded_once(host):
+@pytest.mark.parametrize("form", [0, 1, 3])
+def test_a_request_that_waits_for_blocks_is_passed_and_uploaded_once(host, form):
     """140 of 148 blocks are at work; the next request's 60000 positions need
     more than the other 8.  A small request that comes later does not wait for
     it, and the waiting one's rows go to the device once."""
     long, wide, small = _rows(14000), _rows(60000), _rows(500)
-    prm = make_params(gamma=1.0, cache_mb=10.0)
+    prm = make_params(gamma=1.0, cache_mb=10.0, form=form)
     host.lib.fake_us_per_row(30)
-    loop = Server(host, max_inflight=4, rows_per_block=100)
+    loop = Server(host, max_inflight=4, rows_per_block=100, form=form)
     try:
         alone = 0
         for p in (long, wide, small):
