@@ -301,8 +301,9 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
     if (ok) {
         back.assign(take.begin() + slot.w.count, take.end());
     } else if (rc == kNoRoom && free_blocks < capacity) {
-        // the leader's state needs more blocks than are free now
-        take[0]->need_blocks = slot.w.used;
+        // the leader's state needs more blocks than are free now (whether the idle
+        // device has enough, its own plan will tell)
+        take[0]->need_blocks = std::min(slot.w.used, capacity);
         back = take;
     } else {
         err = last_error();

@@ -112,6 +112,23 @@ def test_a_request_too_large_for_the_device_fails_alone(host):
         loop.close()
 
 
+def test_a_request_too_large_for_the_device_fails_also_when_it_waited(host):
+    p, huge = _rows(14000), _rows(900000, 1)
+    prm = make_params(gamma=1.0, cache_mb=10.0)
+    host.lib.fake_us_per_row(10)
+    loop = Server(host, rows_per_block=100)
+    try:
+        t = loop.submit(p, prm)
+        while loop.stats()["waves"] < 1:
+            time.sleep(0.001)
+        with pytest.raises(EngineError, match="too large"):
+            loop.wait(loop.submit(huge, prm))
+        assert loop.done(t) and loop.wait(t)[1]["iters"] == 14000
+    finally:
+        host.lib.fake_us_per_row(1)
+        loop.close()
+
+
 @pytest.mark.parametrize("form,inflight", [(0, 4), (0, 1), (3, 4), (4, 1)])
 def test_the_loop_does_not_wait_for_the_device(host, form, inflight):
     """A call that waits (a synchronisation, or an allocation or a release that
