@@ -19,13 +19,14 @@
 // more throughput than more blocks per request.
 // A wave's blocks are planned within the free SMs, so all of them are
 // resident at once; launches are therefore plain (not cooperative) and
-// several run concurrently.  The blocks write a request's result into host-mapped
-// memory (a copy would wait in a hardware queue that other streams' launches may
-// fill) and, when all have finished, set its word there; the scheduler then hands
-// the result out and its SMs to the next wave while the rest of the launch runs on.  Rows and solver state stay on the device
-// until the launch ends.  Results equal a solve of the same request
-// alone: the solver's arithmetic does not depend on the number of blocks or
-// on the other instances of a launch.
+// several run concurrently.  The blocks write a request's result into
+// host-mapped memory (a copy would wait in a hardware queue that other streams'
+// launches may fill) and, when all have finished, set its word there; the
+// scheduler then hands the result out and its SMs to the next wave while the
+// rest of the launch runs on.  Rows and solver state stay on the device until
+// the launch ends.  Results equal a solve of the same request alone: the
+// solver's arithmetic does not depend on the number of blocks or on the other
+// instances of a launch.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -91,10 +91,11 @@ from svmb200 import datagen
 from svmb200.lib import Engine, Server, make_params
 eng = Engine()
 form = int(sys.argv[2])
-long, _ = datagen.sparse_text(n=8000, n_test=0, d=2000, seed=31)
+long, _ = datagen.sparse_text(n=12000 if form == 0 else 8000, n_test=0, d=2000, seed=31)
 small, _ = datagen.dense_gauss(n=500, n_test=0, d=16, seed=32)
 srv = Server(eng, form=form)
-t_long = srv.submit(long, make_params(gamma=0.5, C_pos=4.0, cache_mb=0.5, form=form))
+more = dict(C_pos=30.0, eps=1e-4) if form == 0 else dict(C_pos=4.0)     # several seconds
+t_long = srv.submit(long, make_params(gamma=0.5, cache_mb=0.5, form=form, **more))
 while srv.stats()["waves"] < 1:
     time.sleep(0.001)
 time.sleep(0.02)
