@@ -85,6 +85,7 @@ struct Slot {
     char *dev = nullptr;
     char *host = nullptr, *host_dev = nullptr;
     size_t host_bytes = 0;
+    std::vector<char *> outgrown;   // smaller staging of earlier waves
     size_t mem = 0;
     int blocks = 0;
 };
@@ -322,7 +323,9 @@ void Server::admit(Slot &slot, std::unique_lock<std::mutex> &lk)
         }
     }
     if (ok && slot.host_bytes < slot.w.up_bytes + slot.w.down_bytes) {
-        if (slot.host) cudaFreeHost(slot.host);
+        // (freeing page-locked memory waits for the device: what is outgrown, less
+        // than what replaces it, stays until the loop ends)
+        if (slot.host) slot.outgrown.push_back(slot.host);
         slot.host = nullptr;
         slot.host_bytes = 0;
         const size_t want = (slot.w.up_bytes + slot.w.down_bytes) * 2;
@@ -566,6 +569,7 @@ void svmb_server_destroy(svmb_server *h)
             cudaStreamDestroy(sl.stream);
         }
         if (sl.host) cudaFreeHost(sl.host);
+        for (char *p : sl.outgrown) cudaFreeHost(p);
         if (sl.flags_host) cudaFreeHost(sl.flags_host);
     }
     delete h;

@@ -202,7 +202,7 @@ cudaError_t cudaFree(void *p)
     if (p) waits++;
     return free(p), cudaSuccess;
 }
-cudaError_t cudaFreeHost(void *p) { return free(p), cudaSuccess; }
+cudaError_t cudaFreeHost(void *p) { return waits++, free(p), cudaSuccess; }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t s)
 {
     if (!p) return cudaErrorInvalidValue;
